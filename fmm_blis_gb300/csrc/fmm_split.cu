@@ -31,11 +31,11 @@
  *              integer of magnitude <= 2^24 that FP32 holds exactly; the
  *              epilogue warps drain each chunk from TMEM (double-buffered, so
  *              the tensor core keeps running), convert it exactly to int32 and
- *              add it to the level sum L_g. At the end of a level, L_g is
- *              folded into a 64-bit fixed-point accumulator Z in global
- *              memory in units of level G (BF16: G = 6, or 7 when
- *              k_pad <= 128; FP8: G = min(s + 1, 10); the finest units that
- *              keep Z inside int64):
+ *              add it to the level sum L_g. The level sums make up a 64-bit
+ *              fixed-point value Z in units of level G (BF16: G = 6, or 7
+ *              when k_pad <= 128; FP8: G = min(s + 1, 10); the finest units
+ *              that keep Z inside int64), written to global memory digit by
+ *              digit as the levels finish (ZPlanes):
  *                  Z = sum_{g<=G} L_g * 2^(db(G-g)) + sum_{g>G} round(L_g / 2^(db(g-G)))
  *              and M_r[i,j] ~= 2^(E_i + F_j + 2 - db*G) * Z is formed in FP64
  *              and added with alpha*W[p,r] into every C sub-block p (the
@@ -731,9 +731,12 @@ __device__ __forceinline__ double i64_to_double_scaled(int64_t z, int e)
 struct GemmProblem {
     CUtensorMap tmA;      /* A slices [product][s][m_pad][k_pad], box 64 x 128 */
     CUtensorMap tmB;      /* B slices [product][s][n_pad][k_pad], box 64 x 256 */
-    int64_t* Z;           /* [product][n_pad][m_pad] int64 level accumulators */
+    uint8_t* Z;           /* [product] Z planes (ZPlanes) */
     int s;                /* slices */
     int zlevel;           /* G: the level whose unit Z counts in */
+    int zmin;             /* lowest level with a digit plane (ZPlanes) */
+    int znd;              /* digit planes */
+    int zrow0;            /* first Z row of the launch's tile row 0 */
     int nkb;              /* k_pad / kbe */
     int kbe;              /* k elements per 128-byte stage row: 64 (BF16) or 128 (FP8) */
     int db;               /* digit bits: 8 (BF16) or 5 (FP8-E4M3) */
@@ -836,6 +839,132 @@ struct ItemRing {
     }
 };
 
+/* How Z = sum_{g<=G} L_g 2^(db(G-g)) + sum_{g>G} round(L_g / 2^(db(g-G))) is
+ * stored: the GEMM runs the levels from the least significant one down to
+ * g = 2, and at the end of a level g <= G its low db bits are final (every
+ * later level is a multiple of 2^db units of it), so they go to that level's
+ * digit plane and the rest of the sum carries into level g - 1 in the same
+ * 32-bit register; what is left after g = 2 is the high plane:
+ *
+ *     Z = (... (hi << db | d[zmin]) << db | ... | d[gtop]) << db(G - gtop),
+ *     gtop = min(s + 1, G).
+ *
+ * Levels above G carry their rounded value (shifted up to the next level's
+ * unit, so it is rounded exactly once). Every sum stays inside int32: a carry
+ * is at most 2^-5 of the sum it comes from. zmin = 3; 4 in the FP8 format
+ * (|2^5 L_2 + L_3 + carry| <= 2^27 + 2^23 + 2^20) and for BF16 when G = 7
+ * (k_pad <= 128: 2^29 + 2^22 + 2^16), where levels 3 and 2 share the high
+ * plane. Z takes at most 8 bytes per element in the BF16 format, 11 in FP8.
+ *
+ * Layout of one product, by groups of four columns: for each group m_pad x
+ * int4 (high plane, a row's four columns side by side), then per digit plane
+ * (zmin first) m_pad x 4 bytes. An epilogue thread owns one row, so a warp
+ * stores whole 512- and 128-byte lines, each byte once, with plain stores.
+ * Adding each level into an int64 Z with red.global.add.u64 instead moved
+ * 6 x 8 bytes per element through the L2 atomic units (6 slices); the GEMM of
+ * 222 x1 at 3000 x 2500 x 2049 took 455 us that way and takes 402 us now, of
+ * a 300 x 700 x 450 classical problem 93 and 71 us. */
+struct ZPlanes {
+    int zmin, nd;
+    __host__ __device__ static ZPlanes of(int s, int G, int fmt)
+    {
+        ZPlanes z;
+        z.zmin = fmt != 0 || G == 7 ? 4 : 3;
+        const int gtop = s + 1 < G ? s + 1 : G;
+        z.nd = gtop >= z.zmin ? gtop - z.zmin + 1 : 0;
+        return z;
+    }
+};
+
+/* bytes of one 4-column group of Z */
+__host__ __device__ __forceinline__ int64_t z_group_bytes(int64_t m_pad, int nd) { return m_pad * 4 * (4 + nd); }
+
+/* the same index, in a way the compiler cannot carry loads across: the
+ * epilogue's 64 sums leave no room to keep a problem's fields in registers
+ * for a whole item, so they are read from the launch parameter where they are
+ * used */
+__device__ __forceinline__ int opaque(int x)
+{
+    asm volatile("" : "+r"(x));
+    return x;
+}
+
+/* Drains one work item from the accumulator into Z (one epilogue warp: 32
+ * TMEM lanes, kEpiCols columns from tmem address `tl`, one row per thread):
+ * every chunk of every level, levels s+1 .. 2. zh is the address of Z row zi
+ * in the high plane of the thread's first column group. `arrive(buf)` reports
+ * a TMEM buffer read. */
+template <class Arrive>
+__device__ __forceinline__ bool drain_item(const GemmLaunch& L, int p, uint8_t* zh, int zi, uint32_t tl, uint64_t* accf,
+                                           int& buf, uint32_t& aph, int lane, volatile int* abort_flag, int code,
+                                           Arrive arrive)
+{
+    int lsum[kEpiCols];
+#pragma unroll
+    for (int x = 0; x < kEpiCols; ++x) lsum[x] = 0;
+    for (int g = L.prob[p].s + 1; g >= 2; --g) {
+        int left, mul;
+        {
+            const GemmProblem& P = L.prob[opaque(p)];
+            left = (level_pairs(g, P.s) * P.nkb + kChunkKB - 1) / kChunkKB;   /* chunks */
+            mul = g == 2 && P.zmin == 4 ? 1 << P.db : 1;                      /* levels 3 and 2 in one register */
+        }
+        for (; left > 0; --left) {
+            if (!sm103::mbar_wait(&accf[buf], aph, abort_flag, L.err, code)) return false;
+            sm103::tc_fence_after();
+#pragma unroll
+            for (int h = 0; h < kEpiCols / 8; ++h) {
+                uint32_t v[8];
+                SM103_TMEM_LD_X8(tl + buf * kTileN + h * 8, v);
+                sm103::tmem_wait_ld();
+#pragma unroll
+                for (int x = 0; x < 8; ++x)
+                    lsum[h * 8 + x] += __float2int_rn(__uint_as_float(v[x])) * mul;   /* exact: integer, |v| <= 2^24 */
+            }
+            sm103::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) arrive(buf);
+            buf ^= 1;
+            if (buf == 0) aph ^= 1;
+        }
+        const GemmProblem& P = L.prob[opaque(p)];
+        const int G = P.zlevel, db = P.db, zmin = P.zmin, m_pad = P.m_pad;
+        /* the GEMM never reads Z back: its lines leave L2 before the slices' */
+        uint64_t pol;
+        asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
+        if (g > G) {
+            /* round to units of G (ties up), back up to the next level's unit */
+            const int sh = db * (g - G), up = g - 1 > G ? sh - db : 0;
+#pragma unroll
+            for (int x = 0; x < kEpiCols; ++x) lsum[x] = (((lsum[x] >> (sh - 1)) + 1) >> 1) << up;
+        } else if (g >= zmin) {
+            const uint64_t gstep = (uint64_t)z_group_bytes(m_pad, P.znd);
+            const uint32_t dmask = db == 8 ? 0xffffffffu : 0x1f1f1f1fu;
+            uint8_t* q = zh + ((int64_t)m_pad * 4 * (4 + g - zmin) - (int64_t)zi * 12);
+#pragma unroll
+            for (int x = 0; x < kEpiCols; x += 4) {
+                const uint32_t w01 = __byte_perm((uint32_t)lsum[x], (uint32_t)lsum[x + 1], 0x0040u);
+                const uint32_t w23 = __byte_perm((uint32_t)lsum[x + 2], (uint32_t)lsum[x + 3], 0x0040u);
+                const uint32_t w = __byte_perm(w01, w23, 0x5410u) & dmask;
+                asm volatile("st.global.L2::cache_hint.u32 [%0], %1, %3;\n\tadd.u64 %0, %0, %2;"
+                             : "+l"(q) : "r"(w), "l"(gstep), "l"(pol) : "memory");
+#pragma unroll
+                for (int y = 0; y < 4; ++y) lsum[x + y] >>= db;
+            }
+        } else if (g == 2) {
+            const uint64_t gstep = (uint64_t)z_group_bytes(m_pad, P.znd);
+            uint8_t* q = zh;
+#pragma unroll
+            for (int x = 0; x < kEpiCols; x += 4) {
+                asm volatile("st.global.L2::cache_hint.v4.u32 [%0], {%1, %2, %3, %4}, %6;\n\tadd.u64 %0, %0, %5;"
+                             : "+l"(q) : "r"(lsum[x]), "r"(lsum[x + 1]), "r"(lsum[x + 2]), "r"(lsum[x + 3]),
+                               "l"(gstep), "l"(pol) : "memory");
+            }
+        }
+    }
+    return true;
+}
+
 /* Persistent GEMM over a list of work items (problem, product of its group,
  * 128 x 256 output tile), drawn dynamically: the producer takes the next item
  * from L.sched and passes it to the other roles through a CTA-local item
@@ -844,10 +973,10 @@ struct ItemRing {
  * tcgen05.mma (M=128, N=256, K=16 BF16 or K=32 FP8 per the item's problem:
  * 128 clocks per MMA hide the accumulator dependency), warps 2..17 drain
  * each exact chunk (16 stage rows: 1024 BF16 or 2048 FP8 terms) from the
- * double-buffered TMEM accumulator into int32 level sums and fold finished
- * levels into the product's 64-bit Z tile in global memory. The pipeline,
- * TMEM allocation and barrier phases run on across items, so one item's last
- * fold overlaps the next item's first MMAs. */
+ * double-buffered TMEM accumulator into int32 level sums and write the
+ * digits of Z that a finished level settles (drain_item). The pipeline, TMEM
+ * allocation and barrier phases run on across items, so one item's last
+ * stores overlap the next item's first MMAs. */
 __global__ void __launch_bounds__(kGemmThreads, 1)
 split_gemm_kernel(const __grid_constant__ GemmLaunch L)
 {
@@ -912,9 +1041,10 @@ split_gemm_kernel(const __grid_constant__ GemmLaunch L)
                 const int s = P.s, nkb = P.nkb;
                 const int arow = it.r * s * P.m_pad + it.tile_m * kTileM;
                 const int brow = it.r * s * P.n_pad + it.tile_n * kTileN;
-                /* Pair order: t ascending in even levels and descending in odd
-                 * ones, so the last pair of a level and the first of the next
-                 * share a slice ((1,2)->(1,3), (3,1)->(4,1), ...), and k runs
+                /* Pair order: levels from s+1 down to 2 (ZPlanes), t ascending
+                 * in odd levels and descending in even ones, so the last pair
+                 * of a level and the first of the next share a slice
+                 * ((4,1)->(3,1), (1,3)->(1,2), ...), and k runs
                  * forward and backward on alternate pairs, so a shared slice's
                  * most recently loaded blocks are read again first, while they
                  * are still in L2. The MMA side only counts stages; every
@@ -922,10 +1052,10 @@ split_gemm_kernel(const __grid_constant__ GemmLaunch L)
                  * eight stages ahead measured 3x slower, with 7x the DRAM
                  * reads.) */
                 int pi = 0;
-                for (int g = 2; g <= s + 1 && ok; ++g) {
+                for (int g = s + 1; g >= 2 && ok; --g) {
                     const int tlo = max(1, g - s), thi = min(s, g - 1);
                     for (int x = 0; x <= thi - tlo && ok; ++x, ++pi) {
-                        const int t = (g & 1) ? thi - x : tlo + x;
+                        const int t = (g & 1) ? tlo + x : thi - x;
                         const int u = g - t;
                         for (int y = 0; y < nkb; ++y) {
                             const int kb = (pi & 1) ? nkb - 1 - y : y;
@@ -966,7 +1096,7 @@ split_gemm_kernel(const __grid_constant__ GemmLaunch L)
                 if (b < 0) break;
                 const Item it = decode_item(L, b);
                 const int s = L.prob[it.p].s, nkb = L.prob[it.p].nkb, fmt = L.prob[it.p].fmt;
-                for (int g = 2; g <= s + 1 && ok; ++g) {
+                for (int g = s + 1; g >= 2 && ok; --g) {
                     const int level_kb = level_pairs(g, s) * nkb;
                     int jl = 0;
                     for (int t = max(1, g - s); t <= min(s, g - 1) && ok; ++t)
@@ -1018,85 +1148,19 @@ split_gemm_kernel(const __grid_constant__ GemmLaunch L)
         const uint32_t tl = tmem + ((uint32_t)(quarter * 32) << 16);
         int buf = 0;
         uint32_t aph = 0;
-        bool ok = true;
-        /* Z lines stay in L2 between the level folds of an item (evict_last);
-         * the last fold marks them evict_first, as the GEMM is done with them */
-        uint64_t pol_keep, pol_drop;
-        asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol_keep));
-        asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol_drop));
         ItemRing ring{sm103::smem_u32(sfull), 0, 0};
         for (;;) {
             int b;
-            if (!ring.take_warp(&b, lane, abort_flag, L.err, 9)) { ok = false; break; }
+            if (!ring.take_warp(&b, lane, abort_flag, L.err, 9)) break;
             if (b < 0) break;
             const Item it = decode_item(L, b);
             const GemmProblem& P = L.prob[it.p];
-            const int s = P.s, nkb = P.nkb;
-            int64_t* zrow = P.Z + (int64_t)it.r * P.n_pad * P.m_pad +
-                            (int64_t)(it.tile_n * kTileN + colbase) * P.m_pad + it.tile_m * kTileM + row;
-            const struct { int zlevel, m_pad, db; } a = {P.zlevel, P.m_pad, P.db};
-            for (int g = 2; g <= s + 1 && ok; ++g) {
-                int lsum[kEpiCols];
-#pragma unroll
-                for (int x = 0; x < kEpiCols; ++x) lsum[x] = 0;
-                const int nchunks = (level_pairs(g, s) * nkb + kChunkKB - 1) / kChunkKB;
-                for (int c = 0; c < nchunks; ++c) {
-                    if (!sm103::mbar_wait(&accf[buf], aph, abort_flag, L.err, 4)) { ok = false; break; }
-                    sm103::tc_fence_after();
-#pragma unroll
-                    for (int h = 0; h < kEpiCols / 8; ++h) {
-                        uint32_t v[8];
-                        SM103_TMEM_LD_X8(tl + buf * kTileN + colbase + h * 8, v);
-                        sm103::tmem_wait_ld();
-#pragma unroll
-                        for (int x = 0; x < 8; ++x)
-                            lsum[h * 8 + x] += __float2int_rn(__uint_as_float(v[x]));   /* exact: integer, |v| <= 2^24 */
-                    }
-                    sm103::tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) sm103::mbar_arrive(&acce[buf]);
-                    buf ^= 1;
-                    if (buf == 0) aph ^= 1;
-                }
-                if (!ok) break;
-                /* fold L_g into the Z tile (units of level G): D = G - g, exact
-                 * left shift by db*D for D >= 0, rounded right shift by -db*D
-                 * (ties up) for D < 0. The first level stores; later levels add with
-                 * fire-and-forget 64-bit reductions (two's-complement addition
-                 * is exact and order-free), so the warps go straight back to
-                 * draining the accumulator. */
-                {
-                    const int D = a.zlevel - g;
-                    const uint32_t lsh = D >= 0 ? a.db * D : 0;
-                    const uint32_t rsh = D >= 0 ? 0 : -a.db * D;
-                    const uint64_t rnd = D >= 0 ? 0 : (1ull << (rsh - 1));
-                    uint64_t zp = (uint64_t)zrow;
-                    const uint64_t zstep = (uint64_t)a.m_pad * 8;
-                    const uint64_t pol = g == s + 1 ? pol_drop : pol_keep;
-                    if (g == 2) {
-#pragma unroll
-                        for (int x = 0; x < kEpiCols; ++x)
-                            asm volatile("{\n\t.reg .b64 t;\n\t"
-                                         "cvt.s64.s32 t, %1;\n\t"
-                                         "shl.b64 t, t, %2;\n\t"
-                                         "st.global.L2::cache_hint.u64 [%0], t, %4;\n\t"
-                                         "add.u64 %0, %0, %3;\n\t}"
-                                         : "+l"(zp) : "r"(lsum[x]), "r"(lsh), "l"(zstep), "l"(pol) : "memory");
-                    } else {
-#pragma unroll
-                        for (int x = 0; x < kEpiCols; ++x)
-                            asm volatile("{\n\t.reg .b64 t;\n\t"
-                                         "cvt.s64.s32 t, %1;\n\t"
-                                         "shl.b64 t, t, %2;\n\t"
-                                         "add.s64 t, t, %4;\n\t"
-                                         "shr.s64 t, t, %3;\n\t"
-                                         "red.global.add.L2::cache_hint.u64 [%0], t, %6;\n\t"
-                                         "add.u64 %0, %0, %5;\n\t}"
-                                         : "+l"(zp) : "r"(lsum[x]), "r"(lsh), "r"(rsh), "l"(rnd), "l"(zstep), "l"(pol)
-                                         : "memory");
-                    }
-                }
-            }
+            const int zi = P.zrow0 + it.tile_m * kTileM + row;
+            uint8_t* z0 = P.Z + ((int64_t)it.r * P.n_pad + it.tile_n * kTileN + colbase) / 4 *
+                                    z_group_bytes(P.m_pad, P.znd);
+            if (!drain_item(L, it.p, z0 + (int64_t)zi * 16, zi, tl + colbase, accf, buf, aph, lane, abort_flag, 4,
+                            [&](int q) { sm103::mbar_arrive(&acce[q]); }))
+                break;
         }
     }
     sm103::tc_fence_before();
@@ -1211,10 +1275,10 @@ split_gemm_pair_kernel(const __grid_constant__ GemmLaunch L)
                 const int arow = it.r * s * P.m_pad + it.tile_m * kPairTileM + 128 * (int)rank;
                 const int brow = it.r * s * P.n_pad + it.tile_n * kTileN + 128 * (int)rank;
                 int pi = 0;   /* the single-CTA kernel's pair order */
-                for (int g = 2; g <= s + 1 && ok; ++g) {
+                for (int g = s + 1; g >= 2 && ok; --g) {
                     const int tlo = max(1, g - s), thi = min(s, g - 1);
                     for (int x = 0; x <= thi - tlo && ok; ++x, ++pi) {
-                        const int t = (g & 1) ? thi - x : tlo + x;
+                        const int t = (g & 1) ? tlo + x : thi - x;
                         const int u = g - t;
                         for (int y = 0; y < nkb; ++y) {
                             const int kb = (pi & 1) ? nkb - 1 - y : y;
@@ -1258,7 +1322,7 @@ split_gemm_pair_kernel(const __grid_constant__ GemmLaunch L)
                 if (b < 0) break;
                 const Item it = decode_item(L, b, kPairRasterGroup);
                 const int s = L.prob[it.p].s, nkb = L.prob[it.p].nkb, fmt = L.prob[it.p].fmt;
-                for (int g = 2; g <= s + 1 && ok; ++g) {
+                for (int g = s + 1; g >= 2 && ok; --g) {
                     const int level_kb = level_pairs(g, s) * nkb;
                     for (int jl = 0; jl < level_kb && ok; ) {
                         if (jl % kChunkKB == 0) {
@@ -1307,79 +1371,19 @@ split_gemm_pair_kernel(const __grid_constant__ GemmLaunch L)
         const uint32_t acce0 = sm103::mapa(sm103::smem_u32(acce), 0);
         int buf = 0;
         uint32_t aph = 0;
-        bool ok = true;
-        uint64_t pol_keep, pol_drop;
-        asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol_keep));
-        asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol_drop));
         ItemRing ring{sm103::smem_u32(sfull), 0, 0};
         for (;;) {
             int b;
-            if (!ring.take_warp(&b, lane, abort_flag, L.err, 20)) { ok = false; break; }
+            if (!ring.take_warp(&b, lane, abort_flag, L.err, 20)) break;
             if (b < 0) break;
             const Item it = decode_item(L, b, kPairRasterGroup);
             const GemmProblem& P = L.prob[it.p];
-            const int s = P.s, nkb = P.nkb;
-            int64_t* zrow = P.Z + (int64_t)it.r * P.n_pad * P.m_pad +
-                            (int64_t)(it.tile_n * kTileN + colbase) * P.m_pad + it.tile_m * kPairTileM +
-                            128 * (int)rank + row;
-            const struct { int zlevel, m_pad, db; } a = {P.zlevel, P.m_pad, P.db};
-            for (int g = 2; g <= s + 1 && ok; ++g) {
-                int lsum[kEpiCols];
-#pragma unroll
-                for (int x = 0; x < kEpiCols; ++x) lsum[x] = 0;
-                const int nchunks = (level_pairs(g, s) * nkb + kChunkKB - 1) / kChunkKB;
-                for (int c = 0; c < nchunks; ++c) {
-                    if (!sm103::mbar_wait(&accf[buf], aph, abort_flag, L.err, 16)) { ok = false; break; }
-                    sm103::tc_fence_after();
-#pragma unroll
-                    for (int h = 0; h < kEpiCols / 8; ++h) {
-                        uint32_t v[8];
-                        SM103_TMEM_LD_X8(tl + buf * kTileN + colbase + h * 8, v);
-                        sm103::tmem_wait_ld();
-#pragma unroll
-                        for (int x = 0; x < 8; ++x)
-                            lsum[h * 8 + x] += __float2int_rn(__uint_as_float(v[x]));   /* exact: integer, |v| <= 2^24 */
-                    }
-                    sm103::tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) sm103::mbar_arrive_cluster(acce0 + buf * 8);
-                    buf ^= 1;
-                    if (buf == 0) aph ^= 1;
-                }
-                if (!ok) break;
-                /* fold L_g into the Z tile, as in split_gemm_kernel */
-                {
-                    const int D = a.zlevel - g;
-                    const uint32_t lsh = D >= 0 ? a.db * D : 0;
-                    const uint32_t rsh = D >= 0 ? 0 : -a.db * D;
-                    const uint64_t rnd = D >= 0 ? 0 : (1ull << (rsh - 1));
-                    uint64_t zp = (uint64_t)zrow;
-                    const uint64_t zstep = (uint64_t)a.m_pad * 8;
-                    const uint64_t pol = g == s + 1 ? pol_drop : pol_keep;
-                    if (g == 2) {
-#pragma unroll
-                        for (int x = 0; x < kEpiCols; ++x)
-                            asm volatile("{\n\t.reg .b64 t;\n\t"
-                                         "cvt.s64.s32 t, %1;\n\t"
-                                         "shl.b64 t, t, %2;\n\t"
-                                         "st.global.L2::cache_hint.u64 [%0], t, %4;\n\t"
-                                         "add.u64 %0, %0, %3;\n\t}"
-                                         : "+l"(zp) : "r"(lsum[x]), "r"(lsh), "l"(zstep), "l"(pol) : "memory");
-                    } else {
-#pragma unroll
-                        for (int x = 0; x < kEpiCols; ++x)
-                            asm volatile("{\n\t.reg .b64 t;\n\t"
-                                         "cvt.s64.s32 t, %1;\n\t"
-                                         "shl.b64 t, t, %2;\n\t"
-                                         "add.s64 t, t, %4;\n\t"
-                                         "shr.s64 t, t, %3;\n\t"
-                                         "red.global.add.L2::cache_hint.u64 [%0], t, %6;\n\t"
-                                         "add.u64 %0, %0, %5;\n\t}"
-                                         : "+l"(zp) : "r"(lsum[x]), "r"(lsh), "r"(rsh), "l"(rnd), "l"(zstep), "l"(pol)
-                                         : "memory");
-                    }
-                }
-            }
+            const int zi = P.zrow0 + it.tile_m * kPairTileM + 128 * (int)rank + row;
+            uint8_t* z0 = P.Z + ((int64_t)it.r * P.n_pad + it.tile_n * kTileN + colbase) / 4 *
+                                    z_group_bytes(P.m_pad, P.znd);
+            if (!drain_item(L, it.p, z0 + (int64_t)zi * 16, zi, tl + colbase, accf, buf, aph, lane, abort_flag, 16,
+                            [&](int q) { sm103::mbar_arrive_cluster(acce0 + q * 8); }))
+                break;
         }
     }
     sm103::tc_fence_before();
@@ -1398,10 +1402,82 @@ split_gemm_pair_kernel(const __grid_constant__ GemmLaunch L)
  * once per product). */
 constexpr int kScatterMaxEnt = 1024;
 
-__global__ void __launch_bounds__(256)
-scatter_kernel(const int* __restrict__ tab, int r0, int nprod, int64_t m, int64_t n,
-               int m_pad, int n_pad, int ebase, double alpha, const int64_t* __restrict__ Z,
-               const int* __restrict__ e_row, const int* __restrict__ f_col, double* __restrict__ C,
+/* Z of a product group as the C updates read it (see ZPlanes) */
+struct ZView {
+    const uint8_t* base;
+    int64_t prod;     /* bytes per product */
+    int64_t group;    /* bytes per 4-column group */
+    int m_pad, n_pad;
+    int nd;           /* digit planes */
+    int ebase;        /* exponent of Z's unit relative to 2^(E_i + F_j) */
+};
+
+constexpr int kScatterCols = 4;   /* columns per thread: one column group of Z */
+
+/* One row of a column group of one product: the loads (one int4, nd words, the
+ * exponents), then the four Z values. FMT 0: at most four byte digits below
+ * the high word, absent ones zero (Z counts in units of level G whatever the
+ * slice count); FMT 1: nd = G - 3 five-bit digits. */
+template <int FMT>
+struct ZRow {
+    static constexpr int NP = FMT ? 7 : 4;
+    int4 hi;
+    int4 f;
+    int e;
+    uint32_t w[NP];
+
+    __device__ __forceinline__ void load(const ZView& v, const int* __restrict__ e_row, const int* __restrict__ f_col,
+                                         int q, int i, int j)
+    {
+        const uint8_t* g = v.base + q * v.prod + (int64_t)(j >> 2) * v.group;
+        hi = *(const int4*)(g + (int64_t)i * 16);
+        const uint8_t* d = g + ((int64_t)v.m_pad * 16 + (int64_t)i * 4);
+#pragma unroll
+        for (int p = 0; p < NP; ++p) w[p] = p < v.nd ? *(const uint32_t*)(d + (int64_t)p * v.m_pad * 4) : 0u;
+        e = e_row[(int64_t)q * v.m_pad + i];
+        f = *(const int4*)(f_col + (int64_t)q * v.n_pad + j);
+    }
+    /* M[i, j + u] = 2^(ebase + E_i + F_j) * Z */
+    __device__ __forceinline__ void values(const ZView& v, double (&M)[kScatterCols]) const
+    {
+        const int h[4] = {hi.x, hi.y, hi.z, hi.w}, fc[4] = {f.x, f.y, f.z, f.w};
+        const int er = e + v.ebase;
+        if (FMT == 0) {
+            /* the four words' bytes, transposed: digit 0 on top */
+            const uint32_t a0 = __byte_perm(w[1], w[0], 0x5140u), a1 = __byte_perm(w[1], w[0], 0x7362u);
+            const uint32_t b0 = __byte_perm(w[3], w[2], 0x5140u), b1 = __byte_perm(w[3], w[2], 0x7362u);
+            const uint32_t lo[4] = {__byte_perm(b0, a0, 0x5410u), __byte_perm(b0, a0, 0x7632u),
+                                    __byte_perm(b1, a1, 0x5410u), __byte_perm(b1, a1, 0x7632u)};
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                M[u] = i64_to_double_scaled((int64_t)(((uint64_t)(uint32_t)h[u] << 32) | lo[u]), er + fc[u]);
+        } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                uint64_t lo = 0;
+#pragma unroll
+                for (int p = 0; p < NP; ++p)
+                    if (p < v.nd) lo = (lo << 5) | __byte_perm(w[p], 0u, 0x4440u + (unsigned)u);
+                M[u] = i64_to_double_scaled((int64_t)(((uint64_t)(int64_t)h[u] << (5 * v.nd)) | lo), er + fc[u]);
+            }
+        }
+    }
+};
+
+/* beta*c of the C update, as scale_c_kernel forms it */
+__device__ __forceinline__ double beta_c(double beta, const double* c)
+{
+    if (beta == 1.0) return *c;
+    return beta == 0.0 ? 0.0 : beta * *c;
+}
+
+/* C updates of one C sub-block p = blockIdx.y: tiles of blockDim.x rows x 4
+ * columns, a thread a row of a column group. For algorithms whose sub-block
+ * values do not fit scatter_all_kernel's shared memory. */
+template <int FMT>
+__global__ void __launch_bounds__(128)
+scatter_kernel(const int* __restrict__ tab, int r0, int nprod, int64_t m, int64_t n, double alpha, double beta,
+               const ZView Z, const int* __restrict__ e_row, const int* __restrict__ f_col, double* __restrict__ C,
                int64_t ldc)
 {
     __shared__ double lam[kScatterMaxEnt];
@@ -1428,111 +1504,85 @@ scatter_kernel(const int* __restrict__ tab, int r0, int nprod, int64_t m, int64_
     }
     __syncthreads();
     const int ne = nsel;
-    const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ne == 0 || idx >= (uint32_t)rl * (uint32_t)cl) return;
-    const int i = (int)(idx % (uint32_t)rl), j = (int)(idx / (uint32_t)rl);
+    const uint32_t me = (uint32_t)((m + t.mt - 1) / t.mt), tiles_i = (me + blockDim.x - 1) / blockDim.x;
+    const int i = (int)(blockIdx.x % tiles_i * blockDim.x + threadIdx.x), j = (int)(blockIdx.x / tiles_i) * 4;
+    if ((ne == 0 && beta == 1.0) || i >= rl || j >= cl) return;
     double* cp = C + ro + i + (int64_t)(co + j) * ldc;
-    double c = *cp;
-    const int64_t zij = (int64_t)j * m_pad + i;
-    const int64_t zstride = (int64_t)n_pad * m_pad;
-    int q = 0;
-    for (; q + 4 <= ne; q += 4) {
-        int64_t z[4];
-        int ex[4];
+    double c[kScatterCols];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int r = prod[q + u];
-            z[u] = Z[r * zstride + zij];
-            ex[u] = e_row[r * m_pad + i] + f_col[r * n_pad + j] + ebase;
-        }
+    for (int u = 0; u < 4; ++u) c[u] = j + u < cl ? beta_c(beta, cp + u * ldc) : 0.0;
+    ZRow<FMT> z;
+    if (ne > 0) z.load(Z, e_row, f_col, prod[0], i, j);
+    for (int q = 0; q < ne; ++q) {
+        double M[kScatterCols];
+        z.values(Z, M);
+        if (q + 1 < ne) z.load(Z, e_row, f_col, prod[q + 1], i, j);   /* in flight under this product's updates */
 #pragma unroll
-        for (int u = 0; u < 4; ++u) c = fma(lam[q + u], i64_to_double_scaled(z[u], ex[u]), c);
+        for (int u = 0; u < 4; ++u) c[u] = fma(lam[q], M[u], c[u]);
     }
-    for (; q < ne; ++q) {
-        const int r = prod[q];
-        c = fma(lam[q], i64_to_double_scaled(Z[r * zstride + zij], e_row[r * m_pad + i] + f_col[r * n_pad + j] + ebase), c);
-    }
-    *cp = c;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+        if (j + u < cl) cp[u * ldc] = c[u];
 }
 
-/* one element (i, j) of the product grid for scatter_all_kernel */
-__device__ __forceinline__ void scatter_all_element(uint64_t idx, uint32_t rows, uint32_t i_lo, int P, int T, int tid,
-                                                    int nprod,
-                                                    int m_pad, int n_pad, int ebase, const int (&geo)[4][64],
-                                                    double* cs, const double* lam, const int* pidx, const int* off,
-                                                    const int64_t* __restrict__ Z, const int* __restrict__ e_row,
-                                                    const int* __restrict__ f_col, double* __restrict__ C,
-                                                    int64_t ldc)
-{
-    const int i = (int)(i_lo + (uint32_t)idx % rows), j = (int)((uint32_t)idx / rows);
-    uint64_t live = 0;
-    for (int p = 0; p < P; ++p) {
-        if (i < geo[1][p] && j < geo[3][p]) {
-            live |= 1ull << p;
-            cs[p * T + tid] = C[geo[0][p] + i + (int64_t)(geo[2][p] + j) * ldc];
-        }
-    }
-    const int64_t zij = (int64_t)j * m_pad + i;
-    const int64_t zstride = (int64_t)n_pad * m_pad;
-    int q = 0;
-    for (; q + 4 <= nprod; q += 4) {
-        int64_t z[4];
-        int ex[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            z[u] = Z[(q + u) * zstride + zij];
-            ex[u] = e_row[(int64_t)(q + u) * m_pad + i] + f_col[(int64_t)(q + u) * n_pad + j] + ebase;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int b = off[q + u], e = off[q + u + 1];
-            if (b == e) continue;
-            const double M = i64_to_double_scaled(z[u], ex[u]);
-            for (int x = b; x < e; ++x) {
-                const int p = pidx[x];
-                if ((live >> p) & 1ull) cs[p * T + tid] = fma(lam[x], M, cs[p * T + tid]);
-            }
-        }
-    }
-    for (; q < nprod; ++q) {
-        const int b = off[q], e = off[q + 1];
-        if (b == e) continue;
-        const double M = i64_to_double_scaled(Z[q * zstride + zij],
-                                              e_row[(int64_t)q * m_pad + i] + f_col[(int64_t)q * n_pad + j] + ebase);
-        for (int x = b; x < e; ++x) {
-            const int p = pidx[x];
-            if ((live >> p) & 1ull) cs[p * T + tid] = fma(lam[x], M, cs[p * T + tid]);
-        }
-    }
-    for (int p = 0; p < P; ++p)
-        if ((live >> p) & 1ull) C[geo[0][p] + i + (int64_t)(geo[2][p] + j) * ldc] = cs[p * T + tid];
-}
-
-/* Multi-C epilogue, element-major: one thread per element (i, j) of the
- * product grid (element index i + j*m_e in [idx_first, idx_end), grid-stride)
- * updates that element of every C sub-block p, so each product's
- * Z_r[i,j] is read and converted once and shared by all sub-blocks it feeds.
- * The sub-blocks' running values live in shared memory (cs[p][thread]); for
- * every sub-block the updates still come in increasing product order, so the
- * result is identical to scatter_kernel's. Used when the sub-block count and
- * the group's W entries fit the shared-memory budget. */
-constexpr int kScatterAllSmem = 32 * 1024;   /* cs[] budget: P * threads * 8 */
+/* Multi-C epilogue, element-major: a thread takes a row of a 4-column group
+ * of the product grid (rows [i_lo, i_lo + i_rows), all m_e rows when i_rows is
+ * 0; columns [c0, c1)) and updates those elements of every C sub-block p, so
+ * each product's Z_r is read (whole words: 5 to 10 loads for four elements)
+ * and converted once and shared by all sub-blocks it feeds. The sub-blocks'
+ * running values live in shared memory (cs[p][2][thread], two columns each);
+ * for every sub-block the updates still come in increasing product order, so
+ * the result is identical to scatter_kernel's. Used when the sub-block count
+ * and the group's W entries fit the shared-memory budget.
+ *
+ * Bound by the FP64 pipe (2 FMA/clk/SM) once an algorithm has several
+ * sub-blocks; four independent chains per thread keep it fed (222 x1 at
+ * 3000 x 2500: 66 us, 107 us with one element per thread; its 12 FMAs per
+ * element of the product grid take 37 us of the pipe). The classical
+ * case is bound by HBM instead (8 bytes of Z, 16 of C per element). */
+constexpr int kScatterAllSmem = 32 * 1024;   /* cs[] budget: P * threads * 32 */
+constexpr int kScatterAllMaxSmem = 96 * 1024;
 
 /* vb, vg: the block's index among the vg blocks that share the element range */
+template <int FMT>
 __device__ __forceinline__ void scatter_all_body(const int* __restrict__ tab, int r0, int nprod, int64_t m, int64_t n,
-                                                 int m_pad, int n_pad, int ebase, double alpha,
-                                                 const int64_t* __restrict__ Z, const int* __restrict__ e_row,
-                                                 const int* __restrict__ f_col, double* __restrict__ C, int64_t ldc,
-                                                 uint64_t idx_first, uint64_t idx_end, uint64_t vb, uint64_t vg,
-                                                 uint32_t i_lo = 0, uint32_t i_rows = 0)
+                                                 double alpha, double beta, const ZView& Z,
+                                                 const int* __restrict__ e_row, const int* __restrict__ f_col,
+                                                 double* __restrict__ C, int64_t ldc, int c0, int c1, uint32_t vb,
+                                                 uint32_t vg, uint32_t i_lo = 0, uint32_t i_rows = 0)
 {
-    extern __shared__ double sm_all[];
+    extern __shared__ __align__(16) double sm_all[];
     __shared__ int geo[4][64];           /* per sub-block p: ro, rl, co, cl */
     const Tab t = tab_view(tab);
     const int P = t.mt * t.nt, T = (int)blockDim.x, tid = (int)threadIdx.x;
     const int eb = t.w_off[r0], E = t.w_off[r0 + nprod] - eb;
-    double* cs = sm_all;                 /* [P][T] */
-    double* lam = cs + (size_t)P * T;    /* [E] */
+    const uint32_t me = (uint32_t)((m + t.mt - 1) / t.mt);
+    const uint32_t rows = i_rows ? i_rows : me;
+    const uint32_t tiles_i = (rows + T - 1) / T;
+    const uint32_t tiles = tiles_i * (uint32_t)((c1 + 3) / 4 - c0 / 4);   /* row tiles fastest */
+    if (P == 1 && E == 1 && nprod == 1) {
+        /* one sub-block fed by one product (the classical split GEMM): no
+         * shared memory, the C values in registers; HBM-bound (Z and C) */
+        const double l = alpha * (double)t.w_ent[2 * eb + 1];
+        const int jl = min((int)n, c1);
+        for (uint32_t x = vb; x < tiles; x += vg) {
+            const int i = (int)(i_lo + x % tiles_i * T) + tid, j = (int)(c0 / 4 + x / tiles_i) * 4;
+            if (i >= (int)(i_lo + rows)) continue;
+            ZRow<FMT> z;
+            z.load(Z, e_row, f_col, 0, i, j);
+            double* cp = C + i + (int64_t)j * ldc;
+            double c[kScatterCols], M[kScatterCols];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) c[u] = j + u >= c0 && j + u < jl ? beta_c(beta, cp + u * ldc) : 0.0;
+            z.values(Z, M);
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (j + u >= c0 && j + u < jl) cp[u * ldc] = fma(l, M[u], c[u]);
+        }
+        return;
+    }
+    double2* cs = (double2*)sm_all;      /* [P][2][T] */
+    double* lam = sm_all + (size_t)P * T * 4;    /* [E] */
     int* pidx = (int*)(lam + E);         /* [E] */
     int* off = pidx + E;                 /* [nprod + 1] */
     for (int x = tid; x < E; x += T) {
@@ -1545,61 +1595,59 @@ __device__ __forceinline__ void scatter_all_body(const int* __restrict__ tab, in
         fmm_part_geom32((int)n, t.nt, p % t.nt, &geo[2][p], &geo[3][p]);
     }
     __syncthreads();
-    const uint32_t me = (uint32_t)((m + t.mt - 1) / t.mt), ne = (uint32_t)((n + t.nt - 1) / t.nt);
-    /* the product-grid rows [i_lo, i_lo + rows) of every column, element
-     * index (i - i_lo) + j * rows (all rows when i_rows is 0); rows * ne <
-     * 2^32 (checked on the host), so the element index fits 32 bits */
-    const uint32_t rows = i_rows ? i_rows : me;
-    const uint64_t idx = idx_first + vb * (uint64_t)T + (uint64_t)tid;
-    const uint64_t end = idx_end < (uint64_t)rows * (uint64_t)ne ? idx_end : (uint64_t)rows * (uint64_t)ne;
-    if (P == 1 && E == 1 && nprod == 1) {
-        /* one sub-block fed by one product (the classical split GEMM): the
-         * same conversion and FMA per element without the per-sub-block
-         * bookkeeping, the element's C value kept in a register */
-        const double l = lam[0];
-        const uint64_t step = vg * (uint64_t)T;
-        constexpr int U = 2;   /* elements per thread per round: their loads go out together */
-        const int ro = geo[0][0], rl = geo[1][0], co = geo[2][0], cl = geo[3][0];
-        for (uint64_t idx2 = idx; idx2 < end; idx2 += U * step) {
-            int64_t z[U];
-            int ex[U];
-            double c[U];
-            int ii[U], jj[U];
+    for (uint32_t x = vb; x < tiles; x += vg) {
+        const int i = (int)(i_lo + x % tiles_i * T) + tid, j = (int)(c0 / 4 + x / tiles_i) * 4;
+        if (i >= (int)(i_lo + rows)) continue;
+        ZRow<FMT> z;
+        z.load(Z, e_row, f_col, 0, i, j);
+        /* elements outside a smaller sub-block or the column range are
+         * carried along as zeros and not stored */
+        for (int p = 0; p < P; ++p) {
+            const int jl = i < geo[1][p] ? min(geo[3][p], c1) : 0;
+            const double* cp = C + geo[0][p] + i + (int64_t)(geo[2][p] + j) * ldc;
+            double c[kScatterCols];
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const uint64_t e = idx2 + u * step;
-                ii[u] = (int)(i_lo + (uint32_t)e % rows);
-                jj[u] = e < end ? (int)((uint32_t)e / rows) : cl;   /* past the end: not live */
-                z[u] = 0;
-                ex[u] = 0;
-                c[u] = 0.0;
-                if (ii[u] < rl && jj[u] < cl) {
-                    z[u] = Z[(int64_t)jj[u] * m_pad + ii[u]];
-                    ex[u] = e_row[ii[u]] + f_col[jj[u]] + ebase;
-                    c[u] = C[ro + ii[u] + (int64_t)(co + jj[u]) * ldc];
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-                if (ii[u] < rl && jj[u] < cl)
-                    C[ro + ii[u] + (int64_t)(co + jj[u]) * ldc] = fma(l, i64_to_double_scaled(z[u], ex[u]), c[u]);
+            for (int u = 0; u < 4; ++u) c[u] = j + u >= c0 && j + u < jl ? beta_c(beta, cp + u * ldc) : 0.0;
+            cs[(2 * p) * T + tid] = make_double2(c[0], c[1]);
+            cs[(2 * p + 1) * T + tid] = make_double2(c[2], c[3]);
         }
-        return;
+        for (int q = 0; q < nprod; ++q) {
+            double M[kScatterCols];
+            z.values(Z, M);
+            if (q + 1 < nprod) z.load(Z, e_row, f_col, q + 1, i, j);   /* in flight under this product's updates */
+            const int e = off[q + 1];
+            for (int y = off[q]; y < e; ++y) {
+                const double l = lam[y];
+                double2* c = cs + 2 * pidx[y] * T + tid;
+                double2 a = c[0], b = c[T];
+                a.x = fma(l, M[0], a.x);
+                a.y = fma(l, M[1], a.y);
+                b.x = fma(l, M[2], b.x);
+                b.y = fma(l, M[3], b.y);
+                c[0] = a;
+                c[T] = b;
+            }
+        }
+        for (int p = 0; p < P; ++p) {
+            const int jl = i < geo[1][p] ? min(geo[3][p], c1) : 0;
+            double* cp = C + geo[0][p] + i + (int64_t)(geo[2][p] + j) * ldc;
+            const double2 a = cs[(2 * p) * T + tid], b = cs[(2 * p + 1) * T + tid];
+            const double c[kScatterCols] = {a.x, a.y, b.x, b.y};
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (j + u >= c0 && j + u < jl) cp[u * ldc] = c[u];
+        }
     }
-    /* grid-stride: a block's set-up above serves many elements */
-    for (uint64_t idx2 = idx; idx2 < end; idx2 += vg * (uint64_t)T)
-        scatter_all_element(idx2, rows, i_lo, P, T, tid, nprod, m_pad, n_pad, ebase, geo, cs, lam, pidx, off, Z,
-                            e_row, f_col, C, ldc);
 }
 
+template <int FMT>
 __global__ void __launch_bounds__(256)
-scatter_all_kernel(const int* __restrict__ tab, int r0, int nprod, int64_t m, int64_t n,
-                   int m_pad, int n_pad, int ebase, double alpha, const int64_t* __restrict__ Z,
-                   const int* __restrict__ e_row, const int* __restrict__ f_col, double* __restrict__ C,
-                   int64_t ldc, uint64_t idx_first, uint64_t idx_end, uint32_t i_lo, uint32_t i_rows)
+scatter_all_kernel(const int* __restrict__ tab, int r0, int nprod, int64_t m, int64_t n, double alpha, double beta,
+                   const ZView Z, const int* __restrict__ e_row, const int* __restrict__ f_col,
+                   double* __restrict__ C, int64_t ldc, int c0, int c1, uint32_t i_lo, uint32_t i_rows)
 {
-    scatter_all_body(tab, r0, nprod, m, n, m_pad, n_pad, ebase, alpha, Z, e_row, f_col, C, ldc, idx_first, idx_end,
-                     blockIdx.x, gridDim.x, i_lo, i_rows);
+    scatter_all_body<FMT>(tab, r0, nprod, m, n, alpha, beta, Z, e_row, f_col, C, ldc, c0, c1, blockIdx.x, gridDim.x,
+                          i_lo, i_rows);
 }
 
 
@@ -1623,13 +1671,13 @@ struct WaveProb {
     int* f_col;
     uint8_t* sa;
     uint8_t* sb;
-    const int64_t* Z;
+    ZView Z;
     int64_t lda, ldb, ldc, m, n, k, m_pad, n_pad, k_pad;
     int64_t b0;   /* the problem's first block in this launch */
     int64_t nb;   /* its blocks */
     int64_t gx;   /* blocks along the first coordinate of its per-problem grid */
     double alpha, beta;
-    int R, kt, ebase;
+    int R, kt, fmt;
 };
 struct WaveLaunch {
     int nprob;
@@ -1647,23 +1695,17 @@ __device__ __forceinline__ int wave_find(const WaveLaunch& W, int64_t b)
     return lo;
 }
 
-/* C := beta*C (when beta != 1) and the maxima arrays zeroed, grid-stride over each problem's range */
+/* the maxima arrays zeroed, grid-stride over each problem's range */
 __global__ void __launch_bounds__(256) wave_prep_kernel(const __grid_constant__ WaveLaunch W)
 {
     const WaveProb& P = W.p[wave_find(W, blockIdx.x)];
     const int64_t vb = blockIdx.x - P.b0;
     const int64_t za = (int64_t)P.kt * P.m, zb = (int64_t)P.kt * P.n;
-    const int64_t total = za + zb + (P.beta != 1.0 ? P.m * P.n : 0);
-    for (int64_t x = vb * blockDim.x + threadIdx.x; x < total; x += P.nb * (int64_t)blockDim.x) {
-        if (x < za) {
+    for (int64_t x = vb * blockDim.x + threadIdx.x; x < za + zb; x += P.nb * (int64_t)blockDim.x) {
+        if (x < za)
             P.amax[x] = 0;
-        } else if (x < za + zb) {
+        else
             P.bmax[x - za] = 0;
-        } else {
-            const int64_t e = x - za - zb;
-            double* c = P.C + e % P.m + (e / P.m) * P.ldc;
-            *c = P.beta == 0.0 ? 0.0 : P.beta * *c;
-        }
     }
 }
 
@@ -1709,11 +1751,12 @@ __global__ void __launch_bounds__(COLS * 8, COLS == 32 ? 4 : 8) wave_pack_b_kern
 __global__ void __launch_bounds__(256) wave_scatter_kernel(const __grid_constant__ WaveLaunch W)
 {
     const WaveProb& P = W.p[wave_find(W, blockIdx.x)];
-    const int64_t vb = blockIdx.x - P.b0;
-    const Tab t = tab_view(P.tab);
-    const uint64_t me = (uint64_t)((P.m + t.mt - 1) / t.mt), ne = (uint64_t)((P.n + t.nt - 1) / t.nt);
-    scatter_all_body(P.tab, 0, P.R, P.m, P.n, (int)P.m_pad, (int)P.n_pad, P.ebase, P.alpha, P.Z, P.e_row, P.f_col,
-                     P.C, P.ldc, 0, me * ne, (uint64_t)vb, (uint64_t)P.nb);
+    const uint32_t vb = (uint32_t)(blockIdx.x - P.b0), vg = (uint32_t)P.nb;
+    const int nt = P.tab[2], c1 = (int)((P.n + nt - 1) / nt);
+    if (P.fmt)
+        scatter_all_body<1>(P.tab, 0, P.R, P.m, P.n, P.alpha, P.beta, P.Z, P.e_row, P.f_col, P.C, P.ldc, 0, c1, vb, vg);
+    else
+        scatter_all_body<0>(P.tab, 0, P.R, P.m, P.n, P.alpha, P.beta, P.Z, P.e_row, P.f_col, P.C, P.ldc, 0, c1, vb, vg);
 }
 
 /* --------------------------------------------------------- host -------- */
@@ -1778,10 +1821,24 @@ Dims dims_of(const AlgView& alg, int64_t m, int64_t n, int64_t k, int fmt = 0)
     return d;
 }
 
+/* G, the level whose unit Z counts in: BF16 6, or 7 when k_pad <= 128 (the
+ * finest unit keeping Z inside int64); FP8 s + 1 up to 10 (exact for s <= 9) */
+int zlevel_of(const Dims& d, int s, int fmt)
+{
+    if (fmt) return std::min(s + 1, 10);
+    return d.k_pad <= 128 ? 7 : 6;
+}
+
+/* bytes of one product's Z planes */
+size_t z_bytes(const Dims& d, int s, int fmt)
+{
+    return (size_t)d.n_pad / 4 * (size_t)z_group_bytes(d.m_pad, ZPlanes::of(s, zlevel_of(d, s, fmt), fmt).nd);
+}
+
 size_t per_product_bytes(const Dims& d, int s, int fmt)
 {
-    return (fmt ? 1 : 2) * (size_t)s * (size_t)(d.m_pad + d.n_pad) * (size_t)d.k_pad +
-           8 * (size_t)d.m_pad * (size_t)d.n_pad + 4 * (size_t)(d.m_pad + d.n_pad) + 1024;
+    return (fmt ? 1 : 2) * (size_t)s * (size_t)(d.m_pad + d.n_pad) * (size_t)d.k_pad + z_bytes(d, s, fmt) +
+           4 * (size_t)(d.m_pad + d.n_pad) + 1024;
 }
 
 int group_size(const AlgView& alg, const Dims& d, int s, size_t budget, int fmt)
@@ -1814,7 +1871,7 @@ WsLayout ws_layout_g(const AlgView& alg, const Dims& d, int64_t m, int64_t n, in
     L.fcol = take(sizeof(int) * (size_t)G * (size_t)d.n_pad);
     L.sa = take(esz * (size_t)G * s * (size_t)d.m_pad * (size_t)d.k_pad);
     L.sb = take(esz * (size_t)G * s * (size_t)d.n_pad * (size_t)d.k_pad);
-    L.z = take(8 * (size_t)G * (size_t)d.m_pad * (size_t)d.n_pad);
+    L.z = take((size_t)G * z_bytes(d, s, fmt));
     L.total = off;
     return L;
 }
@@ -2105,12 +2162,12 @@ static void job_maxima_b(SplitJob& j, cudaStream_t st, int64_t c0 = 0, int64_t c
     fmm_count_launch(1);
 }
 
-/* C := beta*C and the per-sub-block row/column maxima of A and B; with a
+/* the per-sub-block row/column maxima of A and B; with a
  * side pool the B maxima run on its stream s[0], which job_pack joins back */
 static int job_prologue(SplitJob& j, cudaStream_t st, SidePool* sp = nullptr)
 {
-    int rc = fmm_scale_c(j.m, j.n, j.beta, j.C, j.ldc, st);
-    if (rc != FMM_OK || j.trivial) return rc;
+    int rc;
+    if (j.trivial) return fmm_scale_c(j.m, j.n, j.beta, j.C, j.ldc, st);   /* else beta goes with the C updates */
     if ((rc = job_maxima_a(j, st)) != FMM_OK) return rc;
     if (sp && (rc = side_fork1(sp, st)) != FMM_OK) return rc;
     job_maxima_b(j, sp ? sp->s[0] : st);
@@ -2226,16 +2283,24 @@ static void job_pack_a_rows(SplitJob& j, int r0, int np, int64_t a, int64_t b, c
     fmm_count_launch(2);
 }
 
-/* G, the level whose unit Z counts in: BF16 6, or 7 when k_pad <= 128 (the
- * finest unit keeping Z inside int64); FP8 s + 1 up to 10 (exact for s <= 9) */
-static int job_zlevel(const SplitJob& j)
-{
-    if (j.fmt) return std::min(j.s + 1, 10);
-    return j.d.k_pad <= 128 ? 7 : 6;
-}
+static int job_zlevel(const SplitJob& j) { return zlevel_of(j.d, j.s, j.fmt); }
 static int job_db(const SplitJob& j) { return j.fmt ? 5 : 8; }
 /* exponent of Z's unit relative to 2^(E_i + F_j) */
 static int job_ebase(const SplitJob& j) { return 2 - job_db(j) * job_zlevel(j); }
+
+/* the job's Z planes for the C updates */
+static ZView job_zview(const SplitJob& j)
+{
+    ZView v;
+    v.base = j.w + j.L.z;
+    v.prod = (int64_t)z_bytes(j.d, j.s, j.fmt);
+    v.nd = ZPlanes::of(j.s, job_zlevel(j), j.fmt).nd;
+    v.group = z_group_bytes(j.d.m_pad, v.nd);
+    v.m_pad = (int)j.d.m_pad;
+    v.n_pad = (int)j.d.n_pad;
+    v.ebase = job_ebase(j);
+    return v;
+}
 
 /* the job's product group as one problem of a GEMM launch */
 /* pair tiles for this job's single-call GEMM launches */
@@ -2256,9 +2321,13 @@ static int job_fill(const SplitJob& j, GemmProblem& gp, int np, int item_begin, 
         return FMM_ERR_CUDA;
     if (make_slice_map(&gp.tmB, sb, d.k_pad, (int64_t)np * j.s * d.n_pad, pair ? kTileN / 2 : kTileN, j.fmt) != FMM_OK)
         return FMM_ERR_CUDA;
-    gp.Z = (int64_t*)(j.w + j.L.z) + (size_t)r_first * d.m_pad * d.n_pad;
+    gp.Z = j.w + j.L.z + (size_t)r_first * z_bytes(d, j.s, j.fmt);
     gp.s = j.s;
     gp.zlevel = job_zlevel(j);
+    const ZPlanes zp = ZPlanes::of(j.s, gp.zlevel, j.fmt);
+    gp.zmin = zp.zmin;
+    gp.znd = zp.nd;
+    gp.zrow0 = 0;
     gp.kbe = kbe_of(j.fmt);
     gp.nkb = (int)(d.k_pad / gp.kbe);
     gp.db = job_db(j);
@@ -2339,7 +2408,8 @@ static int job_gemm_block(const SplitJob& j, int np, int64_t it0, int64_t it1, i
             make_slice_map(&gp.tmB, sb, j.d.k_pad, (int64_t)cnt * j.s * j.d.n_pad - c0, pair ? kTileN / 2 : kTileN,
                            j.fmt) != FMM_OK)
             return FMM_ERR_CUDA;
-        gp.Z += r0 + c0 * j.d.m_pad;
+        gp.Z += c0 / 4 * z_group_bytes(j.d.m_pad, gp.znd);
+        gp.zrow0 = (int)r0;
         gp.tiles_m = (int)tm;
         gp.tiles_n = (int)tn;
         if (int rc = launch_gemm(gl, (int64_t)cnt * tiles, cnt, st, pair); rc != FMM_OK) return rc;
@@ -2347,25 +2417,34 @@ static int job_gemm_block(const SplitJob& j, int np, int64_t it0, int64_t it1, i
     return FMM_OK;
 }
 
-/* blocks of the grid-stride element-major scatter: one per T elements, at
- * most 16 per SM (each then serves several elements) */
-static unsigned scatter_blocks(uint64_t elems, int T)
-{
-    return (unsigned)std::min<uint64_t>((elems + T - 1) / T, 16 * 152);
-}
+/* tiles of T rows x 4 columns of the element-major scatter over rows x cols
+ * elements (a column range may start inside a group) */
+static int64_t scatter_tiles(int64_t rows, int64_t cols, int T) { return (rows + T - 1) / T * ((cols + 3) / 4 + 1); }
 
-/* the element-major scatter applies to this job (see job_scatter) */
-static bool job_scatter_all(const SplitJob& j, int r0, int np, int* T_out, size_t* smem_out)
+/* blocks of one element-major scatter launch: one per tile, at most 16 per SM
+ * (each then serves several tiles with one set-up) */
+static unsigned scatter_blocks(int64_t tiles) { return (unsigned)std::min<int64_t>(tiles, 16 * 152); }
+
+/* Whether the element-major C update applies to products [r0, r0 + np): at
+ * most 64 sub-blocks whose values (T threads x 4 columns) and the group's W
+ * entries fit its shared memory. T: 32 KB of values, a multiple of 32 up to
+ * 256, at least 32; with `small` 16 KB and at most 128, which fits on an SM
+ * beside a resident GEMM CTA while P <= 16. */
+static bool job_scatter_all(const SplitJob& j, int r0, int np, int* T_out, size_t* smem_out, bool small = false)
 {
     const Tab ht = tab_view(j.alg.htab);
     const int P = j.alg.mt * j.alg.nt;
     const int E = ht.w_off[r0 + np] - ht.w_off[r0];
-    const int T = std::min(256, kScatterAllSmem / (8 * P)) / 32 * 32;
-    const size_t smem = (size_t)P * std::max(T, 0) * 8 + (size_t)E * 12 + (size_t)(np + 1) * 4;
+    const int T =
+        std::max(32, std::min(small ? 128 : 256, (small ? kScatterAllSmem / 2 : kScatterAllSmem) / (32 * P)) / 32 * 32);
+    const size_t smem = (size_t)P * T * 32 + (size_t)E * 12 + (size_t)(np + 1) * 4;
     *T_out = T;
     *smem_out = smem;
-    return P <= 64 && T >= 32 && smem <= 47 * 1024;
+    return P <= 64 && smem <= (size_t)kScatterAllMaxSmem;
 }
+
+/* beta*C comes with the C updates of the first product group */
+static double job_beta(const SplitJob& j, int r0) { return r0 == 0 ? j.beta : 1.0; }
 
 /* the C updates of products [r0, r0 + np) for the product-grid rows
  * [i0, i1) of the columns [j0, j1), element-major form only */
@@ -2374,20 +2453,14 @@ static void job_scatter_block(const SplitJob& j, int r0, int np, int64_t i0, int
 {
     int T;
     size_t smem;
-    job_scatter_all(j, r0, np, &T, &smem);
-    if (small && T > 128) {   /* 128-thread blocks fit on an SM beside a resident GEMM CTA */
-        const Tab ht = tab_view(j.alg.htab);
-        const int P = j.alg.mt * j.alg.nt, E = ht.w_off[r0 + np] - ht.w_off[r0];
-        T = 128;
-        smem = (size_t)P * T * 8 + (size_t)E * 12 + (size_t)(np + 1) * 4;
-    }
-    const uint64_t rows = (uint64_t)(i1 - i0);
-    const uint64_t first = (uint64_t)j0 * rows, end = (uint64_t)j1 * rows;
-    if (end <= first) return;
-    scatter_all_kernel<<<scatter_blocks(end - first, T), (unsigned)T, smem, st>>>(
-        j.alg.tab, r0, np, j.m, j.n, (int)j.d.m_pad, (int)j.d.n_pad, job_ebase(j), j.alpha,
-        (const int64_t*)(j.w + j.L.z), (const int*)(j.w + j.L.erow), (const int*)(j.w + j.L.fcol), j.C, j.ldc, first,
-        end, (uint32_t)i0, (uint32_t)rows);
+    job_scatter_all(j, r0, np, &T, &smem, small);
+    if (j1 <= j0 || i1 <= i0) return;
+    T = (int)std::min<int64_t>(T, round_up(i1 - i0, 32));   /* fewer values than smem has room for */
+    const unsigned nb = scatter_blocks(scatter_tiles(i1 - i0, j1 - j0, T));
+    auto* k = j.fmt ? scatter_all_kernel<1> : scatter_all_kernel<0>;
+    k<<<nb, (unsigned)T, smem, st>>>(j.alg.tab, r0, np, j.m, j.n, j.alpha, job_beta(j, r0), job_zview(j),
+                                     (const int*)(j.w + j.L.erow), (const int*)(j.w + j.L.fcol), j.C, j.ldc, (int)j0,
+                                     (int)j1, (uint32_t)i0, (uint32_t)(i1 - i0));
     fmm_count_launch(1);
 }
 
@@ -2399,30 +2472,18 @@ static void job_scatter_cols(const SplitJob& j, int r0, int np, int64_t j0, int6
     job_scatter_block(j, r0, np, 0, j.d.me, j0, j1, st, small);
 }
 
-/* small: blocks of at most 128 threads (and so at most 16 KB of sub-block
- * values), which fit on an SM beside a resident GEMM CTA */
 static void job_scatter(const SplitJob& j, int r0, int np, cudaStream_t st, bool small = false)
 {
-    const int64_t elems = j.d.me * j.d.ne;   /* the largest part's extent */
-    /* element-major form when the sub-block values and the group's W entries
-     * fit beside the kernel's 1 KB of static geometry in 48 KB: threads per
-     * block T = 32 KB / (8 P), a multiple of 32, at least 32 */
-    const Tab ht = tab_view(j.alg.htab);
-    const int P = j.alg.mt * j.alg.nt;
-    const int E = ht.w_off[r0 + np] - ht.w_off[r0];
-    int T = std::min(small ? 128 : 256, kScatterAllSmem / (8 * P)) / 32 * 32;
-    const size_t smem = (size_t)P * std::max(T, 0) * 8 + (size_t)E * 12 + (size_t)(np + 1) * 4;
-    if (P <= 64 && T >= 32 && smem <= 47 * 1024) {
-        scatter_all_kernel<<<scatter_blocks((uint64_t)elems, T), (unsigned)T, smem, st>>>(
-            j.alg.tab, r0, np, j.m, j.n, (int)j.d.m_pad, (int)j.d.n_pad, job_ebase(j), j.alpha,
-            (const int64_t*)(j.w + j.L.z), (const int*)(j.w + j.L.erow), (const int*)(j.w + j.L.fcol), j.C, j.ldc,
-            (uint64_t)0, (uint64_t)elems, 0u, 0u);
-        fmm_count_launch(1);
+    int T;
+    size_t smem;
+    if (job_scatter_all(j, r0, np, &T, &smem)) {
+        job_scatter_block(j, r0, np, 0, j.d.me, 0, j.d.ne, st, small);
         return;
     }
-    scatter_kernel<<<dim3((unsigned)((elems + 255) / 256), (unsigned)(j.alg.mt * j.alg.nt)), 256, 0, st>>>(
-        j.alg.tab, r0, np, j.m, j.n, (int)j.d.m_pad, (int)j.d.n_pad, job_ebase(j), j.alpha,
-        (const int64_t*)(j.w + j.L.z), (const int*)(j.w + j.L.erow), (const int*)(j.w + j.L.fcol), j.C, j.ldc);
+    auto* k = j.fmt ? scatter_kernel<1> : scatter_kernel<0>;
+    k<<<dim3((unsigned)((j.d.me + 127) / 128 * ((j.d.ne + 3) / 4)), (unsigned)(j.alg.mt * j.alg.nt)), 128, 0, st>>>(
+        j.alg.tab, r0, np, j.m, j.n, j.alpha, job_beta(j, r0), job_zview(j), (const int*)(j.w + j.L.erow),
+        (const int*)(j.w + j.L.fcol), j.C, j.ldc);
     fmm_count_launch(1);
 }
 
@@ -2434,10 +2495,14 @@ static int launch_gemm(GemmLaunch& gl, int64_t nitems, int nprod_timed, cudaStre
     if (cudaGetDevice(&dev) != cudaSuccess) return FMM_ERR_CUDA;
     const uint64_t bit = dev < 64 ? 1ull << dev : 0;
     if (bit == 0 || !(attr_set.load(std::memory_order_acquire) & bit)) {
-        if (cudaFuncSetAttribute(split_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kGemmSmem) != cudaSuccess ||
-            cudaFuncSetAttribute(split_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kPairSmem) != cudaSuccess)
+        auto smem_limit = [](const void* f, size_t bytes) {
+            return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
+        };
+        if (!smem_limit((const void*)split_gemm_kernel, kGemmSmem) ||
+            !smem_limit((const void*)split_gemm_pair_kernel, kPairSmem) ||
+            !smem_limit((const void*)scatter_all_kernel<0>, kScatterAllMaxSmem) ||
+            !smem_limit((const void*)scatter_all_kernel<1>, kScatterAllMaxSmem) ||
+            !smem_limit((const void*)wave_scatter_kernel, kScatterAllMaxSmem))
             return FMM_ERR_CUDA;
         attr_set.fetch_or(bit, std::memory_order_acq_rel);
     }
@@ -2633,7 +2698,7 @@ int fmm_split_host(const AlgView& alg, int64_t m, int64_t n, int64_t k, double a
         if (int rc = fmm_scale_c(m, n, beta, dC, m, st); rc != FMM_OK) return rc;
     } else {
         SplitJob j;
-        int rc = job_init(j, alg, m, n, k, alpha, dA, m, dB, ka, 0.0, dC, m, s, fmt);
+        int rc = job_init(j, alg, m, n, k, alpha, dA, m, dB, ka, beta, dC, m, s, fmt);
         if (rc != FMM_OK) return rc;
         if ((rc = job_bind(j, ws, wsb, wsb)) != FMM_OK) return rc;
         const int G = j.L.group, nt = alg.nt;
@@ -2728,12 +2793,11 @@ int fmm_split_host(const AlgView& alg, int64_t m, int64_t n, int64_t k, double a
                 }
                 if (CH == 2 && (rc = up_b(1)) != FMM_OK) return rc;
                 mark(2, cs);
-                /* C up behind A and B, then C := beta*C, on s[3] */
+                /* C up behind A and B, for the C updates on s[3] */
                 if (beta != 0.0 &&
                     (!ok(fmm_copy2d_async(dC, row, C, sizeof(double) * ldc, row, n, cudaMemcpyHostToDevice, cs)) ||
                      !ok(cudaEventRecord(sp->gate[2], cs)) || !ok(cudaStreamWaitEvent(ss, sp->gate[2], 0))))
                     return FMM_ERR_CUDA;
-                if ((rc = fmm_scale_c(m, n, beta, dC, m, ss)) != FMM_OK) return rc;
                 /* the GEMM blocks on the call's stream */
                 const int order[4][2] = {{0, 0}, {1, 0}, {0, 1}, {1, 1}};
                 int nq = 0;
@@ -2852,12 +2916,11 @@ int fmm_split_host(const AlgView& alg, int64_t m, int64_t n, int64_t k, double a
             if ((rc = job_gemm(j, np, st)) != FMM_OK) return rc;
             if (r0 + np >= alg.R) mark(4, st);
             if (r0 == 0) {
-                /* C under the first GEMM, then C := beta*C before the first scatter */
+                /* C under the first GEMM, before the first C updates */
                 if (beta != 0.0 &&
                     (!ok(fmm_copy2d_async(dC, row, C, sizeof(double) * ldc, row, n, cudaMemcpyHostToDevice, cs)) ||
                      !ok(cudaEventRecord(sp->gate[2], cs)) || !ok(cudaStreamWaitEvent(st, sp->gate[2], 0))))
                     return FMM_ERR_CUDA;
-                if ((rc = fmm_scale_c(m, n, beta, dC, m, st)) != FMM_OK) return rc;
             }
             int T;
             size_t smem;
@@ -2945,13 +3008,12 @@ static WaveProb wave_prob(const SplitJob& j)
     w.f_col = (int*)(j.w + j.L.fcol);
     w.sa = j.w + j.L.sa;
     w.sb = j.w + j.L.sb;
-    w.Z = (const int64_t*)(j.w + j.L.z);
+    w.Z = job_zview(j);
     w.lda = j.lda; w.ldb = j.ldb; w.ldc = j.ldc;
     w.m = j.m; w.n = j.n; w.k = j.k;
     w.m_pad = j.d.m_pad; w.n_pad = j.d.n_pad; w.k_pad = j.d.k_pad;
     w.alpha = j.alpha; w.beta = j.beta;
-    w.R = j.alg.R; w.kt = j.alg.kt;
-    w.ebase = job_ebase(j);
+    w.R = j.alg.R; w.kt = j.alg.kt; w.fmt = j.fmt;
     return w;
 }
 
@@ -3033,7 +3095,7 @@ static int wave_side_pack(const std::vector<SplitJob*>& qs, bool small, cudaStre
     if (qs.empty()) return FMM_OK;
     WaveLaunch L;
     int64_t nb = wave_table(L, qs, [](const SplitJob& j, WaveProb& w) {
-        const int64_t total = (int64_t)j.alg.kt * (j.m + j.n) + (j.beta != 1.0 ? j.m * j.n : 0);
+        const int64_t total = (int64_t)j.alg.kt * (j.m + j.n);
         w.gx = 1;
         w.nb = std::min<int64_t>(std::max<int64_t>((total + 2047) / 2048, 1), 2048);
     });
@@ -3073,7 +3135,7 @@ static int wave_side_scatter(const std::vector<SplitJob*>& qs, bool small, cudaS
     for (SplitJob* j : qs) {
         int Tj;
         size_t sm;
-        if (job_scatter_all(*j, 0, j->alg.R, &Tj, &sm) && Tj >= 32) {
+        if (job_scatter_all(*j, 0, j->alg.R, &Tj, &sm, small)) {
             all.push_back(j);
             T = std::min(T, Tj);
         } else {
@@ -3085,12 +3147,17 @@ static int wave_side_scatter(const std::vector<SplitJob*>& qs, bool small, cudaS
         for (SplitJob* j : all) {
             const Tab ht = tab_view(j->alg.htab);
             const int P = j->alg.mt * j->alg.nt, E = ht.w_off[j->alg.R] - ht.w_off[0];
-            smem = std::max(smem, (size_t)P * T * 8 + (size_t)E * 12 + (size_t)(j->alg.R + 1) * 4);
+            smem = std::max(smem, (size_t)P * T * 32 + (size_t)E * 12 + (size_t)(j->alg.R + 1) * 4);
         }
+        /* the launch's blocks are shared out by the problems' tiles, so a
+         * block's set-up serves several tiles in a wave of many problems too */
+        int64_t tiles = 0;
+        for (SplitJob* j : all) tiles += scatter_tiles(j->d.me, j->d.ne, T);
+        const double share = (double)scatter_blocks(tiles) / (double)tiles;
         WaveLaunch L;
         const int64_t nb = wave_table(L, all, [&](const SplitJob& j, WaveProb& w) {
             w.gx = 1;
-            w.nb = scatter_blocks((uint64_t)(j.d.me * j.d.ne), T);
+            w.nb = std::max<int64_t>(1, (int64_t)(share * (double)scatter_tiles(j.d.me, j.d.ne, T)));
         });
         wave_scatter_kernel<<<(unsigned)nb, (unsigned)T, smem, st>>>(L);
         fmm_count_launch(1);
