@@ -517,6 +517,7 @@ extern "C" int fmm_gpu_split_strassen_ab_ex(double alpha, const double* A, int64
 extern "C" void fmm_gpu_release_host_buffers(void)
 {
     fmm_split_host_release();
+    fmm_f64_release_temp();
     std::lock_guard<std::mutex> lk(g_gen_mu);
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;

@@ -30,6 +30,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 namespace cg = cooperative_groups;
@@ -369,6 +370,180 @@ fmm_f64_kernel(const int* __restrict__ tab, int64_t m, int64_t n, int64_t k,
                                       (int)(blockIdx.x / tiles_m), As, Bs, ue, ve, r_begin, r_end, Sp, Tp);
 }
 
+/* ------------------------------------- pipelined single-term tiles ---- */
+
+/* 8-byte global -> shared copy, zero when !ok (nothing is read then) */
+__device__ __forceinline__ void cp_async8(double* dst, const double* src, bool ok)
+{
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(ok ? 8 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+/* Tile geometry of the pipelined kernels: BM x BN outputs per CTA, TM x TN per
+ * thread, k steps of kPipeBk in a ring of kPipeStages shared-memory stages
+ * (A as [k][m]; B as [k][n] with an odd pitch, as its copies run along k). */
+constexpr int kPipeBk = 16, kPipeStages = 4;
+template <int BM, int BN, int TM, int TN>
+struct PipeTile {
+    static constexpr int RT = BM / TM, CT = BN / TN, NT = RT * CT;
+    static constexpr int PB = BN + 1;
+    static constexpr int STAGE = kPipeBk * (BM + PB);            /* doubles */
+    static constexpr size_t SMEM = sizeof(double) * STAGE * kPipeStages;
+    static_assert(NT % BM == 0 && NT % kPipeBk == 0, "tile/thread mapping");
+
+    /* the stage's copies: rows [i0, i0 + BM) x k [k0, k0 + kPipeBk) of A and
+     * the same k x columns [j0, j0 + BN) of B, zero outside rows/cols/kend */
+    __device__ static __forceinline__ void issue(double* st, const double* __restrict__ A, int64_t lda, int64_t rows,
+                                                 const double* __restrict__ B, int64_t ldb, int64_t cols, int64_t i0,
+                                                 int64_t j0, int64_t k0, int64_t kend)
+    {
+        const int tid = threadIdx.x;
+        {
+            const int li = tid % BM, lk = tid / BM;
+            const int64_t gi = i0 + li;
+            const bool ok = gi < rows;
+            const double* p = A + (ok ? gi : 0) + k0 * lda;
+            double* d = st + li;
+#pragma unroll
+            for (int t = 0; t < kPipeBk * BM / NT; ++t) {
+                const int kk = lk + t * (NT / BM);
+                const bool in = ok && k0 + kk < kend;
+                cp_async8(d + kk * BM, in ? p + kk * lda : A, in);
+            }
+        }
+        {
+            const int kk = tid % kPipeBk, lj = tid / kPipeBk;
+            const bool ok = k0 + kk < kend;
+            const double* p = B + (ok ? k0 + kk : 0);
+            double* d = st + kPipeBk * BM + kk * PB;
+#pragma unroll
+            for (int t = 0; t < kPipeBk * BN / NT; ++t) {
+                const int jj = lj + t * (NT / kPipeBk);
+                const bool in = ok && j0 + jj < cols;
+                cp_async8(d + jj, in ? p + (j0 + jj) * ldb : B, in);
+            }
+        }
+    }
+
+    /* acc += the stage's kn rows, k in increasing order */
+    __device__ static __forceinline__ void multiply(const double* st, int kn, double (&acc)[TM][TN])
+    {
+        const int tr = threadIdx.x % RT, tc = threadIdx.x / RT;
+        const double* as = st + tr;
+        const double* bs = st + kPipeBk * BM + tc;
+#pragma unroll 4
+        for (int kk = 0; kk < kn; ++kk) {
+            double a[TM], b[TN];
+#pragma unroll
+            for (int x = 0; x < TM; ++x) a[x] = as[kk * BM + x * RT];
+#pragma unroll
+            for (int y = 0; y < TN; ++y) b[y] = bs[kk * PB + y * CT];
+#pragma unroll
+            for (int x = 0; x < TM; ++x)
+#pragma unroll
+                for (int y = 0; y < TN; ++y) acc[x][y] = fma(a[x], b[y], acc[x][y]);
+        }
+    }
+};
+
+/* The FP64 FMM GEMM over single-term operands (the classical GEMM, or the
+ * pre-formed S_r, T_r of the products r_begin..): one CTA per output tile
+ * position runs every product over it, as fmm_f64_kernel does and in the same
+ * order (the same bits), with the operand copies of the next steps, across
+ * products too, in flight under the DFMAs. Bound by the FP64 pipe, 2 FMA per
+ * clock and SM, which eight warps keep busy; the CTAs are small so that the
+ * SMs' shares of the tiles differ little. */
+template <int BM, int BN, int TM, int TN, int MINB>
+__global__ void __launch_bounds__(PipeTile<BM, BN, TM, TN>::NT, MINB)
+fmm_f64_pipe_kernel(const int* __restrict__ tab, int64_t m, int64_t n, int64_t k, double alpha,
+                    const double* __restrict__ A, int64_t lda, const double* __restrict__ B, int64_t ldb,
+                    double* __restrict__ C, int64_t ldc, int tiles_m, int r_begin, int r_end,
+                    const double* __restrict__ Sp, const double* __restrict__ Tp)
+{
+    using PT = PipeTile<BM, BN, TM, TN>;
+    extern __shared__ double f64_stages[];
+    const int mt = tab[0], kt = tab[1], nt = tab[2], R = tab[3];
+    const int* u_off = tab + FMM_ALG_HDR;
+    const int* v_off = u_off + (R + 1);
+    const int* w_off = v_off + (R + 1);
+    const int* w_ent = w_off + (R + 1) + 2 * u_off[R] + 2 * v_off[R];
+    const int64_t me = (m + mt - 1) / mt, ne = (n + nt - 1) / nt, ke = (k + kt - 1) / kt;
+    const int64_t i0 = (int64_t)(blockIdx.x % (unsigned)tiles_m) * BM, j0 = (int64_t)(blockIdx.x / (unsigned)tiles_m) * BN;
+    const int tr = threadIdx.x % PT::RT, tc = threadIdx.x / PT::RT;
+    if (Sp) {
+        A = Sp;
+        lda = me;
+        B = Tp;
+        ldb = ke;
+    }
+    const int64_t sa = Sp ? me * ke : 0, sb = Sp ? ke * ne : 0;   /* operands of the next product */
+    const int64_t nk = (ke + kPipeBk - 1) / kPipeBk;
+    int lr = r_begin;      /* the next step to copy: product lr, k from lk */
+    int64_t lk = 0;
+    const double *la = A, *lb = B;
+    int ls = 0;            /* its stage */
+    auto copy_next = [&]() {
+        if (lr < r_end) {
+            PT::issue(f64_stages + ls * PT::STAGE, la, lda, me, lb, ldb, ne, i0, j0, lk, ke);
+            lk += kPipeBk;
+            if (lk >= ke) {
+                lk = 0;
+                ++lr;
+                la += sa;
+                lb += sb;
+            }
+            ls = ls + 1 == kPipeStages ? 0 : ls + 1;
+        }
+        cp_async_commit();
+    };
+#pragma unroll
+    for (int x = 0; x < kPipeStages - 1; ++x) copy_next();
+    int cs = 0;            /* the stage to multiply */
+    for (int r = r_begin; r < r_end; ++r) {
+        double acc[TM][TN];
+#pragma unroll
+        for (int x = 0; x < TM; ++x)
+#pragma unroll
+            for (int y = 0; y < TN; ++y) acc[x][y] = 0.0;
+        for (int64_t q = 0; q < nk; ++q) {
+            cp_async_wait<kPipeStages - 2>();
+            __syncthreads();   /* the step's copies are in, and the stage copied to next is read out */
+            copy_next();
+            const int64_t left = ke - q * kPipeBk;
+            if (left >= kPipeBk)
+                PT::multiply(f64_stages + cs * PT::STAGE, kPipeBk, acc);
+            else
+                PT::multiply(f64_stages + cs * PT::STAGE, (int)left, acc);
+            cs = cs + 1 == kPipeStages ? 0 : cs + 1;
+        }
+        /* multi-C epilogue */
+        for (int e = w_off[r]; e < w_off[r + 1]; ++e) {
+            const int part = w_ent[2 * e];
+            const double lam = alpha * (double)w_ent[2 * e + 1];
+            int64_t ro, rl, co, cl;
+            fmm_part_geom(m, mt, part / nt, &ro, &rl);
+            fmm_part_geom(n, nt, part % nt, &co, &cl);
+            double* cb = C + (ro + i0 + tr) + (co + j0 + tc) * ldc;
+            const int64_t il = rl - i0 - tr, jl = cl - j0 - tc;   /* rows and columns left from this thread's first */
+            double c[TM][TN];
+#pragma unroll
+            for (int y = 0; y < TN; ++y)
+#pragma unroll
+                for (int x = 0; x < TM; ++x)
+                    if (x * PT::RT < il && y * PT::CT < jl) c[x][y] = cb[x * PT::RT + y * PT::CT * ldc];
+#pragma unroll
+            for (int y = 0; y < TN; ++y)
+#pragma unroll
+                for (int x = 0; x < TM; ++x)
+                    if (x * PT::RT < il && y * PT::CT < jl)
+                        cb[x * PT::RT + y * PT::CT * ldc] = fma(lam, acc[x][y], c[x][y]);
+        }
+    }
+}
+
 /* ------------------------------------------------------------ batched -- */
 
 /* One problem of a batched FP64 launch; problems are laid out in the order
@@ -384,10 +559,10 @@ struct F64Prob {
     double* C;
     int64_t ldc;
     int64_t item_begin;   /* first (tile position) item of this problem */
-    int tiles_m, tiles_n;
+    int tiles_m, tile;    /* tile: items are tile x tile positions (64, 32 or 16) */
 };
 
-constexpr int kF64Bm = 64, kF64Bn = 64, kF64Bk = 32, kF64Tm = 4, kF64Tn = 4;
+constexpr int kF64BatchThreads = 256;
 constexpr int kF64TableChunk = 256;   /* problems per table-writer launch (parameter space) */
 
 struct F64TableChunk {
@@ -403,29 +578,58 @@ __global__ void f64_table_write(const __grid_constant__ F64TableChunk c)
     for (int i = threadIdx.x; i < c.count; i += blockDim.x) c.dst[i] = c.p[i];
 }
 
+/* One item: beta applied to the C elements its threads own in every
+ * sub-block of the tile position, then the tile as the single-problem kernels
+ * run it (every tile shape accumulates in the same order: the same bits). */
+template <int B, int T, bool MMA>
+__device__ __forceinline__ void f64_batch_item(const F64Prob& P, int ti, int tj, double* As, double* Bs, Entry* ue,
+                                               Entry* ve)
+{
+    constexpr int RT = B / T;
+    const int tr = threadIdx.x % RT, tc = threadIdx.x / RT;
+    const int mt = P.tab[0], nt = P.tab[2];
+    if (P.beta != 1.0) {
+        for (int part = 0; part < mt * nt; ++part) {
+            int64_t ro, rl, co, cl;
+            fmm_part_geom(P.m, mt, part / nt, &ro, &rl);
+            fmm_part_geom(P.n, nt, part % nt, &co, &cl);
+            for (int y = 0; y < T; ++y) {
+                const int64_t gj = (int64_t)tj * B + tc + y * RT;
+                if (gj >= cl) continue;
+                for (int x = 0; x < T; ++x) {
+                    const int64_t gi = (int64_t)ti * B + tr + x * RT;
+                    if (gi < rl) {
+                        double* q = P.C + ro + gi + (co + gj) * P.ldc;
+                        *q = P.beta == 0.0 ? 0.0 : P.beta * *q;
+                    }
+                }
+            }
+        }
+    }
+    if (P.k == 0 || P.alpha == 0.0) return;
+    f64_tile<B, B, 32, T, T, MMA>(P.tab, P.m, P.n, P.k, P.alpha, P.A, P.lda, P.B, P.ldb, P.C, P.ldc, ti, tj, As, Bs, ue,
+                                  ve, 0, P.tab[3], nullptr, nullptr);
+}
+
 /* Batched FP64 FMM GEMM: one persistent launch over all (problem, tile
  * position) items of a batch. A CTA takes the next item from an atomic
  * counter (problems sorted by per-item work, largest first, so the long
- * items go out first), applies beta to the C elements its threads own in
- * every sub-block of that tile position, then runs the tile exactly as the
- * single-problem kernel does, so each result is identical to the problem
- * issued alone. */
+ * items go out first). The FP64 MMA engine has no 16 x 16 tile (its eight
+ * warps need 8 x 8 fragments). */
 template <bool MMA>
-__global__ void __launch_bounds__((kF64Bm / kF64Tm) * (kF64Bn / kF64Tn))
+__global__ void __launch_bounds__(kF64BatchThreads)
 fmm_f64_batch_kernel(const F64Prob* __restrict__ probs, int nprob, int64_t nitems,
                      unsigned long long* __restrict__ counter)
 {
-    constexpr int RT = kF64Bm / kF64Tm, CT = kF64Bn / kF64Tn;
-    using SM = F64Smem<kF64Bm, kF64Bn, kF64Bk, MMA>;
+    using SM = F64Smem<64, 64, 32, MMA>;
     __shared__ double As[SM::A_ELEMS];
     __shared__ double Bs[SM::B_ELEMS];
     __shared__ Entry ue[kMaxEntries];
     __shared__ Entry ve[kMaxEntries];
     __shared__ long long next;
-    const int tid = threadIdx.x, tr = tid % RT, tc = tid / RT;
     for (;;) {
         __syncthreads();   /* the previous item is done with next, ue and ve */
-        if (tid == 0) next = (long long)atomicAdd(counter, 1ull);
+        if (threadIdx.x == 0) next = (long long)atomicAdd(counter, 1ull);
         __syncthreads();
         const int64_t b = next;
         if (b >= nitems) break;
@@ -437,29 +641,12 @@ fmm_f64_batch_kernel(const F64Prob* __restrict__ probs, int nprob, int64_t nitem
         const F64Prob P = probs[lo];
         const int64_t local = b - P.item_begin;
         const int ti = (int)(local % P.tiles_m), tj = (int)(local / P.tiles_m);
-        const int mt = P.tab[0], nt = P.tab[2];
-        if (P.beta != 1.0) {
-            for (int part = 0; part < mt * nt; ++part) {
-                int64_t ro, rl, co, cl;
-                fmm_part_geom(P.m, mt, part / nt, &ro, &rl);
-                fmm_part_geom(P.n, nt, part % nt, &co, &cl);
-                for (int y = 0; y < kF64Tn; ++y) {
-                    const int64_t gj = (int64_t)tj * kF64Bn + tc + y * CT;
-                    if (gj >= cl) continue;
-                    for (int x = 0; x < kF64Tm; ++x) {
-                        const int64_t gi = (int64_t)ti * kF64Bm + tr + x * RT;
-                        if (gi < rl) {
-                            double* q = P.C + ro + gi + (co + gj) * P.ldc;
-                            *q = P.beta == 0.0 ? 0.0 : P.beta * *q;
-                        }
-                    }
-                }
-            }
-        }
-        if (P.k == 0 || P.alpha == 0.0) continue;
-        f64_tile<kF64Bm, kF64Bn, kF64Bk, kF64Tm, kF64Tn, MMA>(P.tab, P.m, P.n, P.k, P.alpha, P.A, P.lda, P.B, P.ldb,
-                                                        P.C, P.ldc, ti, tj, As, Bs, ue, ve, 0, P.tab[3],
-                                                        nullptr, nullptr);
+        if (P.tile == 64)
+            f64_batch_item<64, 4, MMA>(P, ti, tj, As, Bs, ue, ve);
+        else if (MMA || P.tile == 32)
+            f64_batch_item<32, 2, MMA>(P, ti, tj, As, Bs, ue, ve);
+        else
+            f64_batch_item<16, 1, false>(P, ti, tj, As, Bs, ue, ve);
     }
 }
 
@@ -531,74 +718,63 @@ __global__ void scale_c_kernel(int64_t m, int64_t n, double beta, double* C, int
  * with a long k (the BLIS "sup" shapes, blis/kernels/haswell/3/sup): the
  * regular kernel would run one CTA per tile down the whole of k on a few
  * SMs. Here a cluster of ks CTAs (one per k chunk of kc elements) computes
- * each tile: every CTA accumulates its chunk in k order with the DFMA
- * micro-kernel, leaves its partial tile in shared memory, and after a cluster
+ * each tile: every CTA accumulates its chunk in k order (the pipelined tile),
+ * leaves its partial tile in shared memory, and after a cluster
  * barrier each CTA sums a share of the tile's elements over the ks partials
  * through distributed shared memory, always in chunk order
  * (((p_0 + p_1) + p_2) + ...), and applies C := fma(alpha, sum, C). The
  * result depends only on (m, n, k): the batched call runs these problems
  * through the same kernel. */
-constexpr int kSupB = 32, kSupBk = 32, kSupT = 2, kSupThreads = (kSupB / kSupT) * (kSupB / kSupT);
-constexpr int kSupMaxTiles = 128, kSupMaxSplits = 8, kSupMinChunk = 256;
-
-__global__ void __launch_bounds__(kSupThreads)
+template <int BM, int BN, int TM, int TN, int MINB>
+__global__ void __launch_bounds__(PipeTile<BM, BN, TM, TN>::NT, MINB)
 fmm_f64_sup_kernel(int64_t m, int64_t n, int64_t k, double alpha, const double* __restrict__ A, int64_t lda,
                    const double* __restrict__ B, int64_t ldb, double* __restrict__ C, int64_t ldc, int tiles_m,
                    int ks, int64_t kc)
 {
-    constexpr int RT = kSupB / kSupT;   /* thread rows (and columns) */
-    __shared__ double As[kSupBk][kSupB + 1];
-    __shared__ double Bs[kSupBk][kSupB + 1];
-    __shared__ double Ps[kSupB * kSupB];          /* this CTA's partial tile, element i + 32 j */
+    using PT = PipeTile<BM, BN, TM, TN>;
+    extern __shared__ double f64_stages[];
+    __shared__ double Ps[BM * BN];                /* this CTA's partial tile, element i + BM j */
     cg::cluster_group cl = cg::this_cluster();
     const int rank = (int)cl.block_rank();        /* the k chunk */
     const int tile = (int)(blockIdx.x / (unsigned)ks);
-    const int64_t i0 = (int64_t)(tile % tiles_m) * kSupB, j0 = (int64_t)(tile / tiles_m) * kSupB;
+    const int64_t i0 = (int64_t)(tile % tiles_m) * BM, j0 = (int64_t)(tile / tiles_m) * BN;
     const int64_t kb = (int64_t)rank * kc, kend = kb + kc < k ? kb + kc : k;
-    const int tid = threadIdx.x, tr = tid % RT, tc = tid / RT;
-    double acc[kSupT][kSupT];
+    const int tid = threadIdx.x, tr = tid % PT::RT, tc = tid / PT::RT;
+    double acc[TM][TN];
 #pragma unroll
-    for (int x = 0; x < kSupT; ++x)
+    for (int x = 0; x < TM; ++x)
 #pragma unroll
-        for (int y = 0; y < kSupT; ++y) acc[x][y] = 0.0;
-    for (int64_t k0 = kb; k0 < kend; k0 += kSupBk) {
-        /* A: 32 rows x 32 k, B: 32 k x 32 columns, zero past the edges */
-#pragma unroll
-        for (int t = 0; t < kSupB * kSupBk / kSupThreads; ++t) {
-            const int e = tid + t * kSupThreads;
-            const int li = e % kSupB, lk = e / kSupB;
-            const int64_t gi = i0 + li, gk = k0 + lk;
-            As[lk][li] = (gi < m && gk < kend) ? __ldg(A + gi + gk * lda) : 0.0;
-            const int lk2 = e % kSupBk, lj = e / kSupBk;
-            const int64_t gk2 = k0 + lk2, gj = j0 + lj;
-            Bs[lk2][lj] = (gk2 < kend && gj < n) ? __ldg(B + gk2 + gj * ldb) : 0.0;
+        for (int y = 0; y < TN; ++y) acc[x][y] = 0.0;
+    int64_t lk = kb;
+    int ls = 0, cs = 0;
+    auto copy_next = [&]() {
+        if (lk < kend) {
+            PT::issue(f64_stages + ls * PT::STAGE, A, lda, m, B, ldb, n, i0, j0, lk, kend);
+            lk += kPipeBk;
+            ls = ls + 1 == kPipeStages ? 0 : ls + 1;
         }
-        __syncthreads();
-#pragma unroll 8
-        for (int kk = 0; kk < kSupBk; ++kk) {
-            double a[kSupT], b[kSupT];
+        cp_async_commit();
+    };
 #pragma unroll
-            for (int x = 0; x < kSupT; ++x) a[x] = As[kk][tr + x * RT];
-#pragma unroll
-            for (int y = 0; y < kSupT; ++y) b[y] = Bs[kk][tc + y * RT];
-#pragma unroll
-            for (int x = 0; x < kSupT; ++x)
-#pragma unroll
-                for (int y = 0; y < kSupT; ++y) acc[x][y] = fma(a[x], b[y], acc[x][y]);
-        }
-        __syncthreads();
+    for (int x = 0; x < kPipeStages - 1; ++x) copy_next();
+    for (int64_t k0 = kb; k0 < kend; k0 += kPipeBk) {
+        cp_async_wait<kPipeStages - 2>();
+        __syncthreads();   /* the step's copies are in, and the stage copied to next is read out */
+        copy_next();
+        PT::multiply(f64_stages + cs * PT::STAGE, (int)(kend - k0 < kPipeBk ? kend - k0 : kPipeBk), acc);
+        cs = cs + 1 == kPipeStages ? 0 : cs + 1;
     }
 #pragma unroll
-    for (int x = 0; x < kSupT; ++x)
+    for (int x = 0; x < TM; ++x)
 #pragma unroll
-        for (int y = 0; y < kSupT; ++y) Ps[(tr + x * RT) + kSupB * (tc + y * RT)] = acc[x][y];
+        for (int y = 0; y < TN; ++y) Ps[(tr + x * PT::RT) + BM * (tc + y * PT::CT)] = acc[x][y];
     cl.sync();   /* every partial tile of the cluster is in place */
-    /* the tile's 1024 elements in groups of 256, group g summed by CTA g % ks */
-    for (int g = rank; g < kSupB * kSupB / kSupThreads; g += ks) {
-        const int e = g * kSupThreads + tid;
+    /* the tile's elements in groups of NT, group g summed by CTA g % ks */
+    for (int g = rank; g < BM * BN / PT::NT; g += ks) {
+        const int e = g * PT::NT + tid;
         double s = *cl.map_shared_rank(Ps + e, 0);
         for (int q = 1; q < ks; ++q) s = s + *cl.map_shared_rank(Ps + e, q);
-        const int64_t gi = i0 + e % kSupB, gj = j0 + e / kSupB;
+        const int64_t gi = i0 + e % BM, gj = j0 + e / BM;
         if (gi < m && gj < n) {
             double* p = C + gi + gj * ldc;
             *p = fma(alpha, s, *p);
@@ -622,15 +798,17 @@ bool plain_classical(const AlgView& alg)
     return u_off[1] == 1 && v_off[1] == 1 && w_off[1] == 1 && u_ent[1] == 1 && v_ent[1] == 1 && w_ent[1] == 1;
 }
 
-int sup_launch(int64_t m, int64_t n, int64_t k, double alpha, const double* A, int64_t lda, const double* B,
-               int64_t ldb, double* C, int64_t ldc, int ks, cudaStream_t st)
+template <int BM, int BN, int TM, int TN, int MINB>
+int sup_launch_t(int64_t m, int64_t n, int64_t k, double alpha, const double* A, int64_t lda, const double* B,
+                 int64_t ldb, double* C, int64_t ldc, int ks, cudaStream_t st)
 {
-    const int64_t tm = (m + kSupB - 1) / kSupB, tn = (n + kSupB - 1) / kSupB;
+    using PT = PipeTile<BM, BN, TM, TN>;
+    const int64_t tm = (m + BM - 1) / BM, tn = (n + BN - 1) / BN;
     const int64_t kc = fmm_f64_sup_chunk(k, ks);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(tm * tn * ks));
-    cfg.blockDim = dim3(kSupThreads);
-    cfg.dynamicSmemBytes = 0;
+    cfg.blockDim = dim3(PT::NT);
+    cfg.dynamicSmemBytes = PT::SMEM;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -639,13 +817,34 @@ int sup_launch(int64_t m, int64_t n, int64_t k, double alpha, const double* A, i
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, fmm_f64_sup_kernel, m, n, k, alpha, A, lda, B, ldb, C, ldc,
-                                             (int)tm, ks, kc);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, fmm_f64_sup_kernel<BM, BN, TM, TN, MINB>, m, n, k, alpha, A, lda, B,
+                                             ldb, C, ldc, (int)tm, ks, kc);
     fmm_count_launch(1);
     return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? FMM_OK : FMM_ERR_CUDA;
 }
 
-template <int BM, int BN, int BK, int TM, int TN>
+/* Tile of the cluster path: 16 x 8 or 8 x 8, whichever loads the busiest SM
+ * less (ks CTAs per tile), the smaller one at the lower measured efficiency.
+ * The bits do not depend on it. Measured (us, 16 x 8 / 8 x 8; 32 x 32 before):
+ * 128 x 128 x 16384 536 / 522 (1047), 250 x 120 x 12000 676 / 753,
+ * 257 x 129 x 2048 146 / 166 (218), 33 x 700 x 3000 197 / 162 (316),
+ * 8 x 320 x 16384 201 / 131. */
+int sup_launch(int64_t m, int64_t n, int64_t k, double alpha, const double* A, int64_t lda, const double* B,
+               int64_t ldb, double* C, int64_t ldc, int ks, cudaStream_t st)
+{
+    int dev = 0, sms = 152;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    auto load = [&](int bm, int bn, double eff) {
+        const int64_t ctas = ((m + bm - 1) / bm) * ((n + bn - 1) / bn) * ks;
+        return (double)((ctas + sms - 1) / sms) * (bm * bn) / eff;
+    };
+    if (load(8, 8, 0.85) < load(16, 8, 0.95))
+        return sup_launch_t<8, 8, 1, 1, 8>(m, n, k, alpha, A, lda, B, ldb, C, ldc, ks, st);
+    return sup_launch_t<16, 8, 1, 1, 6>(m, n, k, alpha, A, lda, B, ldb, C, ldc, ks, st);
+}
+
+template <int BM, int BN, int BK, int TM, int TN, bool MMA>
 int launch_cfg(const AlgView& alg, int64_t m, int64_t n, int64_t k, double alpha,
                const double* A, int64_t lda, const double* B, int64_t ldb, double* C,
                int64_t ldc, int r_begin, int r_end, const double* Sp, const double* Tp, cudaStream_t st)
@@ -653,26 +852,144 @@ int launch_cfg(const AlgView& alg, int64_t m, int64_t n, int64_t k, double alpha
     const int64_t me = (m + alg.mt - 1) / alg.mt, ne = (n + alg.nt - 1) / alg.nt;
     const int64_t tm = (me + BM - 1) / BM, tn = (ne + BN - 1) / BN;
     if (tm * tn > 0x7fffffffLL) return FMM_ERR_UNSUPPORTED;
-    if (g_f64_engine.load(std::memory_order_relaxed) == FMM_F64_MMA)
-        fmm_f64_kernel<BM, BN, BK, TM, TN, true><<<(unsigned)(tm * tn), (BM / TM) * (BN / TN), 0, st>>>(
-            alg.tab, m, n, k, alpha, A, lda, B, ldb, C, ldc, (int)tm, r_begin, r_end, Sp, Tp);
-    else
-        fmm_f64_kernel<BM, BN, BK, TM, TN, false><<<(unsigned)(tm * tn), (BM / TM) * (BN / TN), 0, st>>>(
-            alg.tab, m, n, k, alpha, A, lda, B, ldb, C, ldc, (int)tm, r_begin, r_end, Sp, Tp);
+    fmm_f64_kernel<BM, BN, BK, TM, TN, MMA><<<(unsigned)(tm * tn), (BM / TM) * (BN / TN), 0, st>>>(
+        alg.tab, m, n, k, alpha, A, lda, B, ldb, C, ldc, (int)tm, r_begin, r_end, Sp, Tp);
     fmm_count_launch(1);
     return cudaGetLastError() == cudaSuccess ? FMM_OK : FMM_ERR_CUDA;
 }
 
-int launch_pick(int pick, const AlgView& alg, int64_t m, int64_t n, int64_t k, double alpha, const double* A,
+template <int BM, int BN, int TM, int TN, int MINB>
+int launch_pipe(const AlgView& alg, int64_t m, int64_t n, int64_t k, double alpha, const double* A, int64_t lda,
+                const double* B, int64_t ldb, double* C, int64_t ldc, int r_begin, int r_end, const double* Sp,
+                const double* Tp, cudaStream_t st)
+{
+    using PT = PipeTile<BM, BN, TM, TN>;
+    const int64_t me = (m + alg.mt - 1) / alg.mt, ne = (n + alg.nt - 1) / alg.nt;
+    const int64_t tm = (me + BM - 1) / BM, tn = (ne + BN - 1) / BN;
+    if (tm * tn > 0x7fffffffLL) return FMM_ERR_UNSUPPORTED;
+    if (PT::SMEM > 48 * 1024) {
+        static std::atomic<uint64_t> attr_set{0};   /* a per-device attribute of the kernel: set once per device */
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess) return FMM_ERR_CUDA;
+        const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+        if (bit == 0 || !(attr_set.load(std::memory_order_acquire) & bit)) {
+            if (cudaFuncSetAttribute(fmm_f64_pipe_kernel<BM, BN, TM, TN, MINB>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PT::SMEM) != cudaSuccess)
+                return FMM_ERR_CUDA;
+            attr_set.fetch_or(bit, std::memory_order_acq_rel);
+        }
+    }
+    fmm_f64_pipe_kernel<BM, BN, TM, TN, MINB><<<(unsigned)(tm * tn), PT::NT, PT::SMEM, st>>>(
+        alg.tab, m, n, k, alpha, A, lda, B, ldb, C, ldc, (int)tm, r_begin, r_end, Sp, Tp);
+    fmm_count_launch(1);
+    return cudaGetLastError() == cudaSuccess ? FMM_OK : FMM_ERR_CUDA;
+}
+
+/* the kernels a call runs its tiles on */
+enum F64Pick {
+    kPipe64, kPipe16x8, kPipe8,                       /* pipelined DFMA tiles, single-term operands */
+    kFused64, kFused32,                               /* DFMA with the packs fused in */
+    kMma64, kMma128x64, kMma64x128, kMma32            /* FP64 MMA engine */
+};
+
+int launch_pick(F64Pick pick, const AlgView& alg, int64_t m, int64_t n, int64_t k, double alpha, const double* A,
                 int64_t lda, const double* B, int64_t ldb, double* C, int64_t ldc, int r_begin, int r_end,
                 const double* Sp, const double* Tp, cudaStream_t st)
 {
+    auto go = [&](auto f) { return f(alg, m, n, k, alpha, A, lda, B, ldb, C, ldc, r_begin, r_end, Sp, Tp, st); };
     switch (pick) {
-    case 3: return launch_cfg<64, 64, 32, 4, 4>(alg, m, n, k, alpha, A, lda, B, ldb, C, ldc, r_begin, r_end, Sp, Tp, st);
-    case 4: return launch_cfg<128, 64, 16, 8, 4>(alg, m, n, k, alpha, A, lda, B, ldb, C, ldc, r_begin, r_end, Sp, Tp, st);
-    case 5: return launch_cfg<64, 128, 16, 4, 8>(alg, m, n, k, alpha, A, lda, B, ldb, C, ldc, r_begin, r_end, Sp, Tp, st);
-    default: return launch_cfg<32, 32, 32, 2, 2>(alg, m, n, k, alpha, A, lda, B, ldb, C, ldc, r_begin, r_end, Sp, Tp, st);
+    case kPipe64: return go(launch_pipe<64, 64, 4, 4, 2>);
+    case kPipe16x8: return go(launch_pipe<16, 8, 1, 1, 6>);
+    case kPipe8: return go(launch_pipe<8, 8, 1, 1, 8>);
+    case kFused64: return go(launch_cfg<64, 64, 32, 4, 4, false>);
+    case kFused32: return go(launch_cfg<32, 32, 32, 2, 2, false>);
+    case kMma64: return go(launch_cfg<64, 64, 32, 4, 4, true>);
+    case kMma128x64: return go(launch_cfg<128, 64, 16, 8, 4, true>);
+    case kMma64x128: return go(launch_cfg<64, 128, 16, 4, 8, true>);
+    default: return go(launch_cfg<32, 32, 32, 2, 2, true>);
     }
+}
+
+/* the cheapest of a list of tiles, by the most loaded SM's FP64 work */
+struct F64Cand {
+    F64Pick pick;
+    int bm, bn;
+    double eff;   /* measured share of the FP64 pipe's rate when the SMs' shares are equal */
+};
+
+/* Pipelined tiles: an SM's CTAs share its FP64 pipe and a finished CTA's place
+ * is taken at once, so the SM with the most tiles sets the time. Measured
+ * (us, tiles 64 x 64 / 16 x 8 / 8 x 8; the kernel before: 64 or 32 wide):
+ * classical 4096^3 110038 / 110443 / 109979, classical 1000 x 1200 x 900
+ * 1811 / 1787 / 1779 (1876), 222 x1 2048^3 14502 / 12360 / 12578 (12895),
+ * 333 x1 4097 x 3001 x 3500 81199 / 61521 / 61097 (69717), classical 512^3
+ * 525 / 234 / 247 (265), 222 x1 400^3 - / 159 / 137 (463). */
+constexpr F64Cand kPipeCands[] = {{kPipe64, 64, 64, 0.985}, {kPipe16x8, 16, 8, 0.97}, {kPipe8, 8, 8, 0.85}};
+
+F64Pick pick_pipe(int64_t me, int64_t ne, int sms)
+{
+    F64Pick best = kPipe64;
+    double least = 0.0;
+    for (const F64Cand& c : kPipeCands) {
+        const int64_t tiles = ((me + c.bm - 1) / c.bm) * ((ne + c.bn - 1) / c.bn);
+        const double est = (double)((tiles + sms - 1) / sms) * (c.bm * c.bn) / c.eff;
+        if (least == 0.0 || est < least) { least = est; best = c.pick; }
+    }
+    return best;
+}
+
+/* Tiles with the packs fused in (and the MMA engine's): waves of two CTAs per
+ * SM, times the FMAs per tile including the pack additions (nu, nv terms per
+ * operand), over the tile's efficiency. */
+F64Pick pick_fused(bool mma, int64_t me, int64_t ne, double nu, double nv, int sms)
+{
+    static constexpr F64Cand dfma[] = {{kFused64, 64, 64, 1.0}, {kFused32, 32, 32, 0.8}};
+    static constexpr F64Cand mmac[] = {{kMma64, 64, 64, 1.0}, {kMma128x64, 128, 64, 0.99}, {kMma64x128, 64, 128, 0.99},
+                                       {kMma32, 32, 32, 0.8}};
+    F64Pick best = kFused64;
+    double least = 0.0;
+    for (int x = 0; x < (mma ? 4 : 2); ++x) {
+        const F64Cand& c = mma ? mmac[x] : dfma[x];
+        const int64_t tiles = ((me + c.bm - 1) / c.bm) * ((ne + c.bn - 1) / c.bn);
+        const double waves = (double)((tiles + 2 * (int64_t)sms - 1) / (2 * (int64_t)sms));
+        const double work = (double)(c.bm * c.bn) *
+                            (1.0 + (nu - 1.0) / c.bn + (nv - 1.0) / c.bm + 4.0 / c.bm);
+        if (least == 0.0 || waves * work / c.eff < least) { least = waves * work / c.eff; best = c.pick; }
+    }
+    return best;
+}
+
+/* Stream-ordered temporaries (pre-formed operands) from the library's own
+ * memory pool of the device, which keeps up to 256 MiB between calls: the
+ * device's default pool gives everything back at each synchronization, and
+ * getting it again cost a synchronous caller about 200 us per call. Given back
+ * by fmm_gpu_release_host_buffers. */
+constexpr uint64_t kTempPoolKeep = (uint64_t)256 << 20;
+std::mutex g_pool_mu;
+cudaMemPool_t g_pools[64];
+
+cudaMemPool_t temp_pool()
+{
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    if (g_pools[dev] == nullptr) {
+        cudaMemPoolProps props;
+        memset(&props, 0, sizeof(props));
+        props.allocType = cudaMemAllocationTypePinned;
+        props.handleTypes = cudaMemHandleTypeNone;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t p = nullptr;
+        uint64_t keep = kTempPoolKeep;
+        if (cudaMemPoolCreate(&p, &props) != cudaSuccess) return nullptr;
+        if (cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+            cudaMemPoolDestroy(p);
+            return nullptr;
+        }
+        g_pools[dev] = p;
+    }
+    return g_pools[dev];
 }
 
 /* bytes of pre-formed operands a product group may hold at once */
@@ -690,14 +1007,14 @@ int fmm_scale_c(int64_t m, int64_t n, double beta, double* C, int64_t ldc, cudaS
     return cudaGetLastError() == cudaSuccess ? FMM_OK : FMM_ERR_CUDA;
 }
 
-/* Tile choice: the FP64 pipe is the bottleneck, so estimate each SM's FP64
- * work for every candidate (waves of CTAs over the SMs, two resident per SM,
- * times the FMAs per tile including the fused pack additions, over the
- * configuration's measured efficiency) and take the cheapest. Measured on
- * GB300 at m=n=k=16384: the 64-wide tiles with two CTAs per SM run classical
- * FP64 at 99% of the DFMA peak, the 128 x 128 tile with one CTA per SM
- * (248 registers) about 2% and FMM forms 5-14% slower, so it is not a
- * candidate; 32 x 32 serves grids too small to fill the SMs. */
+void fmm_f64_release_temp()
+{
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    if (g_pools[dev]) cudaMemPoolTrimTo(g_pools[dev], 0);
+}
+
 int fmm_f64_launch(const AlgView& alg, int64_t m, int64_t n, int64_t k, double alpha,
                    const double* A, int64_t lda, const double* B, int64_t ldb,
                    double beta, double* C, int64_t ldc, cudaStream_t st)
@@ -707,10 +1024,12 @@ int fmm_f64_launch(const AlgView& alg, int64_t m, int64_t n, int64_t k, double a
     if (m == 0 || n == 0 || k == 0 || alpha == 0.0) return FMM_OK;
     if (alg.max_nnz_u > kMaxEntries || alg.max_nnz_v > kMaxEntries) return FMM_ERR_UNSUPPORTED;
 
-    if (plain_classical(alg)) {
+    const bool classical = plain_classical(alg);
+    if (classical) {
         const int ks = fmm_gpu_f64_sup_splits(m, n, k);
         if (ks >= 2) return sup_launch(m, n, k, alpha, A, lda, B, ldb, C, ldc, ks, st);
     }
+    const bool mma = g_f64_engine.load(std::memory_order_relaxed) == FMM_F64_MMA;
     int dev = 0, sms = 152;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -719,26 +1038,13 @@ int fmm_f64_launch(const AlgView& alg, int64_t m, int64_t n, int64_t k, double a
      * the tiles (a stream-ordered temporary of at most kPrepackBudget per
      * product group), instead of once per tile position inside the kernel;
      * the values, and so the results, are the same either way. */
-    const bool prepack = alg.R > 1;
-    const double nu = prepack ? 1.0 : alg.avg_nnz_u, nv = prepack ? 1.0 : alg.avg_nnz_v;
-    struct Cand { int id, bm, bn; double eff; };
-    const Cand cands[4] = {{3, 64, 64, 1.0}, {4, 128, 64, 0.99}, {5, 64, 128, 0.99}, {2, 32, 32, 0.8}};
-    double best = 0;
-    int pick = 3;
-    for (int c = 0; c < 4; ++c) {
-        const int64_t bm = cands[c].bm, bn = cands[c].bn;
-        const int64_t tiles = ((me + bm - 1) / bm) * ((ne + bn - 1) / bn);
-        const double waves = (double)((tiles + 2 * (int64_t)sms - 1) / (2 * (int64_t)sms));
-        const double work = (double)(bm * bn) * (1.0 + (nu - 1.0) / (double)bn + (nv - 1.0) / (double)bm +
-                                                 4.0 / (double)bm);
-        const double est = waves * work / cands[c].eff;
-        if (c == 0 || est < best) { best = est; pick = cands[c].id; }
-    }
-    if (prepack) {
+    if (alg.R > 1) {
+        const F64Pick pick = mma ? pick_fused(true, me, ne, 1.0, 1.0, sms) : pick_pipe(me, ne, sms);
         const size_t per = (size_t)(me * ke + ke * ne) * sizeof(double);
         const int G = (int)std::max<size_t>(1, std::min<size_t>((size_t)alg.R, kPrepackBudget / std::max<size_t>(per, 1)));
         void* buf = nullptr;
-        if (cudaMallocAsync(&buf, (size_t)G * per, st) == cudaSuccess) {
+        const cudaMemPool_t pool = temp_pool();
+        if (pool != nullptr && cudaMallocFromPoolAsync(&buf, (size_t)G * per, pool, st) == cudaSuccess) {
             double* Sbuf = (double*)buf;
             double* Tbuf = Sbuf + (size_t)G * me * ke;
             for (int r0 = 0; r0 < alg.R && rc == FMM_OK; r0 += G) {
@@ -755,6 +1061,8 @@ int fmm_f64_launch(const AlgView& alg, int64_t m, int64_t n, int64_t k, double a
         }
         cudaGetLastError();   /* no temporary: the combinations stay fused into the kernel */
     }
+    const F64Pick pick = classical && !mma ? pick_pipe(me, ne, sms)
+                                           : pick_fused(mma, me, ne, alg.avg_nnz_u, alg.avg_nnz_v, sms);
     return launch_pick(pick, alg, m, n, k, alpha, A, lda, B, ldb, C, ldc, 0, alg.R, nullptr, nullptr, st);
 }
 
@@ -801,9 +1109,38 @@ int fmm_f64_batch_launch(int count, const F64BatchItem* items, void* ws, size_t 
                 continue;
             }
         }
-        const int64_t ke = (it.k + it.alg.kt - 1) / it.alg.kt;
-        cost[i] = (it.k == 0 || it.alpha == 0.0) ? 1.0 : (double)it.alg.R * (double)(ke + 1);
         order.push_back(i);
+    }
+    int dev = 0, sms = 152;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const bool mma = g_f64_engine.load(std::memory_order_relaxed) == FMM_F64_MMA;
+    /* Item tiles: 64 x 64 costs the fewest pack additions, but one item of a
+     * deep problem can last as long as the whole batch (1024^3 222 x1: 14.7 M
+     * FMAs, 7 ms on half an SM). A problem's tile shrinks to 32, then 16,
+     * while its items hold more than an eighth of a CTA's share of the
+     * batch. 24 problems of 256 to 1024: 7.1 ms with 64 x 64 alone. */
+    int64_t ctas = 2 * (int64_t)sms;
+    const int cap = g_f64_batch_ctas.load();
+    if (cap > 0) ctas = std::min<int64_t>(ctas, cap);
+    auto item_fmas = [&](int i, int tile) {
+        const F64BatchItem& it = items[i];
+        if (it.k == 0 || it.alpha == 0.0) return 1.0;
+        return (double)tile * tile * it.alg.R * (double)((it.k + it.alg.kt - 1) / it.alg.kt + 1);
+    };
+    auto tiles_of = [&](int i, int tile, int64_t* tm) {
+        const F64BatchItem& it = items[i];
+        const int64_t me = (it.m + it.alg.mt - 1) / it.alg.mt, ne = (it.n + it.alg.nt - 1) / it.alg.nt;
+        *tm = (me + tile - 1) / tile;
+        return *tm * ((ne + tile - 1) / tile);
+    };
+    double total = 0.0;
+    int64_t tm = 0;
+    for (int i : order) total += item_fmas(i, 32) * (double)tiles_of(i, 32, &tm);
+    std::vector<int> tile(count, 64);
+    for (int i : order) {
+        while (tile[i] > (mma ? 32 : 16) && item_fmas(i, tile[i]) > total / (double)ctas / 8) tile[i] /= 2;
+        cost[i] = item_fmas(i, tile[i]);
     }
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
     std::vector<F64Prob> tab(order.size());
@@ -815,12 +1152,12 @@ int fmm_f64_batch_launch(int count, const F64BatchItem* items, void* ws, size_t 
         P.m = it.m; P.n = it.n; P.k = it.k;
         P.alpha = it.alpha; P.beta = it.beta;
         P.A = it.A; P.lda = it.lda; P.B = it.B; P.ldb = it.ldb; P.C = it.C; P.ldc = it.ldc;
-        const int64_t me = (it.m + it.alg.mt - 1) / it.alg.mt, ne = (it.n + it.alg.nt - 1) / it.alg.nt;
-        const int64_t tm = (me + kF64Bm - 1) / kF64Bm, tn = (ne + kF64Bn - 1) / kF64Bn;
-        if (tm > 0x7fffffffLL || tn > 0x7fffffffLL) return FMM_ERR_UNSUPPORTED;
-        P.tiles_m = (int)tm; P.tiles_n = (int)tn;
+        P.tile = tile[order[q]];
+        const int64_t tiles = tiles_of(order[q], P.tile, &tm);
+        if (tm > 0x7fffffffLL || tiles / tm > 0x7fffffffLL) return FMM_ERR_UNSUPPORTED;
+        P.tiles_m = (int)tm;
         P.item_begin = items_total;
-        items_total += tm * tn;
+        items_total += tiles;
     }
     if (tab.empty()) return FMM_OK;
     unsigned long long* counter = (unsigned long long*)ws;
@@ -834,18 +1171,11 @@ int fmm_f64_batch_launch(int count, const F64BatchItem* items, void* ws, size_t 
         f64_table_write<<<1, 128, 0, st>>>(ch);
         fmm_count_launch(1);
     }
-    int dev = 0, sms = 152;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int64_t grid = std::min<int64_t>(items_total, 2 * (int64_t)sms);
-    const int cap = g_f64_batch_ctas.load();
-    if (cap > 0) grid = std::min<int64_t>(grid, cap);   /* items are drawn from a counter: any grid finishes them */
-    if (g_f64_engine.load(std::memory_order_relaxed) == FMM_F64_MMA)
-        fmm_f64_batch_kernel<true><<<(unsigned)grid, (kF64Bm / kF64Tm) * (kF64Bn / kF64Tn), 0, st>>>(
-            dtab, (int)tab.size(), items_total, counter);
+    const int64_t grid = std::min<int64_t>(items_total, ctas);   /* items are drawn from a counter: any grid finishes them */
+    if (mma)
+        fmm_f64_batch_kernel<true><<<(unsigned)grid, kF64BatchThreads, 0, st>>>(dtab, (int)tab.size(), items_total, counter);
     else
-        fmm_f64_batch_kernel<false><<<(unsigned)grid, (kF64Bm / kF64Tm) * (kF64Bn / kF64Tn), 0, st>>>(
-            dtab, (int)tab.size(), items_total, counter);
+        fmm_f64_batch_kernel<false><<<(unsigned)grid, kF64BatchThreads, 0, st>>>(dtab, (int)tab.size(), items_total, counter);
     fmm_count_launch(1);
     return cudaGetLastError() == cudaSuccess ? FMM_OK : FMM_ERR_CUDA;
 }

@@ -70,6 +70,9 @@ int fmm_f64_launch(const AlgView& alg, int64_t m, int64_t n, int64_t k,
                    const double* B, int64_t ldb, double beta, double* C, int64_t ldc,
                    cudaStream_t st);
 
+/* gives the current device's kept temporary memory back (fmm_f64.cu) */
+void fmm_f64_release_temp();
+
 /* batched FP64 form (fmm_f64.cu): one persistent launch over every
  * (problem, tile position) item */
 struct F64BatchItem {

@@ -249,7 +249,8 @@ int fmm_gpu_split_strassen_ab_gen(double alpha, const double* A, int64_t rs_a, i
                                   int64_t m, int64_t n, int64_t k,
                                   fmm_t fmm, int levels, int slices, int format);
 
-/* Frees the current device's buffers kept by fmm_gpu_split_strassen_ab_ex. */
+/* Frees the current device's buffers kept by fmm_gpu_split_strassen_ab_ex and
+ * the temporary memory kept by the plain FP64 form (at most 256 MiB). */
 void fmm_gpu_release_host_buffers(void);
 
 /* Pinned host memory for the operands of the host-buffer entry points:
