@@ -478,7 +478,7 @@ extern "C" size_t fmm_gpu_split_workspace_size_fmt(const fmm_t* fmm, int levels,
     fmm_t flat;
     int owned = 0;
     if (fmm_flatten(fmm, levels, &flat, &owned) != FMM_OK) return 0;
-    AlgView v;
+    AlgView v = {};
     v.mt = flat.m_tilde; v.kt = flat.k_tilde; v.nt = flat.n_tilde; v.R = flat.R;
     size_t b = fmm_split_ws_bytes(v, m, n, k, slices, format);
     if (owned) free_fmm(flat);

@@ -24,6 +24,7 @@
  *    (product, sub-block) instead of one per KC block.
  */
 #include "fmm_internal.h"
+#include "sm103_ptx.cuh"
 
 #include <cooperative_groups.h>
 
@@ -54,6 +55,21 @@ extern "C" int fmm_gpu_f64_sup_splits(int64_t m, int64_t n, int64_t k)
 int64_t fmm_f64_sup_chunk(int64_t k, int ks)
 {
     return ((k + ks - 1) / ks + 31) / 32 * 32;
+}
+
+/* the trivial 1 x 1 x 1 algorithm with all three coefficients +1: the
+ * classical GEMM C += alpha * A * B */
+bool fmm_plain_classical(const AlgView& alg)
+{
+    if (alg.R != 1 || alg.mt != 1 || alg.kt != 1 || alg.nt != 1 || alg.htab == nullptr) return false;
+    const int* t = alg.htab;
+    const int* u_off = t + FMM_ALG_HDR;
+    const int* v_off = u_off + 2;
+    const int* w_off = v_off + 2;
+    const int* u_ent = w_off + 2;
+    const int* v_ent = u_ent + 2 * u_off[1];
+    const int* w_ent = v_ent + 2 * v_off[1];
+    return u_off[1] == 1 && v_off[1] == 1 && w_off[1] == 1 && u_ent[1] == 1 && v_ent[1] == 1 && w_ent[1] == 1;
 }
 
 namespace {
@@ -372,15 +388,9 @@ fmm_f64_kernel(const int* __restrict__ tab, int64_t m, int64_t n, int64_t k,
 
 /* ------------------------------------- pipelined single-term tiles ---- */
 
-/* 8-byte global -> shared copy, zero when !ok (nothing is read then) */
-__device__ __forceinline__ void cp_async8(double* dst, const double* src, bool ok)
-{
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(ok ? 8 : 0) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+using sm103::cp_async8;
+using sm103::cp_async_commit;
+using sm103::cp_async_wait;
 
 /* Tile geometry of the pipelined kernels: BM x BN outputs per CTA, TM x TN per
  * thread, k steps of kPipeBk in a ring of kPipeStages shared-memory stages
@@ -783,21 +793,6 @@ fmm_f64_sup_kernel(int64_t m, int64_t n, int64_t k, double alpha, const double* 
     cl.sync();   /* no CTA leaves while another still reads its partial */
 }
 
-/* the trivial 1 x 1 x 1 algorithm with all three coefficients +1: the
- * classical GEMM C += alpha * A * B */
-bool plain_classical(const AlgView& alg)
-{
-    if (alg.R != 1 || alg.mt != 1 || alg.kt != 1 || alg.nt != 1 || alg.htab == nullptr) return false;
-    const int* t = alg.htab;
-    const int* u_off = t + FMM_ALG_HDR;
-    const int* v_off = u_off + 2;
-    const int* w_off = v_off + 2;
-    const int* u_ent = w_off + 2;
-    const int* v_ent = u_ent + 2 * u_off[1];
-    const int* w_ent = v_ent + 2 * v_off[1];
-    return u_off[1] == 1 && v_off[1] == 1 && w_off[1] == 1 && u_ent[1] == 1 && v_ent[1] == 1 && w_ent[1] == 1;
-}
-
 template <int BM, int BN, int TM, int TN, int MINB>
 int sup_launch_t(int64_t m, int64_t n, int64_t k, double alpha, const double* A, int64_t lda, const double* B,
                  int64_t ldb, double* C, int64_t ldc, int ks, cudaStream_t st)
@@ -959,7 +954,7 @@ F64Pick pick_fused(bool mma, int64_t me, int64_t ne, double nu, double nv, int s
     return best;
 }
 
-/* Stream-ordered temporaries (pre-formed operands) from the library's own
+/* Stream-ordered temporaries (pre-formed operands, work units' planes) from the library's own
  * memory pool of the device, which keeps up to 256 MiB between calls: the
  * device's default pool gives everything back at each synchronization, and
  * getting it again cost a synchronous caller about 200 us per call. Given back
@@ -968,7 +963,9 @@ constexpr uint64_t kTempPoolKeep = (uint64_t)256 << 20;
 std::mutex g_pool_mu;
 cudaMemPool_t g_pools[64];
 
-cudaMemPool_t temp_pool()
+}  // namespace
+
+cudaMemPool_t fmm_temp_pool()
 {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
@@ -991,6 +988,8 @@ cudaMemPool_t temp_pool()
     }
     return g_pools[dev];
 }
+
+namespace {
 
 /* bytes of pre-formed operands a product group may hold at once */
 constexpr size_t kPrepackBudget = (size_t)4 << 30;
@@ -1024,7 +1023,7 @@ int fmm_f64_launch(const AlgView& alg, int64_t m, int64_t n, int64_t k, double a
     if (m == 0 || n == 0 || k == 0 || alpha == 0.0) return FMM_OK;
     if (alg.max_nnz_u > kMaxEntries || alg.max_nnz_v > kMaxEntries) return FMM_ERR_UNSUPPORTED;
 
-    const bool classical = plain_classical(alg);
+    const bool classical = fmm_plain_classical(alg);
     if (classical) {
         const int ks = fmm_gpu_f64_sup_splits(m, n, k);
         if (ks >= 2) return sup_launch(m, n, k, alpha, A, lda, B, ldb, C, ldc, ks, st);
@@ -1043,7 +1042,7 @@ int fmm_f64_launch(const AlgView& alg, int64_t m, int64_t n, int64_t k, double a
         const size_t per = (size_t)(me * ke + ke * ne) * sizeof(double);
         const int G = (int)std::max<size_t>(1, std::min<size_t>((size_t)alg.R, kPrepackBudget / std::max<size_t>(per, 1)));
         void* buf = nullptr;
-        const cudaMemPool_t pool = temp_pool();
+        const cudaMemPool_t pool = fmm_temp_pool();
         if (pool != nullptr && cudaMallocFromPoolAsync(&buf, (size_t)G * per, pool, st) == cudaSuccess) {
             double* Sbuf = (double*)buf;
             double* Tbuf = Sbuf + (size_t)G * me * ke;
@@ -1097,7 +1096,7 @@ int fmm_f64_batch_launch(int count, const F64BatchItem* items, void* ws, size_t 
         const F64BatchItem& it = items[i];
         if (it.alg.max_nnz_u > kMaxEntries || it.alg.max_nnz_v > kMaxEntries) return FMM_ERR_UNSUPPORTED;
         if (it.m == 0 || it.n == 0) continue;   /* nothing to do at all */
-        if (it.k > 0 && it.alpha != 0.0 && plain_classical(it.alg)) {
+        if (it.k > 0 && it.alpha != 0.0 && fmm_plain_classical(it.alg)) {
             /* small/skinny classical problems take the same kernel as their
              * single calls (C := beta*C first, as there) */
             const int ks = fmm_gpu_f64_sup_splits(it.m, it.n, it.k);

@@ -55,6 +55,9 @@ __host__ __device__ __forceinline__ void fmm_part_geom32(int d, int t, int i, in
     *len = base + (i < rem ? 1 : 0);
 }
 
+/* the trivial 1 x 1 x 1 algorithm with coefficients +1: C += alpha * A * B (fmm_f64.cu) */
+bool fmm_plain_classical(const AlgView& alg);
+
 /* Host helpers implemented in fmm_api.cu */
 int fmm_flatten(const fmm_t* fmm, int levels, fmm_t* flat, int* owned);
 int fmm_alg_get(const fmm_t* flat, AlgView* out);  /* upload/cache */
@@ -70,6 +73,9 @@ int fmm_f64_launch(const AlgView& alg, int64_t m, int64_t n, int64_t k,
                    const double* B, int64_t ldb, double beta, double* C, int64_t ldc,
                    cudaStream_t st);
 
+/* the library's memory pool of the current device for stream-ordered
+ * temporaries (null: none); keeps a bounded amount between calls */
+cudaMemPool_t fmm_temp_pool();
 /* gives the current device's kept temporary memory back (fmm_f64.cu) */
 void fmm_f64_release_temp();
 

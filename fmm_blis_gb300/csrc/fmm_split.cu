@@ -70,6 +70,7 @@
 #include "sm103_ptx.cuh"
 
 #include <cuda.h>
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
 
@@ -79,6 +80,7 @@
 #include <cstring>
 #include <deque>
 #include <mutex>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -143,18 +145,21 @@ __host__ __device__ constexpr uint64_t digit_offset()
 template <int S, int DB>
 __device__ __forceinline__ Digits split_offset(double x, int E)
 {
-    const uint64_t bits = (uint64_t)__double_as_longlong(x);
-    const bool neg = (bits >> 63) != 0;
-    const int bexp = (int)((bits >> 52) & 0x7ff);
-    uint64_t mant = bits & 0x000fffffffffffffull;
-    int ex;
-    if (bexp == 0) ex = -1074; else { mant |= 0x0010000000000000ull; ex = bexp - 1075; }
+    const uint32_t hi = (uint32_t)__double2hiint(x);
+    const int bexp = (int)(hi >> 20) & 0x7ff;
+    /* |x| = mant * 2^ex; a subnormal has exponent field 1 without the implicit bit */
+    const int ex = (bexp > 1 ? bexp : 1) - 1075;
+    const uint64_t mant = ((uint64_t)((hi & 0x000fffffu) | (bexp ? 0x00100000u : 0u)) << 32) | (uint32_t)__double2loint(x);
+    /* round(mant * 2^sh), ties away: ((mant >> (r - 1)) + 1) >> 1 with r = -sh.
+     * PTX shifts by 64 and more give 0, as the rounding does there. For a
+     * normal |x| < 2^E sh is at most DB*S - 54: left shifts are rare. */
     const int sh = ex + DB * S - E - 1;
-    int64_t X;
-    if (mant == 0 || sh < -62) X = 0;
-    else if (sh >= 0) X = (int64_t)(mant << sh);
-    else X = (int64_t)((mant + (1ull << (-sh - 1))) >> (-sh));
-    if (neg) X = -X;
+    uint64_t t;
+    asm("shr.u64 %0, %1, %2;" : "=l"(t) : "l"(mant), "r"((uint32_t)(-sh - 1)));
+    uint64_t u = (t + 1) >> 1;
+    if (sh >= 0) u = mant << sh;
+    const int64_t neg = (int64_t)(int32_t)hi >> 31;   /* 0 or -1 */
+    const int64_t X = ((int64_t)u ^ neg) - neg;
     return Digits{X, (uint64_t)X + digit_offset<S, DB>()};
 }
 
@@ -222,6 +227,28 @@ __device__ __forceinline__ void store_digits8(uint8_t* __restrict__ base, int64_
             for (int x = 0; x < 4; ++x)
                 h[x] = pack_e4m3x2_exact(digit_f<S, DB>(Y[2 * x], tt), digit_f<S, DB>(Y[2 * x + 1], tt));
             *(uint2*)(base + e) = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
+        }
+    }
+}
+
+/* store_digits8 for 4 consecutive k elements (8 or 4 bytes per slice) */
+template <int S, int DB>
+__device__ __forceinline__ void store_digits4(uint8_t* __restrict__ base, int64_t off, int64_t slice_stride,
+                                              const Digits (&Y)[4])
+{
+#pragma unroll
+    for (int tt = 0; tt < S; ++tt) {
+        const int64_t e = off + (int64_t)tt * slice_stride;
+        if (DB == 8) {
+            uint32_t w[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                w[h] = pack_bf16x2_exact(digit_f<S, DB>(Y[2 * h], tt), digit_f<S, DB>(Y[2 * h + 1], tt));
+            *(uint2*)(base + 2 * e) = make_uint2(w[0], w[1]);
+        } else {
+            const uint32_t lo = pack_e4m3x2_exact(digit_f<S, DB>(Y[0], tt), digit_f<S, DB>(Y[1], tt));
+            const uint32_t hi = pack_e4m3x2_exact(digit_f<S, DB>(Y[2], tt), digit_f<S, DB>(Y[3], tt));
+            *(uint32_t*)(base + e) = lo | (hi << 16);
         }
     }
 }
@@ -619,6 +646,38 @@ pack_b_kernel(const int* __restrict__ tab, int r0, int np, const double* __restr
     pack_b_body<S, DB, COLS>(tab, r0, np, B, ldb, k, n, n_pad, k_pad, f_col, sb, j_first, blockIdx.x, blockIdx.y);
 }
 
+/* a call of f(integral_constant S, integral_constant DB) for a slice count and format */
+template <class F>
+auto with_slices(int fmt, int s, F f)
+{
+#define FMM_CASE(S_, DB_) return f(std::integral_constant<int, S_>(), std::integral_constant<int, DB_>())
+    if (fmt == 0) {
+        switch (s) {
+        case 2: FMM_CASE(2, 8);
+        case 3: FMM_CASE(3, 8);
+        case 4: FMM_CASE(4, 8);
+        case 5: FMM_CASE(5, 8);
+        case 6: FMM_CASE(6, 8);
+        case 7: FMM_CASE(7, 8);
+        default: FMM_CASE(8, 8);
+        }
+    }
+    switch (s) {
+    case 2: FMM_CASE(2, 5);
+    case 3: FMM_CASE(3, 5);
+    case 4: FMM_CASE(4, 5);
+    case 5: FMM_CASE(5, 5);
+    case 6: FMM_CASE(6, 5);
+    case 7: FMM_CASE(7, 5);
+    case 8: FMM_CASE(8, 5);
+    case 9: FMM_CASE(9, 5);
+    case 10: FMM_CASE(10, 5);
+    case 11: FMM_CASE(11, 5);
+    default: FMM_CASE(12, 5);
+    }
+#undef FMM_CASE
+}
+
 /* Which packs a launch_packs call issues: both sides, or one side only; the
  * A side over the S_r rows [ia0, ia1) (multiples of 64, or ia1 = m_pad), the
  * B side over the T_r columns [jb0, jb1) (multiples of 32, or jb1 = n_pad). */
@@ -659,35 +718,167 @@ void launch_packs(int fmt, int s, const int* tab, int r, int np, const double* A
                   int64_t k_pad, const int* e_row, const int* f_col, uint8_t* sa, uint8_t* sb,
                   cudaStream_t st, cudaStream_t st_b, const PackSel& sel = PackSel())
 {
-#define FMM_PACKS(S_, DB_) \
-    launch_packs_t<S_, DB_>(tab, r, np, A, lda, B, ldb, m, n, k, m_pad, n_pad, k_pad, e_row, f_col, sa, sb, st, \
-                            st_b, sel)
-    if (fmt == 0) {
-        switch (s) {
-        case 2: FMM_PACKS(2, 8); break;
-        case 3: FMM_PACKS(3, 8); break;
-        case 4: FMM_PACKS(4, 8); break;
-        case 5: FMM_PACKS(5, 8); break;
-        case 6: FMM_PACKS(6, 8); break;
-        case 7: FMM_PACKS(7, 8); break;
-        default: FMM_PACKS(8, 8); break;
+    with_slices(fmt, s, [&](auto S, auto DB) {
+        launch_packs_t<S(), DB()>(tab, r, np, A, lda, B, ldb, m, n, k, m_pad, n_pad, k_pad, e_row, f_col, sa, sb, st,
+                                  st_b, sel);
+    });
+}
+
+/* ------------------------------- classical: maxima, exponents, digits ---- */
+
+/* The classical GEMM's whole operand side in one launch: a cluster of CTAs
+ * owns 16 rows of A (or 16 columns of B), each CTA a k chunk. Every CTA takes
+ * its chunk's maxima, the cluster combines them through distributed shared
+ * memory, and the CTA reads its chunk again (from L2 mostly) and splits the
+ * digits. The same exponents and digits as the general path's maxima,
+ * exponents and packs (one term of coefficient 1), which takes seven launches.
+ * Bound by latency (loads in flight) and instruction issue: 8192 x 8192 of both
+ * operands, 6 slices, 575 us (4.7 TB/s of the 2.7 GB it cannot do without);
+ * 690 us with 64-bit maxima and general shifts, 680 us through cp.async tiles. */
+constexpr int kPrepLines = 16, kPrepK = 128, kPrepThreads = 256;
+constexpr int kPrepPitch = kPrepK + kPrepK / 16 + 1;   /* one pad per 16 k, odd row pitch: no bank conflicts either way */
+
+struct PrepShared {
+    double tile[2][kPrepLines * kPrepPitch];
+    uint2 part[kPrepThreads / kPrepLines][kPrepLines];   /* (OR of low words, maximum of high words) */
+    uint2 mx[kPrepLines];                                /* this CTA's, read by the cluster */
+};
+
+/* lines [l0, l0 + 16) of A (rows) or B (columns), k chunk `rank` of `nrank` */
+template <int S, int DB, bool A_SIDE>
+__device__ __forceinline__ void prep_body(PrepShared& sh, const double* __restrict__ X, int64_t ld, int64_t lines,
+                                          int64_t k, int64_t l_pad, int64_t k_pad, int* __restrict__ ex,
+                                          uint8_t* __restrict__ out, int64_t l0, int rank, int nrank)
+{
+    namespace cgr = cooperative_groups;
+    const int tid = threadIdx.x;
+    const int64_t chunk = ((k_pad + nrank - 1) / nrank + kPrepK - 1) / kPrepK * kPrepK;
+    const int64_t p0 = rank * chunk, p1 = p0 + chunk < k_pad ? p0 + chunk : k_pad;
+    const int64_t pe = p1 < k ? p1 : k;   /* the chunk's k with data */
+    const int tiles = p1 > p0 ? (int)((p1 - p0 + kPrepK - 1) / kPrepK) : 0;
+    /* a thread's eight elements of a 16 x 128 tile, lanes along the operand's
+     * contiguous direction: A one line, every 16th k; B one k, every 2nd line */
+    const int line = A_SIDE ? tid % kPrepLines : tid / kPrepK;
+    const int kq = A_SIDE ? tid / kPrepLines : tid % kPrepK;
+    const int lines_left = (int)(lines - l0 < kPrepLines ? lines - l0 : kPrepLines) - line;
+    const double* x0 = A_SIDE ? X + (l0 + line) + (p0 + kq) * ld : X + (p0 + kq) + (l0 + line) * ld;
+    const int64_t ystep = (A_SIDE ? 16 : 2) * ld, tstep = A_SIDE ? kPrepK * ld : kPrepK;
+    const int k_left = pe > p0 ? (int)(pe - p0) - kq : -kq;   /* this thread's k from the chunk's start */
+    auto load = [&](int t, double (&v)[8]) {                  /* tile t of the chunk */
+        const double* q = x0 + t * tstep;
+        const int kl = k_left - t * kPrepK;
+        const int lim = A_SIDE ? (lines_left > 0 ? kl : 0) : (kl > 0 ? lines_left : 0);
+#pragma unroll
+        for (int y = 0; y < 8; ++y) v[y] = (A_SIDE ? 16 : 2) * y < lim ? __ldg(q + y * ystep) : 0.0;
+    };
+    /* What the exponent needs of a line's largest |x|: its high word, and where
+     * that is 0 (below 2^-1042) the leading bit of the low words. A side: one
+     * line per thread, B side: eight. */
+    constexpr int NL = A_SIDE ? 1 : 8;
+    uint32_t mh[NL], ml[NL];
+#pragma unroll
+    for (int y = 0; y < NL; ++y) mh[y] = ml[y] = 0;
+    auto take = [&](const double (&v)[8]) {
+#pragma unroll
+        for (int y = 0; y < 8; ++y) {
+            const int z = A_SIDE ? 0 : y;
+            mh[z] = max(mh[z], (uint32_t)__double2hiint(v[y]) & 0x7fffffffu);
+            ml[z] |= (uint32_t)__double2loint(v[y]);
         }
-    } else {
-        switch (s) {
-        case 2: FMM_PACKS(2, 5); break;
-        case 3: FMM_PACKS(3, 5); break;
-        case 4: FMM_PACKS(4, 5); break;
-        case 5: FMM_PACKS(5, 5); break;
-        case 6: FMM_PACKS(6, 5); break;
-        case 7: FMM_PACKS(7, 5); break;
-        case 8: FMM_PACKS(8, 5); break;
-        case 9: FMM_PACKS(9, 5); break;
-        case 10: FMM_PACKS(10, 5); break;
-        case 11: FMM_PACKS(11, 5); break;
-        default: FMM_PACKS(12, 5); break;
+    };
+    double v[8];
+    {
+        double w[8];
+        for (int t = 0; t < tiles; t += 2) {   /* sixteen loads in flight */
+            load(t, v);
+            load(t + 1, w);
+            take(v);
+            take(w);
         }
     }
-#undef FMM_PACKS
+    if (A_SIDE) {
+        sh.part[tid / kPrepLines][tid % kPrepLines] = make_uint2(ml[0], mh[0]);
+    } else {
+#pragma unroll
+        for (int y = 0; y < NL; ++y) {
+            const uint32_t h = __reduce_max_sync(0xffffffffu, mh[y]), l = __reduce_or_sync(0xffffffffu, ml[y]);
+            /* line = tid / 128 + 2 y; the four warps of a line each leave one maximum */
+            if (tid % 32 == 0) sh.part[tid / 32 % 4][line + 2 * y] = make_uint2(l, h);
+        }
+    }
+    __syncthreads();
+    if (tid < kPrepLines) {
+        uint2 m = make_uint2(0, 0);
+        for (int q = 0; q < (A_SIDE ? kPrepThreads / kPrepLines : 4); ++q) {
+            m.x |= sh.part[q][tid].x;
+            m.y = max(m.y, sh.part[q][tid].y);
+        }
+        sh.mx[tid] = m;
+    }
+    if (nrank > 1) {
+        cgr::cluster_group cl = cgr::this_cluster();
+        cl.sync();
+        uint2 m = make_uint2(0, 0);
+        if (tid < kPrepLines)
+            for (int q = 0; q < nrank; ++q) {
+                const uint2 z = *cl.map_shared_rank(&sh.mx[tid], q);
+                m.x |= z.x;
+                m.y = max(m.y, z.y);
+            }
+        cl.sync();   /* every CTA has read the others' maxima */
+        if (tid < kPrepLines) sh.mx[tid] = m;
+    }
+    if (tiles > 0) load(0, v);
+    __syncthreads();
+    /* exponent of the line's maximum (exp_above: normal numbers by the exponent
+     * field, subnormal ones by the leading bit) */
+    auto exponent = [&](int x) {
+        const uint2 m = sh.mx[x];
+        return exp_above(__hiloint2double((int)m.y, (int)(m.y ? 0u : m.x)));
+    };
+    if (rank == 0 && tid < kPrepLines) ex[l0 + tid] = exponent(tid);
+    /* digits: a warp takes lines w and w + 8, four consecutive k per lane:
+     * 256-byte stores per line and slice */
+    const int rl = tid / 32, k4 = tid % 32 * 4;
+    const int E0 = exponent(rl), E1 = exponent(rl + 8);
+    const int64_t off = (l0 + rl) * k_pad + p0 + k4;
+    const int pos = rl * kPrepPitch + k4 + k4 / 16;
+    for (int t = 0; t < tiles; ++t) {
+        double* tile = sh.tile[t & 1];   /* the other one may still be read */
+#pragma unroll
+        for (int y = 0; y < 8; ++y) {
+            const int li = A_SIDE ? line : line + 2 * y, kk = A_SIDE ? kq + 16 * y : kq;
+            tile[li * kPrepPitch + kk + kk / 16] = v[y];
+        }
+        __syncthreads();
+        if (t + 1 < tiles) load(t + 1, v);   /* in flight under this tile's digits */
+        if (p0 + t * kPrepK + k4 < p1) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                Digits Y[4];
+#pragma unroll
+                for (int x = 0; x < 4; ++x) Y[x] = split_offset<S, DB>(tile[pos + h * 8 * kPrepPitch + x], h ? E1 : E0);
+                store_digits4<S, DB>(out, off + h * 8 * k_pad + (int64_t)t * kPrepK, l_pad * k_pad, Y);
+            }
+        }
+    }
+}
+
+template <int S, int DB>
+__global__ void __launch_bounds__(kPrepThreads, DB == 8 ? 4 : 3)   /* more digits spill at 64 registers */
+prep_kernel(const double* __restrict__ A, int64_t lda, const double* __restrict__ B, int64_t ldb, int64_t m,
+            int64_t n, int64_t k, int64_t m_pad, int64_t n_pad, int64_t k_pad, int* __restrict__ e_row,
+            int* __restrict__ f_col, uint8_t* __restrict__ sa, uint8_t* __restrict__ sb,
+            unsigned int* __restrict__ sched, int nrank)
+{
+    __shared__ PrepShared sh;
+    const int64_t c = blockIdx.x / (unsigned)nrank, ca = m_pad / kPrepLines;
+    const int rank = (int)(blockIdx.x % (unsigned)nrank);
+    if (blockIdx.x == 0 && threadIdx.x == 0) *sched = 0;   /* the GEMM's work-item counter */
+    if (c < ca)
+        prep_body<S, DB, true>(sh, A, lda, m, k, m_pad, k_pad, e_row, sa, c * kPrepLines, rank, nrank);
+    else
+        prep_body<S, DB, false>(sh, B, ldb, n, k, n_pad, k_pad, f_col, sb, (c - ca) * kPrepLines, rank, nrank);
 }
 
 /* ------------------------------------------------------ GEMM kernel ---- */
@@ -737,6 +928,7 @@ struct GemmProblem {
     int zmin;             /* lowest level with a digit plane (ZPlanes) */
     int znd;              /* digit planes */
     int zrow0;            /* first Z row of the launch's tile row 0 */
+    int nunits, unit_kb;  /* work units per tile, k blocks per unit at most; nunits 0: whole tiles (UnitSpan) */
     int nkb;              /* k_pad / kbe */
     int kbe;              /* k elements per 128-byte stage row: 64 (BF16) or 128 (FP8) */
     int db;               /* digit bits: 8 (BF16) or 5 (FP8-E4M3) */
@@ -762,13 +954,51 @@ struct GemmLaunch {
 };
 static_assert(sizeof(GemmLaunch) <= 32764, "GemmLaunch must fit the kernel parameter space");
 
-__device__ __forceinline__ int level_pairs(int g, int s) { return min(s, g - 1) - max(1, g - s) + 1; }
+__host__ __device__ __forceinline__ int level_pairs(int g, int s)
+{
+    return (g - 1 < s ? g - 1 : s) - (g - s > 1 ? g - s : 1) + 1;
+}
+
+/* A tile's k blocks of all slice pairs as work units, for a product grid too
+ * small to give every SM a tile: a unit is part of one level, its k blocks
+ * [q0, q1) in the producer's order, at most unit_kb of them. Each unit leaves
+ * its sums as one int32 plane ([n_pad/4][m_pad] int4, below); the C
+ * update adds a level's planes (an exact integer sum) before it rounds and
+ * combines the levels, so Z is the same value. */
+struct UnitSpan {
+    int g, q0, q1;
+};
+
+__host__ __device__ __forceinline__ int level_units(int g, int s, int nkb, int unit_kb)
+{
+    return (level_pairs(g, s) * nkb + unit_kb - 1) / unit_kb;
+}
+
+__host__ __device__ __forceinline__ UnitSpan unit_span(int s, int nkb, int unit_kb, int u)
+{
+    for (int g = s + 1; g > 2; --g) {
+        const int cnt = level_units(g, s, nkb, unit_kb);
+        if (u < cnt) {
+            const int lk = level_pairs(g, s) * nkb, len = (lk + cnt - 1) / cnt;
+            return UnitSpan{g, u * len, u * len + len < lk ? u * len + len : lk};
+        }
+        u -= cnt;
+    }
+    const int cnt = level_units(2, s, nkb, unit_kb), len = (nkb + cnt - 1) / cnt;
+    return UnitSpan{2, u * len, u * len + len < nkb ? u * len + len : nkb};
+}
+
+/* the k blocks [q0, q1) of level g that an item runs: all of every level, or its unit's */
+__device__ __forceinline__ UnitSpan level_span(const GemmProblem& P, const UnitSpan& u, int g)
+{
+    return P.nunits ? u : UnitSpan{g, 0, level_pairs(g, P.s) * P.nkb};
+}
 
 /* Work item b -> problem, product and tile: problems in order, products in
  * order within a problem, then a grouped raster of kRasterGroup tile rows so
  * the CTAs resident together share slice panels in L2. */
 struct Item {
-    int p, r, tile_m, tile_n;
+    int p, r, tile_m, tile_n, unit;
 };
 
 __device__ __forceinline__ Item decode_item(const GemmLaunch& L, int b, int raster = kRasterGroup)
@@ -784,6 +1014,11 @@ __device__ __forceinline__ Item decode_item(const GemmLaunch& L, int b, int rast
     Item it;
     it.p = p;
     it.r = local / per_prod;
+    it.unit = 0;
+    if (P.nunits) {   /* one product: the tiles of unit 0, then of unit 1, ... */
+        it.unit = it.r;
+        it.r = 0;
+    }
     const int id = local % per_prod;
     const int per_group = raster * P.tiles_n;
     const int grp = id / per_group, first_m = grp * raster;
@@ -965,6 +1200,41 @@ __device__ __forceinline__ bool drain_item(const GemmLaunch& L, int p, uint8_t* 
     return true;
 }
 
+/* drain_item for a work unit: its chunks' sums, stored as they are. zp: the
+ * thread's row in the unit's plane of its first column group. */
+template <class Arrive>
+__device__ __forceinline__ bool drain_unit(const GemmLaunch& L, int4* zp, int64_t gstep, int nkb_unit, uint32_t tl,
+                                           uint64_t* accf, int& buf, uint32_t& aph, int lane,
+                                           volatile int* abort_flag, int code, Arrive arrive)
+{
+    int lsum[kEpiCols];
+#pragma unroll
+    for (int x = 0; x < kEpiCols; ++x) lsum[x] = 0;
+    for (int left = (nkb_unit + kChunkKB - 1) / kChunkKB; left > 0; --left) {
+        if (!sm103::mbar_wait(&accf[buf], aph, abort_flag, L.err, code)) return false;
+        sm103::tc_fence_after();
+#pragma unroll
+        for (int h = 0; h < kEpiCols / 8; ++h) {
+            uint32_t v[8];
+            SM103_TMEM_LD_X8(tl + buf * kTileN + h * 8, v);
+            sm103::tmem_wait_ld();
+#pragma unroll
+            for (int x = 0; x < 8; ++x) lsum[h * 8 + x] += __float2int_rn(__uint_as_float(v[x]));
+        }
+        sm103::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) arrive(buf);
+        buf ^= 1;
+        if (buf == 0) aph ^= 1;
+    }
+#pragma unroll
+    for (int x = 0; x < kEpiCols; x += 4) {
+        *zp = make_int4(lsum[x], lsum[x + 1], lsum[x + 2], lsum[x + 3]);
+        zp += gstep;
+    }
+    return true;
+}
+
 /* Persistent GEMM over a list of work items (problem, product of its group,
  * 128 x 256 output tile), drawn dynamically: the producer takes the next item
  * from L.sched and passes it to the other roles through a CTA-local item
@@ -1051,24 +1321,28 @@ split_gemm_kernel(const __grid_constant__ GemmLaunch L)
                  * chunk sum is exact in any order. (An L2 prefetch of the boxes
                  * eight stages ahead measured 3x slower, with 7x the DRAM
                  * reads.) */
+                const UnitSpan us = P.nunits ? unit_span(s, nkb, P.unit_kb, it.unit) : UnitSpan{0, 0, 0};
+                const int g_hi = P.nunits ? us.g : s + 1, g_lo = P.nunits ? us.g : 2;
                 int pi = 0;
-                for (int g = s + 1; g >= 2 && ok; --g) {
+                for (int g = g_hi; g >= g_lo && ok; --g) {
                     const int tlo = max(1, g - s), thi = min(s, g - 1);
-                    for (int x = 0; x <= thi - tlo && ok; ++x, ++pi) {
+                    const UnitSpan sp = level_span(P, us, g);
+                    int x = sp.q0 / nkb, y = sp.q0 - x * nkb;
+                    for (int q = sp.q0; q < sp.q1; ++q) {
                         const int t = (g & 1) ? tlo + x : thi - x;
                         const int u = g - t;
-                        for (int y = 0; y < nkb; ++y) {
-                            const int kb = (pi & 1) ? nkb - 1 - y : y;
-                            if (!sm103::mbar_wait(&empty[st], ph ^ 1, abort_flag, L.err, 1)) { ok = false; break; }
-                            sm103::mbar_arrive_expect_tx(&full[st], kStageBytes);
-                            sm103::tma_load_2d(sA + st * kATileBytes, &P.tmA, &full[st], kb * P.kbe,
-                                               arow + (t - 1) * P.m_pad);
-                            sm103::tma_load_2d(sB + st * kBTileBytes, &P.tmB, &full[st], kb * P.kbe,
-                                               brow + (u - 1) * P.n_pad);
-                            armed |= 1u << st;
-                            if (++st == kStages) { st = 0; ph ^= 1; armed = 0; }
-                        }
+                        const int kb = ((pi + x) & 1) ? nkb - 1 - y : y;
+                        if (!sm103::mbar_wait(&empty[st], ph ^ 1, abort_flag, L.err, 1)) { ok = false; break; }
+                        sm103::mbar_arrive_expect_tx(&full[st], kStageBytes);
+                        sm103::tma_load_2d(sA + st * kATileBytes, &P.tmA, &full[st], kb * P.kbe,
+                                           arow + (t - 1) * P.m_pad);
+                        sm103::tma_load_2d(sB + st * kBTileBytes, &P.tmB, &full[st], kb * P.kbe,
+                                           brow + (u - 1) * P.n_pad);
+                        armed |= 1u << st;
+                        if (++st == kStages) { st = 0; ph ^= 1; armed = 0; }
+                        if (++y == nkb) { y = 0; ++x; }
                     }
+                    pi += thi - tlo + 1;
                 }
             }
             if (!ok) {
@@ -1095,44 +1369,46 @@ split_gemm_kernel(const __grid_constant__ GemmLaunch L)
                 if (!ring.take(&b, abort_flag, L.err, 8)) { ok = false; break; }
                 if (b < 0) break;
                 const Item it = decode_item(L, b);
-                const int s = L.prob[it.p].s, nkb = L.prob[it.p].nkb, fmt = L.prob[it.p].fmt;
-                for (int g = s + 1; g >= 2 && ok; --g) {
-                    const int level_kb = level_pairs(g, s) * nkb;
-                    int jl = 0;
-                    for (int t = max(1, g - s); t <= min(s, g - 1) && ok; ++t)
-                        for (int kb = 0; kb < nkb; ++kb) {
-                            if (jl % kChunkKB == 0) {
-                                if (!sm103::mbar_wait(&acce[buf], aph ^ 1, abort_flag, L.err, 2)) { ok = false; break; }
-                                sm103::tc_fence_after();
-                            }
-                            if (!sm103::mbar_wait(&full[st], ph, abort_flag, L.err, 3)) { ok = false; break; }
+                const GemmProblem& P = L.prob[it.p];
+                const int fmt = P.fmt;
+                const UnitSpan us = P.nunits ? unit_span(P.s, P.nkb, P.unit_kb, it.unit) : UnitSpan{0, 0, 0};
+                const int g_hi = P.nunits ? us.g : P.s + 1, g_lo = P.nunits ? us.g : 2;
+                for (int g = g_hi; g >= g_lo && ok; --g) {
+                    const UnitSpan sp = level_span(P, us, g);
+                    const int level_kb = sp.q1 - sp.q0;
+                    for (int jl = 0; jl < level_kb; ) {
+                        if (jl % kChunkKB == 0) {
+                            if (!sm103::mbar_wait(&acce[buf], aph ^ 1, abort_flag, L.err, 2)) { ok = false; break; }
                             sm103::tc_fence_after();
-                            const uint32_t a0 = sm103::smem_u32(sA + st * kATileBytes);
-                            const uint32_t b0 = sm103::smem_u32(sB + st * kBTileBytes);
-                            /* four MMAs per 128-byte stage row: K = 16 BF16 or 32 FP8
-                             * elements each, 32 bytes apart */
-                            if (fmt) {
-#pragma unroll
-                                for (int kk = 0; kk < 4; ++kk)
-                                    sm103::mma_f8(tmem + buf * kTileN, sm103::smem_desc_sw128(a0 + kk * 32),
-                                                  sm103::smem_desc_sw128(b0 + kk * 32), idesc8,
-                                                  (jl % kChunkKB != 0 || kk != 0) ? 1u : 0u);
-                            } else {
-#pragma unroll
-                                for (int kk = 0; kk < 4; ++kk)
-                                    sm103::mma_bf16(tmem + buf * kTileN, sm103::smem_desc_sw128(a0 + kk * 32),
-                                                    sm103::smem_desc_sw128(b0 + kk * 32), idesc16,
-                                                    (jl % kChunkKB != 0 || kk != 0) ? 1u : 0u);
-                            }
-                            sm103::mma_commit(&empty[st]);
-                            if (++st == kStages) { st = 0; ph ^= 1; }
-                            ++jl;
-                            if (jl % kChunkKB == 0 || jl == level_kb) {
-                                sm103::mma_commit(&accf[buf]);
-                                buf ^= 1;
-                                if (buf == 0) aph ^= 1;
-                            }
                         }
+                        if (!sm103::mbar_wait(&full[st], ph, abort_flag, L.err, 3)) { ok = false; break; }
+                        sm103::tc_fence_after();
+                        const uint32_t a0 = sm103::smem_u32(sA + st * kATileBytes);
+                        const uint32_t b0 = sm103::smem_u32(sB + st * kBTileBytes);
+                        /* four MMAs per 128-byte stage row: K = 16 BF16 or 32 FP8
+                         * elements each, 32 bytes apart */
+                        if (fmt) {
+#pragma unroll
+                            for (int kk = 0; kk < 4; ++kk)
+                                sm103::mma_f8(tmem + buf * kTileN, sm103::smem_desc_sw128(a0 + kk * 32),
+                                              sm103::smem_desc_sw128(b0 + kk * 32), idesc8,
+                                              (jl % kChunkKB != 0 || kk != 0) ? 1u : 0u);
+                        } else {
+#pragma unroll
+                            for (int kk = 0; kk < 4; ++kk)
+                                sm103::mma_bf16(tmem + buf * kTileN, sm103::smem_desc_sw128(a0 + kk * 32),
+                                                sm103::smem_desc_sw128(b0 + kk * 32), idesc16,
+                                                (jl % kChunkKB != 0 || kk != 0) ? 1u : 0u);
+                        }
+                        sm103::mma_commit(&empty[st]);
+                        if (++st == kStages) { st = 0; ph ^= 1; }
+                        ++jl;
+                        if (jl % kChunkKB == 0 || jl == level_kb) {
+                            sm103::mma_commit(&accf[buf]);
+                            buf ^= 1;
+                            if (buf == 0) aph ^= 1;
+                        }
+                    }
                 }
             }
             /* all issued MMAs complete before TMEM is released */
@@ -1156,6 +1432,14 @@ split_gemm_kernel(const __grid_constant__ GemmLaunch L)
             const Item it = decode_item(L, b);
             const GemmProblem& P = L.prob[it.p];
             const int zi = P.zrow0 + it.tile_m * kTileM + row;
+            if (P.nunits) {
+                const UnitSpan us = unit_span(P.s, P.nkb, P.unit_kb, it.unit);
+                int4* zp = (int4*)P.Z + ((int64_t)it.unit * P.n_pad + it.tile_n * kTileN + colbase) / 4 * P.m_pad + zi;
+                if (!drain_unit(L, zp, P.m_pad, us.q1 - us.q0, tl + colbase, accf, buf, aph, lane, abort_flag, 4,
+                                [&](int q) { sm103::mbar_arrive(&acce[q]); }))
+                    break;
+                continue;
+            }
             uint8_t* z0 = P.Z + ((int64_t)it.r * P.n_pad + it.tile_n * kTileN + colbase) / 4 *
                                     z_group_bytes(P.m_pad, P.znd);
             if (!drain_item(L, it.p, z0 + (int64_t)zi * 16, zi, tl + colbase, accf, buf, aph, lane, abort_flag, 4,
@@ -1651,6 +1935,60 @@ scatter_all_kernel(const int* __restrict__ tab, int r0, int nprod, int64_t m, in
 }
 
 
+/* C update of a classical GEMM whose tiles ran as work units: a thread takes
+ * a row of a column group, adds each level's planes, rounds and combines the
+ * levels into Z and updates C as scatter_all_kernel does. Blocks of 32 rows x
+ * 16 columns; reads nunits x 4 bytes per element, mostly from L2. */
+__global__ void __launch_bounds__(128)
+scatter_units_kernel(int m, int n, double alpha, double beta, const int4* __restrict__ Zp, int m_pad, int n_pad, int s,
+                     int nkb, int unit_kb, int nunits, int G, int db, int ebase, const int* __restrict__ e_row,
+                     const int* __restrict__ f_col, double* __restrict__ C, int64_t ldc)
+{
+    const int i = (int)blockIdx.x * 32 + (int)threadIdx.x % 32, j = ((int)blockIdx.y * 4 + (int)threadIdx.x / 32) * 4;
+    if (i >= m || j >= n) return;
+    double* cp = C + i + (int64_t)j * ldc;
+    double c[kScatterCols];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) c[u] = j + u < n ? beta_c(beta, cp + u * ldc) : 0.0;
+    const int er = e_row[i] + ebase;
+    const int4 f = *(const int4*)(f_col + j);
+    const int fc[4] = {f.x, f.y, f.z, f.w};
+    const int4* q = Zp + (int64_t)(j / 4) * m_pad + i;
+    const int64_t plane = (int64_t)n_pad / 4 * m_pad;
+    int64_t z[kScatterCols] = {0, 0, 0, 0};
+    int l[kScatterCols] = {0, 0, 0, 0};
+    int g = s + 1, left = level_units(g, s, nkb, unit_kb);
+    constexpr int U = 8;   /* planes in flight */
+    for (int p0 = 0; p0 < nunits; p0 += U) {
+        int4 v[U];
+#pragma unroll
+        for (int x = 0; x < U; ++x)
+            if (p0 + x < nunits) v[x] = q[(p0 + x) * plane];
+#pragma unroll
+        for (int x = 0; x < U; ++x) {
+            if (p0 + x >= nunits) break;
+            l[0] += v[x].x;
+            l[1] += v[x].y;
+            l[2] += v[x].z;
+            l[3] += v[x].w;
+            if (--left > 0) continue;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {   /* the level is complete */
+                if (g > G)
+                    z[u] += ((l[u] >> (db * (g - G) - 1)) + 1) >> 1;
+                else
+                    z[u] += (int64_t)((uint64_t)(int64_t)l[u] << (db * (G - g)));
+                l[u] = 0;
+            }
+            --g;
+            left = level_units(g, s, nkb, unit_kb);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+        if (j + u < n) cp[u * ldc] = fma(alpha, i64_to_double_scaled(z[u], er + fc[u]), c[u]);
+}
+
 /* ------------------------------------- batched waves: side work per wave ---- */
 
 /* A wave of a batch runs each side kernel (C scaling and maxima zeroing,
@@ -1746,6 +2084,21 @@ __global__ void __launch_bounds__(COLS * 8, COLS == 32 ? 4 : 8) wave_pack_b_kern
     const int64_t vb = blockIdx.x - P.b0;
     pack_b_body<S, DB, COLS>(P.tab, 0, P.R, P.B, P.ldb, P.k, P.n, P.n_pad, P.k_pad, P.f_col, P.sb, 0, vb % P.gx,
                              vb / P.gx);
+}
+
+/* the classical problems' maxima, exponents and digits (prep_kernel), clusters of nrank CTAs */
+template <int S, int DB>
+__global__ void __launch_bounds__(kPrepThreads, 3) wave_classical_kernel(const __grid_constant__ WaveLaunch W, int nrank)
+{
+    __shared__ PrepShared sh;
+    const WaveProb& P = W.p[wave_find(W, blockIdx.x)];
+    const int64_t c = (blockIdx.x - P.b0) / nrank, ca = P.m_pad / kPrepLines;
+    const int rank = (int)(blockIdx.x % (unsigned)nrank);
+    if (c < ca)
+        prep_body<S, DB, true>(sh, P.A, P.lda, P.m, P.k, P.m_pad, P.k_pad, P.e_row, P.sa, c * kPrepLines, rank, nrank);
+    else
+        prep_body<S, DB, false>(sh, P.B, P.ldb, P.n, P.k, P.n_pad, P.k_pad, P.f_col, P.sb, (c - ca) * kPrepLines, rank,
+                                nrank);
 }
 
 __global__ void __launch_bounds__(256) wave_scatter_kernel(const __grid_constant__ WaveLaunch W)
@@ -1888,6 +2241,53 @@ WsLayout ws_layout(const AlgView& alg, int64_t m, int64_t n, int64_t k, int s, s
     return L;
 }
 
+/* Work units of a classical GEMM (UnitSpan), for a product grid whose tiles
+ * leave SMs idle: the units per tile that the model below finds cheapest, none
+ * when whole tiles do as well (planes of at most kUnitBytes). A k block costs about 760 clocks on the single-SM kernel and 640 on
+ * CTA pairs, a unit or tile 3000 beside them, the extra planes the C update
+ * reads about one clock per 2000 bytes. 300 x 700 x 450, 6 slices: 9 tiles of
+ * 168 k blocks, 71 us; as 9 x 17 units 14 us. */
+constexpr size_t kUnitBytes = (size_t)128 << 20;
+
+struct UnitPlan {
+    int nunits = 0, unit_kb = 0;
+    size_t bytes = 0;
+};
+
+UnitPlan unit_plan(const Dims& d, int s, int fmt, bool pair)
+{
+    constexpr int64_t sms = 152;
+    constexpr double kb_single = 760, kb_pair = 640, per_unit = 3000, bytes_per_clk = 2000;
+    const int64_t tiles = d.m_pad / kTileM * (d.n_pad / kTileN);
+    const int nkb = (int)(d.k_pad / kbe_of(fmt));
+    UnitPlan best;
+    if (tiles >= sms) return best;
+    const size_t plane = 4 * (size_t)d.m_pad * (size_t)d.n_pad;
+    const double all = (double)nkb * s * (s + 1) / 2;
+    double least = all * kb_single + per_unit;   /* one round of whole tiles */
+    if (pair) least = (double)((tiles / 2 + sms / 2 - 1) / (sms / 2)) * (all * kb_pair + per_unit);
+    least *= 0.9;
+    for (int parts = 2; parts <= 64; ++parts) {
+        const int T = std::max(2, (int)((all + parts - 1) / parts));
+        int nu = 0, longest = 0;
+        for (int g = s + 1; g >= 2; --g) {
+            const int cnt = level_units(g, s, nkb, T), lk = level_pairs(g, s) * nkb;
+            nu += cnt;
+            longest = std::max(longest, (lk + cnt - 1) / cnt);
+        }
+        if (nu * plane > kUnitBytes) continue;
+        const double t = (double)((tiles * nu + sms - 1) / sms) * (longest * kb_single + per_unit) +
+                         (double)(nu - 2) * (double)plane / bytes_per_clk;
+        if (t < least) {
+            least = t;
+            best.nunits = nu;
+            best.unit_kb = T;
+            best.bytes = (size_t)nu * plane;
+        }
+    }
+    return best;
+}
+
 /* opt-in event timing of the GEMM launches */
 std::mutex g_timing_mu;
 bool g_timing = false;
@@ -1977,6 +2377,8 @@ struct SplitJob {
     int s;
     int fmt;       /* 0: BF16 slices, 1: FP8-E4M3 slices */
     bool trivial;  /* nothing beyond C := beta*C */
+    bool classical; /* one product of coefficient 1: prep_kernel forms its operands */
+    int nunits, unit_kb; /* its tiles run as work units (0: whole) */
     WsLayout L;
     uint8_t* w;
 };
@@ -1995,6 +2397,8 @@ static int job_init(SplitJob& j, const AlgView& alg, int64_t m, int64_t n, int64
     j.s = s;
     j.w = nullptr;
     j.trivial = m == 0 || n == 0 || k == 0 || alpha == 0.0;
+    j.classical = fmm_plain_classical(alg);
+    j.nunits = j.unit_kb = 0;
     if (j.trivial) return FMM_OK;
     if (alg.max_nnz_u > kPackMaxEnt || alg.max_nnz_v > kPackMaxEnt) return FMM_ERR_UNSUPPORTED;
     if (m > 0x7fffffffLL || n > 0x7fffffffLL) return FMM_ERR_UNSUPPORTED;
@@ -2328,6 +2732,7 @@ static int job_fill(const SplitJob& j, GemmProblem& gp, int np, int item_begin, 
     gp.zmin = zp.zmin;
     gp.znd = zp.nd;
     gp.zrow0 = 0;
+    gp.nunits = gp.unit_kb = 0;
     gp.kbe = kbe_of(j.fmt);
     gp.nkb = (int)(d.k_pad / gp.kbe);
     gp.db = job_db(j);
@@ -2345,7 +2750,8 @@ static int64_t job_items(const SplitJob& j, int np, bool pair = false)
     return (int64_t)np * (j.d.m_pad / (pair ? kPairTileM : kTileM)) * (j.d.n_pad / kTileN);
 }
 
-static int launch_gemm(GemmLaunch& gl, int64_t nitems, int nprod_timed, cudaStream_t st, bool pair);
+static int launch_gemm(GemmLaunch& gl, int64_t nitems, int nprod_timed, cudaStream_t st, bool pair,
+                       bool sched_zeroed = false);
 
 /* The GEMM of the job's current product group, as back-to-back launches of
  * at most K products, K the fewest products that give each launch about 24
@@ -2487,7 +2893,7 @@ static void job_scatter(const SplitJob& j, int r0, int np, cudaStream_t st, bool
     fmm_count_launch(1);
 }
 
-static int launch_gemm(GemmLaunch& gl, int64_t nitems, int nprod_timed, cudaStream_t st, bool pair)
+static int launch_gemm(GemmLaunch& gl, int64_t nitems, int nprod_timed, cudaStream_t st, bool pair, bool sched_zeroed)
 {
     /* the kernels' shared-memory limit is a per-device attribute: set once per device */
     static std::atomic<uint64_t> attr_set{0};
@@ -2518,8 +2924,8 @@ static int launch_gemm(GemmLaunch& gl, int64_t nitems, int nprod_timed, cudaStre
         g_timed_products += (uint64_t)nprod_timed;
     }
     /* both kernels draw their work items from gl.sched, zero at launch */
-    if (gl.sched == nullptr || cudaMemsetAsync(gl.sched, 0, sizeof(unsigned int), st) != cudaSuccess)
-        return FMM_ERR_CUDA;
+    if (gl.sched == nullptr) return FMM_ERR_CUDA;
+    if (!sched_zeroed && cudaMemsetAsync(gl.sched, 0, sizeof(unsigned int), st) != cudaSuccess) return FMM_ERR_CUDA;
     if (pair)   /* clusters of two CTAs, one pair tile each at a time */
         split_gemm_pair_kernel<<<(unsigned)(2 * std::min<int64_t>(nitems, sms / 2)), kGemmThreads, kPairSmem, st>>>(gl);
     else
@@ -2596,6 +3002,93 @@ static int split_overlap(SplitJob& j, const OverlapPlan& o, void* ws, cudaStream
     return cudaGetLastError() == cudaSuccess ? FMM_OK : FMM_ERR_CUDA;
 }
 
+/* CTAs per cluster (k chunks) of prep_kernel for `groups` line groups of depth
+ * k_pad: more while the launch has fewer than three CTAs per SM, or a chunk is
+ * longer than 1024 k (its 16 lines are read twice, the second time from L2:
+ * 128 KB for each of the 608 CTAs in flight), of at least one tile each */
+static int prep_ranks(int64_t groups, int64_t k_pad)
+{
+    int r = 1;
+    while (r < 8 && k_pad >= (int64_t)kPrepK * 2 * r && (groups * r < 3 * 152 || k_pad > (int64_t)1024 * r)) r *= 2;
+    return r;
+}
+
+template <class K, class... Args>
+static int launch_clusters(K* kernel, int64_t blocks, int cluster, cudaStream_t st, Args... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(kPrepThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)cluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+    fmm_count_launch(1);
+    return e == cudaSuccess ? FMM_OK : FMM_ERR_CUDA;
+}
+
+/* exponents and digit slices of both operands of a classical job */
+static int job_prep(SplitJob& j, cudaStream_t st)
+{
+    const Dims& d = j.d;
+    const int64_t groups = (d.m_pad + d.n_pad) / kPrepLines;
+    const int nrank = prep_ranks(groups, d.k_pad);
+    return with_slices(j.fmt, j.s, [&](auto S, auto DB) {
+        return launch_clusters(prep_kernel<S(), DB()>, groups * nrank, nrank, st, j.A, j.lda, j.B, j.ldb, j.m, j.n, j.k,
+                               d.m_pad, d.n_pad, d.k_pad, (int*)(j.w + j.L.erow), (int*)(j.w + j.L.fcol),
+                               j.w + j.L.sa, j.w + j.L.sb, (unsigned int*)(j.w + j.L.sched), nrank);
+    });
+}
+
+/* A classical GEMM: one launch for the operands, one for the tiles (or their
+ * work units), one for C. The units' planes are a stream-ordered temporary
+ * (with `alloc`; without it, or without memory, the tiles run whole). */
+static int split_classical(SplitJob& j, bool alloc, cudaStream_t st)
+{
+    if (int rc = job_prep(j, st); rc != FMM_OK) return rc;
+    UnitPlan up;
+    if (alloc) up = unit_plan(j.d, j.s, j.fmt, job_pair(j));
+    void* planes = nullptr;
+    if (up.nunits != 0) {
+        const cudaMemPool_t pool = fmm_temp_pool();
+        if (pool == nullptr || cudaMallocFromPoolAsync(&planes, up.bytes, pool, st) != cudaSuccess) {
+            cudaGetLastError();
+            up = UnitPlan();
+        }
+    }
+    const bool pair = job_pair(j) && up.nunits == 0;
+    GemmLaunch gl;
+    memset(&gl, 0, sizeof(gl));
+    gl.nprob = 1;
+    gl.sched = (unsigned int*)(j.w + j.L.sched);   /* zeroed by prep_kernel */
+    GemmProblem& gp = gl.prob[0];
+    if (int rc = job_fill(j, gp, 1, 0, pair); rc != FMM_OK) return rc;
+    if (up.nunits == 0) {
+        if (int rc = launch_gemm(gl, job_items(j, 1, pair), 1, st, pair, true); rc != FMM_OK) return rc;
+        job_scatter(j, 0, 1, st);
+        return cudaGetLastError() == cudaSuccess ? FMM_OK : FMM_ERR_CUDA;
+    }
+    gp.nunits = up.nunits;
+    gp.unit_kb = up.unit_kb;
+    gp.Z = (uint8_t*)planes;
+    int rc = launch_gemm(gl, job_items(j, 1) * up.nunits, 1, st, false, true);
+    if (rc == FMM_OK) {
+        scatter_units_kernel<<<dim3((unsigned)((j.m + 31) / 32), (unsigned)((j.n + 15) / 16)), 128, 0, st>>>(
+            (int)j.m, (int)j.n, j.alpha, j.beta, (const int4*)planes, (int)j.d.m_pad, (int)j.d.n_pad, j.s, gp.nkb,
+            up.unit_kb, up.nunits, job_zlevel(j), job_db(j), job_ebase(j), (const int*)(j.w + j.L.erow),
+            (const int*)(j.w + j.L.fcol), j.C, j.ldc);
+        fmm_count_launch(1);
+        rc = cudaGetLastError() == cudaSuccess ? FMM_OK : FMM_ERR_CUDA;
+    }
+    if (cudaFreeAsync(planes, st) != cudaSuccess && rc == FMM_OK) rc = FMM_ERR_CUDA;
+    return rc;
+}
+
 static int split_launch_budget(const AlgView& alg, int64_t m, int64_t n, int64_t k, double alpha,
                                const double* A, int64_t lda, const double* B, int64_t ldb, double beta,
                                double* C, int64_t ldc, int s, int fmt, void* ws, size_t ws_bytes, size_t budget,
@@ -2609,6 +3102,7 @@ static int split_launch_budget(const AlgView& alg, int64_t m, int64_t n, int64_t
         if (o.ok) return split_overlap(j, o, ws, st, sp);
     }
     if (!j.trivial && (rc = job_bind(j, ws, ws_bytes, budget)) != FMM_OK) return rc;
+    if (!j.trivial && j.classical) return split_classical(j, sp != nullptr, st);
     if ((rc = job_prologue(j, st, sp)) != FMM_OK || j.trivial) return rc;
     const int G = j.L.group;
     for (int r0 = 0; r0 < alg.R; r0 += G) {
@@ -3056,71 +3550,76 @@ static void wave_packs_t(WaveLaunch& L, const std::vector<SplitJob*>& qs, bool s
     fmm_count_launch(2);
 }
 
-static void wave_packs(int fmt, int s, WaveLaunch& L, const std::vector<SplitJob*>& qs, bool small, cudaStream_t st)
+/* maxima, exponents and digits of classical jobs of one format and slice
+ * count: one launch per cluster size among them (chunks of at most 1024 k) */
+static int wave_classical(int fmt, int s, WaveLaunch& L, const std::vector<SplitJob*>& qs, cudaStream_t st)
 {
-#define FMM_WPACKS(S_, DB_) wave_packs_t<S_, DB_>(L, qs, small, st)
-    if (fmt == 0) {
-        switch (s) {
-        case 2: FMM_WPACKS(2, 8); break;
-        case 3: FMM_WPACKS(3, 8); break;
-        case 4: FMM_WPACKS(4, 8); break;
-        case 5: FMM_WPACKS(5, 8); break;
-        case 6: FMM_WPACKS(6, 8); break;
-        case 7: FMM_WPACKS(7, 8); break;
-        default: FMM_WPACKS(8, 8); break;
-        }
-    } else {
-        switch (s) {
-        case 2: FMM_WPACKS(2, 5); break;
-        case 3: FMM_WPACKS(3, 5); break;
-        case 4: FMM_WPACKS(4, 5); break;
-        case 5: FMM_WPACKS(5, 5); break;
-        case 6: FMM_WPACKS(6, 5); break;
-        case 7: FMM_WPACKS(7, 5); break;
-        case 8: FMM_WPACKS(8, 5); break;
-        case 9: FMM_WPACKS(9, 5); break;
-        case 10: FMM_WPACKS(10, 5); break;
-        case 11: FMM_WPACKS(11, 5); break;
-        default: FMM_WPACKS(12, 5); break;
-        }
+    for (int nrank = 1; nrank <= 8; nrank *= 2) {
+        std::vector<SplitJob*> sel;
+        for (SplitJob* j : qs)
+            if (prep_ranks(3 * 152, j->d.k_pad) == nrank) sel.push_back(j);
+        if (sel.empty()) continue;
+        const int64_t nb = wave_table(L, sel, [&](const SplitJob& j, WaveProb& w) {
+            w.gx = 1;
+            w.nb = (j.d.m_pad + j.d.n_pad) / kPrepLines * nrank;
+        });
+        const int rc = with_slices(fmt, s, [&](auto S, auto DB) {
+            return launch_clusters(wave_classical_kernel<S(), DB()>, nb, nrank, st, L, nrank);
+        });
+        if (rc != FMM_OK) return rc;
     }
-#undef FMM_WPACKS
+    return FMM_OK;
 }
 
 /* The side work before a wave's GEMM, one launch per kernel over the bound
- * jobs qs (all products of each as one group): C scaling and maxima zeroing,
- * maxima, exponents, then the packs per (slice count, format). */
-static int wave_side_pack(const std::vector<SplitJob*>& qs, bool small, cudaStream_t st)
+ * jobs qs (all products of each as one group). Classical jobs: prep_kernel's
+ * work per (slice count, format). Others: maxima zeroing, maxima, exponents,
+ * then the packs per (slice count, format). */
+static int wave_side_pack(const std::vector<SplitJob*>& all, bool small, cudaStream_t st)
 {
-    if (qs.empty()) return FMM_OK;
     WaveLaunch L;
-    int64_t nb = wave_table(L, qs, [](const SplitJob& j, WaveProb& w) {
-        const int64_t total = (int64_t)j.alg.kt * (j.m + j.n);
-        w.gx = 1;
-        w.nb = std::min<int64_t>(std::max<int64_t>((total + 2047) / 2048, 1), 2048);
-    });
-    wave_prep_kernel<<<(unsigned)nb, 256, 0, st>>>(L);
-    nb = wave_table(L, qs, [](const SplitJob& j, WaveProb& w) {
-        w.gx = (j.m + 255) / 256 * j.alg.kt * ((j.d.ke + 255) / 256);
-        w.nb = w.gx + ((int64_t)j.alg.kt * j.n * 32 + 255) / 256;
-    });
-    wave_maxima_kernel<<<(unsigned)nb, 256, 0, st>>>(L);
-    nb = wave_table(L, qs, [](const SplitJob& j, WaveProb& w) {
-        w.gx = (j.d.m_pad + j.d.n_pad + 255) / 256;
-        w.nb = w.gx * j.alg.R;
-    });
-    wave_exps_kernel<<<(unsigned)nb, 256, 0, st>>>(L);
-    fmm_count_launch(3);
-    /* packs, one pair of launches per (format, slice count) present */
-    std::vector<std::pair<int, int>> kinds;
-    for (SplitJob* j : qs)
-        if (std::find(kinds.begin(), kinds.end(), std::make_pair(j->fmt, j->s)) == kinds.end())
-            kinds.emplace_back(j->fmt, j->s);
-    for (auto [fmt, sl] : kinds) {
-        std::vector<SplitJob*> sel;
-        for (SplitJob* j : qs)
-            if (j->fmt == fmt && j->s == sl) sel.push_back(j);
-        wave_packs(fmt, sl, L, sel, small, st);
+    std::vector<SplitJob*> qs, cl;
+    for (SplitJob* j : all) (j->classical ? cl : qs).push_back(j);
+    auto each_kind = [](const std::vector<SplitJob*>& js, auto f) -> int {
+        std::vector<std::pair<int, int>> kinds;
+        for (SplitJob* j : js)
+            if (std::find(kinds.begin(), kinds.end(), std::make_pair(j->fmt, j->s)) == kinds.end())
+                kinds.emplace_back(j->fmt, j->s);
+        for (auto [fmt, sl] : kinds) {
+            std::vector<SplitJob*> sel;
+            for (SplitJob* j : js)
+                if (j->fmt == fmt && j->s == sl) sel.push_back(j);
+            if (int rc = f(fmt, sl, sel); rc != FMM_OK) return rc;
+        }
+        return FMM_OK;
+    };
+    if (int rc = each_kind(cl, [&](int fmt, int sl, auto& sel) { return wave_classical(fmt, sl, L, sel, st); });
+        rc != FMM_OK)
+        return rc;
+    if (!qs.empty()) {
+        int64_t nb = wave_table(L, qs, [](const SplitJob& j, WaveProb& w) {
+            const int64_t total = (int64_t)j.alg.kt * (j.m + j.n);
+            w.gx = 1;
+            w.nb = std::min<int64_t>(std::max<int64_t>((total + 2047) / 2048, 1), 2048);
+        });
+        wave_prep_kernel<<<(unsigned)nb, 256, 0, st>>>(L);
+        nb = wave_table(L, qs, [](const SplitJob& j, WaveProb& w) {
+            w.gx = (j.m + 255) / 256 * j.alg.kt * ((j.d.ke + 255) / 256);
+            w.nb = w.gx + ((int64_t)j.alg.kt * j.n * 32 + 255) / 256;
+        });
+        wave_maxima_kernel<<<(unsigned)nb, 256, 0, st>>>(L);
+        nb = wave_table(L, qs, [](const SplitJob& j, WaveProb& w) {
+            w.gx = (j.d.m_pad + j.d.n_pad + 255) / 256;
+            w.nb = w.gx * j.alg.R;
+        });
+        wave_exps_kernel<<<(unsigned)nb, 256, 0, st>>>(L);
+        fmm_count_launch(3);
+        each_kind(qs, [&](int fmt, int sl, auto& sel) {
+            return with_slices(fmt, sl, [&](auto S, auto DB) {
+                wave_packs_t<S(), DB()>(L, sel, small, st);
+                return (int)FMM_OK;
+            });
+        });
     }
     return cudaGetLastError() == cudaSuccess ? FMM_OK : FMM_ERR_CUDA;
 }

@@ -81,6 +81,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     }
 }
 
+/* 8-byte global -> shared copy, zero when !ok (nothing is read then) */
+__device__ __forceinline__ void cp_async8(double* dst, const double* src, bool ok)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(ok ? 8 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
 /* ---- clusters (CTA pairs) ---- */
 
 __device__ __forceinline__ uint32_t cluster_ctarank()

@@ -188,7 +188,10 @@ size_t fmm_gpu_split_workspace_size(const fmm_t* fmm, int levels,
  * integer-valued FP32 accumulation, and recombined in FP64. slices in 2..8.
  * `workspace` (256-byte aligned) holds at least one product's slices and
  * level accumulators; fmm_gpu_split_workspace_size gives the recommended
- * size. Asynchronous on `stream`. */
+ * size. A classical problem with too few tiles to fill the GPU also takes a
+ * stream-ordered temporary of at most 128 MiB from the library's memory pool
+ * (without it the tiles run whole; the result is the same). Asynchronous on
+ * `stream`. */
 int fmm_gpu_split_dgemm(const fmm_t* fmm, int levels,
                         int64_t m, int64_t n, int64_t k,
                         double alpha, const double* A, int64_t lda,
@@ -250,7 +253,7 @@ int fmm_gpu_split_strassen_ab_gen(double alpha, const double* A, int64_t rs_a, i
                                   fmm_t fmm, int levels, int slices, int format);
 
 /* Frees the current device's buffers kept by fmm_gpu_split_strassen_ab_ex and
- * the temporary memory kept by the plain FP64 form (at most 256 MiB). */
+ * the temporary memory its pool kept (at most 256 MiB). */
 void fmm_gpu_release_host_buffers(void);
 
 /* Pinned host memory for the operands of the host-buffer entry points:
