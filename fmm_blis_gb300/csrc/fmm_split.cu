@@ -2219,7 +2219,7 @@ WsLayout ws_layout_g(const AlgView& alg, const Dims& d, int64_t m, int64_t n, in
     L.group = G;
     L.amax = take(sizeof(unsigned long long) * (size_t)alg.kt * (size_t)m);
     L.bmax = take(sizeof(unsigned long long) * (size_t)alg.kt * (size_t)n);
-    L.sched = take(sizeof(unsigned int));   /* the pair GEMM's work-item counter */
+    L.sched = take(2 * sizeof(unsigned int));   /* work-item counters of GEMM launches in flight together */
     L.erow = take(sizeof(int) * (size_t)G * (size_t)d.m_pad);
     L.fcol = take(sizeof(int) * (size_t)G * (size_t)d.n_pad);
     L.sa = take(esz * (size_t)G * s * (size_t)d.m_pad * (size_t)d.k_pad);
@@ -2464,9 +2464,10 @@ struct SidePool {
     cudaEvent_t wave_sc[2][kWaveStreams];   /* a workspace half's C updates done */
     cudaEvent_t gate[3];   /* host-buffer calls: A, B and C on the device */
     cudaEvent_t chunk[32]; /* host-buffer calls: B chunks in (0..7), C chunks out (8..31) */
-    cudaEvent_t blk[10];   /* host-buffer calls, blocked schedule: A halves up, A and B halves packed, GEMM blocks done */
+    cudaEvent_t blk[16];   /* host-buffer calls, blocked schedule: A halves up, A halves and B parts packed, GEMM blocks done */
     cudaEvent_t tl[kTimelinePoints + 1];  /* host-buffer calls: the call's timeline (timing events) */
     cudaStream_t hi;       /* greatest priority: GEMMs that side work runs beside */
+    cudaStream_t top[3];   /* greatest priority: side work that runs between GEMMs (host-buffer calls) */
 };
 
 std::mutex g_side_mu, g_side_use;
@@ -2485,10 +2486,12 @@ SidePool* side_pool()
     cudaDeviceGetStreamPriorityRange(&least, &greatest);
     bool ok = cudaEventCreateWithFlags(&p->fork, cudaEventDisableTiming) == cudaSuccess &&
               cudaStreamCreateWithPriority(&p->hi, cudaStreamNonBlocking, greatest) == cudaSuccess;
+    for (int i = 0; i < 3 && ok; ++i)
+        ok = cudaStreamCreateWithPriority(&p->top[i], cudaStreamNonBlocking, greatest) == cudaSuccess;
     for (int i = 0; i < 3 && ok; ++i) ok = cudaEventCreateWithFlags(&p->gate[i], cudaEventDisableTiming) == cudaSuccess;
     for (int i = 0; i <= kTimelinePoints && ok; ++i) ok = cudaEventCreate(&p->tl[i]) == cudaSuccess;
     for (int i = 0; i < 32 && ok; ++i) ok = cudaEventCreateWithFlags(&p->chunk[i], cudaEventDisableTiming) == cudaSuccess;
-    for (int i = 0; i < 10 && ok; ++i) ok = cudaEventCreateWithFlags(&p->blk[i], cudaEventDisableTiming) == cudaSuccess;
+    for (int i = 0; i < 16 && ok; ++i) ok = cudaEventCreateWithFlags(&p->blk[i], cudaEventDisableTiming) == cudaSuccess;
     for (int h = 0; h < 2 && ok; ++h) {
         ok = cudaEventCreateWithFlags(&p->wave_gm[h], cudaEventDisableTiming) == cudaSuccess;
         for (int i = 0; i < kWaveStreams && ok; ++i)
@@ -2788,7 +2791,7 @@ static int job_gemm(const SplitJob& j, int np, cudaStream_t st)
  * jt0 * 256 columns), with the same row strides, so each (product, tile)
  * item computes exactly what the full launch computes for it. */
 static int job_gemm_block(const SplitJob& j, int np, int64_t it0, int64_t it1, int64_t jt0, int64_t jt1,
-                          cudaStream_t st)
+                          cudaStream_t st, int slot)
 {
     const bool pair = job_pair(j);
     const int64_t tm = it1 - it0, tn = jt1 - jt0;
@@ -2805,7 +2808,7 @@ static int job_gemm_block(const SplitJob& j, int np, int64_t it0, int64_t it1, i
         const int cnt = std::min(K, np - r);
         memset(&gl, 0, sizeof(gl));
         gl.nprob = 1;
-        gl.sched = (unsigned int*)(j.w + j.L.sched);
+        gl.sched = (unsigned int*)(j.w + j.L.sched) + slot;
         GemmProblem& gp = gl.prob[0];
         if (int rc = job_fill(j, gp, cnt, 0, pair, r); rc != FMM_OK) return rc;
         const uint8_t* sa = j.w + j.L.sa + ((size_t)r * j.s * j.d.m_pad + (size_t)r0) * j.d.k_pad * esz;
@@ -3157,6 +3160,7 @@ static uint8_t* host_buffers(size_t bytes)
 static size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
 constexpr int kChunks = 8;   /* B uploads and C downloads per host-buffer call */
+constexpr size_t kHostSimpleBytes = (size_t)32 << 20;   /* operands up to this size go without the overlapped schedules */
 
 int fmm_split_host(const AlgView& alg, int64_t m, int64_t n, int64_t k, double alpha, const double* A,
                    int64_t lda, const double* B, int64_t ldb, double beta, double* C, int64_t ldc, int s, int fmt)
@@ -3185,12 +3189,53 @@ int fmm_split_host(const AlgView& alg, int64_t m, int64_t n, int64_t k, double a
     const bool tline = g_timeline.load() && !trivial;
     const auto host_t0 = std::chrono::steady_clock::now();
     auto mark = [&](int x, cudaStream_t on) { if (tline) cudaEventRecord(sp->tl[x], on); };
+    auto read_timeline = [&]() {
+        std::lock_guard<std::mutex> lk(g_timeline_mu);
+        for (int x = 1; x <= kTimelinePoints; ++x) {
+            float t = 0.f;
+            cudaEventElapsedTime(&t, sp->tl[0], sp->tl[x]);
+            g_timeline_ms[x - 1] = t;
+        }
+        g_timeline_ms[kTimelinePoints] =
+            std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - host_t0).count();
+    };
     if (trivial) {
         /* C := beta*C */
         if (beta != 0.0 && !ok(fmm_copy2d_async(dC, row, C, sizeof(double) * ldc, row, n, cudaMemcpyHostToDevice, st)))
             return FMM_ERR_CUDA;
         if (int rc = fmm_scale_c(m, n, beta, dC, m, st); rc != FMM_OK) return rc;
     } else {
+        /* Small operands, or many sub-blocks: the device call between plain
+         * copies. Overlapping the copies with the work saves at most their
+         * time (at about 200 bytes per ns), and the blocked schedule's copies,
+         * one per C piece and sub-block, cost about 4 us each: 444 x1 at
+         * 1715 x 1867 x 1620, 16 sub-blocks, 1.9 ms blocked. */
+        const double piece_ns = 4000.0 * ((double)alg.mt * alg.nt * (double)std::min<int64_t>(16, 1 + (m * n * 8 >> 21)) +
+                                          2.0 * alg.mt + 8.0 * alg.nt);
+        if (bA + bB + bC <= kHostSimpleBytes || piece_ns > (double)(bA + bB + bC) / 200.0) {
+            mark(0, st);
+            if (!ok(fmm_copy2d_async(dA, row, A, sizeof(double) * lda, row, k, cudaMemcpyHostToDevice, st)))
+                return FMM_ERR_CUDA;
+            mark(1, st);
+            if (!ok(fmm_copy2d_async(dB, sizeof(double) * k, B, sizeof(double) * ldb, sizeof(double) * k, n,
+                                     cudaMemcpyHostToDevice, st)))
+                return FMM_ERR_CUDA;
+            mark(2, st);
+            if (beta != 0.0 &&
+                !ok(fmm_copy2d_async(dC, row, C, sizeof(double) * ldc, row, n, cudaMemcpyHostToDevice, st)))
+                return FMM_ERR_CUDA;
+            mark(3, st);
+            if (int rc = split_launch_budget(alg, m, n, k, alpha, dA, m, dB, ka, beta, dC, m, s, fmt, ws, wsb, wsb, st,
+                                             sp); rc != FMM_OK)
+                return rc;
+            mark(4, st);
+            if (!ok(fmm_copy2d_async(C, sizeof(double) * ldc, dC, row, row, n, cudaMemcpyDeviceToHost, st)))
+                return FMM_ERR_CUDA;
+            mark(5, st);
+            if (!ok(cudaStreamSynchronize(st))) return FMM_ERR_CUDA;
+            if (tline) read_timeline();
+            return cudaGetLastError() == cudaSuccess ? fmm_device_error_status() : FMM_ERR_CUDA;
+        }
         SplitJob j;
         int rc = job_init(j, alg, m, n, k, alpha, dA, m, dB, ka, beta, dC, m, s, fmt);
         if (rc != FMM_OK) return rc;
@@ -3200,35 +3245,40 @@ int fmm_split_host(const AlgView& alg, int64_t m, int64_t n, int64_t k, double a
         cudaStream_t sb = sp->s[0];
         /* Blocked schedule, for one product group with the element-major C
          * update and a product grid of at least two GEMM tiles along a side:
-         * the grid splits into up to 2 x 2 blocks of tiles (row halves of A,
-         * column halves of B). A's first row half and B's first column half
-         * go up first, so the GEMM of block (0, 0) starts after half of each
-         * operand; A's second half follows, then B's, and the blocks run in
-         * the order (0,0), (1,0), (0,1), (1,1). A block's C elements are final
-         * when its GEMM ends: they are updated (beside the next block's GEMM)
-         * and read back in four column chunks, so after the last GEMM only
-         * the last block's C is left. The work a block's GEMM meets beside
-         * it (the other halves' slices, the earlier blocks' C updates) runs
-         * in the 128-thread forms that fit on an SM beside a GEMM CTA. Every
-         * (product, tile) item and every C element is computed as in the
-         * unblocked call: the same bits. */
+         * the grid splits into up to 2 x 4 blocks of tiles (row halves of A,
+         * column parts of B), column by column. A's first row half and B's
+         * first column part go up first, so the GEMM of block (0, 0) starts
+         * after those; A's second half follows, then B's other parts. A
+         * block's C elements are final when its GEMM ends: they are updated
+         * and read back while later blocks run, so after the last GEMM only
+         * the last block's C is left. Every (product, tile) item and every C
+         * element is computed as in the unblocked call: the same bits. */
         {
             const bool pair = job_pair(j);
             const int64_t me = j.d.me, ne = j.d.ne, m_pad = j.d.m_pad, n_pad = j.d.n_pad;
             const int64_t U = pair ? kPairTileM : kTileM;
             const int64_t tiles_m = m_pad / U, tiles_n = n_pad / kTileN;
-            const int RH = tiles_m >= 2 ? 2 : 1, CH = tiles_n >= 2 ? 2 : 1;
+            const int RH = tiles_m >= 2 ? 2 : 1;
+            /* four column parts where a block still has half a round of items
+             * (two blocks are in flight at a time) */
+            const int CH = tiles_n >= 4 && alg.R * (tiles_m / RH) * (tiles_n / 4) >= (pair ? 38 : 76) ? 4
+                           : tiles_n >= 2 ? 2 : 1;
             int Tchk;
             size_t smchk;
             if (one_group && RH * CH >= 2 && job_scatter_all(j, 0, alg.R, &Tchk, &smchk)) {
                 const int mt = alg.mt;
-                const int64_t tcm[3] = {0, RH == 2 ? (tiles_m + 1) / 2 : tiles_m, tiles_m};
-                const int64_t tcn[3] = {0, CH == 2 ? (tiles_n + 1) / 2 : tiles_n, tiles_n};
-                const int64_t rcut[3] = {0, tcm[1] * U, m_pad};          /* S_r row halves */
-                const int64_t ccut[3] = {0, tcn[1] * kTileN, n_pad};     /* T_r column halves */
-                cudaStream_t ss = sp->s[3], sa = sp->s[4];
+                const int64_t rcut[3] = {0, RH == 2 ? (tiles_m + 1) / 2 * U : m_pad, m_pad};   /* S_r row halves */
+                int64_t ccut[5];                                                               /* T_r column parts */
+                for (int x = 0; x <= CH; ++x) ccut[x] = (tiles_n * x + CH - 1) / CH * kTileN;
+                /* copies per B part and per block's C: pieces of at least 2 MiB
+                 * (a copy and the launches behind it cost about 10 us) */
+                auto pieces = [](int64_t elems, int most) {
+                    return (int)std::min<int64_t>(most, std::max<int64_t>(1, elems * 8 >> 21));
+                };
+                const int bchunks = pieces(k * n / CH, 8 / CH), cchunks = pieces(m * n / (RH * CH), 16 / (RH * CH));
+                const cudaStream_t ss = sp->top[0], sa = sp->top[1], sb = sp->top[2];
                 auto up_a = [&](int h) -> int {
-                    /* the A rows ro_p + [rcut[h], rcut[h+1]) of every row part p, then that half's A side on s[4] */
+                    /* the A rows ro_p + [rcut[h], rcut[h+1]) of every row part p, then that half's A side */
                     if (RH == 1) {
                         if (!ok(fmm_copy2d_async(dA, row, A, sizeof(double) * lda, row, k, cudaMemcpyHostToDevice, cs)))
                             return FMM_ERR_CUDA;
@@ -3248,13 +3298,13 @@ int fmm_split_host(const AlgView& alg, int64_t m, int64_t n, int64_t k, double a
                                                       sizeof(unsigned long long) * (size_t)alg.kt * (size_t)m, sa)))
                         return FMM_ERR_CUDA;
                     job_maxima_a_rows(j, sa, rcut[h], rcut[h + 1]);
-                    job_pack_a_rows(j, 0, alg.R, rcut[h], rcut[h + 1], sa, h == 1);
+                    job_pack_a_rows(j, 0, alg.R, rcut[h], rcut[h + 1], sa);
                     return ok(cudaEventRecord(sp->blk[2 + h], sa)) ? FMM_OK : FMM_ERR_CUDA;
                 };
                 int xb = 0;
                 auto up_b = [&](int h) -> int {
-                    /* the T_r columns [ccut[h], ccut[h+1]) in four chunks, each chunk's B side on s[0] */
-                    const int64_t w = round_up((ccut[h + 1] - ccut[h] + 3) / 4, 32);
+                    /* the T_r columns [ccut[h], ccut[h+1]) in chunks, each chunk's B side behind it */
+                    const int64_t w = round_up((ccut[h + 1] - ccut[h] + bchunks - 1) / bchunks, 32);
                     for (int64_t j0 = ccut[h]; j0 < ccut[h + 1]; j0 += w, ++xb) {
                         const int64_t j1 = std::min(j0 + w, ccut[h + 1]);
                         for (int c = 0; c < nt; ++c) {
@@ -3273,93 +3323,120 @@ int fmm_split_host(const AlgView& alg, int64_t m, int64_t n, int64_t k, double a
                             fmm_part_geom(n, nt, c, &co, &cl);
                             job_maxima_b(j, sb, co + std::min(j0, cl), co + std::min(j1, cl));
                         }
-                        job_pack_b_cols(j, 0, alg.R, j0, j1, sb, h == 1);
+                        job_pack_b_cols(j, 0, alg.R, j0, j1, sb);
                     }
                     return ok(cudaEventRecord(sp->blk[4 + h], sb)) ? FMM_OK : FMM_ERR_CUDA;
                 };
+                const int nq = RH * CH;   /* block q: rows q % RH, columns q / RH */
+                /* GEMM blocks alternate between two streams, each with its
+                 * own item counter: a block's CTAs leave as its items run out
+                 * and the next block's take their place (a block at 4096 with
+                 * one Strassen level is 112 items on 76 CTA pairs). The side
+                 * work has priority, or the GEMMs would keep the SMs from the
+                 * C updates until the last block. */
+                const cudaStream_t gst[2] = {st, sp->s[5]}, ds = sp->s[6];
+                auto gemm = [&](int q) -> int {
+                    const cudaStream_t on = gst[q & 1];
+                    if (!ok(cudaStreamWaitEvent(on, sp->blk[2 + q % RH], 0)) ||
+                        !ok(cudaStreamWaitEvent(on, sp->blk[4 + q / RH], 0)))
+                        return FMM_ERR_CUDA;
+                    if (q == 0) mark(3, on);
+                    if (int e = job_gemm_block(j, alg.R, rcut[q % RH] / U, rcut[q % RH + 1] / U,
+                                               ccut[q / RH] / kTileN, ccut[q / RH + 1] / kTileN, on, q & 1); e != FMM_OK)
+                        return e;
+                    if (q + 1 == nq) mark(4, on);
+                    return ok(cudaEventRecord(sp->blk[8 + q], on)) ? FMM_OK : FMM_ERR_CUDA;
+                };
+                /* a block's C updates in column chunks, each with its event */
+                struct CChunk {
+                    int64_t i0, i1, j0, j1;
+                };
+                CChunk chunks[16];
+                int xc = 0;
+                auto update = [&](int q) -> int {
+                    if (!ok(cudaStreamWaitEvent(ss, sp->blk[8 + q], 0))) return FMM_ERR_CUDA;
+                    const int64_t i0 = rcut[q % RH], i1 = std::min(rcut[q % RH + 1], me);
+                    const int64_t a0 = ccut[q / RH], b0 = std::min(ccut[q / RH + 1], ne);
+                    if (i1 <= i0 || b0 <= a0) return FMM_OK;
+                    const int64_t w = std::max<int64_t>((b0 - a0 + cchunks - 1) / cchunks, 1);
+                    for (int64_t j0 = a0; j0 < b0; j0 += w, ++xc) {
+                        chunks[xc] = CChunk{i0, i1, j0, std::min(j0 + w, b0)};
+                        job_scatter_block(j, 0, alg.R, i0, i1, j0, chunks[xc].j1, ss);
+                        if (!ok(cudaEventRecord(sp->chunk[8 + xc], ss))) return FMM_ERR_CUDA;
+                    }
+                    return FMM_OK;
+                };
+                /* a block's C elements up, for its updates */
+                auto up_c = [&](int q) -> int {
+                    if (beta == 0.0) return FMM_OK;
+                    for (int p = 0; p < mt; ++p) {
+                        int64_t ro, rl;
+                        fmm_part_geom(m, mt, p, &ro, &rl);
+                        const int64_t ra = ro + std::min(rcut[q % RH], rl), rb = ro + std::min(rcut[q % RH + 1], rl);
+                        if (rb <= ra) continue;
+                        for (int y = 0; y < nt; ++y) {
+                            int64_t co, cl;
+                            fmm_part_geom(n, nt, y, &co, &cl);
+                            const int64_t ca = co + std::min(ccut[q / RH], cl), cb = co + std::min(ccut[q / RH + 1], cl);
+                            if (cb > ca &&
+                                !ok(fmm_copy2d_async(dC + ra + ca * m, row, C + ra + ca * ldc, sizeof(double) * ldc,
+                                                     sizeof(double) * (rb - ra), cb - ca, cudaMemcpyHostToDevice, cs)))
+                                return FMM_ERR_CUDA;
+                        }
+                    }
+                    return ok(cudaEventRecord(sp->chunk[24 + q], cs)) &&
+                                   ok(cudaStreamWaitEvent(ss, sp->chunk[24 + q], 0))
+                               ? FMM_OK : FMM_ERR_CUDA;
+                };
+                /* Everything in the order it is needed: what a block's GEMM
+                 * waits for, the GEMM, then C for the blocks under way (its
+                 * copy and the updates fit under the GEMMs; C last of all
+                 * would hold the first update until 3/4 of the call's time).
+                 * Streams that share a hardware queue run in enqueue order. */
                 mark(0, cs);
                 if ((rc = up_a(0)) != FMM_OK) return rc;
                 if (RH == 1) mark(1, cs);
-                if ((rc = up_b(0)) != FMM_OK) return rc;
-                if (RH == 2) {
-                    if ((rc = up_a(1)) != FMM_OK) return rc;
-                    mark(1, cs);
-                }
-                if (CH == 2 && (rc = up_b(1)) != FMM_OK) return rc;
-                mark(2, cs);
-                /* C up behind A and B, for the C updates on s[3] */
-                if (beta != 0.0 &&
-                    (!ok(fmm_copy2d_async(dC, row, C, sizeof(double) * ldc, row, n, cudaMemcpyHostToDevice, cs)) ||
-                     !ok(cudaEventRecord(sp->gate[2], cs)) || !ok(cudaStreamWaitEvent(ss, sp->gate[2], 0))))
-                    return FMM_ERR_CUDA;
-                /* the GEMM blocks on the call's stream */
-                const int order[4][2] = {{0, 0}, {1, 0}, {0, 1}, {1, 1}};
-                int nq = 0;
-                int qr[4], qc[4];
-                for (const auto& o : order)
-                    if (o[0] < RH && o[1] < CH) {
-                        qr[nq] = o[0];
-                        qc[nq] = o[1];
-                        ++nq;
+                int c_next = 0;   /* the next block whose C goes up */
+                for (int x = 0; x < CH; ++x) {
+                    if ((rc = up_b(x)) != FMM_OK) return rc;
+                    if (x + 1 == CH) mark(2, cs);
+                    if ((rc = gemm(x * RH)) != FMM_OK) return rc;
+                    if (RH == 2) {
+                        if (x == 0) {
+                            if ((rc = up_a(1)) != FMM_OK) return rc;
+                            mark(1, cs);
+                        }
+                        if ((rc = gemm(x * RH + 1)) != FMM_OK) return rc;
                     }
-                for (int q = 0; q < nq; ++q) {
-                    if (!ok(cudaStreamWaitEvent(st, sp->blk[2 + qr[q]], 0)) ||
-                        !ok(cudaStreamWaitEvent(st, sp->blk[4 + qc[q]], 0)))
-                        return FMM_ERR_CUDA;
-                    if (q == 0) mark(3, st);
-                    if ((rc = job_gemm_block(j, alg.R, tcm[qr[q]], tcm[qr[q] + 1], tcn[qc[q]], tcn[qc[q] + 1], st)) !=
-                        FMM_OK)
-                        return rc;
-                    if (!ok(cudaEventRecord(sp->blk[6 + q], st))) return FMM_ERR_CUDA;
+                    for (; c_next < (x + 1 == CH ? nq : x * RH + 1); ++c_next)
+                        if ((rc = up_c(c_next)) != FMM_OK || (rc = update(c_next)) != FMM_OK) return rc;
                 }
-                mark(4, st);
-                /* each block's C updates on s[3] in four column chunks, each
-                 * chunk's C elements read back on s[1] */
-                int xc = 0;
-                for (int q = 0; q < nq; ++q) {
-                    if (!ok(cudaStreamWaitEvent(ss, sp->blk[6 + q], 0))) return FMM_ERR_CUDA;
-                    const int64_t i0 = rcut[qr[q]], i1 = std::min(rcut[qr[q] + 1], me);
-                    const int64_t a0 = ccut[qc[q]], b0 = std::min(ccut[qc[q] + 1], ne);
-                    if (i1 <= i0 || b0 <= a0) continue;
-                    const int64_t w = std::max<int64_t>((b0 - a0 + 3) / 4, 1);
-                    for (int64_t j0 = a0; j0 < b0; j0 += w, ++xc) {
-                        const int64_t j1 = std::min(j0 + w, b0);
-                        job_scatter_block(j, 0, alg.R, i0, i1, j0, j1, ss, q + 1 < nq);
-                        if (!ok(cudaEventRecord(sp->chunk[8 + xc], ss)) ||
-                            !ok(cudaStreamWaitEvent(cs, sp->chunk[8 + xc], 0)))
-                            return FMM_ERR_CUDA;
-                        for (int p = 0; p < mt; ++p) {
-                            int64_t ro, rl;
-                            fmm_part_geom(m, mt, p, &ro, &rl);
-                            const int64_t ra = ro + std::min(i0, rl), rb = ro + std::min(i1, rl);
-                            if (rb <= ra) continue;
-                            for (int c = 0; c < nt; ++c) {
-                                int64_t co, cl;
-                                fmm_part_geom(n, nt, c, &co, &cl);
-                                const int64_t ca = co + std::min(j0, cl), cb = co + std::min(j1, cl);
-                                if (cb > ca &&
-                                    !ok(fmm_copy2d_async(C + ra + ca * ldc, sizeof(double) * ldc, dC + ra + ca * m, row,
-                                                          sizeof(double) * (rb - ra), cb - ca, cudaMemcpyDeviceToHost,
-                                                          cs)))
-                                    return FMM_ERR_CUDA;
-                            }
+                /* each chunk's C elements back on s[6], beside the uploads (enqueued
+                 * last: a copy to pageable memory holds the host) */
+                for (int x = 0; x < xc; ++x) {
+                    const CChunk& c = chunks[x];
+                    if (!ok(cudaStreamWaitEvent(ds, sp->chunk[8 + x], 0))) return FMM_ERR_CUDA;
+                    for (int p = 0; p < mt; ++p) {
+                        int64_t ro, rl;
+                        fmm_part_geom(m, mt, p, &ro, &rl);
+                        const int64_t ra = ro + std::min(c.i0, rl), rb = ro + std::min(c.i1, rl);
+                        if (rb <= ra) continue;
+                        for (int y = 0; y < nt; ++y) {
+                            int64_t co, cl;
+                            fmm_part_geom(n, nt, y, &co, &cl);
+                            const int64_t ca = co + std::min(c.j0, cl), cb = co + std::min(c.j1, cl);
+                            if (cb > ca &&
+                                !ok(fmm_copy2d_async(C + ra + ca * ldc, sizeof(double) * ldc, dC + ra + ca * m, row,
+                                                     sizeof(double) * (rb - ra), cb - ca, cudaMemcpyDeviceToHost, ds)))
+                                return FMM_ERR_CUDA;
                         }
                     }
                 }
-                mark(5, cs);
-                if (!ok(cudaStreamSynchronize(cs)) || !ok(cudaStreamSynchronize(st)) ||
-                    !ok(cudaStreamSynchronize(ss)) || !ok(cudaStreamSynchronize(sa)) || !ok(cudaStreamSynchronize(sb)))
+                mark(5, ds);
+                if (!ok(cudaStreamSynchronize(ds)) || !ok(cudaStreamSynchronize(cs)) || !ok(cudaStreamSynchronize(gst[0])) ||
+                    !ok(cudaStreamSynchronize(gst[1])) || !ok(cudaStreamSynchronize(ss)) || !ok(cudaStreamSynchronize(sa)) || !ok(cudaStreamSynchronize(sb)))
                     return FMM_ERR_CUDA;
-                if (tline) {
-                    std::lock_guard<std::mutex> lk(g_timeline_mu);
-                    for (int y = 1; y <= kTimelinePoints; ++y) {
-                        float t = 0.f;
-                        cudaEventElapsedTime(&t, sp->tl[0], sp->tl[y]);
-                        g_timeline_ms[y - 1] = t;
-                    }
-                    g_timeline_ms[kTimelinePoints] =
-                        std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - host_t0).count();
-                }
+                if (tline) read_timeline();
                 return cudaGetLastError() == cudaSuccess ? fmm_device_error_status() : FMM_ERR_CUDA;
             }
         }
@@ -3446,16 +3523,7 @@ int fmm_split_host(const AlgView& alg, int64_t m, int64_t n, int64_t k, double a
             if (!ok(cudaEventRecord(sp->gate[1], cs)) || !ok(cudaStreamSynchronize(cs)) ||
                 !ok(cudaStreamSynchronize(st)))
                 return FMM_ERR_CUDA;
-            if (tline) {
-                std::lock_guard<std::mutex> lk(g_timeline_mu);
-                for (int x = 1; x <= kTimelinePoints; ++x) {
-                    float t = 0.f;
-                    cudaEventElapsedTime(&t, sp->tl[0], sp->tl[x]);
-                    g_timeline_ms[x - 1] = t;
-                }
-                g_timeline_ms[kTimelinePoints] =
-                    std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - host_t0).count();
-            }
+            if (tline) read_timeline();
             return cudaGetLastError() == cudaSuccess ? fmm_device_error_status() : FMM_ERR_CUDA;
         }
     }
