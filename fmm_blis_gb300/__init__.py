@@ -285,8 +285,20 @@ def set_split_pair_rows(min_rows: int) -> int:
 
 # ------------------------------------------------------------ GPU calls --
 
+_torch = None
+
+
+def _get_torch():
+    """the torch module (the package itself imports without it)"""
+    global _torch
+    if _torch is None:
+        import torch
+        _torch = torch
+    return _torch
+
+
 def _colmajor_ld(t, rows: int, name: str) -> int:
-    if t.dtype.__str__() != "torch.float64":
+    if t.dtype is not (_torch or _get_torch()).float64:
         raise TypeError(f"{name} must be float64")
     if not t.is_cuda:
         raise TypeError(f"{name} must be a CUDA tensor")
@@ -306,7 +318,10 @@ def colmajor(t):
 
 def _stream_ptr(stream) -> int | None:
     if stream is None:
-        import torch
+        torch = _torch or _get_torch()
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        if raw is not None and torch.cuda.is_initialized():
+            return raw(torch._C._cuda_getDevice())   # a tenth of current_stream()'s time
         return torch.cuda.current_stream().cuda_stream
     return int(getattr(stream, "cuda_stream", stream))
 

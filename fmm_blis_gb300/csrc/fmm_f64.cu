@@ -554,6 +554,157 @@ fmm_f64_pipe_kernel(const int* __restrict__ tab, int64_t m, int64_t n, int64_t k
     }
 }
 
+/* --------------------------------------------- small FMM problems ---- */
+
+/* A whole small FMM GEMM in one launch: a CTA owns an 8 x 8 tile position, its
+ * groups of 64 threads (one element each) take the products in turn, packs
+ * fused in with the terms' loads one k step ahead, and leave each M_r in shared
+ * memory; then every C sub-block's element gets beta*C and the products in
+ * increasing order. The values and orders are the general path's (the same
+ * bits). Bound by latency: a product's k sum is one chain of dependent DFMAs
+ * per element (about 120 clocks each), so the products run side by side, and
+ * the general path's two packing launches, its C scaling and its temporary
+ * cost more than the whole problem. 222 x1 at 97 x 61 x 45: 28.7 us general. */
+constexpr int kSmallTile = 8, kSmallBk = 16, kSmallGroup = kSmallTile * kSmallTile, kSmallGroups = 8;
+constexpr int kSmallMaxR = 64;
+constexpr int kSmallA = kSmallBk * kSmallTile, kSmallB = kSmallBk * (kSmallTile + 1);   /* one operand tile, doubles */
+constexpr int kSmallTerms = 4;   /* terms in flight together */
+
+/* shared memory: operand tiles (two per group), M_r, entries */
+size_t small_smem(int R, int nu, int nv)
+{
+    const int G = std::min(R, kSmallGroups);
+    return sizeof(double) * ((size_t)2 * G * (kSmallA + kSmallB) + (size_t)R * kSmallGroup) +
+           sizeof(Entry) * (size_t)(nu + nv);
+}
+
+/* this thread's two elements of the terms [x0, x0 + kSmallTerms) of a
+ * combination at (i, j) and (i + di, j + dj) of its sub-blocks */
+struct SmallTerms {
+    double v[kSmallTerms][2];
+
+    __device__ __forceinline__ void load(const Entry* e, int n, int64_t i, int64_t j, int64_t di, int64_t dj, int64_t ld)
+    {
+#pragma unroll
+        for (int x = 0; x < kSmallTerms; ++x)
+            if (x < n) {
+#pragma unroll
+                for (int t = 0; t < 2; ++t) {
+                    const int64_t a = i + t * di, b = j + t * dj;
+                    v[x][t] = a < e[x].rows && b < e[x].cols ? e[x].base[a + b * ld] : 0.0;
+                }
+            }
+    }
+    /* s (+)= the terms, in order; the first one by its kind */
+    __device__ __forceinline__ void sum(const Entry* e, int n, bool first, double (&s)[2]) const
+    {
+#pragma unroll
+        for (int x = 0; x < kSmallTerms; ++x)
+            if (x < n) {
+                if (x == 0 && first) {
+                    s[0] = v[0][0];
+                    s[1] = v[0][1];
+                    scale_first(e[0], s);
+                } else {
+                    s[0] = fma(e[x].coef, v[x][0], s[0]);
+                    s[1] = fma(e[x].coef, v[x][1], s[1]);
+                }
+            }
+    }
+    /* the whole combination, its first terms already loaded */
+    __device__ __forceinline__ void combine(const Entry* e, int n, int64_t i, int64_t j, int64_t di, int64_t dj,
+                                            int64_t ld, double (&s)[2])
+    {
+        s[0] = s[1] = 0.0;
+        sum(e, n, true, s);
+        for (int x = kSmallTerms; x < n; x += kSmallTerms) {
+            load(e + x, n - x, i, j, di, dj, ld);
+            sum(e + x, n - x, false, s);
+        }
+    }
+};
+
+__global__ void __launch_bounds__(kSmallGroup * kSmallGroups)
+fmm_f64_small_kernel(const int* __restrict__ tab, int64_t m, int64_t n, int64_t k, double alpha,
+                     const double* __restrict__ A, int64_t lda, const double* __restrict__ B, int64_t ldb, double beta,
+                     double* __restrict__ C, int64_t ldc, int tiles_m)
+{
+    extern __shared__ double f64_stages[];
+    const int mt = tab[0], kt = tab[1], nt = tab[2], R = tab[3];
+    const int* u_off = tab + FMM_ALG_HDR;
+    const int* v_off = u_off + (R + 1);
+    const int* w_off = v_off + (R + 1);
+    const int* u_ent = w_off + (R + 1);
+    const int nu = u_off[R], nv = v_off[R], nw = w_off[R];
+    const int* v_ent = u_ent + 2 * nu;
+    const int* wp_off = v_ent + 2 * nv + 2 * nw;
+    const int* wp_ent = wp_off + (mt * nt + 1);
+    const int G = (int)blockDim.x / kSmallGroup, g = (int)threadIdx.x / kSmallGroup, tid = (int)threadIdx.x % kSmallGroup;
+    double* tiles = f64_stages + (size_t)g * 2 * (kSmallA + kSmallB);                  /* [2][A, B] */
+    double* M = f64_stages + (size_t)G * 2 * (kSmallA + kSmallB);                      /* [R][64] */
+    Entry* ue = (Entry*)(M + (size_t)R * kSmallGroup);
+    Entry* ve = ue + nu;
+    stage_entries(u_ent, 0, nu, kt, mt, A, lda, m, k, ue);
+    stage_entries(v_ent, 0, nv, nt, kt, B, ldb, k, n, ve);
+    __syncthreads();
+    const int64_t ke = (k + kt - 1) / kt;
+    const int64_t i0 = (int64_t)(blockIdx.x % (unsigned)tiles_m) * kSmallTile;
+    const int64_t j0 = (int64_t)(blockIdx.x / (unsigned)tiles_m) * kSmallTile;
+    const int tr = tid % kSmallTile, tc = tid / kSmallTile;   /* the thread's element, and its A copies (row, k) */
+    const int bk = tid % kSmallBk, bj = tid / kSmallBk;       /* its B copies: k, columns bj and bj + 4 */
+    SmallTerms ta, tb;
+    auto fetch = [&](int r, int64_t k0) {
+        ta.load(ue + u_off[r], u_off[r + 1] - u_off[r], i0 + tr, k0 + tc, 0, 8, lda);
+        tb.load(ve + v_off[r], v_off[r + 1] - v_off[r], k0 + bk, j0 + bj, 0, 4, ldb);
+    };
+    auto put = [&](int r, int64_t k0, double* t) {
+        double s[2];
+        ta.combine(ue + u_off[r], u_off[r + 1] - u_off[r], i0 + tr, k0 + tc, 0, 8, lda, s);
+        t[tc * kSmallTile + tr] = s[0];
+        t[(tc + 8) * kSmallTile + tr] = s[1];
+        tb.combine(ve + v_off[r], v_off[r + 1] - v_off[r], k0 + bk, j0 + bj, 0, 4, ldb, s);
+        t[kSmallA + bk * (kSmallTile + 1) + bj] = s[0];
+        t[kSmallA + bk * (kSmallTile + 1) + bj + 4] = s[1];
+    };
+    auto group_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(g + 1) : "memory"); };
+    int buf = 0;
+    if (g < R) {
+        fetch(g, 0);
+        put(g, 0, tiles);
+    }
+    for (int r = g; r < R; r += G) {
+        double acc = 0.0;
+        for (int64_t k0 = 0; k0 < ke; k0 += kSmallBk) {
+            group_sync();   /* the step's tile is in, the other one read out */
+            const bool last = k0 + kSmallBk >= ke;
+            const int rn = last ? r + G : r;
+            const int64_t kn = last ? 0 : k0 + kSmallBk;
+            if (rn < R) fetch(rn, kn);
+            const double* t = tiles + buf * (kSmallA + kSmallB);
+            const int kc = (int)(ke - k0 < kSmallBk ? ke - k0 : kSmallBk);
+#pragma unroll 4
+            for (int kk = 0; kk < kc; ++kk)
+                acc = fma(t[kk * kSmallTile + tr], t[kSmallA + kk * (kSmallTile + 1) + tc], acc);
+            buf ^= 1;
+            if (rn < R) put(rn, kn, tiles + buf * (kSmallA + kSmallB));
+        }
+        M[r * kSmallGroup + tid] = acc;
+    }
+    __syncthreads();
+    /* the C sub-blocks, shared out over the groups */
+    for (int p = g; p < mt * nt; p += G) {
+        int64_t ro, rl, co, cl;
+        fmm_part_geom(m, mt, p / nt, &ro, &rl);
+        fmm_part_geom(n, nt, p % nt, &co, &cl);
+        if (i0 + tr >= rl || j0 + tc >= cl) continue;
+        double* cp = C + ro + i0 + tr + (co + j0 + tc) * ldc;
+        double c = beta == 1.0 ? *cp : (beta == 0.0 ? 0.0 : beta * *cp);
+        for (int e = wp_off[p]; e < wp_off[p + 1]; ++e)
+            c = fma(alpha * (double)wp_ent[2 * e + 1], M[wp_ent[2 * e] * kSmallGroup + tid], c);
+        *cp = c;
+    }
+}
+
 /* ------------------------------------------------------------ batched -- */
 
 /* One problem of a batched FP64 launch; problems are laid out in the order
@@ -1006,6 +1157,48 @@ int fmm_scale_c(int64_t m, int64_t n, double beta, double* C, int64_t ldc, cudaS
     return cudaGetLastError() == cudaSuccess ? FMM_OK : FMM_ERR_CUDA;
 }
 
+namespace {
+
+/* Whether a problem runs as fmm_f64_small_kernel: its busiest SM's FP64 work
+ * (8 x 8 tiles, the packs adding about a quarter) within 50000 clocks, about
+ * where the general path's fewer DFMAs make up for its launches (256^3 222 x1
+ * is just past it), and the shared memory it needs. */
+bool small_fmm(const AlgView& alg, int64_t me, int64_t ne, int64_t ke, int sms, size_t* smem)
+{
+    if (alg.R < 2 || alg.R > kSmallMaxR || alg.htab == nullptr) return false;
+    const int* u_off = alg.htab + FMM_ALG_HDR;
+    const int nu = u_off[alg.R], nv = u_off[alg.R + 1 + alg.R];
+    if (nu > kMaxEntries || nv > kMaxEntries) return false;
+    const int64_t tiles = ((me + kSmallTile - 1) / kSmallTile) * ((ne + kSmallTile - 1) / kSmallTile);
+    if (tiles > (int64_t)64 * sms) return false;
+    const double clocks = (double)((tiles + sms - 1) / sms) * kSmallGroup * alg.R * (double)ke * 1.25 / 2.0;
+    *smem = small_smem(alg.R, nu, nv);
+    return clocks <= 50000.0 && *smem <= (size_t)100 * 1024;
+}
+
+int launch_small(const AlgView& alg, int64_t m, int64_t n, int64_t k, double alpha, const double* A, int64_t lda,
+                 const double* B, int64_t ldb, double beta, double* C, int64_t ldc, size_t smem, cudaStream_t st)
+{
+    static std::atomic<uint64_t> attr_set{0};   /* a per-device attribute of the kernel: set once per device */
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return FMM_ERR_CUDA;
+    const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+    if (bit == 0 || !(attr_set.load(std::memory_order_acquire) & bit)) {
+        if (cudaFuncSetAttribute(fmm_f64_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024) !=
+            cudaSuccess)
+            return FMM_ERR_CUDA;
+        attr_set.fetch_or(bit, std::memory_order_acq_rel);
+    }
+    const int64_t me = (m + alg.mt - 1) / alg.mt, ne = (n + alg.nt - 1) / alg.nt;
+    const int64_t tm = (me + kSmallTile - 1) / kSmallTile, tn = (ne + kSmallTile - 1) / kSmallTile;
+    fmm_f64_small_kernel<<<(unsigned)(tm * tn), kSmallGroup * std::min(alg.R, kSmallGroups), smem, st>>>(
+        alg.tab, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, (int)tm);
+    fmm_count_launch(1);
+    return cudaGetLastError() == cudaSuccess ? FMM_OK : FMM_ERR_CUDA;
+}
+
+}  // namespace
+
 void fmm_f64_release_temp()
 {
     int dev = 0;
@@ -1018,21 +1211,24 @@ int fmm_f64_launch(const AlgView& alg, int64_t m, int64_t n, int64_t k, double a
                    const double* A, int64_t lda, const double* B, int64_t ldb,
                    double beta, double* C, int64_t ldc, cudaStream_t st)
 {
-    int rc = fmm_scale_c(m, n, beta, C, ldc, st);
-    if (rc != FMM_OK) return rc;
-    if (m == 0 || n == 0 || k == 0 || alpha == 0.0) return FMM_OK;
+    if (m == 0 || n == 0 || k == 0 || alpha == 0.0) return fmm_scale_c(m, n, beta, C, ldc, st);
     if (alg.max_nnz_u > kMaxEntries || alg.max_nnz_v > kMaxEntries) return FMM_ERR_UNSUPPORTED;
 
-    const bool classical = fmm_plain_classical(alg);
-    if (classical) {
-        const int ks = fmm_gpu_f64_sup_splits(m, n, k);
-        if (ks >= 2) return sup_launch(m, n, k, alpha, A, lda, B, ldb, C, ldc, ks, st);
-    }
     const bool mma = g_f64_engine.load(std::memory_order_relaxed) == FMM_F64_MMA;
     int dev = 0, sms = 152;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int64_t me = (m + alg.mt - 1) / alg.mt, ne = (n + alg.nt - 1) / alg.nt, ke = (k + alg.kt - 1) / alg.kt;
+    size_t smem = 0;
+    if (!mma && small_fmm(alg, me, ne, ke, sms, &smem))
+        return launch_small(alg, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, smem, st);
+    int rc = fmm_scale_c(m, n, beta, C, ldc, st);
+    if (rc != FMM_OK) return rc;
+    const bool classical = fmm_plain_classical(alg);
+    if (classical) {
+        const int ks = fmm_gpu_f64_sup_splits(m, n, k);
+        if (ks >= 2) return sup_launch(m, n, k, alpha, A, lda, B, ldb, C, ldc, ks, st);
+    }
     /* FMM algorithms form each product's operand combinations once, ahead of
      * the tiles (a stream-ordered temporary of at most kPrepackBudget per
      * product group), instead of once per tile position inside the kernel;

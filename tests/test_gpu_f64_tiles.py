@@ -1,5 +1,6 @@
 """The plain FP64 form's tiles at their edges: every pipelined tile (64 x 64,
-16 x 8, 8 x 8 by the size of the product grid), k below, at and past a copy
+16 x 8, 8 x 8 by the size of the product grid), the one-launch small FMM
+problems, k below, at and past a copy
 step and the stages of the ring, sub-arrays with odd leading dimensions, the
 cluster path's two tiles; against the oracle within the FP64 bound, and the
 batched call (64, 32 and 16 wide items) bit for bit against the single calls."""
@@ -33,6 +34,8 @@ def sub(x, pad):
     (500, 520, 63, None, 0), (1300, 1290, 64, None, 0), (2049, 700, 65, None, 0), (5000, 9, 31, None, 0),
     (40, 3000, 100, None, 0), (300, 299, 301, "222", 1), (700, 640, 33, "333", 1), (1100, 1030, 128, "222", 1),
     (257, 258, 130, "444", 1), (260, 200, 190, "232", 2), (50, 60, 3, "322", 1),
+    (97, 61, 45, "222", 1), (3, 13, 7, "222", 1), (16, 16, 32, "222", 1), (17, 200, 35, "333", 1),
+    (100, 90, 81, "444", 1), (130, 120, 150, "322", 1), (40, 44, 130, "222", 2),
     (128, 128, 4096, None, 0), (65, 7, 2050, None, 0), (257, 129, 1300, None, 0), (310, 320, 900, None, 0)])
 @pytest.mark.parametrize("alpha,beta,pad", [(1.0, 1.0, 0), (-0.5, 0.0, 3), (2.0, 0.25, 8)])
 def test_tiles_match_oracle(fmm, orc, algs, torch_cuda, m, n, k, alg, levels, alpha, beta, pad):
