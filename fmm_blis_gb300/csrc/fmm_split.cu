@@ -872,6 +872,7 @@ prep_kernel(const double* __restrict__ A, int64_t lda, const double* __restrict_
             unsigned int* __restrict__ sched, int nrank)
 {
     __shared__ PrepShared sh;
+    sm103::grid_launch_dependents();
     const int64_t c = blockIdx.x / (unsigned)nrank, ca = m_pad / kPrepLines;
     const int rank = (int)(blockIdx.x % (unsigned)nrank);
     if (blockIdx.x == 0 && threadIdx.x == 0) *sched = 0;   /* the GEMM's work-item counter */
@@ -944,14 +945,19 @@ struct GemmProblem {
 constexpr int kMaxLaunchProblems = 80;
 
 /* Everything a launch needs, passed by value (tensor maps included), so a
- * launch copies nothing to the device and can be captured in a graph. */
-struct GemmLaunch {
+ * launch copies nothing to the device and can be captured in a graph. Single
+ * calls launch kernels of their own with room for one problem: 32 KB of
+ * parameters cost a launch several microseconds. */
+template <int N>
+struct GemmLaunchOf {
     int nprob;
     int nitems;           /* sum over problems of products * tiles */
     int* err;
-    unsigned int* sched;  /* pair kernel: next work item, zero at launch */
-    GemmProblem prob[kMaxLaunchProblems];
+    unsigned int* sched;  /* next work item, zero at launch */
+    GemmProblem prob[N];
 };
+using GemmLaunch = GemmLaunchOf<kMaxLaunchProblems>;
+using GemmLaunch1 = GemmLaunchOf<1>;
 static_assert(sizeof(GemmLaunch) <= 32764, "GemmLaunch must fit the kernel parameter space");
 
 __host__ __device__ __forceinline__ int level_pairs(int g, int s)
@@ -1001,7 +1007,8 @@ struct Item {
     int p, r, tile_m, tile_n, unit;
 };
 
-__device__ __forceinline__ Item decode_item(const GemmLaunch& L, int b, int raster = kRasterGroup)
+template <class GL>
+__device__ __forceinline__ Item decode_item(const GL& L, int b, int raster = kRasterGroup)
 {
     int p = 0, hi = L.nprob - 1;        /* last problem with item_begin <= b */
     while (p < hi) {
@@ -1129,8 +1136,8 @@ __device__ __forceinline__ int opaque(int x)
  * every chunk of every level, levels s+1 .. 2. zh is the address of Z row zi
  * in the high plane of the thread's first column group. `arrive(buf)` reports
  * a TMEM buffer read. */
-template <class Arrive>
-__device__ __forceinline__ bool drain_item(const GemmLaunch& L, int p, uint8_t* zh, int zi, uint32_t tl, uint64_t* accf,
+template <class GL, class Arrive>
+__device__ __forceinline__ bool drain_item(const GL& L, int p, uint8_t* zh, int zi, uint32_t tl, uint64_t* accf,
                                            int& buf, uint32_t& aph, int lane, volatile int* abort_flag, int code,
                                            Arrive arrive)
 {
@@ -1202,8 +1209,8 @@ __device__ __forceinline__ bool drain_item(const GemmLaunch& L, int p, uint8_t* 
 
 /* drain_item for a work unit: its chunks' sums, stored as they are. zp: the
  * thread's row in the unit's plane of its first column group. */
-template <class Arrive>
-__device__ __forceinline__ bool drain_unit(const GemmLaunch& L, int4* zp, int64_t gstep, int nkb_unit, uint32_t tl,
+template <class GL, class Arrive>
+__device__ __forceinline__ bool drain_unit(const GL& L, int4* zp, int64_t gstep, int nkb_unit, uint32_t tl,
                                            uint64_t* accf, int& buf, uint32_t& aph, int lane,
                                            volatile int* abort_flag, int code, Arrive arrive)
 {
@@ -1247,8 +1254,9 @@ __device__ __forceinline__ bool drain_unit(const GemmLaunch& L, int4* zp, int64_
  * digits of Z that a finished level settles (drain_item). The pipeline, TMEM
  * allocation and barrier phases run on across items, so one item's last
  * stores overlap the next item's first MMAs. */
+template <class GL>
 __global__ void __launch_bounds__(kGemmThreads, 1)
-split_gemm_kernel(const __grid_constant__ GemmLaunch L)
+split_gemm_kernel(const __grid_constant__ GL L)
 {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -1284,6 +1292,8 @@ split_gemm_kernel(const __grid_constant__ GemmLaunch L)
     sm103::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
+    sm103::grid_launch_dependents();
+    sm103::grid_wait();   /* the slices, L.sched and (a reused) Z are the launches' before this one */
     if (warp == 0) {
         /* ---------------- TMA producer ---------------- */
         if (lane == 0) {
@@ -1481,8 +1491,9 @@ constexpr size_t kPairSmem = (size_t)kPairStages * kPairStageBytes + 1024 + 512;
  * as in split_gemm_kernel and reports the buffer free to the even CTA. All
  * waits are bounded; the two cluster barriers (after barrier set-up, before
  * TMEM release) are reached by every thread of both CTAs. */
+template <class GL>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
-split_gemm_pair_kernel(const __grid_constant__ GemmLaunch L)
+split_gemm_pair_kernel(const __grid_constant__ GL L)
 {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -1945,6 +1956,7 @@ scatter_units_kernel(int m, int n, double alpha, double beta, const int4* __rest
                      const int* __restrict__ f_col, double* __restrict__ C, int64_t ldc)
 {
     const int i = (int)blockIdx.x * 32 + (int)threadIdx.x % 32, j = ((int)blockIdx.y * 4 + (int)threadIdx.x / 32) * 4;
+    sm103::grid_wait();
     if (i >= m || j >= n) return;
     double* cp = C + i + (int64_t)j * ldc;
     double c[kScatterCols];
@@ -2753,8 +2765,9 @@ static int64_t job_items(const SplitJob& j, int np, bool pair = false)
     return (int64_t)np * (j.d.m_pad / (pair ? kPairTileM : kTileM)) * (j.d.n_pad / kTileN);
 }
 
-static int launch_gemm(GemmLaunch& gl, int64_t nitems, int nprod_timed, cudaStream_t st, bool pair,
-                       bool sched_zeroed = false);
+template <class GL>
+static int launch_gemm(GL& gl, int64_t nitems, int nprod_timed, cudaStream_t st, bool pair,
+                       bool after_prep = false);
 
 /* The GEMM of the job's current product group, as back-to-back launches of
  * at most K products, K the fewest products that give each launch about 24
@@ -2773,7 +2786,7 @@ static int job_gemm(const SplitJob& j, int np, cudaStream_t st)
     int K = (int)std::min<int64_t>(np, std::max<int64_t>(1, (24 * units + tiles - 1) / tiles));
     const int nl = (np + K - 1) / K;
     K = (np + nl - 1) / nl;
-    GemmLaunch gl;
+    GemmLaunch1 gl;
     for (int r = 0; r < np; r += K) {
         const int cnt = std::min(K, np - r);
         memset(&gl, 0, sizeof(gl));
@@ -2803,7 +2816,7 @@ static int job_gemm_block(const SplitJob& j, int np, int64_t it0, int64_t it1, i
     K = (np + nl - 1) / nl;
     const size_t esz = j.fmt ? 1 : 2;
     const int64_t r0 = it0 * (pair ? kPairTileM : kTileM), c0 = jt0 * kTileN;
-    GemmLaunch gl;
+    GemmLaunch1 gl;
     for (int r = 0; r < np; r += K) {
         const int cnt = std::min(K, np - r);
         memset(&gl, 0, sizeof(gl));
@@ -2896,25 +2909,53 @@ static void job_scatter(const SplitJob& j, int r0, int np, cudaStream_t st, bool
     fmm_count_launch(1);
 }
 
-static int launch_gemm(GemmLaunch& gl, int64_t nitems, int nprod_timed, cudaStream_t st, bool pair, bool sched_zeroed)
+/* dynamic shared memory limits of this file's kernels: per-device attributes, set once per device */
+static int kernel_attributes(int dev)
 {
-    /* the kernels' shared-memory limit is a per-device attribute: set once per device */
     static std::atomic<uint64_t> attr_set{0};
+    const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+    if (bit != 0 && (attr_set.load(std::memory_order_acquire) & bit)) return FMM_OK;
+    auto limit = [](const void* f, size_t bytes) {
+        return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
+    };
+    if (!limit((const void*)split_gemm_kernel<GemmLaunch>, kGemmSmem) ||
+        !limit((const void*)split_gemm_kernel<GemmLaunch1>, kGemmSmem) ||
+        !limit((const void*)split_gemm_pair_kernel<GemmLaunch>, kPairSmem) ||
+        !limit((const void*)split_gemm_pair_kernel<GemmLaunch1>, kPairSmem) ||
+        !limit((const void*)scatter_all_kernel<0>, kScatterAllMaxSmem) ||
+        !limit((const void*)scatter_all_kernel<1>, kScatterAllMaxSmem) ||
+        !limit((const void*)wave_scatter_kernel, kScatterAllMaxSmem))
+        return FMM_ERR_CUDA;
+    attr_set.fetch_or(bit, std::memory_order_acq_rel);
+    return FMM_OK;
+}
+
+/* a launch that may start its blocks while the kernel before it on the stream
+ * still runs; the kernel waits (sm103::grid_wait) before it reads anything */
+template <class K, class... Args>
+static int launch_after(K* kernel, dim3 grid, int threads, size_t smem, cudaStream_t st, const Args&... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess ? FMM_OK : FMM_ERR_CUDA;
+}
+
+/* after_prep: the kernel before it on the stream is prep_kernel, which zeroes
+ * gl.sched and lets this one's blocks start */
+template <class GL>
+static int launch_gemm(GL& gl, int64_t nitems, int nprod_timed, cudaStream_t st, bool pair, bool after_prep)
+{
     int dev = 0, sms = 152;
     if (cudaGetDevice(&dev) != cudaSuccess) return FMM_ERR_CUDA;
-    const uint64_t bit = dev < 64 ? 1ull << dev : 0;
-    if (bit == 0 || !(attr_set.load(std::memory_order_acquire) & bit)) {
-        auto smem_limit = [](const void* f, size_t bytes) {
-            return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
-        };
-        if (!smem_limit((const void*)split_gemm_kernel, kGemmSmem) ||
-            !smem_limit((const void*)split_gemm_pair_kernel, kPairSmem) ||
-            !smem_limit((const void*)scatter_all_kernel<0>, kScatterAllMaxSmem) ||
-            !smem_limit((const void*)scatter_all_kernel<1>, kScatterAllMaxSmem) ||
-            !smem_limit((const void*)wave_scatter_kernel, kScatterAllMaxSmem))
-            return FMM_ERR_CUDA;
-        attr_set.fetch_or(bit, std::memory_order_acq_rel);
-    }
+    if (int rc = kernel_attributes(dev); rc != FMM_OK) return rc;
     if (nitems > 0x7fffffffLL) return FMM_ERR_UNSUPPORTED;
     if (nitems == 0) return FMM_OK;
     gl.nitems = (int)nitems;
@@ -2928,11 +2969,16 @@ static int launch_gemm(GemmLaunch& gl, int64_t nitems, int nprod_timed, cudaStre
     }
     /* both kernels draw their work items from gl.sched, zero at launch */
     if (gl.sched == nullptr) return FMM_ERR_CUDA;
-    if (!sched_zeroed && cudaMemsetAsync(gl.sched, 0, sizeof(unsigned int), st) != cudaSuccess) return FMM_ERR_CUDA;
+    if (!after_prep && cudaMemsetAsync(gl.sched, 0, sizeof(unsigned int), st) != cudaSuccess) return FMM_ERR_CUDA;
     if (pair)   /* clusters of two CTAs, one pair tile each at a time */
         split_gemm_pair_kernel<<<(unsigned)(2 * std::min<int64_t>(nitems, sms / 2)), kGemmThreads, kPairSmem, st>>>(gl);
-    else
+    else if (after_prep && !timed) {   /* an event between the two kernels ends the overlap */
+        if (int rc = launch_after(split_gemm_kernel<GL>, dim3((unsigned)std::min<int64_t>(nitems, sms)), kGemmThreads,
+                                  kGemmSmem, st, gl); rc != FMM_OK)
+            return rc;
+    } else {
         split_gemm_kernel<<<(unsigned)std::min<int64_t>(nitems, sms), kGemmThreads, kGemmSmem, st>>>(gl);
+    }
     if (timed) timing_mark(st, false);
     fmm_count_launch(1);
     return FMM_OK;
@@ -3065,7 +3111,7 @@ static int split_classical(SplitJob& j, bool alloc, cudaStream_t st)
         }
     }
     const bool pair = job_pair(j) && up.nunits == 0;
-    GemmLaunch gl;
+    GemmLaunch1 gl;
     memset(&gl, 0, sizeof(gl));
     gl.nprob = 1;
     gl.sched = (unsigned int*)(j.w + j.L.sched);   /* zeroed by prep_kernel */
@@ -3081,12 +3127,12 @@ static int split_classical(SplitJob& j, bool alloc, cudaStream_t st)
     gp.Z = (uint8_t*)planes;
     int rc = launch_gemm(gl, job_items(j, 1) * up.nunits, 1, st, false, true);
     if (rc == FMM_OK) {
-        scatter_units_kernel<<<dim3((unsigned)((j.m + 31) / 32), (unsigned)((j.n + 15) / 16)), 128, 0, st>>>(
-            (int)j.m, (int)j.n, j.alpha, j.beta, (const int4*)planes, (int)j.d.m_pad, (int)j.d.n_pad, j.s, gp.nkb,
-            up.unit_kb, up.nunits, job_zlevel(j), job_db(j), job_ebase(j), (const int*)(j.w + j.L.erow),
-            (const int*)(j.w + j.L.fcol), j.C, j.ldc);
+        rc = launch_after(scatter_units_kernel, dim3((unsigned)((j.m + 31) / 32), (unsigned)((j.n + 15) / 16)), 128, 0,
+                          st, (int)j.m, (int)j.n, j.alpha, j.beta, (const int4*)planes, (int)j.d.m_pad,
+                          (int)j.d.n_pad, j.s, gp.nkb, up.unit_kb, up.nunits, job_zlevel(j), job_db(j), job_ebase(j),
+                          (const int*)(j.w + j.L.erow), (const int*)(j.w + j.L.fcol), j.C, j.ldc);
         fmm_count_launch(1);
-        rc = cudaGetLastError() == cudaSuccess ? FMM_OK : FMM_ERR_CUDA;
+        if (rc == FMM_OK && cudaGetLastError() != cudaSuccess) rc = FMM_ERR_CUDA;
     }
     if (cudaFreeAsync(planes, st) != cudaSuccess && rc == FMM_OK) rc = FMM_ERR_CUDA;
     return rc;

@@ -81,6 +81,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     }
 }
 
+/* Programmatic launches: the stream's next kernel, when launched so, may start
+ * its blocks from here on; grid_wait returns once every kernel this one
+ * depends on has completed (at once in an ordinary launch). */
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 /* 8-byte global -> shared copy, zero when !ok (nothing is read then) */
 __device__ __forceinline__ void cp_async8(double* dst, const double* src, bool ok)
 {
