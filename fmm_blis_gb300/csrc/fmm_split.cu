@@ -1759,6 +1759,48 @@ struct ZRow {
     }
 };
 
+/* ZRow for two columns of a group (j even) */
+template <int FMT>
+struct ZPair {
+    static constexpr int NP = FMT ? 7 : 4;
+    int2 hi, f;
+    int e;
+    uint32_t w[NP];
+
+    __device__ __forceinline__ void load(const ZView& v, const int* __restrict__ e_row, const int* __restrict__ f_col,
+                                         int q, int i, int j)
+    {
+        const uint8_t* g = v.base + q * v.prod + (int64_t)(j >> 2) * v.group;
+        hi = *(const int2*)(g + (int64_t)i * 16 + (j & 2) * 4);
+        const uint8_t* d = g + ((int64_t)v.m_pad * 16 + (int64_t)i * 4 + (j & 2));
+#pragma unroll
+        for (int p = 0; p < NP; ++p) w[p] = p < v.nd ? *(const uint16_t*)(d + (int64_t)p * v.m_pad * 4) : 0u;
+        e = e_row[(int64_t)q * v.m_pad + i];
+        f = *(const int2*)(f_col + (int64_t)q * v.n_pad + j);
+    }
+    __device__ __forceinline__ void values(const ZView& v, double (&M)[2]) const
+    {
+        const int h[2] = {hi.x, hi.y}, fc[2] = {f.x, f.y};
+        const int er = e + v.ebase;
+        if (FMT == 0) {
+            const uint32_t a = __byte_perm(w[0], w[1], 0x5410u), b = __byte_perm(w[2], w[3], 0x5410u);
+            const uint32_t lo[2] = {__byte_perm(a, b, 0x0246u), __byte_perm(a, b, 0x1357u)};
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+                M[u] = i64_to_double_scaled((int64_t)(((uint64_t)(uint32_t)h[u] << 32) | lo[u]), er + fc[u]);
+        } else {
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                uint64_t lo = 0;
+#pragma unroll
+                for (int p = 0; p < NP; ++p)
+                    if (p < v.nd) lo = (lo << 5) | __byte_perm(w[p], 0u, 0x4440u + (unsigned)u);
+                M[u] = i64_to_double_scaled((int64_t)(((uint64_t)(int64_t)h[u] << (5 * v.nd)) | lo), er + fc[u]);
+            }
+        }
+    }
+};
+
 /* beta*c of the C update, as scale_c_kernel forms it */
 __device__ __forceinline__ double beta_c(double beta, const double* c)
 {
@@ -1820,26 +1862,29 @@ scatter_kernel(const int* __restrict__ tab, int r0, int nprod, int64_t m, int64_
         if (j + u < cl) cp[u * ldc] = c[u];
 }
 
-/* Multi-C epilogue, element-major: a thread takes a row of a 4-column group
- * of the product grid (rows [i_lo, i_lo + i_rows), all m_e rows when i_rows is
- * 0; columns [c0, c1)) and updates those elements of every C sub-block p, so
- * each product's Z_r is read (whole words: 5 to 10 loads for four elements)
- * and converted once and shared by all sub-blocks it feeds. The sub-blocks'
- * running values live in shared memory (cs[p][2][thread], two columns each);
- * for every sub-block the updates still come in increasing product order, so
- * the result is identical to scatter_kernel's. Used when the sub-block count
- * and the group's W entries fit the shared-memory budget.
+/* Multi-C epilogue, element-major: a thread takes a row of a 4-column group, or
+ * of half of one, of the product grid (rows [i_lo, i_lo + i_rows), all m_e rows
+ * when i_rows is 0; columns [c0, c1)) and updates those elements of every C
+ * sub-block p, so each product's Z_r is read (whole words) and converted once
+ * and shared by all sub-blocks it feeds. The sub-blocks' running values live
+ * in shared memory (cs[p][pair][thread], two columns each); for every
+ * sub-block the updates still come in increasing product order, so the result
+ * is identical to scatter_kernel's. Used when the sub-block count and the
+ * group's W entries fit the shared-memory budget.
  *
  * Bound by the FP64 pipe (2 FMA/clk/SM) once an algorithm has several
- * sub-blocks; four independent chains per thread keep it fed (222 x1 at
- * 3000 x 2500: 66 us, 107 us with one element per thread; its 12 FMAs per
- * element of the product grid take 37 us of the pipe). The classical
- * case is bound by HBM instead (8 bytes of Z, 16 of C per element). */
-constexpr int kScatterAllSmem = 32 * 1024;   /* cs[] budget: P * threads * 32 */
+ * sub-blocks, if four independent chains per thread and enough threads feed it
+ * (222 x1 at 3000 x 2500: 66 us, 107 us with one element per thread; its 12
+ * FMAs per element of the product grid take 37 us of the pipe). Shared memory
+ * limits the threads, so above 6 sub-blocks a thread takes two columns (222
+ * x2 at 4096, 16 sub-blocks: 326 us, 416 with four; 333 x1: 260 and 270), up
+ * to that four, which read fewer and wider words (222 x1: 73 us with two). The
+ * classical case is bound by HBM instead (8 bytes of Z, 16 of C per element). */
+constexpr int kScatterAllSmem = 32 * 1024;   /* cs[] budget: P * threads * columns * 8 */
 constexpr int kScatterAllMaxSmem = 96 * 1024;
 
 /* vb, vg: the block's index among the vg blocks that share the element range */
-template <int FMT>
+template <int FMT, int NC>
 __device__ __forceinline__ void scatter_all_body(const int* __restrict__ tab, int r0, int nprod, int64_t m, int64_t n,
                                                  double alpha, double beta, const ZView& Z,
                                                  const int* __restrict__ e_row, const int* __restrict__ f_col,
@@ -1853,9 +1898,11 @@ __device__ __forceinline__ void scatter_all_body(const int* __restrict__ tab, in
     const int eb = t.w_off[r0], E = t.w_off[r0 + nprod] - eb;
     const uint32_t me = (uint32_t)((m + t.mt - 1) / t.mt);
     const uint32_t rows = i_rows ? i_rows : me;
-    const uint32_t tiles_i = (rows + T - 1) / T;
+    const bool one = P == 1 && E == 1 && nprod == 1;
+    const int TR = one ? T : T * NC / 4;                                  /* rows per tile */
+    const uint32_t tiles_i = (rows + TR - 1) / TR;
     const uint32_t tiles = tiles_i * (uint32_t)((c1 + 3) / 4 - c0 / 4);   /* row tiles fastest */
-    if (P == 1 && E == 1 && nprod == 1) {
+    if (one) {
         /* one sub-block fed by one product (the classical split GEMM): no
          * shared memory, the C values in registers; HBM-bound (Z and C) */
         const double l = alpha * (double)t.w_ent[2 * eb + 1];
@@ -1876,8 +1923,9 @@ __device__ __forceinline__ void scatter_all_body(const int* __restrict__ tab, in
         }
         return;
     }
-    double2* cs = (double2*)sm_all;      /* [P][2][T] */
-    double* lam = sm_all + (size_t)P * T * 4;    /* [E] */
+    constexpr int NH = NC / 2;           /* column pairs of a thread */
+    double2* cs = (double2*)sm_all;      /* [P][NH][T] */
+    double* lam = sm_all + P * T * NC;   /* [E] */
     int* pidx = (int*)(lam + E);         /* [E] */
     int* off = pidx + E;                 /* [nprod + 1] */
     for (int x = tid; x < E; x += T) {
@@ -1890,59 +1938,72 @@ __device__ __forceinline__ void scatter_all_body(const int* __restrict__ tab, in
         fmm_part_geom32((int)n, t.nt, p % t.nt, &geo[2][p], &geo[3][p]);
     }
     __syncthreads();
+    const int tr = tid % TR, th = tid / TR * NC;     /* row of the tile, first of the thread's columns */
     for (uint32_t x = vb; x < tiles; x += vg) {
-        const int i = (int)(i_lo + x % tiles_i * T) + tid, j = (int)(c0 / 4 + x / tiles_i) * 4;
+        const int i = (int)(i_lo + x % tiles_i * TR) + tr, j = (int)(c0 / 4 + x / tiles_i) * 4 + th;
         if (i >= (int)(i_lo + rows)) continue;
-        ZRow<FMT> z;
+        std::conditional_t<NC == 4, ZRow<FMT>, ZPair<FMT>> z;
         z.load(Z, e_row, f_col, 0, i, j);
         /* elements outside a smaller sub-block or the column range are
          * carried along as zeros and not stored */
         for (int p = 0; p < P; ++p) {
             const int jl = i < geo[1][p] ? min(geo[3][p], c1) : 0;
             const double* cp = C + geo[0][p] + i + (int64_t)(geo[2][p] + j) * ldc;
-            double c[kScatterCols];
+            double c[NC];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) c[u] = j + u >= c0 && j + u < jl ? beta_c(beta, cp + u * ldc) : 0.0;
-            cs[(2 * p) * T + tid] = make_double2(c[0], c[1]);
-            cs[(2 * p + 1) * T + tid] = make_double2(c[2], c[3]);
+            for (int u = 0; u < NC; ++u) c[u] = j + u >= c0 && j + u < jl ? beta_c(beta, cp + u * ldc) : 0.0;
+#pragma unroll
+            for (int h = 0; h < NH; ++h) cs[(p * NH + h) * T + tid] = make_double2(c[2 * h], c[2 * h + 1]);
         }
         for (int q = 0; q < nprod; ++q) {
-            double M[kScatterCols];
+            double M[NC];
             z.values(Z, M);
             if (q + 1 < nprod) z.load(Z, e_row, f_col, q + 1, i, j);   /* in flight under this product's updates */
+            /* four values at a time, one sub-block's or two's (a product's are
+             * distinct): their loads and FMAs are under way together */
             const int e = off[q + 1];
-            for (int y = off[q]; y < e; ++y) {
-                const double l = lam[y];
-                double2* c = cs + 2 * pidx[y] * T + tid;
-                double2 a = c[0], b = c[T];
+            for (int y = off[q]; y < e; y += 4 / NC) {
+                const bool two = NC == 4 || y + 1 < e;
+                double2* c = cs + pidx[y] * NH * T + tid;
+                double2* d = NC == 4 ? c + T : cs + pidx[two ? y + 1 : y] * T + tid;
+                const double l = lam[y], l2 = NC == 4 ? l : (two ? lam[y + 1] : 0.0);
+                double2 a = *c, b = *d;
                 a.x = fma(l, M[0], a.x);
                 a.y = fma(l, M[1], a.y);
-                b.x = fma(l, M[2], b.x);
-                b.y = fma(l, M[3], b.y);
-                c[0] = a;
-                c[T] = b;
+                if (two) {
+                    b.x = fma(l2, M[NC - 2], b.x);
+                    b.y = fma(l2, M[NC - 1], b.y);
+                }
+                *c = a;
+                if (two) *d = b;
             }
         }
         for (int p = 0; p < P; ++p) {
             const int jl = i < geo[1][p] ? min(geo[3][p], c1) : 0;
             double* cp = C + geo[0][p] + i + (int64_t)(geo[2][p] + j) * ldc;
-            const double2 a = cs[(2 * p) * T + tid], b = cs[(2 * p + 1) * T + tid];
-            const double c[kScatterCols] = {a.x, a.y, b.x, b.y};
+            double2 a[NH];
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (j + u >= c0 && j + u < jl) cp[u * ldc] = c[u];
+            for (int h = 0; h < NH; ++h) a[h] = cs[(p * NH + h) * T + tid];
+#pragma unroll
+            for (int h = 0; h < NH; ++h) {
+                if (j + 2 * h >= c0 && j + 2 * h < jl) cp[2 * h * ldc] = a[h].x;
+                if (j + 2 * h + 1 >= c0 && j + 2 * h + 1 < jl) cp[(2 * h + 1) * ldc] = a[h].y;
+            }
         }
     }
 }
 
-template <int FMT>
+/* columns per thread of the element-major C update of P sub-blocks: see above */
+__host__ __device__ __forceinline__ int scatter_cols(int P) { return P <= 6 ? 4 : 2; }
+
+template <int FMT, int NC>
 __global__ void __launch_bounds__(256)
 scatter_all_kernel(const int* __restrict__ tab, int r0, int nprod, int64_t m, int64_t n, double alpha, double beta,
                    const ZView Z, const int* __restrict__ e_row, const int* __restrict__ f_col,
                    double* __restrict__ C, int64_t ldc, int c0, int c1, uint32_t i_lo, uint32_t i_rows)
 {
-    scatter_all_body<FMT>(tab, r0, nprod, m, n, alpha, beta, Z, e_row, f_col, C, ldc, c0, c1, blockIdx.x, gridDim.x,
-                          i_lo, i_rows);
+    scatter_all_body<FMT, NC>(tab, r0, nprod, m, n, alpha, beta, Z, e_row, f_col, C, ldc, c0, c1, blockIdx.x, gridDim.x,
+                              i_lo, i_rows);
 }
 
 
@@ -2118,10 +2179,19 @@ __global__ void __launch_bounds__(256) wave_scatter_kernel(const __grid_constant
     const WaveProb& P = W.p[wave_find(W, blockIdx.x)];
     const uint32_t vb = (uint32_t)(blockIdx.x - P.b0), vg = (uint32_t)P.nb;
     const int nt = P.tab[2], c1 = (int)((P.n + nt - 1) / nt);
-    if (P.fmt)
-        scatter_all_body<1>(P.tab, 0, P.R, P.m, P.n, P.alpha, P.beta, P.Z, P.e_row, P.f_col, P.C, P.ldc, 0, c1, vb, vg);
-    else
-        scatter_all_body<0>(P.tab, 0, P.R, P.m, P.n, P.alpha, P.beta, P.Z, P.e_row, P.f_col, P.C, P.ldc, 0, c1, vb, vg);
+    auto go = [&](auto F, auto N) {
+        scatter_all_body<decltype(F)::value, decltype(N)::value>(P.tab, 0, P.R, P.m, P.n, P.alpha, P.beta, P.Z,
+                                                                 P.e_row, P.f_col, P.C, P.ldc, 0, c1, vb, vg);
+    };
+    constexpr std::integral_constant<int, 0> bf16{};
+    constexpr std::integral_constant<int, 1> fp8{};
+    constexpr std::integral_constant<int, 2> pair{};
+    constexpr std::integral_constant<int, 4> row{};
+    if (scatter_cols(P.tab[0] * nt) == 4) {
+        if (P.fmt) go(fp8, row); else go(bf16, row);
+    } else {
+        if (P.fmt) go(fp8, pair); else go(bf16, pair);
+    }
 }
 
 /* --------------------------------------------------------- host -------- */
@@ -2839,27 +2909,37 @@ static int job_gemm_block(const SplitJob& j, int np, int64_t it0, int64_t it1, i
     return FMM_OK;
 }
 
-/* tiles of T rows x 4 columns of the element-major scatter over rows x cols
- * elements (a column range may start inside a group) */
-static int64_t scatter_tiles(int64_t rows, int64_t cols, int T) { return (rows + T - 1) / T * ((cols + 3) / 4 + 1); }
+/* rows of a tile of the element-major scatter with T threads; its width is 4 columns */
+static int scatter_tile_rows(const SplitJob& j, int T)
+{
+    return j.classical ? T : T * scatter_cols(j.alg.mt * j.alg.nt) / 4;
+}
+
+/* tiles over rows x cols elements of a job (a column range may start inside a group) */
+static int64_t scatter_tiles(const SplitJob& j, int64_t rows, int64_t cols, int T)
+{
+    const int tr = scatter_tile_rows(j, T);
+    return (rows + tr - 1) / tr * ((cols + 3) / 4 + 1);
+}
 
 /* blocks of one element-major scatter launch: one per tile, at most 16 per SM
  * (each then serves several tiles with one set-up) */
 static unsigned scatter_blocks(int64_t tiles) { return (unsigned)std::min<int64_t>(tiles, 16 * 152); }
 
 /* Whether the element-major C update applies to products [r0, r0 + np): at
- * most 64 sub-blocks whose values (T threads x 4 columns) and the group's W
+ * most 64 sub-blocks whose values (T threads x 2 or 4 columns) and the group's W
  * entries fit its shared memory. T: 32 KB of values, a multiple of 32 up to
  * 256, at least 32; with `small` 16 KB and at most 128, which fits on an SM
- * beside a resident GEMM CTA while P <= 16. */
+ * beside a resident GEMM CTA while P <= 32. */
 static bool job_scatter_all(const SplitJob& j, int r0, int np, int* T_out, size_t* smem_out, bool small = false)
 {
     const Tab ht = tab_view(j.alg.htab);
     const int P = j.alg.mt * j.alg.nt;
     const int E = ht.w_off[r0 + np] - ht.w_off[r0];
+    const int per = 8 * P * scatter_cols(P);   /* bytes of values per thread */
     const int T =
-        std::max(32, std::min(small ? 128 : 256, (small ? kScatterAllSmem / 2 : kScatterAllSmem) / (32 * P)) / 32 * 32);
-    const size_t smem = (size_t)P * T * 32 + (size_t)E * 12 + (size_t)(np + 1) * 4;
+        std::max(32, std::min(small ? 128 : 256, (small ? kScatterAllSmem / 2 : kScatterAllSmem) / per) / 32 * 32);
+    const size_t smem = (size_t)T * per + (size_t)E * 12 + (size_t)(np + 1) * 4;
     *T_out = T;
     *smem_out = smem;
     return P <= 64 && smem <= (size_t)kScatterAllMaxSmem;
@@ -2877,9 +2957,11 @@ static void job_scatter_block(const SplitJob& j, int r0, int np, int64_t i0, int
     size_t smem;
     job_scatter_all(j, r0, np, &T, &smem, small);
     if (j1 <= j0 || i1 <= i0) return;
-    T = (int)std::min<int64_t>(T, round_up(i1 - i0, 32));   /* fewer values than smem has room for */
-    const unsigned nb = scatter_blocks(scatter_tiles(i1 - i0, j1 - j0, T));
-    auto* k = j.fmt ? scatter_all_kernel<1> : scatter_all_kernel<0>;
+    T = (int)std::min<int64_t>(T, round_up((i1 - i0) * T / scatter_tile_rows(j, T), 32));   /* fewer than smem has room for */
+    const unsigned nb = scatter_blocks(scatter_tiles(j, i1 - i0, j1 - j0, T));
+    const bool row = scatter_cols(j.alg.mt * j.alg.nt) == 4;
+    auto* k = j.fmt ? (row ? scatter_all_kernel<1, 4> : scatter_all_kernel<1, 2>)
+                    : (row ? scatter_all_kernel<0, 4> : scatter_all_kernel<0, 2>);
     k<<<nb, (unsigned)T, smem, st>>>(j.alg.tab, r0, np, j.m, j.n, j.alpha, job_beta(j, r0), job_zview(j),
                                      (const int*)(j.w + j.L.erow), (const int*)(j.w + j.L.fcol), j.C, j.ldc, (int)j0,
                                      (int)j1, (uint32_t)i0, (uint32_t)(i1 - i0));
@@ -2922,8 +3004,10 @@ static int kernel_attributes(int dev)
         !limit((const void*)split_gemm_kernel<GemmLaunch1>, kGemmSmem) ||
         !limit((const void*)split_gemm_pair_kernel<GemmLaunch>, kPairSmem) ||
         !limit((const void*)split_gemm_pair_kernel<GemmLaunch1>, kPairSmem) ||
-        !limit((const void*)scatter_all_kernel<0>, kScatterAllMaxSmem) ||
-        !limit((const void*)scatter_all_kernel<1>, kScatterAllMaxSmem) ||
+        !limit((const void*)scatter_all_kernel<0, 2>, kScatterAllMaxSmem) ||
+        !limit((const void*)scatter_all_kernel<1, 2>, kScatterAllMaxSmem) ||
+        !limit((const void*)scatter_all_kernel<0, 4>, kScatterAllMaxSmem) ||
+        !limit((const void*)scatter_all_kernel<1, 4>, kScatterAllMaxSmem) ||
         !limit((const void*)wave_scatter_kernel, kScatterAllMaxSmem))
         return FMM_ERR_CUDA;
     attr_set.fetch_or(bit, std::memory_order_acq_rel);
@@ -3760,17 +3844,17 @@ static int wave_side_scatter(const std::vector<SplitJob*>& qs, bool small, cudaS
         for (SplitJob* j : all) {
             const Tab ht = tab_view(j->alg.htab);
             const int P = j->alg.mt * j->alg.nt, E = ht.w_off[j->alg.R] - ht.w_off[0];
-            smem = std::max(smem, (size_t)P * T * 32 + (size_t)E * 12 + (size_t)(j->alg.R + 1) * 4);
+            smem = std::max(smem, (size_t)P * T * 8 * scatter_cols(P) + (size_t)E * 12 + (size_t)(j->alg.R + 1) * 4);
         }
         /* the launch's blocks are shared out by the problems' tiles, so a
          * block's set-up serves several tiles in a wave of many problems too */
         int64_t tiles = 0;
-        for (SplitJob* j : all) tiles += scatter_tiles(j->d.me, j->d.ne, T);
+        for (SplitJob* j : all) tiles += scatter_tiles(*j, j->d.me, j->d.ne, T);
         const double share = (double)scatter_blocks(tiles) / (double)tiles;
         WaveLaunch L;
         const int64_t nb = wave_table(L, all, [&](const SplitJob& j, WaveProb& w) {
             w.gx = 1;
-            w.nb = std::max<int64_t>(1, (int64_t)(share * (double)scatter_tiles(j.d.me, j.d.ne, T)));
+            w.nb = std::max<int64_t>(1, (int64_t)(share * (double)scatter_tiles(j, j.d.me, j.d.ne, T)));
         });
         wave_scatter_kernel<<<(unsigned)nb, (unsigned)T, smem, st>>>(L);
         fmm_count_launch(1);

@@ -28,6 +28,8 @@ def torch_cuda():
     ("232", 1, 130, 259, 260, 12, "fp8"),   # all seven FP8 planes, three levels above G
     ("333", 1, 100, 101, 60, 8, "bf16"),    # k_pad 64: levels 3 and 2 share the high plane
     ("222", 1, 66, 65, 90, 2, "fp8"),       # no digit plane at all
+    ("322", 1, 200, 67, 40, 7, "fp8"),      # 6 and
+    ("232", 2, 260, 31, 50, 6, "bf16"),     # 16 sub-blocks: four and two columns per thread
 ])
 @pytest.mark.parametrize("alpha,beta", [(1.0, 1.0), (-0.75, 0.5), (2.0, 0.0)])
 @pytest.mark.parametrize("groups", ["one", "several"])
