@@ -143,7 +143,7 @@ __host__ __device__ constexpr uint64_t digit_offset()
 }
 
 template <int S, int DB>
-__device__ __forceinline__ Digits split_offset(double x, int E)
+__device__ __forceinline__ Digits split_offset_any(double x, int E)
 {
     const uint32_t hi = (uint32_t)__double2hiint(x);
     const int bexp = (int)(hi >> 20) & 0x7ff;
@@ -163,6 +163,41 @@ __device__ __forceinline__ Digits split_offset(double x, int E)
     return Digits{X, (uint64_t)X + digit_offset<S, DB>()};
 }
 
+/* split_offset_any for N elements of one line, in about half the integer
+ * instructions (which bound the packs): with t = mant >> (r - 1), OFF =
+ * digit_offset and s = 0 or -1 for the sign, Y = X + OFF is
+ * ((t ^ s) + 2 OFF + 1) >> 1 for either sign (-floor(a / 2) =
+ * floor((1 - a) / 2)), so rounding, negation and offset are one 64-bit
+ * addition (a batch's classical problems: 785 -> 739 us of digits in all). Where
+ * r - 1 could be negative (down to -7: |x| < 2^E, DB*S > 53) the mantissa is
+ * shifted up by 10 first; not by more, so that its top bit stays below bit 63
+ * and a shift held at 63 leaves 0. Needs Y and its extra bit inside 64 bits
+ * (DB*S <= 60) and no left shift: E >= DB*S - 1074 (lines below that hold
+ * subnormal numbers only). */
+template <int S, int DB, int N>
+__device__ __forceinline__ void split_offsets(const double (&x)[N], int E, Digits (&Y)[N])
+{
+    constexpr bool kTop = DB * S > 53;
+    if (DB * S > 60 || E < DB * S - 1074) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) Y[i] = split_offset_any<S, DB>(x[i], E);
+        return;
+    }
+    const int K = E + 1075 - DB * S + (kTop ? 10 : 0);   /* r - 1 = K - max(exponent field, 1) */
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const uint32_t hi = (uint32_t)__double2hiint(x[i]);
+        const int bexp = (int)(hi >> 20) & 0x7ff;
+        uint64_t mant = ((uint64_t)((hi & 0x000fffffu) | ((uint32_t)min(bexp, 1) << 20)) << 32) |
+                        (uint32_t)__double2loint(x[i]);
+        if (kTop) mant <<= 10;
+        const uint64_t t = mant >> min(K - max(bexp, 1), 63);
+        const uint64_t neg = (uint64_t)((int64_t)(int32_t)hi >> 31);
+        Y[i].X = 0;   /* not needed below 64 digit bits */
+        Y[i].Y = (uint64_t)((int64_t)((t ^ neg) + (2 * digit_offset<S, DB>() + 1)) >> 1);
+    }
+}
+
 /* digit t (0 = most significant) as an exact float. A lower digit is field
  * S-1-t of Y minus 2^(DB-1): the field is placed in the mantissa of 2^23 (one
  * byte permute for DB = 8, a shift and mask for DB = 5) and 2^23 + 2^(DB-1)
@@ -176,7 +211,8 @@ __device__ __forceinline__ float digit_f(const Digits& g, int t)
     constexpr uint64_t kOff = digit_offset<S, DB>();
     constexpr uint64_t kMask = (1ull << sh) - 1;
     if (t == 0) {
-        const int d = (int)(g.X >> sh) + (int)((((uint64_t)g.X & kMask) + kOff) >> sh);
+        const int d = DB * S < 64 ? (int)((int64_t)g.Y >> sh)
+                                  : (int)(g.X >> sh) + (int)((((uint64_t)g.X & kMask) + kOff) >> sh);
         return __int_as_float(0x4B400000 + d) - 12582912.0f;   /* exact for |d| < 2^22 */
     }
     const int fi = S - 1 - t;
@@ -556,9 +592,11 @@ __device__ __forceinline__ void pack_a_body(const int* __restrict__ tab, int r0,
     for (int rr = threadIdx.x / 8; rr < ROWS; rr += ROWS / 2) {
         const int64_t gi = i0 + rr;
         const int E = e_row[gi];
-        Digits Y[8];
+        double x8[8];
 #pragma unroll
-        for (int x = 0; x < 8; ++x) Y[x] = split_offset<S, DB>(Sf[kg * 8 + x][rr], E);
+        for (int x = 0; x < 8; ++x) x8[x] = Sf[kg * 8 + x][rr];
+        Digits Y[8];
+        split_offsets<S, DB>(x8, E, Y);
         store_digits8<S, DB>(sa, slice0 + gi * k_pad + p0 + kg * 8, m_pad * k_pad, Y);
     }
 }
@@ -632,8 +670,7 @@ __device__ __forceinline__ void pack_b_body(const int* __restrict__ tab, int r0,
     }
     const int F = f_col[gj];
     Digits Y[8];
-#pragma unroll
-    for (int x = 0; x < 8; ++x) Y[x] = split_offset<S, DB>(v8[x], F);
+    split_offsets<S, DB>(v8, F, Y);
     store_digits8<S, DB>(sb, slice0 + gj * k_pad + p0, n_pad * k_pad, Y);
 }
 
@@ -733,8 +770,9 @@ void launch_packs(int fmt, int s, const int* tab, int r, int np, const double* A
  * digits. The same exponents and digits as the general path's maxima,
  * exponents and packs (one term of coefficient 1), which takes seven launches.
  * Bound by latency (loads in flight) and instruction issue: 8192 x 8192 of both
- * operands, 6 slices, 575 us (4.7 TB/s of the 2.7 GB it cannot do without);
- * 690 us with 64-bit maxima and general shifts, 680 us through cp.async tiles. */
+ * operands, 6 slices, 560 us (4.8 TB/s of the 2.7 GB it cannot do without);
+ * 575 us with split_offset_any, 690 us with 64-bit maxima as well, 680 us
+ * through cp.async tiles. */
 constexpr int kPrepLines = 16, kPrepK = 128, kPrepThreads = 256;
 constexpr int kPrepPitch = kPrepK + kPrepK / 16 + 1;   /* one pad per 16 k, odd row pitch: no bank conflicts either way */
 
@@ -855,9 +893,11 @@ __device__ __forceinline__ void prep_body(PrepShared& sh, const double* __restri
         if (p0 + t * kPrepK + k4 < p1) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                Digits Y[4];
+                double x4[4];
 #pragma unroll
-                for (int x = 0; x < 4; ++x) Y[x] = split_offset<S, DB>(tile[pos + h * 8 * kPrepPitch + x], h ? E1 : E0);
+                for (int x = 0; x < 4; ++x) x4[x] = tile[pos + h * 8 * kPrepPitch + x];
+                Digits Y[4];
+                split_offsets<S, DB>(x4, h ? E1 : E0, Y);
                 store_digits4<S, DB>(out, off + h * 8 * k_pad + (int64_t)t * kPrepK, l_pad * k_pad, Y);
             }
         }
@@ -865,7 +905,7 @@ __device__ __forceinline__ void prep_body(PrepShared& sh, const double* __restri
 }
 
 template <int S, int DB>
-__global__ void __launch_bounds__(kPrepThreads, DB == 8 ? 4 : 3)   /* more digits spill at 64 registers */
+__global__ void __launch_bounds__(kPrepThreads, 3)   /* four per SM would spill */
 prep_kernel(const double* __restrict__ A, int64_t lda, const double* __restrict__ B, int64_t ldb, int64_t m,
             int64_t n, int64_t k, int64_t m_pad, int64_t n_pad, int64_t k_pad, int* __restrict__ e_row,
             int* __restrict__ f_col, uint8_t* __restrict__ sa, uint8_t* __restrict__ sb,

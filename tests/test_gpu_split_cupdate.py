@@ -62,3 +62,26 @@ def test_largest_level_sums(fmm, orc, torch_cuda, s, fmt):
     fmm.split_dgemm(to_dev(A), to_dev(B), dC, None, 0, s, fmt=fmt)
     want = orc.split_fmm_dgemm(oc.classical(), A, B, C.copy(order="F"), s, fmt=fmt)
     assert np.array_equal(to_host(dC), want)
+
+
+@pytest.mark.parametrize("alg,levels", [(None, 0), ("222", 1)])
+@pytest.mark.parametrize("s,fmt", [(6, "bf16"), (7, "bf16"), (8, "bf16"), (11, "fp8"), (12, "fp8")])
+def test_digits_around_the_last_unit(fmm, orc, algs, torch_cuda, alg, levels, s, fmt):
+    """elements from the last digit's unit to far below it, of both signs: the
+    large element that sets a row's exponent meets zeros of B"""
+    from oracle import coeffs as oc
+    m, n, k = 64, 20, 40
+    A, B, C = rand(m, k, 31), rand(k, n, 32), np.zeros((m, n), order="F")
+    A *= 2.0 ** -(np.arange(m, dtype=np.float64)[:, None] % 32 + 38)
+    A[::3, 1::4] = 2.0 ** -(np.arange(0, m, 3, dtype=np.float64)[:, None] % 32 + 38)   # ties among them
+    A[:, [0, k // 2]] = 0.75
+    B[[0, k // 2], :] = 0.0
+    f = fmm.new_fmm(COEFFS / f"{alg}.txt") if alg else None
+    try:
+        dC = to_dev(C)
+        fmm.split_dgemm(to_dev(A), to_dev(B), dC, f, levels, s, fmt=fmt)
+    finally:
+        if f is not None:
+            fmm.free_fmm(f)
+    want = orc.split_fmm_dgemm(oc.power(algs[alg], levels) if alg else oc.classical(), A, B, C.copy(order="F"), s, fmt=fmt)
+    assert np.array_equal(to_host(dC), want)
