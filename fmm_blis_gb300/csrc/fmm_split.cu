@@ -59,9 +59,11 @@
  * updates on pool streams beside the other group's GEMM, and a group's GEMM
  * as launches of about 24 rounds of items. The host-buffer call overlaps the
  * copies with the work (A in row halves and B in column chunks chased by
- * their packs, the GEMM in up to 2 x 2 blocks of tiles that start on half of
- * each operand, each block's C read back in column chunks behind its C
- * updates). Batched calls run waves of up
+ * their packs, the GEMM in up to 2 x 4 blocks of tiles that start on a part of
+ * each operand, each block's C sent and read back with its C updates), unless
+ * the operands are small. A classical call runs three kernels: prep_kernel
+ * (maxima, exponents and digits), the GEMM, with the tiles of a small grid cut
+ * into work units, and the C updates. Batched calls run waves of up
  * to 80 problems, one GEMM launch per tile kind per wave, waves alternating
  * between two workspace halves so a wave's packs overlap the previous wave.
  * Every path gives the same bits for a problem.
@@ -3240,7 +3242,10 @@ static int split_classical(SplitJob& j, bool alloc, cudaStream_t st)
     gl.nprob = 1;
     gl.sched = (unsigned int*)(j.w + j.L.sched);   /* zeroed by prep_kernel */
     GemmProblem& gp = gl.prob[0];
-    if (int rc = job_fill(j, gp, 1, 0, pair); rc != FMM_OK) return rc;
+    if (int rc = job_fill(j, gp, 1, 0, pair); rc != FMM_OK) {
+        if (planes) cudaFreeAsync(planes, st);
+        return rc;
+    }
     if (up.nunits == 0) {
         if (int rc = launch_gemm(gl, job_items(j, 1, pair), 1, st, pair, true); rc != FMM_OK) return rc;
         job_scatter(j, 0, 1, st);
