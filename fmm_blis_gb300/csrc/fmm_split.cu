@@ -643,7 +643,10 @@ pack_a_kernel(const int* __restrict__ tab, int r0, int np, const double* __restr
  * columns x 64 k of T_r, r = r0 + q (column j of T_r is contiguous in k
  * already), and writes its digits into slices sb[q][t][n_pad][k_pad];
  * product index fastest, as on the A side. COLS = 32 (256 threads) for single
- * calls, 16 (128 threads, at most 64 registers) for batched waves. */
+ * calls, 16 (128 threads, at most 64 registers) for batched waves. Eight lanes
+ * read 64 contiguous bytes of a column per load (a load that gives each lane
+ * eight consecutive k touches 16 lines and is bound by L1) and exchange the
+ * sums through shared memory: 222 x2 at 4096, 6 slices, 339 -> 277 us. */
 template <int S, int DB, int COLS>
 __device__ __forceinline__ void pack_b_body(const int* __restrict__ tab, int r0, int np, const double* __restrict__ B,
                                             int64_t ldb, int64_t k, int64_t n, int64_t n_pad, int64_t k_pad,
@@ -651,6 +654,7 @@ __device__ __forceinline__ void pack_b_body(const int* __restrict__ tab, int r0,
                                             int64_t bx, int64_t by)
 {
     __shared__ PEnt ent[kPackMaxEnt];
+    __shared__ double Tf[COLS][72];   /* element k at k + k / 8: no bank conflicts either way */
     const Tab t = tab_view(tab);
     const int64_t ne = (n + t.nt - 1) / t.nt, ke = (k + t.kt - 1) / t.kt;
     const int q = (int)(bx % np);
@@ -668,20 +672,20 @@ __device__ __forceinline__ void pack_b_body(const int* __restrict__ tab, int r0,
     __syncthreads();
     const int kg = threadIdx.x % 8;
     const int64_t gj = j_first + (bx / np) * COLS + threadIdx.x / 8;
-    const int64_t p0 = by * 64 + kg * 8;
-    double v8[8];
+    const int64_t p0 = by * 64;
+    double v8[8];   /* k = p0 + kg + 8 y: a column's eight lanes read 64 bytes side by side */
 #pragma unroll
     for (int x = 0; x < 8; ++x) v8[x] = 0.0;
     if (ne_ > 0 && gj < ne) {
         /* term e + 1's loads go out before term e's FMAs; per term, one
-         * column test and one k limit, then 8 contiguous values at fixed
-         * offsets from one pointer */
+         * column test and one k limit, then 8 values at fixed offsets from
+         * one pointer */
         auto load8 = [&](const PEnt& x, double (&d)[8]) {
-            const int64_t kl = (ke < x.rows ? ke : x.rows) - p0;   /* valid while y < kl */
+            const int64_t kl = (ke < x.rows ? ke : x.rows) - (p0 + kg);   /* valid while 8y < kl */
             const bool cok = gj < x.cols;
-            const double* pt = x.base + gj * ldb + p0;
+            const double* pt = x.base + gj * ldb + p0 + kg;
 #pragma unroll
-            for (int y = 0; y < 8; ++y) d[y] = (cok && y < kl) ? __ldg(pt + y) : 0.0;
+            for (int y = 0; y < 8; ++y) d[y] = (cok && 8 * y < kl) ? __ldg(pt + 8 * y) : 0.0;
         };
         double nx[8];
         load8(ent[0], v8);
@@ -697,10 +701,17 @@ __device__ __forceinline__ void pack_b_body(const int* __restrict__ tab, int r0,
             for (int y = 0; y < 8; ++y) v8[y] = fma(c, cur[y], v8[y]);
         }
     }
+    /* to eight consecutive k per lane, within the column's lanes */
+    double* mine = Tf[threadIdx.x / 8];
+#pragma unroll
+    for (int y = 0; y < 8; ++y) mine[kg + 9 * y] = v8[y];
+    __syncwarp();
+#pragma unroll
+    for (int x = 0; x < 8; ++x) v8[x] = mine[9 * kg + x];
     const int F = f_col[gj];
     Digits Y[8];
     split_offsets<S, DB>(v8, F, Y);
-    store_digits8<S, DB>(sb, slice0 + gj * k_pad + p0, n_pad * k_pad, Y);
+    store_digits8<S, DB>(sb, slice0 + gj * k_pad + p0 + kg * 8, n_pad * k_pad, Y);
 }
 
 template <int S, int DB, int COLS>
