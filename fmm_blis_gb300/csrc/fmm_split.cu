@@ -1889,8 +1889,8 @@ __device__ __forceinline__ double beta_c(double beta, const double* c)
 }
 
 /* C updates of one C sub-block p = blockIdx.y: tiles of blockDim.x rows x 4
- * columns, a thread a row of a column group. For algorithms whose sub-block
- * values do not fit scatter_all_kernel's shared memory. */
+ * columns, a thread a row of a column group. For algorithms of more than 16
+ * sub-blocks (scatter_all_better). */
 template <int FMT>
 __global__ void __launch_bounds__(128)
 scatter_kernel(const int* __restrict__ tab, int r0, int nprod, int64_t m, int64_t n, double alpha, double beta,
@@ -3025,6 +3025,16 @@ static bool job_scatter_all(const SplitJob& j, int r0, int np, int* T_out, size_
     return P <= 64 && smem <= (size_t)kScatterAllMaxSmem;
 }
 
+/* Whether the element-major C update is also the faster one: with more than
+ * 16 sub-blocks its shared memory leaves an SM too few threads (64 sub-blocks:
+ * 32-thread blocks, four per SM), and scatter_kernel, which reads Z once per
+ * sub-block it feeds but keeps nothing in shared memory, is faster at every
+ * grid. Calls of k = 48 per sub-block, 6 slices, element-major / per sub-block,
+ * us: 16 sub-blocks (222 x2) grid 256 x 512 153 / 173, 1000 x 1000 607 / 790;
+ * 36 (322 x2) 424 / 294, 2620 / 1732; 64 (222 x3) 1985 / 1188, 13244 / 7758.
+ * Only calls that need column ranges (host buffers) use it above 16. */
+static bool scatter_all_better(const SplitJob& j) { return j.alg.mt * j.alg.nt <= 16; }
+
 /* beta*C comes with the C updates of the first product group */
 static double job_beta(const SplitJob& j, int r0) { return r0 == 0 ? j.beta : 1.0; }
 
@@ -3060,7 +3070,7 @@ static void job_scatter(const SplitJob& j, int r0, int np, cudaStream_t st, bool
 {
     int T;
     size_t smem;
-    if (job_scatter_all(j, r0, np, &T, &smem)) {
+    if (scatter_all_better(j) && job_scatter_all(j, r0, np, &T, &smem)) {
         job_scatter_block(j, r0, np, 0, j.d.me, 0, j.d.ne, st, small);
         return;
     }
@@ -3915,7 +3925,7 @@ static int wave_side_scatter(const std::vector<SplitJob*>& qs, bool small, cudaS
     for (SplitJob* j : qs) {
         int Tj;
         size_t sm;
-        if (job_scatter_all(*j, 0, j->alg.R, &Tj, &sm, small)) {
+        if (scatter_all_better(*j) && job_scatter_all(*j, 0, j->alg.R, &Tj, &sm, small)) {
             all.push_back(j);
             T = std::min(T, Tj);
         } else {

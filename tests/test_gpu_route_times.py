@@ -1,0 +1,47 @@
+"""Calls whose cost depends on which kernel form or tile a rule picks for them:
+each takes no longer than a bound between the times of the right and the wrong
+pick (best of several, events on the device), so a rule that moves them to the
+wrong one shows."""
+import pytest
+
+from conftest import COEFFS
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def torch_cuda():
+    import torch
+    assert torch.cuda.is_available()
+    return torch
+
+
+def operand(torch, rows, cols):
+    return (torch.rand((cols, rows), device="cuda", dtype=torch.float64) * 2 - 1).t()
+
+
+def device_us(torch, f, reps=5, calls=4):
+    for _ in range(2):
+        f()
+    torch.cuda.synchronize()
+    best = float("inf")
+    for _ in range(reps):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        for _ in range(calls):
+            f()
+        b.record()
+        b.synchronize()
+        best = min(best, a.elapsed_time(b) / calls * 1e3)
+    return best
+
+
+def test_c_updates_of_many_sub_blocks(fmm, torch_cuda):
+    """Three Strassen levels on an 8 x 110 product grid: 64 C sub-blocks, 343
+    products. About 250 us with a C update per sub-block, 530 us with all
+    sub-blocks of an element in one thread."""
+    m, n, k = 64, 880, 384
+    f = fmm.new_fmm(COEFFS / "222.txt")
+    A, B, C = operand(torch_cuda, m, k), operand(torch_cuda, k, n), operand(torch_cuda, m, n)
+    ws = torch_cuda.empty(fmm.split_workspace_size(m, n, k, f, 3, 6), dtype=torch_cuda.uint8, device="cuda")
+    assert device_us(torch_cuda, lambda: fmm.split_dgemm(A, B, C, f, 3, 6, 1.0, 0.5, ws)) < 400
