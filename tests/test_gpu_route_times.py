@@ -45,3 +45,32 @@ def test_c_updates_of_many_sub_blocks(fmm, torch_cuda):
     A, B, C = operand(torch_cuda, m, k), operand(torch_cuda, k, n), operand(torch_cuda, m, n)
     ws = torch_cuda.empty(fmm.split_workspace_size(m, n, k, f, 3, 6), dtype=torch_cuda.uint8, device="cuda")
     assert device_us(torch_cuda, lambda: fmm.split_dgemm(A, B, C, f, 3, 6, 1.0, 0.5, ws)) < 400
+
+
+def test_batch_of_unlike_c_updates(fmm, torch_cuda):
+    """A problem of 36 sub-blocks and 121 products beside a classical one:
+    about 300 us as a batch, 830 us with both in one C update launch whose
+    blocks are shared out by tiles."""
+    torch = torch_cuda
+    f = fmm.new_fmm(COEFFS / "322.txt")
+    ps = [{"A": operand(torch, m, k), "B": operand(torch, k, n), "C": operand(torch, m, n), "fmm": g, "levels": lv,
+           "slices": s, "fmt": fmt}
+          for m, n, k, g, lv, s, fmt in [(963, 267, 134, f, 2, 11, "fp8"), (675, 2091, 595, None, 0, 4, "bf16")]]
+    b = fmm.make_batch(ps)
+    ws = torch.empty(fmm.batch_workspace_size(b), dtype=torch.uint8, device="cuda")
+    assert device_us(torch, lambda: fmm.batch_dgemm(b, workspace=ws)) < 550
+
+
+def test_batch_of_unlike_small_c_updates(fmm, torch_cuda):
+    """16 and 36 sub-blocks of small product grids beside classical problems:
+    1360 us with one C update launch for all, shared out by tiles."""
+    torch = torch_cuda
+    f2, f3 = fmm.new_fmm(COEFFS / "222.txt"), fmm.new_fmm(COEFFS / "322.txt")
+    ps = [{"A": operand(torch, m, k), "B": operand(torch, k, n), "C": operand(torch, m, n), "fmm": g, "levels": lv,
+           "slices": s, "fmt": fmt}
+          for m, n, k, g, lv, s, fmt in [(1069, 935, 147, None, 0, 7, "fp8"), (787, 293, 450, f2, 2, 8, "bf16"),
+                                         (607, 1440, 524, None, 0, 12, "fp8"), (121, 123, 122, None, 0, 3, "bf16"),
+                                         (484, 504, 46, f3, 2, 6, "fp8")]]
+    b = fmm.make_batch(ps)
+    ws = torch.empty(fmm.batch_workspace_size(b), dtype=torch.uint8, device="cuda")
+    assert device_us(torch, lambda: fmm.batch_dgemm(b, workspace=ws)) < 900
