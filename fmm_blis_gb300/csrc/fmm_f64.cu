@@ -30,6 +30,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstring>
 #include <mutex>
 #include <vector>
@@ -1281,6 +1282,89 @@ extern "C" int fmm_gpu_set_f64_batch_ctas(int max_ctas)
     return g_f64_batch_ctas.exchange(max_ctas > 0 ? max_ctas : 0);
 }
 
+namespace {
+
+/* FP64 pipe time of one item of a batch (a tile of all products), in FMAs at a
+ * 64 x 64 tile's rate. Smaller tiles pay for the pack additions of more tiles
+ * per operand element (nu, nv terms per product), 16 x 16 also for fewer FMAs
+ * per shared-memory load and for the C updates of a short k. Measured, tiles
+ * 64 / 32 / 16, us: 2432 x 2048 x 2000 222 x1 (304 tiles of 64) 15249 / 15506 /
+ * 19326, x 64 524 / 564 / 806; classical 1216 x 1024 x 500 1048 / 1052 / 1212,
+ * x 32 84 / 90 / 127; 4864 x 4096 x 400 444 x1 15503 / 17218 / 24942. FP64 MMA
+ * engine, 64 / 32: classical 1216 x 1024 x 500 1184 / 1190, 2048^3 222 x1 16969 /
+ * 17362 (2 and 1.75 rounds of 64 x 64 work). */
+double batch_item_cost(const F64BatchItem& it, int tile, bool mma)
+{
+    if (it.k == 0 || it.alpha == 0.0) return 1.0;
+    const double ke = (double)((it.k + it.alg.kt - 1) / it.alg.kt), nn = it.alg.avg_nnz_u + it.alg.avg_nnz_v;
+    double rel = 1.0;
+    if (tile == 32)
+        rel = mma ? 1.01 + 0.11 * (nn - 2.0) : 1.0 + 0.01 * nn + 1.5 / ke;
+    else if (tile == 16)
+        rel = 1.0 + 0.08 * nn + 11.0 / ke;
+    return rel * tile * tile * it.alg.R * (ke + 1.0);
+}
+
+/* Each problem's tile and item cost. One 64 x 64 item of a deep problem can last
+ * as long as the whole batch (1024^3 222 x1: 7 ms on half an SM), smaller
+ * tiles cost more in all (batch_item_cost). Tried are limits on an item's
+ * cost: from the longest 64 x 64 item down to 1/32 of it, and an eighth of a
+ * CTA's share of the batch; a problem takes its largest tile within the limit,
+ * and the limit with the least estimate is kept. The estimate: items go out
+ * longest first to `slots` SMs (an SM's two CTAs share its FP64 pipe, and one
+ * alone nearly fills it), so after each problem's items the time is the work
+ * so far in whole rounds of that item. 64 / 32 / 16 everywhere / this rule, us:
+ * 2048^3 222 x1 15204 / 13633 / 16552 / 13638; 512^3 222 x1 2019 / 586 / 319 /
+ * 319; eight classical 700^3 4957 / 4629 / 5308 / 4631; 200 of 100^3 222 x1
+ * 1033 / 826 / 962 / 829. */
+template <class TilesOf>
+void batch_tiles(const F64BatchItem* items, const std::vector<int>& order, bool mma, int slots, TilesOf tiles_of,
+                 std::vector<int>& tile, std::vector<double>& cost)
+{
+    struct Choice {
+        double cost[3], items[3];   /* at tiles of 64, 32, 16 */
+    };
+    const int sizes = mma ? 2 : 3;
+    std::vector<Choice> ch(order.size());
+    double longest = 0.0, total = 0.0;
+    for (size_t q = 0; q < order.size(); ++q) {
+        for (int t = 0; t < sizes; ++t) {
+            int64_t tm = 0;
+            ch[q].cost[t] = batch_item_cost(items[order[q]], 64 >> t, mma);
+            ch[q].items[t] = (double)tiles_of(order[q], 64 >> t, &tm);
+        }
+        longest = std::max(longest, ch[q].cost[0]);
+        total += ch[q].cost[1] * ch[q].items[1];
+    }
+    std::vector<int> pick(order.size()), best(order.size(), 0);
+    std::vector<std::pair<double, double>> cls(order.size());   /* (item cost, items) */
+    double least = 0.0;
+    for (int x = 0; x <= 6; ++x) {
+        const double limit = x < 6 ? longest / (1 << x) : total / slots / 16;
+        for (size_t q = 0; q < order.size(); ++q) {
+            pick[q] = 0;
+            while (pick[q] + 1 < sizes && ch[q].cost[pick[q]] > limit) ++pick[q];
+            cls[q] = {ch[q].cost[pick[q]], ch[q].items[pick[q]]};
+        }
+        std::sort(cls.begin(), cls.end(), [](auto& a, auto& b) { return a.first > b.first; });
+        double work = 0.0, est = 0.0;
+        for (const auto& c : cls) {
+            work += c.first * c.second;
+            est = std::max(est, c.first * std::ceil(work / (slots * c.first)));
+        }
+        if (x == 0 || est < (x < 6 ? 0.98 : 1.0) * least) {   /* larger tiles at a near tie */
+            least = est;
+            best = pick;
+        }
+    }
+    for (size_t q = 0; q < order.size(); ++q) {
+        tile[order[q]] = 64 >> best[q];
+        cost[order[q]] = ch[q].cost[best[q]];
+    }
+}
+
+}  // namespace
+
 int fmm_f64_batch_launch(int count, const F64BatchItem* items, void* ws, size_t ws_bytes, cudaStream_t st)
 {
     if (count <= 0) return FMM_OK;
@@ -1310,33 +1394,18 @@ int fmm_f64_batch_launch(int count, const F64BatchItem* items, void* ws, size_t 
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const bool mma = g_f64_engine.load(std::memory_order_relaxed) == FMM_F64_MMA;
-    /* Item tiles: 64 x 64 costs the fewest pack additions, but one item of a
-     * deep problem can last as long as the whole batch (1024^3 222 x1: 14.7 M
-     * FMAs, 7 ms on half an SM). A problem's tile shrinks to 32, then 16,
-     * while its items hold more than an eighth of a CTA's share of the
-     * batch. 24 problems of 256 to 1024: 7.1 ms with 64 x 64 alone. */
     int64_t ctas = 2 * (int64_t)sms;
     const int cap = g_f64_batch_ctas.load();
     if (cap > 0) ctas = std::min<int64_t>(ctas, cap);
-    auto item_fmas = [&](int i, int tile) {
-        const F64BatchItem& it = items[i];
-        if (it.k == 0 || it.alpha == 0.0) return 1.0;
-        return (double)tile * tile * it.alg.R * (double)((it.k + it.alg.kt - 1) / it.alg.kt + 1);
-    };
     auto tiles_of = [&](int i, int tile, int64_t* tm) {
         const F64BatchItem& it = items[i];
         const int64_t me = (it.m + it.alg.mt - 1) / it.alg.mt, ne = (it.n + it.alg.nt - 1) / it.alg.nt;
         *tm = (me + tile - 1) / tile;
         return *tm * ((ne + tile - 1) / tile);
     };
-    double total = 0.0;
-    int64_t tm = 0;
-    for (int i : order) total += item_fmas(i, 32) * (double)tiles_of(i, 32, &tm);
     std::vector<int> tile(count, 64);
-    for (int i : order) {
-        while (tile[i] > (mma ? 32 : 16) && item_fmas(i, tile[i]) > total / (double)ctas / 8) tile[i] /= 2;
-        cost[i] = item_fmas(i, tile[i]);
-    }
+    batch_tiles(items, order, mma, (int)std::min<int64_t>(ctas, sms), tiles_of, tile, cost);
+    int64_t tm = 0;
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
     std::vector<F64Prob> tab(order.size());
     int64_t items_total = 0;

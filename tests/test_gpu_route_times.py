@@ -74,3 +74,18 @@ def test_batch_of_unlike_small_c_updates(fmm, torch_cuda):
     b = fmm.make_batch(ps)
     ws = torch.empty(fmm.batch_workspace_size(b), dtype=torch.uint8, device="cuda")
     assert device_us(torch, lambda: fmm.batch_dgemm(b, workspace=ws)) < 900
+
+
+@pytest.mark.parametrize("alg,shapes,bound", [
+    ("222", [(2048, 2048, 2048, 1)], 15000),                    # tiles of 32: 13.6 ms; of 64 15.2, of 16 16.6
+    ("232", [(1912, 2475, 97, 1), (169, 242, 116, 0)], 1800),   # tiles of 64: 1.5 ms; of 16 2.0
+    ("222", [(512, 512, 512, 1)], 450),                         # tiles of 16: 0.32 ms; of 32 0.59, of 64 2.0
+])
+def test_fp64_batch_tiles(fmm, torch_cuda, alg, shapes, bound):
+    torch = torch_cuda
+    f = fmm.new_fmm(COEFFS / f"{alg}.txt")
+    ps = [{"A": operand(torch, m, k), "B": operand(torch, k, n), "C": operand(torch, m, n), "fmm": f if lv else None,
+           "levels": lv, "slices": 0} for m, n, k, lv in shapes]
+    b = fmm.make_batch(ps)
+    ws = torch.empty(max(fmm.batch_workspace_size(b), 256), dtype=torch.uint8, device="cuda")
+    assert device_us(torch, lambda: fmm.batch_dgemm(b, workspace=ws)) < bound
