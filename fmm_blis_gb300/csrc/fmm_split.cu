@@ -1888,14 +1888,19 @@ __device__ __forceinline__ double beta_c(double beta, const double* c)
     return beta == 0.0 ? 0.0 : beta * *c;
 }
 
-/* C updates of one C sub-block p = blockIdx.y: tiles of blockDim.x rows x 4
- * columns, a thread a row of a column group. For algorithms of more than 16
- * sub-blocks (scatter_all_better). */
+/* C updates of one C sub-block p = blockIdx.y: tiles of tr rows (a power of two,
+ * 8 to 128) x 512 / tr columns, a thread a row of a 4-column group. For
+ * algorithms of more than 16 sub-blocks (scatter_all_better). One thread
+ * gathers the sub-block's entries for each tile, which bounds narrow product
+ * grids: with 128 rows x 4 columns on 8 rows, 444 x2 on an 8 x 600 grid takes
+ * 8.5 ms a call instead of 5.2. */
+constexpr int kScatterThreads = 128;
+
 template <int FMT>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kScatterThreads)
 scatter_kernel(const int* __restrict__ tab, int r0, int nprod, int64_t m, int64_t n, double alpha, double beta,
                const ZView Z, const int* __restrict__ e_row, const int* __restrict__ f_col, double* __restrict__ C,
-               int64_t ldc)
+               int64_t ldc, int tr)
 {
     __shared__ double lam[kScatterMaxEnt];
     __shared__ int prod[kScatterMaxEnt];
@@ -1921,8 +1926,9 @@ scatter_kernel(const int* __restrict__ tab, int r0, int nprod, int64_t m, int64_
     }
     __syncthreads();
     const int ne = nsel;
-    const uint32_t me = (uint32_t)((m + t.mt - 1) / t.mt), tiles_i = (me + blockDim.x - 1) / blockDim.x;
-    const int i = (int)(blockIdx.x % tiles_i * blockDim.x + threadIdx.x), j = (int)(blockIdx.x / tiles_i) * 4;
+    const uint32_t me = (uint32_t)((m + t.mt - 1) / t.mt), tiles_i = (me + tr - 1) / tr;
+    const int i = (int)(blockIdx.x % tiles_i * tr + threadIdx.x % tr);
+    const int j = (int)(blockIdx.x / tiles_i * (kScatterThreads / tr) + threadIdx.x / tr) * 4;
     if ((ne == 0 && beta == 1.0) || i >= rl || j >= cl) return;
     double* cp = C + ro + i + (int64_t)(co + j) * ldc;
     double c[kScatterCols];
@@ -3075,9 +3081,13 @@ static void job_scatter(const SplitJob& j, int r0, int np, cudaStream_t st, bool
         return;
     }
     auto* k = j.fmt ? scatter_kernel<1> : scatter_kernel<0>;
-    k<<<dim3((unsigned)((j.d.me + 127) / 128 * ((j.d.ne + 3) / 4)), (unsigned)(j.alg.mt * j.alg.nt)), 128, 0, st>>>(
-        j.alg.tab, r0, np, j.m, j.n, j.alpha, job_beta(j, r0), job_zview(j), (const int*)(j.w + j.L.erow),
-        (const int*)(j.w + j.L.fcol), j.C, j.ldc);
+    int tr = 8;
+    while (tr < kScatterThreads && tr < j.d.me) tr *= 2;
+    const int64_t groups = kScatterThreads / tr;
+    k<<<dim3((unsigned)((j.d.me + tr - 1) / tr * (((j.d.ne + 3) / 4 + groups - 1) / groups)),
+             (unsigned)(j.alg.mt * j.alg.nt)),
+        kScatterThreads, 0, st>>>(j.alg.tab, r0, np, j.m, j.n, j.alpha, job_beta(j, r0), job_zview(j),
+                                  (const int*)(j.w + j.L.erow), (const int*)(j.w + j.L.fcol), j.C, j.ldc, tr);
     fmm_count_launch(1);
 }
 

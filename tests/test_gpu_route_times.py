@@ -89,3 +89,14 @@ def test_fp64_batch_tiles(fmm, torch_cuda, alg, shapes, bound):
     b = fmm.make_batch(ps)
     ws = torch.empty(max(fmm.batch_workspace_size(b), 256), dtype=torch.uint8, device="cuda")
     assert device_us(torch, lambda: fmm.batch_dgemm(b, workspace=ws)) < bound
+
+
+def test_c_updates_of_narrow_product_grids(fmm, torch_cuda):
+    """256 sub-blocks, an 8 x 600 product grid: 5.2 ms with a block's threads
+    on all of a tile's columns, 8.5 ms with 128 rows x 4 columns a block."""
+    torch = torch_cuda
+    m, n, k = 128, 9600, 768
+    f = fmm.new_fmm(COEFFS / "444.txt")
+    A, B, C = operand(torch, m, k), operand(torch, k, n), operand(torch, m, n)
+    ws = torch.empty(fmm.split_workspace_size(m, n, k, f, 2, 6), dtype=torch.uint8, device="cuda")
+    assert device_us(torch, lambda: fmm.split_dgemm(A, B, C, f, 2, 6, 1.0, 0.5, ws), reps=3, calls=2) < 7000
