@@ -2613,7 +2613,9 @@ static int job_bind_group(SplitJob& j, void* ws, size_t ws_bytes, int G)
 /* Timeline of the last host-buffer call (fmm_gpu_set_host_timeline): device
  * times, from the first copy's start, of A on the device, B on the device,
  * the first GEMM launch's start, the last GEMM launch's end, C's last column
- * chunk back on the host; plus the call's host wall time. */
+ * chunk back on the host; plus the call's host wall time. A call without
+ * overlapped schedule has the start and end of its whole device part for the
+ * GEMM's. */
 constexpr int kTimelinePoints = 5;
 std::atomic<bool> g_timeline{false};
 std::mutex g_timeline_mu;
@@ -3395,6 +3397,20 @@ static size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 constexpr int kChunks = 8;   /* B uploads and C downloads per host-buffer call */
 constexpr size_t kHostSimpleBytes = (size_t)32 << 20;   /* operands up to this size go without the overlapped schedules */
 
+/* A host-buffer call that ends early waits for its streams, so nothing is left
+ * in flight on the caller's memory or the kept buffers. */
+struct HostCallEnd {
+    SidePool* sp;
+    bool complete = false;   /* the call waited for its streams itself */
+    ~HostCallEnd()
+    {
+        if (complete) return;
+        for (cudaStream_t s : sp->s) cudaStreamSynchronize(s);
+        for (cudaStream_t s : sp->top) cudaStreamSynchronize(s);
+        cudaStreamSynchronize(sp->hi);
+    }
+};
+
 int fmm_split_host(const AlgView& alg, int64_t m, int64_t n, int64_t k, double alpha, const double* A,
                    int64_t lda, const double* B, int64_t ldb, double beta, double* C, int64_t ldc, int s, int fmt)
 {
@@ -3407,6 +3423,10 @@ int fmm_split_host(const AlgView& alg, int64_t m, int64_t n, int64_t k, double a
     const int64_t ka = std::max<int64_t>(k, 1);
     const bool trivial = k == 0 || alpha == 0.0;
     if (trivial && beta == 1.0) return FMM_OK;
+    /* what the split form refuses is refused before the first copy */
+    SplitJob j;
+    int rc = job_init(j, alg, m, n, k, alpha, nullptr, m, nullptr, ka, beta, nullptr, m, s, fmt);
+    if (rc != FMM_OK) return rc;
     const size_t bA = trivial ? 0 : align256(sizeof(double) * (size_t)(m * ka));
     const size_t bB = trivial ? 0 : align256(sizeof(double) * (size_t)(ka * n));
     const size_t bC = align256(sizeof(double) * (size_t)(m * n));
@@ -3417,6 +3437,11 @@ int fmm_split_host(const AlgView& alg, int64_t m, int64_t n, int64_t k, double a
     double* dB = (double*)(base + bA);
     double* dC = (double*)(base + bA + bB);
     uint8_t* ws = base + bA + bB + bC;
+    j.A = dA;
+    j.B = dB;
+    j.C = dC;
+    if ((rc = job_bind(j, ws, wsb, wsb)) != FMM_OK) return rc;
+    HostCallEnd end{sp};
     const size_t row = sizeof(double) * (size_t)m;
     auto ok = [](cudaError_t e) { return e == cudaSuccess; };
     const bool tline = g_timeline.load() && !trivial;
@@ -3436,7 +3461,7 @@ int fmm_split_host(const AlgView& alg, int64_t m, int64_t n, int64_t k, double a
         /* C := beta*C */
         if (beta != 0.0 && !ok(fmm_copy2d_async(dC, row, C, sizeof(double) * ldc, row, n, cudaMemcpyHostToDevice, st)))
             return FMM_ERR_CUDA;
-        if (int rc = fmm_scale_c(m, n, beta, dC, m, st); rc != FMM_OK) return rc;
+        if ((rc = fmm_scale_c(m, n, beta, dC, m, st)) != FMM_OK) return rc;
     } else {
         /* Small operands, or many sub-blocks: the device call between plain
          * copies. Overlapping the copies with the work saves at most their
@@ -3458,21 +3483,18 @@ int fmm_split_host(const AlgView& alg, int64_t m, int64_t n, int64_t k, double a
                 !ok(fmm_copy2d_async(dC, row, C, sizeof(double) * ldc, row, n, cudaMemcpyHostToDevice, st)))
                 return FMM_ERR_CUDA;
             mark(3, st);
-            if (int rc = split_launch_budget(alg, m, n, k, alpha, dA, m, dB, ka, beta, dC, m, s, fmt, ws, wsb, wsb, st,
-                                             sp); rc != FMM_OK)
+            if ((rc = split_launch_budget(alg, m, n, k, alpha, dA, m, dB, ka, beta, dC, m, s, fmt, ws, wsb, wsb, st,
+                                          sp)) != FMM_OK)
                 return rc;
             mark(4, st);
             if (!ok(fmm_copy2d_async(C, sizeof(double) * ldc, dC, row, row, n, cudaMemcpyDeviceToHost, st)))
                 return FMM_ERR_CUDA;
             mark(5, st);
             if (!ok(cudaStreamSynchronize(st))) return FMM_ERR_CUDA;
+            end.complete = true;
             if (tline) read_timeline();
             return cudaGetLastError() == cudaSuccess ? fmm_device_error_status() : FMM_ERR_CUDA;
         }
-        SplitJob j;
-        int rc = job_init(j, alg, m, n, k, alpha, dA, m, dB, ka, beta, dC, m, s, fmt);
-        if (rc != FMM_OK) return rc;
-        if ((rc = job_bind(j, ws, wsb, wsb)) != FMM_OK) return rc;
         const int G = j.L.group, nt = alg.nt;
         const bool one_group = G >= alg.R;
         cudaStream_t sb = sp->s[0];
@@ -3669,6 +3691,7 @@ int fmm_split_host(const AlgView& alg, int64_t m, int64_t n, int64_t k, double a
                 if (!ok(cudaStreamSynchronize(ds)) || !ok(cudaStreamSynchronize(cs)) || !ok(cudaStreamSynchronize(gst[0])) ||
                     !ok(cudaStreamSynchronize(gst[1])) || !ok(cudaStreamSynchronize(ss)) || !ok(cudaStreamSynchronize(sa)) || !ok(cudaStreamSynchronize(sb)))
                     return FMM_ERR_CUDA;
+                end.complete = true;
                 if (tline) read_timeline();
                 return cudaGetLastError() == cudaSuccess ? fmm_device_error_status() : FMM_ERR_CUDA;
             }
@@ -3756,6 +3779,7 @@ int fmm_split_host(const AlgView& alg, int64_t m, int64_t n, int64_t k, double a
             if (!ok(cudaEventRecord(sp->gate[1], cs)) || !ok(cudaStreamSynchronize(cs)) ||
                 !ok(cudaStreamSynchronize(st)))
                 return FMM_ERR_CUDA;
+            end.complete = true;
             if (tline) read_timeline();
             return cudaGetLastError() == cudaSuccess ? fmm_device_error_status() : FMM_ERR_CUDA;
         }
@@ -3763,6 +3787,7 @@ int fmm_split_host(const AlgView& alg, int64_t m, int64_t n, int64_t k, double a
     if (!ok(fmm_copy2d_async(C, sizeof(double) * ldc, dC, row, row, n, cudaMemcpyDeviceToHost, st)) ||
         !ok(cudaStreamSynchronize(st)))
         return FMM_ERR_CUDA;
+    end.complete = true;
     /* a kernel whose bounded wait expired left C incomplete: report it */
     return cudaGetLastError() == cudaSuccess ? fmm_device_error_status() : FMM_ERR_CUDA;
 }

@@ -273,9 +273,11 @@ int fmm_gpu_host_free(void* ptr);
  * last call: device milliseconds from the start of A's upload to A on the
  * device, B on the device, the first GEMM launch's start, the last GEMM
  * launch's end and C's last column chunk back on the host, then the call's
- * host wall time. Returns how many values it wrote. Recorded when the call
- * takes its overlapped path (all products' C updates in the element-major
- * form). No counterpart in the reference. */
+ * host wall time. Returns how many values it wrote. Small calls, whose copies
+ * do not overlap with the work, have the start and end of the whole device
+ * part in place of the GEMM's. Not recorded when the call overlaps its copies
+ * but not its C updates (more than 64 C sub-blocks). No counterpart in the
+ * reference. */
 void fmm_gpu_set_host_timeline(int enable);
 int fmm_gpu_read_host_timeline(double* ms, int count);
 
