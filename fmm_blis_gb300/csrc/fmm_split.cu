@@ -2546,9 +2546,9 @@ struct SplitJob {
     int fmt;       /* 0: BF16 slices, 1: FP8-E4M3 slices */
     bool trivial;  /* nothing beyond C := beta*C */
     bool classical; /* one product of coefficient 1: prep_kernel forms its operands */
-    int nunits, unit_kb; /* its tiles run as work units (0: whole) */
     WsLayout L;
     uint8_t* w;
+    uint8_t* z;    /* the group's Z planes; null: outside the workspace (job_bind) */
 };
 
 static int job_init(SplitJob& j, const AlgView& alg, int64_t m, int64_t n, int64_t k, double alpha,
@@ -2563,10 +2563,9 @@ static int job_init(SplitJob& j, const AlgView& alg, int64_t m, int64_t n, int64
     j.alpha = alpha; j.beta = beta;
     j.A = A; j.lda = lda; j.B = B; j.ldb = ldb; j.C = C; j.ldc = ldc;
     j.s = s;
-    j.w = nullptr;
+    j.w = j.z = nullptr;
     j.trivial = m == 0 || n == 0 || k == 0 || alpha == 0.0;
     j.classical = fmm_plain_classical(alg);
-    j.nunits = j.unit_kb = 0;
     if (j.trivial) return FMM_OK;
     if (alg.max_nnz_u > kPackMaxEnt || alg.max_nnz_v > kPackMaxEnt) return FMM_ERR_UNSUPPORTED;
     if (m > 0x7fffffffLL || n > 0x7fffffffLL) return FMM_ERR_UNSUPPORTED;
@@ -2580,15 +2579,20 @@ static int job_init(SplitJob& j, const AlgView& alg, int64_t m, int64_t n, int64
     return FMM_OK;
 }
 
-/* workspace of the job for a product group within `budget` bytes */
+/* Workspace of the job for a product group within `budget` bytes. The least
+ * accepted holds one product with 8 bytes of Z per element; FP8 Z planes of 7
+ * slices and more need 9 to 11, and where they do not fit j.z stays null. */
 static int job_bind(SplitJob& j, void* ws, size_t ws_bytes, size_t budget)
 {
     if (j.trivial) return FMM_OK;
     j.L = ws_layout(j.alg, j.m, j.n, j.k, j.s, budget, j.fmt);
     if ((int64_t)j.L.group * j.s * std::max(j.d.m_pad, j.d.n_pad) > 0x7fffffffLL) return FMM_ERR_UNSUPPORTED;
-    if (ws == nullptr || ws_bytes < j.L.total) return FMM_ERR_WORKSPACE;
+    const size_t least = j.L.group > 1 ? j.L.total
+                                       : std::min(j.L.total, j.L.z + 8 * (size_t)j.d.m_pad * (size_t)j.d.n_pad);
+    if (ws == nullptr || ws_bytes < least) return FMM_ERR_WORKSPACE;
     if (((uintptr_t)ws & 255) != 0) return FMM_ERR_ARG;
     j.w = (uint8_t*)ws;
+    j.z = ws_bytes < j.L.total ? nullptr : j.w + j.L.z;
     return FMM_OK;
 }
 
@@ -2601,6 +2605,7 @@ static int job_bind_group(SplitJob& j, void* ws, size_t ws_bytes, int G)
     if (ws == nullptr || ws_bytes < j.L.total) return FMM_ERR_WORKSPACE;
     if (((uintptr_t)ws & 255) != 0) return FMM_ERR_ARG;
     j.w = (uint8_t*)ws;
+    j.z = j.w + j.L.z;
     return FMM_OK;
 }
 
@@ -2869,7 +2874,7 @@ static int job_ebase(const SplitJob& j) { return 2 - job_db(j) * job_zlevel(j); 
 static ZView job_zview(const SplitJob& j)
 {
     ZView v;
-    v.base = j.w + j.L.z;
+    v.base = j.z;
     v.prod = (int64_t)z_bytes(j.d, j.s, j.fmt);
     v.nd = ZPlanes::of(j.s, job_zlevel(j), j.fmt).nd;
     v.group = z_group_bytes(j.d.m_pad, v.nd);
@@ -2898,7 +2903,7 @@ static int job_fill(const SplitJob& j, GemmProblem& gp, int np, int item_begin, 
         return FMM_ERR_CUDA;
     if (make_slice_map(&gp.tmB, sb, d.k_pad, (int64_t)np * j.s * d.n_pad, pair ? kTileN / 2 : kTileN, j.fmt) != FMM_OK)
         return FMM_ERR_CUDA;
-    gp.Z = j.w + j.L.z + (size_t)r_first * z_bytes(d, j.s, j.fmt);
+    gp.Z = j.z + (size_t)r_first * z_bytes(d, j.s, j.fmt);
     gp.s = j.s;
     gp.zlevel = job_zlevel(j);
     const ZPlanes zp = ZPlanes::of(j.s, gp.zlevel, j.fmt);
@@ -3205,12 +3210,14 @@ static int split_overlap(SplitJob& j, const OverlapPlan& o, void* ws, cudaStream
     const int R = j.alg.R, G1 = o.L1.group, G2 = R - G1;
     j.L = o.L1;
     j.w = (uint8_t*)ws;
+    j.z = j.w + j.L.z;
     SplitJob j2 = j;
     j2.L.erow += o.shift;
     j2.L.fcol += o.shift;
     j2.L.sa += o.shift;
     j2.L.sb += o.shift;
     j2.L.z += o.shift;
+    j2.z += o.shift;
     j2.L.total += o.shift;
     /* the GEMMs on the greatest-priority stream, so the block scheduler
      * places their CTAs first and the side work fills the room they leave */
@@ -3327,6 +3334,21 @@ static int split_classical(SplitJob& j, bool alloc, cudaStream_t st)
     return rc;
 }
 
+/* the product groups of a bound job, one after the other */
+static int split_groups(SplitJob& j, cudaStream_t st, SidePool* sp)
+{
+    int rc = job_prologue(j, st, sp);
+    if (rc != FMM_OK) return rc;
+    const int G = j.L.group;
+    for (int r0 = 0; r0 < j.alg.R; r0 += G) {
+        const int np = std::min(G, j.alg.R - r0);
+        if ((rc = job_pack(j, r0, np, st, sp)) != FMM_OK) return rc;
+        if ((rc = job_gemm(j, np, st)) != FMM_OK) return rc;
+        job_scatter(j, r0, np, st);
+    }
+    return cudaGetLastError() == cudaSuccess ? FMM_OK : FMM_ERR_CUDA;
+}
+
 static int split_launch_budget(const AlgView& alg, int64_t m, int64_t n, int64_t k, double alpha,
                                const double* A, int64_t lda, const double* B, int64_t ldb, double beta,
                                double* C, int64_t ldc, int s, int fmt, void* ws, size_t ws_bytes, size_t budget,
@@ -3339,17 +3361,20 @@ static int split_launch_budget(const AlgView& alg, int64_t m, int64_t n, int64_t
         const OverlapPlan o = overlap_plan(alg, j.d, m, n, s, fmt, std::min(ws_bytes, budget));
         if (o.ok) return split_overlap(j, o, ws, st, sp);
     }
-    if (!j.trivial && (rc = job_bind(j, ws, ws_bytes, budget)) != FMM_OK) return rc;
-    if (!j.trivial && j.classical) return split_classical(j, sp != nullptr, st);
-    if ((rc = job_prologue(j, st, sp)) != FMM_OK || j.trivial) return rc;
-    const int G = j.L.group;
-    for (int r0 = 0; r0 < alg.R; r0 += G) {
-        const int np = std::min(G, alg.R - r0);
-        if ((rc = job_pack(j, r0, np, st, sp)) != FMM_OK) return rc;
-        if ((rc = job_gemm(j, np, st)) != FMM_OK) return rc;
-        job_scatter(j, r0, np, st);
+    if (j.trivial) return job_prologue(j, st);
+    if ((rc = job_bind(j, ws, ws_bytes, budget)) != FMM_OK) return rc;
+    void* zbuf = nullptr;
+    if (j.z == nullptr) {
+        const cudaMemPool_t pool = fmm_temp_pool();
+        if (pool == nullptr || cudaMallocFromPoolAsync(&zbuf, z_bytes(j.d, s, fmt), pool, st) != cudaSuccess) {
+            cudaGetLastError();
+            return FMM_ERR_WORKSPACE;
+        }
+        j.z = (uint8_t*)zbuf;
     }
-    return cudaGetLastError() == cudaSuccess ? FMM_OK : FMM_ERR_CUDA;
+    rc = j.classical ? split_classical(j, sp != nullptr, st) : split_groups(j, st, sp);
+    if (zbuf != nullptr && cudaFreeAsync(zbuf, st) != cudaSuccess && rc == FMM_OK) rc = FMM_ERR_CUDA;
+    return rc;
 }
 
 /* ---------------------------------------------------------------------------

@@ -174,9 +174,11 @@ int fmm_gpu_strassen_ab(double alpha, const double* A, int64_t lda,
  * added into C in one pass), and this size holds the largest group that fits
  * in 32 GiB; when that is all R products, it holds two groups of ceil(R/2)
  * instead, whose packs and C updates overlap the other group's GEMM. Any
- * smaller workspace that holds one product's digit slices and level
- * accumulators also works, with smaller groups; the result is the same bit
- * for bit whatever the grouping. */
+ * smaller workspace that holds one product's digit slices and 8 bytes of
+ * level accumulators per element also works, with smaller groups; the result
+ * is the same bit for bit whatever the grouping. (FP8 slices from 7 up use 9
+ * to 11 bytes; with the least workspace the call takes the accumulators as a
+ * stream-ordered temporary and returns FMM_ERR_WORKSPACE without memory.) */
 size_t fmm_gpu_split_workspace_size(const fmm_t* fmm, int levels,
                                     int64_t m, int64_t n, int64_t k,
                                     int slices);
