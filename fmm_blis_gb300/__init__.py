@@ -127,6 +127,8 @@ def lib() -> ctypes.CDLL:
     L.fmm_gpu_split_workspace_size.argtypes = [pf, ci, i64, i64, i64, ci]
     L.fmm_gpu_split_workspace_size_fmt.restype = ctypes.c_size_t
     L.fmm_gpu_split_workspace_size_fmt.argtypes = [pf, ci, i64, i64, i64, ci, ci]
+    L.fmm_gpu_split_full_workspace_size.restype = ctypes.c_size_t
+    L.fmm_gpu_split_full_workspace_size.argtypes = [pf, ci, i64, i64, i64, ci, ci]
     L.fmm_gpu_split_dgemm_fmt.restype = ci
     L.fmm_gpu_split_dgemm_fmt.argtypes = [pf, ci, i64, i64, i64, dbl, vp, i64, vp, i64, dbl, vp, i64, ci, ci, vp,
                                           ctypes.c_size_t, vp]
@@ -352,10 +354,13 @@ def _fmt(fmt) -> int:
     return int(fmt)
 
 
-def split_workspace_size(m: int, n: int, k: int, fmm: FmmT | None, levels: int, slices: int, fmt="bf16") -> int:
+def split_workspace_size(m: int, n: int, k: int, fmm: FmmT | None, levels: int, slices: int, fmt="bf16",
+                         full: bool = False) -> int:
+    """Recommended workspace of a split call; full: with room for what the
+    call would otherwise take as a temporary (captured calls take none)."""
     pf = ctypes.byref(fmm) if fmm is not None else None
-    return int(lib().fmm_gpu_split_workspace_size_fmt(pf, levels if fmm is not None else 0, m, n, k, slices,
-                                                      _fmt(fmt)))
+    size = lib().fmm_gpu_split_full_workspace_size if full else lib().fmm_gpu_split_workspace_size_fmt
+    return int(size(pf, levels if fmm is not None else 0, m, n, k, slices, _fmt(fmt)))
 
 
 def split_dgemm(A, B, C, fmm: FmmT | None = None, levels: int = 1, slices: int = 6, alpha: float = 1.0,

@@ -470,8 +470,8 @@ extern "C" size_t fmm_gpu_split_workspace_size(const fmm_t* fmm, int levels, int
     return fmm_gpu_split_workspace_size_fmt(fmm, levels, m, n, k, slices, FMM_SPLIT_BF16);
 }
 
-extern "C" size_t fmm_gpu_split_workspace_size_fmt(const fmm_t* fmm, int levels, int64_t m, int64_t n, int64_t k,
-                                                   int slices, int format)
+static size_t split_workspace_size(const fmm_t* fmm, int levels, int64_t m, int64_t n, int64_t k, int slices,
+                                   int format, bool full)
 {
     if (format != FMM_SPLIT_BF16 && format != FMM_SPLIT_FP8_E4M3) return 0;
     if (m < 0 || n < 0 || k < 0 || slices < 2 || slices > (format ? 12 : 8)) return 0;
@@ -480,9 +480,22 @@ extern "C" size_t fmm_gpu_split_workspace_size_fmt(const fmm_t* fmm, int levels,
     if (fmm_flatten(fmm, levels, &flat, &owned) != FMM_OK) return 0;
     AlgView v = {};
     v.mt = flat.m_tilde; v.kt = flat.k_tilde; v.nt = flat.n_tilde; v.R = flat.R;
-    size_t b = fmm_split_ws_bytes(v, m, n, k, slices, format);
+    size_t b = full ? fmm_split_full_ws_bytes(v, m, n, k, slices, format)
+                    : fmm_split_ws_bytes(v, m, n, k, slices, format);
     if (owned) free_fmm(flat);
     return b;
+}
+
+extern "C" size_t fmm_gpu_split_workspace_size_fmt(const fmm_t* fmm, int levels, int64_t m, int64_t n, int64_t k,
+                                                   int slices, int format)
+{
+    return split_workspace_size(fmm, levels, m, n, k, slices, format, false);
+}
+
+extern "C" size_t fmm_gpu_split_full_workspace_size(const fmm_t* fmm, int levels, int64_t m, int64_t n, int64_t k,
+                                                    int slices, int format)
+{
+    return split_workspace_size(fmm, levels, m, n, k, slices, format, true);
 }
 
 extern "C" int fmm_gpu_split_dgemm(const fmm_t* fmm, int levels, int64_t m, int64_t n, int64_t k,

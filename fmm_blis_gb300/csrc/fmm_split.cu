@@ -2529,6 +2529,16 @@ size_t fmm_split_ws_bytes(const AlgView& alg, int64_t m, int64_t n, int64_t k, i
     return two <= kGroupBudget ? std::max(L.total, two) : L.total;
 }
 
+/* the same with room for a classical problem's work units (whichever way the
+ * pair threshold stands at the call) */
+size_t fmm_split_full_ws_bytes(const AlgView& alg, int64_t m, int64_t n, int64_t k, int slices, int fmt)
+{
+    const size_t b = fmm_split_ws_bytes(alg, m, n, k, slices, fmt);
+    if (m == 0 || n == 0 || k == 0 || alg.R != 1 || alg.mt != 1 || alg.kt != 1 || alg.nt != 1) return b;
+    const Dims d = dims_of(alg, m, n, k, fmt);
+    return b + std::max(unit_plan(d, slices, fmt, false).bytes, unit_plan(d, slices, fmt, true).bytes);
+}
+
 /* One split-form GEMM problem being executed: its algorithm, geometry,
  * operands and the part of the workspace it uses. */
 struct SplitJob {
@@ -3287,18 +3297,34 @@ static int job_prep(SplitJob& j, cudaStream_t st)
     });
 }
 
+/* whether work enqueued on st is being captured into a graph */
+static bool capturing(cudaStream_t st)
+{
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &c) != cudaSuccess) cudaGetLastError();
+    return c != cudaStreamCaptureStatusNone;
+}
+
 /* A classical GEMM: one launch for the operands, one for the tiles (or their
- * work units), one for C. The units' planes are a stream-ordered temporary
- * (with `alloc`; without it, or without memory, the tiles run whole). */
-static int split_classical(SplitJob& j, bool alloc, cudaStream_t st)
+ * work units), one for C. With `units`, the units' planes lie behind the job's
+ * part of the workspace where the caller's is large enough
+ * (fmm_split_full_ws_bytes), else they are a stream-ordered temporary. Without
+ * memory, and in a captured call whose workspace has no room, the tiles run
+ * whole: a graph with an allocation node could not be cloned or instantiated
+ * twice. */
+static int split_classical(SplitJob& j, size_t ws_bytes, bool units, cudaStream_t st)
 {
     if (int rc = job_prep(j, st); rc != FMM_OK) return rc;
     UnitPlan up;
-    if (alloc) up = unit_plan(j.d, j.s, j.fmt, job_pair(j));
-    void* planes = nullptr;
+    if (units) up = unit_plan(j.d, j.s, j.fmt, job_pair(j));
+    uint8_t* spare = nullptr;   /* planes in the workspace */
+    void* planes = nullptr;     /* planes of their own */
     if (up.nunits != 0) {
-        const cudaMemPool_t pool = fmm_temp_pool();
-        if (pool == nullptr || cudaMallocFromPoolAsync(&planes, up.bytes, pool, st) != cudaSuccess) {
+        cudaMemPool_t pool = nullptr;
+        if (ws_bytes >= j.L.total + up.bytes) {
+            spare = j.w + j.L.total;
+        } else if (capturing(st) || (pool = fmm_temp_pool()) == nullptr ||
+                   cudaMallocFromPoolAsync(&planes, up.bytes, pool, st) != cudaSuccess) {
             cudaGetLastError();
             up = UnitPlan();
         }
@@ -3320,17 +3346,17 @@ static int split_classical(SplitJob& j, bool alloc, cudaStream_t st)
     }
     gp.nunits = up.nunits;
     gp.unit_kb = up.unit_kb;
-    gp.Z = (uint8_t*)planes;
+    gp.Z = spare ? spare : (uint8_t*)planes;
     int rc = launch_gemm(gl, job_items(j, 1) * up.nunits, 1, st, false, true);
     if (rc == FMM_OK) {
         rc = launch_after(scatter_units_kernel, dim3((unsigned)((j.m + 31) / 32), (unsigned)((j.n + 15) / 16)), 128, 0,
-                          st, (int)j.m, (int)j.n, j.alpha, j.beta, (const int4*)planes, (int)j.d.m_pad,
+                          st, (int)j.m, (int)j.n, j.alpha, j.beta, (const int4*)gp.Z, (int)j.d.m_pad,
                           (int)j.d.n_pad, j.s, gp.nkb, up.unit_kb, up.nunits, job_zlevel(j), job_db(j), job_ebase(j),
                           (const int*)(j.w + j.L.erow), (const int*)(j.w + j.L.fcol), j.C, j.ldc);
         fmm_count_launch(1);
         if (rc == FMM_OK && cudaGetLastError() != cudaSuccess) rc = FMM_ERR_CUDA;
     }
-    if (cudaFreeAsync(planes, st) != cudaSuccess && rc == FMM_OK) rc = FMM_ERR_CUDA;
+    if (planes != nullptr && cudaFreeAsync(planes, st) != cudaSuccess && rc == FMM_OK) rc = FMM_ERR_CUDA;
     return rc;
 }
 
@@ -3372,7 +3398,7 @@ static int split_launch_budget(const AlgView& alg, int64_t m, int64_t n, int64_t
         }
         j.z = (uint8_t*)zbuf;
     }
-    rc = j.classical ? split_classical(j, sp != nullptr, st) : split_groups(j, st, sp);
+    rc = j.classical ? split_classical(j, ws_bytes, sp != nullptr, st) : split_groups(j, st, sp);
     if (zbuf != nullptr && cudaFreeAsync(zbuf, st) != cudaSuccess && rc == FMM_OK) rc = FMM_ERR_CUDA;
     return rc;
 }

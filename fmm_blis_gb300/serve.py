@@ -180,7 +180,7 @@ class _GraphSlot:
         self.A = torch.zeros((bk, bm), dtype=torch.float64, device=dev).t()
         self.B = torch.zeros((bn, bk), dtype=torch.float64, device=dev).t()
         self.C = torch.zeros((bn, bm), dtype=torch.float64, device=dev).t()
-        self.ws = torch.empty(max(fmm.split_workspace_size(bm, bn, bk, None, 0, slices, fmt), 256),
+        self.ws = torch.empty(max(fmm.split_workspace_size(bm, bn, bk, None, 0, slices, fmt, full=True), 256),
                               dtype=torch.uint8, device=dev)
         self.busy_event = None
         with torch.cuda.stream(stream):

@@ -191,9 +191,11 @@ size_t fmm_gpu_split_workspace_size(const fmm_t* fmm, int levels,
  * `workspace` (256-byte aligned) holds at least one product's slices and
  * level accumulators; fmm_gpu_split_workspace_size gives the recommended
  * size. A classical problem with too few tiles to fill the GPU also takes a
- * stream-ordered temporary of at most 128 MiB from the library's memory pool
- * (without it the tiles run whole; the result is the same). Asynchronous on
- * `stream`. */
+ * stream-ordered temporary of at most 128 MiB from the library's memory pool,
+ * unless the workspace has fmm_gpu_split_full_workspace_size bytes. Without
+ * memory for it, and in a call captured into a graph (which then holds no
+ * allocation node), the tiles run whole, slower, with the same result.
+ * Asynchronous on `stream`. */
 int fmm_gpu_split_dgemm(const fmm_t* fmm, int levels,
                         int64_t m, int64_t n, int64_t k,
                         double alpha, const double* A, int64_t lda,
@@ -210,6 +212,13 @@ int fmm_gpu_split_dgemm(const fmm_t* fmm, int levels,
 size_t fmm_gpu_split_workspace_size_fmt(const fmm_t* fmm, int levels,
                                         int64_t m, int64_t n, int64_t k,
                                         int slices, int format);
+
+/* The recommended workspace with everything in it that a call would otherwise
+ * take as a temporary: for callers that keep one workspace, such as a captured
+ * call. Equal to fmm_gpu_split_workspace_size_fmt but for classical problems. */
+size_t fmm_gpu_split_full_workspace_size(const fmm_t* fmm, int levels,
+                                         int64_t m, int64_t n, int64_t k,
+                                         int slices, int format);
 
 /* fmm_gpu_split_dgemm with a slice format: FMM_SPLIT_BF16 (identical to
  * fmm_gpu_split_dgemm) or FMM_SPLIT_FP8_E4M3: 5-bit digits in [-16, 16]

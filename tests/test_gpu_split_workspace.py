@@ -49,3 +49,58 @@ def test_fp8_least_workspace(fmm, alg, levels, m, n, k, s, way):
         assert accepted
         assert np.array_equal(to_host(dC), to_host(want))
     assert fmm.take_device_error() == 0
+
+
+MEM_ALLOC, MEM_FREE = 10, 11   # CU_GRAPH_NODE_TYPE_MEM_ALLOC, _MEM_FREE
+
+
+@pytest.mark.parametrize("m,n,k,s,fmt", [(300, 700, 450, 6, "bf16"), (64, 64, 64, 7, "bf16"), (1100, 260, 300, 9, "fp8"),
+                                         (128, 128, 16384, 6, "bf16")])
+@pytest.mark.parametrize("full", [False, True])
+def test_captured_call_holds_no_allocation(fmm, m, n, k, s, fmt, full):
+    """A captured classical call on the caller's workspace is a graph without
+    allocation nodes, so it can be cloned and have two executables at a time;
+    both give the plain call's bits."""
+    import ctypes
+
+    import torch
+    cu = ctypes.CDLL("libcuda.so.1")
+    A, B, C = to_dev(rand(m, k, 51)), to_dev(rand(k, n, 52)), rand(m, n, 53)
+    want = to_dev(C)
+    fmm.split_dgemm(A, B, want, None, 0, s, alpha=-0.75, beta=0.5, fmt=fmt)
+    ws = torch.empty(fmm.split_workspace_size(m, n, k, None, 0, s, fmt, full=full), dtype=torch.uint8, device="cuda")
+    dC = to_dev(C)
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    h, graph = ctypes.c_void_p(st.cuda_stream), ctypes.c_void_p()
+    assert cu.cuStreamBeginCapture_v2(h, 2) == 0   # CU_STREAM_CAPTURE_MODE_RELAXED
+    try:
+        fmm.split_dgemm(A, B, dC, None, 0, s, alpha=-0.75, beta=0.5, workspace=ws, stream=st, fmt=fmt)
+    finally:
+        assert cu.cuStreamEndCapture(h, ctypes.byref(graph)) == 0
+    count = ctypes.c_size_t()
+    assert cu.cuGraphGetNodes(graph, None, ctypes.byref(count)) == 0
+    nodes = (ctypes.c_void_p * count.value)()
+    assert cu.cuGraphGetNodes(graph, nodes, ctypes.byref(count)) == 0
+    kinds = []
+    for x in nodes:
+        kind = ctypes.c_int()
+        assert cu.cuGraphNodeGetType(ctypes.c_void_p(x), ctypes.byref(kind)) == 0
+        kinds.append(kind.value)
+    assert kinds and MEM_ALLOC not in kinds and MEM_FREE not in kinds
+    clone = ctypes.c_void_p()
+    assert cu.cuGraphClone(ctypes.byref(clone), graph) == 0
+    execs = []
+    for g in (graph, clone, graph):
+        e = ctypes.c_void_p()
+        assert cu.cuGraphInstantiateWithFlags(ctypes.byref(e), g, ctypes.c_ulonglong(0)) == 0
+        execs.append(e)
+    for e in execs:
+        dC.copy_(to_dev(C))
+        torch.cuda.synchronize()
+        assert cu.cuGraphLaunch(e, h) == 0
+        st.synchronize()
+        assert np.array_equal(to_host(dC), to_host(want))
+        assert cu.cuGraphExecDestroy(e) == 0
+    assert cu.cuGraphDestroy(graph) == 0 and cu.cuGraphDestroy(clone) == 0
+    assert fmm.take_device_error() == 0
