@@ -1117,12 +1117,28 @@ cudaMemPool_t g_pools[64];
 
 }  // namespace
 
+namespace {
+/* puts the thread's stream capture mode back */
+struct CaptureModeBack {
+    cudaStreamCaptureMode mode;
+    ~CaptureModeBack()
+    {
+        cudaStreamCaptureMode m = mode;
+        cudaThreadExchangeStreamCaptureMode(&m);
+    }
+};
+}  // namespace
+
 cudaMemPool_t fmm_temp_pool()
 {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
     std::lock_guard<std::mutex> lk(g_pool_mu);
     if (g_pools[dev] == nullptr) {
+        /* a pool may be made while the calling thread captures a stream: no stream's work is part of it */
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return nullptr;
+        const CaptureModeBack back{mode};
         cudaMemPoolProps props;
         memset(&props, 0, sizeof(props));
         props.allocType = cudaMemAllocationTypePinned;
