@@ -1789,6 +1789,27 @@ struct ZView {
 
 constexpr int kScatterCols = 4;   /* columns per thread: one column group of Z */
 
+/* The 5-bit digits of two columns in the 16-bit halves of x[p], plane zmin + p,
+ * absent ones zero: three digits of both columns to a word, then each
+ * column's Z from its high word. Digit by digit in 64 bits the conversion took
+ * twice the instructions and bounded the C updates per sub-block (the ALU pipe
+ * 75% busy): 333 x2 at 3101 x 2244 x 73, 5 slices, 1590 us a call, 1400 now. */
+struct Fp8Pair {
+    uint32_t a, b, c;
+
+    __device__ __forceinline__ explicit Fp8Pair(const uint32_t (&x)[7])
+        : a((x[0] * 32 + x[1]) * 32 + x[2]), b((x[3] * 32 + x[4]) * 32 + x[5]), c(x[6])
+    {
+    }
+    /* column u: hi * 32^7 + its seven digits, down to the nd that there are */
+    __device__ __forceinline__ int64_t value(int hi, int u, int nd) const
+    {
+        const uint32_t d0 = u ? a >> 16 : a & 0xffffu, d1 = u ? b >> 16 : b & 0xffffu, d2 = u ? c >> 16 : c & 0xffffu;
+        const uint32_t low = d0 * (1u << 20) + d1 * 32 + d2, high = (uint32_t)hi * 8 + (d0 >> 12);
+        return (int64_t)(((uint64_t)high << 32) | low) >> (5 * (7 - nd));
+    }
+};
+
 /* One row of a column group of one product: the loads (one int4, nd words, the
  * exponents), then the four Z values. FMT 0: at most four byte digits below
  * the high word, absent ones zero (Z counts in units of level G whatever the
@@ -1827,14 +1848,16 @@ struct ZRow {
             for (int u = 0; u < 4; ++u)
                 M[u] = i64_to_double_scaled((int64_t)(((uint64_t)(uint32_t)h[u] << 32) | lo[u]), er + fc[u]);
         } else {
+            uint32_t x[7], y[7];   /* columns 0 and 2, 1 and 3 */
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                uint64_t lo = 0;
-#pragma unroll
-                for (int p = 0; p < NP; ++p)
-                    if (p < v.nd) lo = (lo << 5) | __byte_perm(w[p], 0u, 0x4440u + (unsigned)u);
-                M[u] = i64_to_double_scaled((int64_t)(((uint64_t)(int64_t)h[u] << (5 * v.nd)) | lo), er + fc[u]);
+            for (int p = 0; p < NP; ++p) {
+                x[p] = __byte_perm(w[p], 0u, 0x4240u);
+                y[p] = __byte_perm(w[p], 0u, 0x4341u);
             }
+            const Fp8Pair even(x), odd(y);
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                M[u] = i64_to_double_scaled((u & 1 ? odd : even).value(h[u], u >> 1, v.nd), er + fc[u]);
         }
     }
 };
@@ -1869,14 +1892,12 @@ struct ZPair {
             for (int u = 0; u < 2; ++u)
                 M[u] = i64_to_double_scaled((int64_t)(((uint64_t)(uint32_t)h[u] << 32) | lo[u]), er + fc[u]);
         } else {
+            uint32_t x[7];
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                uint64_t lo = 0;
+            for (int p = 0; p < NP; ++p) x[p] = __byte_perm(w[p], 0u, 0x4140u);
+            const Fp8Pair both(x);
 #pragma unroll
-                for (int p = 0; p < NP; ++p)
-                    if (p < v.nd) lo = (lo << 5) | __byte_perm(w[p], 0u, 0x4440u + (unsigned)u);
-                M[u] = i64_to_double_scaled((int64_t)(((uint64_t)(int64_t)h[u] << (5 * v.nd)) | lo), er + fc[u]);
-            }
+            for (int u = 0; u < 2; ++u) M[u] = i64_to_double_scaled(both.value(h[u], u, v.nd), er + fc[u]);
         }
     }
 };
@@ -1969,6 +1990,32 @@ scatter_kernel(const int* __restrict__ tab, int r0, int nprod, int64_t m, int64_
 constexpr int kScatterAllSmem = 32 * 1024;   /* cs[] budget: P * threads * columns * 8 */
 constexpr int kScatterAllMaxSmem = 96 * 1024;
 
+/* scatter_all_body for one sub-block fed by one product (the classical split GEMM): no shared memory, the C
+ * values in registers; HBM-bound (Z and C). l: alpha times W. Tiles of blockDim.x rows x 4 columns. */
+template <int FMT>
+__device__ __forceinline__ void scatter_one_body(int64_t n, double l, double beta, const ZView& Z,
+                                                 const int* __restrict__ e_row, const int* __restrict__ f_col,
+                                                 double* __restrict__ C, int64_t ldc, int c0, int c1, uint32_t vb,
+                                                 uint32_t vg, uint32_t i_lo, uint32_t rows)
+{
+    const int T = (int)blockDim.x, jl = min((int)n, c1);
+    const uint32_t tiles_i = (rows + T - 1) / T, tiles = tiles_i * (uint32_t)((c1 + 3) / 4 - c0 / 4);
+    for (uint32_t x = vb; x < tiles; x += vg) {
+        const int i = (int)(i_lo + x % tiles_i * T) + (int)threadIdx.x, j = (int)(c0 / 4 + x / tiles_i) * 4;
+        if (i >= (int)(i_lo + rows)) continue;
+        ZRow<FMT> z;
+        z.load(Z, e_row, f_col, 0, i, j);
+        double* cp = C + i + (int64_t)j * ldc;
+        double c[kScatterCols], M[kScatterCols];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) c[u] = j + u >= c0 && j + u < jl ? beta_c(beta, cp + u * ldc) : 0.0;
+        z.values(Z, M);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (j + u >= c0 && j + u < jl) cp[u * ldc] = fma(l, M[u], c[u]);
+    }
+}
+
 /* vb, vg: the block's index among the vg blocks that share the element range */
 template <int FMT, int NC>
 __device__ __forceinline__ void scatter_all_body(const int* __restrict__ tab, int r0, int nprod, int64_t m, int64_t n,
@@ -1978,50 +2025,35 @@ __device__ __forceinline__ void scatter_all_body(const int* __restrict__ tab, in
                                                  uint32_t vg, uint32_t i_lo = 0, uint32_t i_rows = 0)
 {
     extern __shared__ __align__(16) double sm_all[];
-    __shared__ int geo[4][64];           /* per sub-block p: ro, rl, co, cl */
     const Tab t = tab_view(tab);
     const int P = t.mt * t.nt, T = (int)blockDim.x, tid = (int)threadIdx.x;
     const int eb = t.w_off[r0], E = t.w_off[r0 + nprod] - eb;
     const uint32_t me = (uint32_t)((m + t.mt - 1) / t.mt);
     const uint32_t rows = i_rows ? i_rows : me;
-    const bool one = P == 1 && E == 1 && nprod == 1;
-    const int TR = one ? T : T * NC / 4;                                  /* rows per tile */
-    const uint32_t tiles_i = (rows + TR - 1) / TR;
-    const uint32_t tiles = tiles_i * (uint32_t)((c1 + 3) / 4 - c0 / 4);   /* row tiles fastest */
-    if (one) {
-        /* one sub-block fed by one product (the classical split GEMM): no
-         * shared memory, the C values in registers; HBM-bound (Z and C) */
-        const double l = alpha * (double)t.w_ent[2 * eb + 1];
-        const int jl = min((int)n, c1);
-        for (uint32_t x = vb; x < tiles; x += vg) {
-            const int i = (int)(i_lo + x % tiles_i * T) + tid, j = (int)(c0 / 4 + x / tiles_i) * 4;
-            if (i >= (int)(i_lo + rows)) continue;
-            ZRow<FMT> z;
-            z.load(Z, e_row, f_col, 0, i, j);
-            double* cp = C + i + (int64_t)j * ldc;
-            double c[kScatterCols], M[kScatterCols];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) c[u] = j + u >= c0 && j + u < jl ? beta_c(beta, cp + u * ldc) : 0.0;
-            z.values(Z, M);
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (j + u >= c0 && j + u < jl) cp[u * ldc] = fma(l, M[u], c[u]);
-        }
+    if (P == 1 && E == 1 && nprod == 1) {
+        scatter_one_body<FMT>(n, alpha * (double)t.w_ent[2 * eb + 1], beta, Z, e_row, f_col, C, ldc, c0, c1, vb, vg, i_lo,
+                              rows);
         return;
     }
+    const int TR = T * NC / 4;                                            /* rows per tile */
+    const uint32_t tiles_i = (rows + TR - 1) / TR;
+    const uint32_t tiles = tiles_i * (uint32_t)((c1 + 3) / 4 - c0 / 4);   /* row tiles fastest */
     constexpr int NH = NC / 2;           /* column pairs of a thread */
     double2* cs = (double2*)sm_all;      /* [P][NH][T] */
     double* lam = sm_all + P * T * NC;   /* [E] */
     int* pidx = (int*)(lam + E);         /* [E] */
     int* off = pidx + E;                 /* [nprod + 1] */
+    int4* geo = (int4*)(cs + P * NH * T + (E * 12 + (nprod + 1) * 4 + 15) / 16);   /* [P]: ro, rl, co, cl */
     for (int x = tid; x < E; x += T) {
         pidx[x] = t.w_ent[2 * (eb + x)];
         lam[x] = alpha * (double)t.w_ent[2 * (eb + x) + 1];
     }
     for (int x = tid; x <= nprod; x += T) off[x] = t.w_off[r0 + x] - eb;
     for (int p = tid; p < P; p += T) {
-        fmm_part_geom32((int)m, t.mt, p / t.nt, &geo[0][p], &geo[1][p]);
-        fmm_part_geom32((int)n, t.nt, p % t.nt, &geo[2][p], &geo[3][p]);
+        int4 g;
+        fmm_part_geom32((int)m, t.mt, p / t.nt, &g.x, &g.y);
+        fmm_part_geom32((int)n, t.nt, p % t.nt, &g.z, &g.w);
+        geo[p] = g;
     }
     __syncthreads();
     const int tr = tid % TR, th = tid / TR * NC;     /* row of the tile, first of the thread's columns */
@@ -2033,8 +2065,9 @@ __device__ __forceinline__ void scatter_all_body(const int* __restrict__ tab, in
         /* elements outside a smaller sub-block or the column range are
          * carried along as zeros and not stored */
         for (int p = 0; p < P; ++p) {
-            const int jl = i < geo[1][p] ? min(geo[3][p], c1) : 0;
-            const double* cp = C + geo[0][p] + i + (int64_t)(geo[2][p] + j) * ldc;
+            const int4 g = geo[p];
+            const int jl = i < g.y ? min(g.w, c1) : 0;
+            const double* cp = C + g.x + i + (int64_t)(g.z + j) * ldc;
             double c[NC];
 #pragma unroll
             for (int u = 0; u < NC; ++u) c[u] = j + u >= c0 && j + u < jl ? beta_c(beta, cp + u * ldc) : 0.0;
@@ -2065,8 +2098,9 @@ __device__ __forceinline__ void scatter_all_body(const int* __restrict__ tab, in
             }
         }
         for (int p = 0; p < P; ++p) {
-            const int jl = i < geo[1][p] ? min(geo[3][p], c1) : 0;
-            double* cp = C + geo[0][p] + i + (int64_t)(geo[2][p] + j) * ldc;
+            const int4 g = geo[p];
+            const int jl = i < g.y ? min(g.w, c1) : 0;
+            double* cp = C + g.x + i + (int64_t)(g.z + j) * ldc;
             double2 a[NH];
 #pragma unroll
             for (int h = 0; h < NH; ++h) a[h] = cs[(p * NH + h) * T + tid];
@@ -2082,8 +2116,14 @@ __device__ __forceinline__ void scatter_all_body(const int* __restrict__ tab, in
 /* columns per thread of the element-major C update of P sub-blocks: see above */
 __host__ __device__ __forceinline__ int scatter_cols(int P) { return P <= 6 ? 4 : 2; }
 
+/* its dynamic shared memory: the values of T threads, E entries and nprod offsets of the group, the sub-blocks' places */
+size_t scatter_all_smem(int P, int T, int E, int nprod)
+{
+    return (size_t)P * T * scatter_cols(P) * 8 + ((size_t)E * 12 + (size_t)(nprod + 1) * 4 + 15) / 16 * 16 + (size_t)P * 16;
+}
+
 template <int FMT, int NC>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, FMT == 0 ? 0 : NC == 4 ? 3 : 4)
 scatter_all_kernel(const int* __restrict__ tab, int r0, int nprod, int64_t m, int64_t n, double alpha, double beta,
                    const ZView Z, const int* __restrict__ e_row, const int* __restrict__ f_col,
                    double* __restrict__ C, int64_t ldc, int c0, int c1, uint32_t i_lo, uint32_t i_rows)
@@ -2260,7 +2300,19 @@ __global__ void __launch_bounds__(kPrepThreads, 3) wave_classical_kernel(const _
                                 nrank);
 }
 
-__global__ void __launch_bounds__(256) wave_scatter_kernel(const __grid_constant__ WaveLaunch W)
+/* the C updates of the classical problems of a wave */
+__global__ void __launch_bounds__(256, 4) wave_scatter_one_kernel(const __grid_constant__ WaveLaunch W)
+{
+    const WaveProb& P = W.p[wave_find(W, blockIdx.x)];
+    const uint32_t vb = (uint32_t)(blockIdx.x - P.b0), vg = (uint32_t)P.nb;
+    if (P.fmt)
+        scatter_one_body<1>(P.n, P.alpha, P.beta, P.Z, P.e_row, P.f_col, P.C, P.ldc, 0, (int)P.n, vb, vg, 0, (uint32_t)P.m);
+    else
+        scatter_one_body<0>(P.n, P.alpha, P.beta, P.Z, P.e_row, P.f_col, P.C, P.ldc, 0, (int)P.n, vb, vg, 0, (uint32_t)P.m);
+}
+
+/* the others', in the element-major form */
+__global__ void __launch_bounds__(256, 4) wave_scatter_kernel(const __grid_constant__ WaveLaunch W)
 {
     const WaveProb& P = W.p[wave_find(W, blockIdx.x)];
     const uint32_t vb = (uint32_t)(blockIdx.x - P.b0), vg = (uint32_t)P.nb;
@@ -3042,7 +3094,7 @@ static bool job_scatter_all(const SplitJob& j, int r0, int np, int* T_out, size_
     const int per = 8 * P * scatter_cols(P);   /* bytes of values per thread */
     const int T =
         std::max(32, std::min(small ? 128 : 256, (small ? kScatterAllSmem / 2 : kScatterAllSmem) / per) / 32 * 32);
-    const size_t smem = (size_t)T * per + (size_t)E * 12 + (size_t)(np + 1) * 4;
+    const size_t smem = scatter_all_smem(P, T, E, np);
     *T_out = T;
     *smem_out = smem;
     return P <= 64 && smem <= (size_t)kScatterAllMaxSmem;
@@ -4043,8 +4095,7 @@ static int wave_side_scatter(const std::vector<SplitJob*>& qs, On on)
         for (SplitJob* j : kinds[x]) {
             const int P = j->alg.mt * j->alg.nt;
             if (x == 1)
-                smem = std::max(smem, (size_t)P * T[x] * 8 * scatter_cols(P) + (size_t)entries(*j) * 12 +
-                                          (size_t)(j->alg.R + 1) * 4);
+                smem = std::max(smem, scatter_all_smem(P, T[x], entries(*j), j->alg.R));
             all_tiles += tiles(*j);
             all_work += work(*j);
         }
@@ -4054,7 +4105,7 @@ static int wave_side_scatter(const std::vector<SplitJob*>& qs, On on)
             w.nb = std::min<int64_t>(
                 std::max<int64_t>(1, (int64_t)((double)scatter_blocks(all_tiles) * work(j) / all_work)), tiles(j));
         });
-        wave_scatter_kernel<<<(unsigned)nb, (unsigned)T[x], smem, on(x)>>>(L);
+        (x == 0 ? wave_scatter_one_kernel : wave_scatter_kernel)<<<(unsigned)nb, (unsigned)T[x], smem, on(x)>>>(L);
         fmm_count_launch(1);
     }
     for (size_t q = 0; q < other.size(); ++q)
