@@ -2373,6 +2373,9 @@ int make_slice_map(CUtensorMap* map, const void* base, int64_t k_pad, int64_t ro
  * per-group workspace (slices + Z) under kGroupBudget. */
 constexpr size_t kGroupBudget = (size_t)32 << 30;
 
+/* SMs of the GPU that the rules below were measured on (launches ask the device for its own) */
+constexpr int64_t kSms = 152;
+
 struct Dims {
     int64_t me, ne, ke, m_pad, n_pad, k_pad;
 };
@@ -2476,7 +2479,7 @@ struct UnitPlan {
 
 UnitPlan unit_plan(const Dims& d, int s, int fmt, bool pair)
 {
-    constexpr int64_t sms = 152;
+    constexpr int64_t sms = kSms;
     constexpr double kb_single = 760, kb_pair = 640, per_unit = 3000, bytes_per_clk = 2000;
     const int64_t tiles = d.m_pad / kTileM * (d.n_pad / kTileN);
     const int nkb = (int)(d.k_pad / kbe_of(fmt));
@@ -2787,7 +2790,7 @@ static int job_maxima_a(SplitJob& j, cudaStream_t st)
      * than 8 blocks per SM, so short-and-wide A still fills the GPU */
     const int64_t rows_blocks = (j.m + 255) / 256 * j.alg.kt;
     int cpb = 256;
-    while (cpb > 32 && rows_blocks * ((j.d.ke + cpb - 1) / cpb) < 8 * 152) cpb /= 2;
+    while (cpb > 32 && rows_blocks * ((j.d.ke + cpb - 1) / cpb) < 8 * kSms) cpb /= 2;
     dim3 grid((unsigned)((j.m + 255) / 256), (unsigned)j.alg.kt, (unsigned)((j.d.ke + cpb - 1) / cpb));
     amax_kernel<<<grid, 256, 0, st>>>(j.A, j.lda, j.m, j.k, j.alg.kt, amax, cpb, 0, j.m);
     fmm_count_launch(1);
@@ -2901,7 +2904,7 @@ static void job_maxima_a_rows(SplitJob& j, cudaStream_t st, int64_t a, int64_t b
         if (r1 <= r0) continue;
         const int64_t rows_blocks = (r1 - r0 + 255) / 256 * j.alg.kt;
         int cpb = 256;
-        while (cpb > 32 && rows_blocks * ((j.d.ke + cpb - 1) / cpb) < 8 * 152) cpb /= 2;
+        while (cpb > 32 && rows_blocks * ((j.d.ke + cpb - 1) / cpb) < 8 * kSms) cpb /= 2;
         dim3 grid((unsigned)((r1 - r0 + 255) / 256), (unsigned)j.alg.kt, (unsigned)((j.d.ke + cpb - 1) / cpb));
         amax_kernel<<<grid, 256, 0, st>>>(j.A, j.lda, j.m, j.k, j.alg.kt, amax, cpb, r0, r1);
         fmm_count_launch(1);
@@ -3007,7 +3010,7 @@ static int job_gemm(const SplitJob& j, int np, cudaStream_t st)
 {
     const bool pair = job_pair(j);
     const int64_t tiles = job_items(j, 1, pair);
-    const int64_t units = pair ? 76 : 152;
+    const int64_t units = pair ? kSms / 2 : kSms;
     int K = (int)std::min<int64_t>(np, std::max<int64_t>(1, (24 * units + tiles - 1) / tiles));
     const int nl = (np + K - 1) / K;
     K = (np + nl - 1) / nl;
@@ -3035,7 +3038,7 @@ static int job_gemm_block(const SplitJob& j, int np, int64_t it0, int64_t it1, i
     const int64_t tm = it1 - it0, tn = jt1 - jt0;
     if (tm <= 0 || tn <= 0) return FMM_OK;
     const int64_t tiles = tm * tn;
-    const int64_t units = pair ? 76 : 152;
+    const int64_t units = pair ? kSms / 2 : kSms;
     int K = (int)std::min<int64_t>(np, std::max<int64_t>(1, (24 * units + tiles - 1) / tiles));
     const int nl = (np + K - 1) / K;
     K = (np + nl - 1) / nl;
@@ -3079,7 +3082,7 @@ static int64_t scatter_tiles(const SplitJob& j, int64_t rows, int64_t cols, int 
 
 /* blocks of one element-major scatter launch: one per tile, at most 16 per SM
  * (each then serves several tiles with one set-up) */
-static unsigned scatter_blocks(int64_t tiles) { return (unsigned)std::min<int64_t>(tiles, 16 * 152); }
+static unsigned scatter_blocks(int64_t tiles) { return (unsigned)std::min<int64_t>(tiles, 16 * kSms); }
 
 /* Whether the element-major C update applies to products [r0, r0 + np): at
  * most 64 sub-blocks whose values (T threads x 2 or 4 columns) and the group's W
@@ -3100,15 +3103,24 @@ static bool job_scatter_all(const SplitJob& j, int r0, int np, int* T_out, size_
     return P <= 64 && smem <= (size_t)kScatterAllMaxSmem;
 }
 
-/* Whether the element-major C update is also the faster one: with more than
- * 16 sub-blocks its shared memory leaves an SM too few threads (64 sub-blocks:
+/* Whether the element-major C update is also the faster one. With more than 16
+ * sub-blocks its shared memory leaves an SM too few threads (64 sub-blocks:
  * 32-thread blocks, four per SM), and scatter_kernel, which reads Z once per
  * sub-block it feeds but keeps nothing in shared memory, is faster at every
- * grid. Calls of k = 48 per sub-block, 6 slices, element-major / per sub-block,
- * us: 16 sub-blocks (222 x2) grid 256 x 512 153 / 173, 1000 x 1000 607 / 790;
- * 36 (322 x2) 424 / 294, 2620 / 1732; 64 (222 x3) 1985 / 1188, 13244 / 7758.
- * Only calls that need column ranges (host buffers) use it above 16. */
-static bool scatter_all_better(const SplitJob& j) { return j.alg.mt * j.alg.nt <= 16; }
+ * grid. From 7 sub-blocks up it is also faster while the element-major form has
+ * fewer than two blocks per SM, whose threads take all products one after the
+ * other. Calls of k = 48 per sub-block, 6 slices, element-major / per sub-block,
+ * us: 9 sub-blocks (333 x1) on a grid of 128 x 256 87 / 77, 500 x 700 165 / 167;
+ * 16 (222 x2) 128 x 256 110 / 90, 256 x 512 153 / 173, 1000 x 1000 607 / 790;
+ * 16 of 121 products (232 x2) 128 x 256 181 / 121, 500 x 700 544 / 570; 36
+ * (322 x2) 256 x 512 424 / 294, 1000 x 1000 2620 / 1732; 64 (222 x3) 1985 / 1188,
+ * 13244 / 7758. `tiles`: of the element-major launch that the job would be
+ * part of. Calls that need column ranges (host buffers) use it up to 64. */
+static bool scatter_all_better(const SplitJob& j, int64_t tiles)
+{
+    const int P = j.alg.mt * j.alg.nt;
+    return P <= 16 && (P <= 6 || tiles >= 2 * kSms);
+}
 
 /* beta*C comes with the C updates of the first product group */
 static double job_beta(const SplitJob& j, int r0) { return r0 == 0 ? j.beta : 1.0; }
@@ -3145,7 +3157,7 @@ static void job_scatter(const SplitJob& j, int r0, int np, cudaStream_t st, bool
 {
     int T;
     size_t smem;
-    if (scatter_all_better(j) && job_scatter_all(j, r0, np, &T, &smem)) {
+    if (job_scatter_all(j, r0, np, &T, &smem) && scatter_all_better(j, scatter_tiles(j, j.d.me, j.d.ne, T))) {
         job_scatter_block(j, r0, np, 0, j.d.me, 0, j.d.ne, st, small);
         return;
     }
@@ -3262,7 +3274,7 @@ static OverlapPlan overlap_plan(const AlgView& alg, const Dims& d, int64_t m, in
     o.shift = o.L1.total - o.L1.erow;
     /* each group's GEMM keeps every SM busy for at least 8 rounds of items */
     const int64_t tiles = (d.m_pad / (d.me >= kPairMinRows ? kPairTileM : kTileM)) * (d.n_pad / kTileN);
-    o.ok = o.L1.total + o.shift <= bytes && (int64_t)G1 * tiles >= 8 * 152 &&
+    o.ok = o.L1.total + o.shift <= bytes && (int64_t)G1 * tiles >= 8 * kSms &&
            (int64_t)G1 * s * std::max(d.m_pad, d.n_pad) <= 0x7fffffffLL;
     return o;
 }
@@ -3313,7 +3325,7 @@ static int split_overlap(SplitJob& j, const OverlapPlan& o, void* ws, cudaStream
 static int prep_ranks(int64_t groups, int64_t k_pad)
 {
     int r = 1;
-    while (r < 8 && k_pad >= (int64_t)kPrepK * 2 * r && (groups * r < 3 * 152 || k_pad > (int64_t)1024 * r)) r *= 2;
+    while (r < 8 && k_pad >= (int64_t)kPrepK * 2 * r && (groups * r < 3 * kSms || k_pad > (int64_t)1024 * r)) r *= 2;
     return r;
 }
 
@@ -3619,7 +3631,7 @@ int fmm_split_host(const AlgView& alg, int64_t m, int64_t n, int64_t k, double a
             const int RH = tiles_m >= 2 ? 2 : 1;
             /* four column parts where a block still has half a round of items
              * (two blocks are in flight at a time) */
-            const int CH = tiles_n >= 4 && alg.R * (tiles_m / RH) * (tiles_n / 4) >= (pair ? 38 : 76) ? 4
+            const int CH = tiles_n >= 4 && alg.R * (tiles_m / RH) * (tiles_n / 4) >= (pair ? kSms / 4 : kSms / 2) ? 4
                            : tiles_n >= 2 ? 2 : 1;
             int Tchk;
             size_t smchk;
@@ -3986,7 +3998,7 @@ static int wave_classical(int fmt, int s, WaveLaunch& L, const std::vector<Split
     for (int nrank = 1; nrank <= 8; nrank *= 2) {
         std::vector<SplitJob*> sel;
         for (SplitJob* j : qs)
-            if (prep_ranks(3 * 152, j->d.k_pad) == nrank) sel.push_back(j);
+            if (prep_ranks(3 * kSms, j->d.k_pad) == nrank) sel.push_back(j);
         if (sel.empty()) continue;
         const int64_t nb = wave_table(L, sel, [&](const SplitJob& j, WaveProb& w) {
             w.gx = 1;
@@ -4055,8 +4067,8 @@ static int wave_side_pack(const std::vector<SplitJob*>& all, bool small, cudaStr
 
 /* The C updates after a wave's GEMM, on up to kWaveStreams streams `on(x)`:
  * classical jobs (bound by HBM, no shared memory, full blocks) in one
- * element-major launch, other jobs of at most 16 sub-blocks in a second one, the rest
- * each by its own launch. One launch for all of them would run every job with
+ * element-major launch, the other jobs that it is better for in a second one,
+ * the rest each by its own launch. One launch for all of them would run every job with
  * the fewest threads and the most shared memory any of them needs: 322 x2 at
  * 963 x 267 x 134 with a classical 675 x 2091 x 595, 829 us for the batch
  * against 380. Within a launch the blocks, at most 16 per SM in all, are shared
@@ -4070,7 +4082,7 @@ static int wave_side_scatter(const std::vector<SplitJob*>& qs, On on)
     for (SplitJob* j : qs) {
         int Tj;
         size_t sm;
-        if (scatter_all_better(*j) && job_scatter_all(*j, 0, j->alg.R, &Tj, &sm)) {
+        if (job_scatter_all(*j, 0, j->alg.R, &Tj, &sm) && scatter_all_better(*j, INT64_MAX)) {
             const int x = j->classical ? 0 : 1;
             kinds[x].push_back(j);
             T[x] = std::min(T[x], Tj);
@@ -4078,6 +4090,17 @@ static int wave_side_scatter(const std::vector<SplitJob*>& qs, On on)
             other.push_back(j);
         }
     }
+    int64_t together = 0;
+    for (SplitJob* j : kinds[1]) together += scatter_tiles(*j, j->d.me, j->d.ne, T[1]);
+    /* A job of many products has long blocks; where the launch is about one round of blocks (six per SM), other
+     * jobs' blocks push its last ones into a second round: five problems, 861 of 940 blocks of 232 x2 at 1654 x
+     * 1967, 774 us for the batch, 698 with that one by sub-block (alone it takes 356 this way and 397 by sub-block). */
+    const bool unlike = kinds[1].size() > 1;
+    const auto apart = std::stable_partition(kinds[1].begin(), kinds[1].end(), [&](SplitJob* j) {
+        return scatter_all_better(*j, unlike && j->alg.R > 64 ? together / 4 : together);
+    });
+    other.insert(other.end(), apart, kinds[1].end());
+    kinds[1].erase(apart, kinds[1].end());
     auto entries = [](const SplitJob& j) {
         const Tab ht = tab_view(j.alg.htab);
         return ht.w_off[j.alg.R] - ht.w_off[0];

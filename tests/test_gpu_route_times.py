@@ -134,3 +134,30 @@ def test_fp8_digit_planes_bitexact(fmm, orc, algs, alg, levels, m, n, k, s):
     dC = to_dev(C)
     fmm.split_dgemm(to_dev(A), to_dev(B), dC, f, levels, s, alpha=-0.75, beta=0.5, fmt="fp8")
     assert np.array_equal(to_host(dC), want)
+
+
+def test_batch_of_long_and_short_c_updates(fmm, torch_cuda):
+    """121 products of a 414 x 492 product grid beside four small problems:
+    700 us with its C updates by sub-block, 770 in one launch with the others,
+    whose blocks push its last ones into a second round."""
+    torch = torch_cuda
+    algs = {a: fmm.new_fmm(COEFFS / f"{a}.txt") for a in ("232", "333")}
+    ps = [{"A": operand(torch, m, k), "B": operand(torch, k, n), "C": operand(torch, m, n), "fmm": algs.get(a), "levels": lv,
+           "slices": s, "fmt": fmt, "beta": 0.5}
+          for m, n, k, a, lv, s, fmt in [(45, 832, 36, "232", 2, 7, "fp8"), (50, 734, 124, "333", 1, 10, "fp8"),
+                                         (159, 353, 160, "232", 1, 3, "bf16"), (1654, 1967, 276, "232", 2, 4, "bf16"),
+                                         (65, 221, 2192, None, 0, 6, "bf16")]]
+    b = fmm.make_batch(ps)
+    ws = torch.empty(fmm.batch_workspace_size(b), dtype=torch.uint8, device="cuda")
+    assert device_us(torch, lambda: fmm.batch_dgemm(b, workspace=ws)) < 740
+
+
+def test_c_updates_of_many_products_on_small_grids(fmm, torch_cuda):
+    """121 products, 16 sub-blocks, an 8 x 110 product grid: 96 us with a C
+    update per sub-block, 168 with all products in one thread's chain."""
+    torch = torch_cuda
+    m, n, k = 32, 440, 432
+    f = fmm.new_fmm(COEFFS / "232.txt")
+    A, B, C = operand(torch, m, k), operand(torch, k, n), operand(torch, m, n)
+    ws = torch.empty(fmm.split_workspace_size(m, n, k, f, 2, 6), dtype=torch.uint8, device="cuda")
+    assert device_us(torch, lambda: fmm.split_dgemm(A, B, C, f, 2, 6, 1.0, 0.5, ws)) < 135
