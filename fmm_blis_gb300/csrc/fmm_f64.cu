@@ -882,7 +882,7 @@ __global__ void scale_c_kernel(int64_t m, int64_t n, double beta, double* C, int
  * SMs. Here a cluster of ks CTAs (one per k chunk of kc elements) computes
  * each tile: every CTA accumulates its chunk in k order (the pipelined tile),
  * leaves its partial tile in shared memory, and after a cluster
- * barrier each CTA sums a share of the tile's elements over the ks partials
+ * barrier the first CTA, one element per thread, sums the ks partials
  * through distributed shared memory, always in chunk order
  * (((p_0 + p_1) + p_2) + ...), and applies C := fma(alpha, sum, C). The
  * result depends only on (m, n, k): the batched call runs these problems
@@ -931,12 +931,11 @@ fmm_f64_sup_kernel(int64_t m, int64_t n, int64_t k, double alpha, const double* 
 #pragma unroll
         for (int y = 0; y < TN; ++y) Ps[(tr + x * PT::RT) + BM * (tc + y * PT::CT)] = acc[x][y];
     cl.sync();   /* every partial tile of the cluster is in place */
-    /* the tile's elements in groups of NT, group g summed by CTA g % ks */
-    for (int g = rank; g < BM * BN / PT::NT; g += ks) {
-        const int e = g * PT::NT + tid;
-        double s = *cl.map_shared_rank(Ps + e, 0);
-        for (int q = 1; q < ks; ++q) s = s + *cl.map_shared_rank(Ps + e, q);
-        const int64_t gi = i0 + e % BM, gj = j0 + e / BM;
+    static_assert(BM * BN == PT::NT, "one element per thread");
+    if (rank == 0) {
+        double s = Ps[tid];
+        for (int q = 1; q < ks; ++q) s = s + *cl.map_shared_rank(Ps + tid, q);
+        const int64_t gi = i0 + tid % BM, gj = j0 + tid / BM;
         if (gi < m && gj < n) {
             double* p = C + gi + gj * ldc;
             *p = fma(alpha, s, *p);

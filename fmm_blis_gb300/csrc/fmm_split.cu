@@ -545,9 +545,9 @@ __device__ __forceinline__ void scale_first(const PEnt& x, double (&s)[N])
  * row-major (K-major) into slices sa[q][t][m_pad][k_pad]. The product index
  * runs fastest in the block order, so the products at one tile position run
  * together and read their shared A sub-block tiles through L2 once. ROWS = 64
- * (256 threads) for single calls; ROWS = 32 (128 threads, 25 KB of shared
- * memory, at most 64 registers) for batched waves, small enough to run on an
- * SM beside a resident GEMM CTA. */
+ * (256 threads); ROWS = 32 (128 threads, 25 KB of shared memory, at most 64
+ * registers) where the packs run beside a GEMM (split_overlap), small enough
+ * for an SM with a resident GEMM CTA. */
 template <int S, int DB, int ROWS>
 __device__ __forceinline__ void pack_a_body(const int* __restrict__ tab, int r0, int np, const double* __restrict__ A,
                                             int64_t lda, int64_t m, int64_t k, int64_t m_pad, int64_t k_pad,
@@ -642,8 +642,8 @@ pack_a_kernel(const int* __restrict__ tab, int r0, int np, const double* __restr
 /* B side, all products of a group: CTA (q, tile) forms the tile of COLS
  * columns x 64 k of T_r, r = r0 + q (column j of T_r is contiguous in k
  * already), and writes its digits into slices sb[q][t][n_pad][k_pad];
- * product index fastest, as on the A side. COLS = 32 (256 threads) for single
- * calls, 16 (128 threads, at most 64 registers) for batched waves. Eight lanes
+ * product index fastest, as on the A side. COLS = 32 (256 threads), or 16
+ * (128 threads, at most 64 registers) beside a GEMM. Eight lanes
  * read 64 contiguous bytes of a column per load (a load that gives each lane
  * eight consecutive k touches 16 lines and is bound by L1) and exchange the
  * sums through shared memory: 222 x2 at 4096, 6 slices, 339 -> 277 us. */
@@ -2267,21 +2267,21 @@ __global__ void __launch_bounds__(256) wave_exps_kernel(const __grid_constant__ 
               vb % P.gx, (int)(vb / P.gx));
 }
 
-template <int S, int DB, int ROWS>
-__global__ void __launch_bounds__(ROWS * 4, ROWS == 64 ? 4 : 8) wave_pack_a_kernel(const __grid_constant__ WaveLaunch W)
+template <int S, int DB>
+__global__ void __launch_bounds__(256, 4) wave_pack_a_kernel(const __grid_constant__ WaveLaunch W)
 {
     const WaveProb& P = W.p[wave_find(W, blockIdx.x)];
     const int64_t vb = blockIdx.x - P.b0;
-    pack_a_body<S, DB, ROWS>(P.tab, 0, P.R, P.A, P.lda, P.m, P.k, P.m_pad, P.k_pad, P.e_row, P.sa, vb % P.gx,
+    pack_a_body<S, DB, 64>(P.tab, 0, P.R, P.A, P.lda, P.m, P.k, P.m_pad, P.k_pad, P.e_row, P.sa, vb % P.gx,
                              vb / P.gx);
 }
 
-template <int S, int DB, int COLS>
-__global__ void __launch_bounds__(COLS * 8, COLS == 32 ? 4 : 8) wave_pack_b_kernel(const __grid_constant__ WaveLaunch W)
+template <int S, int DB>
+__global__ void __launch_bounds__(256, 4) wave_pack_b_kernel(const __grid_constant__ WaveLaunch W)
 {
     const WaveProb& P = W.p[wave_find(W, blockIdx.x)];
     const int64_t vb = blockIdx.x - P.b0;
-    pack_b_body<S, DB, COLS>(P.tab, 0, P.R, P.B, P.ldb, P.k, P.n, P.n_pad, P.k_pad, P.f_col, P.sb, 0, vb % P.gx,
+    pack_b_body<S, DB, 32>(P.tab, 0, P.R, P.B, P.ldb, P.k, P.n, P.n_pad, P.k_pad, P.f_col, P.sb, 0, vb % P.gx,
                              vb / P.gx);
 }
 
@@ -2871,10 +2871,7 @@ static void job_pack_a(SplitJob& j, int r0, int np, cudaStream_t st)
     fmm_count_launch(2);
 }
 
-/* small: the 128-thread pack tiles, which fit on an SM beside a resident
- * GEMM CTA */
-static void job_pack_b_cols(SplitJob& j, int r0, int np, int64_t j0, int64_t j1, cudaStream_t st,
-                            bool small = false)
+static void job_pack_b_cols(SplitJob& j, int r0, int np, int64_t j0, int64_t j1, cudaStream_t st)
 {
     const Dims& d = j.d;
     if (j1 <= j0) return;
@@ -2886,7 +2883,6 @@ static void job_pack_b_cols(SplitJob& j, int r0, int np, int64_t j0, int64_t j1,
     sel.a = false;
     sel.jb0 = j0;
     sel.jb1 = j1;
-    sel.small = small;
     launch_packs(j.fmt, j.s, j.alg.tab, r0, np, j.A, j.lda, j.B, j.ldb, j.m, j.n, j.k, d.m_pad, d.n_pad, d.k_pad,
                  (int*)(j.w + j.L.erow), (int*)(j.w + j.L.fcol), j.w + j.L.sa, j.w + j.L.sb, st, st, sel);
     fmm_count_launch(2);
@@ -2913,7 +2909,7 @@ static void job_maxima_a_rows(SplitJob& j, cudaStream_t st, int64_t a, int64_t b
 
 /* row exponents and A slices of the products r0 .. r0+np-1 for the S_r rows
  * [a, b) (multiples of 64, or b = m_pad) */
-static void job_pack_a_rows(SplitJob& j, int r0, int np, int64_t a, int64_t b, cudaStream_t st, bool small = false)
+static void job_pack_a_rows(SplitJob& j, int r0, int np, int64_t a, int64_t b, cudaStream_t st)
 {
     const Dims& d = j.d;
     if (b <= a) return;
@@ -2924,7 +2920,6 @@ static void job_pack_a_rows(SplitJob& j, int r0, int np, int64_t a, int64_t b, c
     sel.b = false;
     sel.ia0 = a;
     sel.ia1 = b;
-    sel.small = small;
     launch_packs(j.fmt, j.s, j.alg.tab, r0, np, j.A, j.lda, j.B, j.ldb, j.m, j.n, j.k, d.m_pad, d.n_pad, d.k_pad,
                  (int*)(j.w + j.L.erow), (int*)(j.w + j.L.fcol), j.w + j.L.sa, j.w + j.L.sb, st, st, sel);
     fmm_count_launch(2);
@@ -3147,10 +3142,9 @@ static void job_scatter_block(const SplitJob& j, int r0, int np, int64_t i0, int
 
 /* the C updates of products [r0, r0 + np) for the product-grid columns
  * [j0, j1) (all rows), element-major form only */
-static void job_scatter_cols(const SplitJob& j, int r0, int np, int64_t j0, int64_t j1, cudaStream_t st,
-                             bool small = false)
+static void job_scatter_cols(const SplitJob& j, int r0, int np, int64_t j0, int64_t j1, cudaStream_t st)
 {
-    job_scatter_block(j, r0, np, 0, j.d.me, j0, j1, st, small);
+    job_scatter_block(j, r0, np, 0, j.d.me, j0, j1, st);
 }
 
 static void job_scatter(const SplitJob& j, int r0, int np, cudaStream_t st, bool small = false)
@@ -3969,25 +3963,18 @@ static int64_t wave_table(WaveLaunch& L, const std::vector<SplitJob*>& qs, F siz
 }
 
 template <int S, int DB>
-static void wave_packs_t(WaveLaunch& L, const std::vector<SplitJob*>& qs, bool small, cudaStream_t st)
+static void wave_packs_t(WaveLaunch& L, const std::vector<SplitJob*>& qs, cudaStream_t st)
 {
-    const int rows = small ? 32 : 64, cols = small ? 16 : 32;
     int64_t nb = wave_table(L, qs, [&](const SplitJob& j, WaveProb& w) {
-        w.gx = (int64_t)j.alg.R * (j.d.m_pad / rows);
+        w.gx = (int64_t)j.alg.R * (j.d.m_pad / 64);
         w.nb = w.gx * (j.d.k_pad / 64);
     });
-    if (small)
-        wave_pack_a_kernel<S, DB, 32><<<(unsigned)nb, 128, 0, st>>>(L);
-    else
-        wave_pack_a_kernel<S, DB, 64><<<(unsigned)nb, 256, 0, st>>>(L);
+    wave_pack_a_kernel<S, DB><<<(unsigned)nb, 256, 0, st>>>(L);
     nb = wave_table(L, qs, [&](const SplitJob& j, WaveProb& w) {
-        w.gx = (int64_t)j.alg.R * ((j.d.n_pad + cols - 1) / cols);
+        w.gx = (int64_t)j.alg.R * ((j.d.n_pad + 31) / 32);
         w.nb = w.gx * (j.d.k_pad / 64);
     });
-    if (small)
-        wave_pack_b_kernel<S, DB, 16><<<(unsigned)nb, 128, 0, st>>>(L);
-    else
-        wave_pack_b_kernel<S, DB, 32><<<(unsigned)nb, 256, 0, st>>>(L);
+    wave_pack_b_kernel<S, DB><<<(unsigned)nb, 256, 0, st>>>(L);
     fmm_count_launch(2);
 }
 
@@ -4016,7 +4003,7 @@ static int wave_classical(int fmt, int s, WaveLaunch& L, const std::vector<Split
  * jobs qs (all products of each as one group). Classical jobs: prep_kernel's
  * work per (slice count, format). Others: maxima zeroing, maxima, exponents,
  * then the packs per (slice count, format). */
-static int wave_side_pack(const std::vector<SplitJob*>& all, bool small, cudaStream_t st)
+static int wave_side_pack(const std::vector<SplitJob*>& all, cudaStream_t st)
 {
     WaveLaunch L;
     std::vector<SplitJob*> qs, cl;
@@ -4057,7 +4044,7 @@ static int wave_side_pack(const std::vector<SplitJob*>& all, bool small, cudaStr
         fmm_count_launch(3);
         each_kind(qs, [&](int fmt, int sl, auto& sel) {
             return with_slices(fmt, sl, [&](auto S, auto DB) {
-                wave_packs_t<S(), DB()>(L, sel, small, st);
+                wave_packs_t<S(), DB()>(L, sel, st);
                 return (int)FMM_OK;
             });
         });
@@ -4184,7 +4171,7 @@ int fmm_split_batch(int count, const SplitJob* jobs_in, void* ws, size_t ws_byte
         }
         /* the full-size tiles: measured, a wave's side kernels do not overlap the previous wave's GEMM (its
          * CTAs hold the SMs), so the tiles that fit beside a GEMM CTA only make them slower */
-        if (int rc = wave_side_pack(qs, false, pack_st(0)); rc != FMM_OK) return rc;
+        if (int rc = wave_side_pack(qs, pack_st(0)); rc != FMM_OK) return rc;
         if (sp)
             for (int x = 0; x < kWaveStreams; ++x)
                 if (!ok(cudaEventRecord(sp->wave_pk[W.h][x], pack_st(x)))) return FMM_ERR_CUDA;
