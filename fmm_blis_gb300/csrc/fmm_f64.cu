@@ -1299,83 +1299,102 @@ extern "C" int fmm_gpu_set_f64_batch_ctas(int max_ctas)
 
 namespace {
 
-/* FP64 pipe time of one item of a batch (a tile of all products), in FMAs at a
- * 64 x 64 tile's rate. Smaller tiles pay for the pack additions of more tiles
- * per operand element (nu, nv terms per product), 16 x 16 also for fewer FMAs
- * per shared-memory load and for the C updates of a short k. Measured, tiles
- * 64 / 32 / 16, us: 2432 x 2048 x 2000 222 x1 (304 tiles of 64) 15249 / 15506 /
- * 19326, x 64 524 / 564 / 806; classical 1216 x 1024 x 500 1048 / 1052 / 1212,
- * x 32 84 / 90 / 127; 4864 x 4096 x 400 444 x1 15503 / 17218 / 24942. FP64 MMA
- * engine, 64 / 32: classical 1216 x 1024 x 500 1184 / 1190, 2048^3 222 x1 16969 /
- * 17362 (2 and 1.75 rounds of 64 x 64 work). */
+/* Item tiles of a batch. One 64 x 64 item of a deep problem can last as long as
+ * the whole batch (1024^3 222 x1: 14.7 M FMAs, 7 ms on half an SM), so a
+ * problem's tile shrinks to 32, then 16, while its items hold more than an
+ * eighth of a CTA's share of the batch: 24 problems of 256 to 1024 7.25 ms, 7.8
+ * with 64 x 64 alone. That is within 3% of the best limit for 258 drawn
+ * batches but for those whose items are nearly all alike, where smaller tiles
+ * only cost more and whole rounds of items decide: for these the tile with the
+ * least batch_rounds times batch_item_cost is taken if it saves 5%. Tiles of 64
+ * / 32 / 16 / the rule, us: 2048^3 222 x1 15204 / 13633 / 16552 / 13640; 1912 x
+ * 2475 x 97 232 x1 1522 / 1580 / 2015 / 1522; 1024^3 222 x1 3992 / 1966 / 2388
+ * / 1966; 512^3 222 x1 2019 / 586 / 319 / 319; classical 1216 x 1024 x 500 1048
+ * / 1052 / 1212 / 1048. */
+
+/* FP64 pipe time of an item (a tile of all products) in FMAs at a 64 x 64
+ * tile's rate. Smaller tiles pay for the pack additions of more tiles per
+ * operand element (nn terms per product on both sides), 16 x 16 also for fewer
+ * FMAs per shared-memory load and for the C updates of a short k. */
 double batch_item_cost(const F64BatchItem& it, int tile, bool mma)
 {
-    if (it.k == 0 || it.alpha == 0.0) return 1.0;
     const double ke = (double)((it.k + it.alg.kt - 1) / it.alg.kt), nn = it.alg.avg_nnz_u + it.alg.avg_nnz_v;
     double rel = 1.0;
     if (tile == 32)
-        rel = mma ? 1.01 + 0.11 * (nn - 2.0) : 1.0 + 0.01 * nn + 1.5 / ke;
+        rel = mma ? 1.01 + 0.11 * (nn - 2.0) : 1.0 + 0.016 * (nn - 2.0) + 1.6 / ke;
     else if (tile == 16)
-        rel = 1.0 + 0.08 * nn + 11.0 / ke;
+        rel = 1.14 + 0.085 * (nn - 2.0) + 11.0 / ke;
     return rel * tile * tile * it.alg.R * (ke + 1.0);
 }
 
-/* Each problem's tile and item cost. One 64 x 64 item of a deep problem can last
- * as long as the whole batch (1024^3 222 x1: 7 ms on half an SM), smaller
- * tiles cost more in all (batch_item_cost). Tried are limits on an item's
- * cost: from the longest 64 x 64 item down to 1/32 of it, and an eighth of a
- * CTA's share of the batch; a problem takes its largest tile within the limit,
- * and the limit with the least estimate is kept. The estimate: items go out
- * longest first to `slots` SMs (an SM's two CTAs share its FP64 pipe, and one
- * alone nearly fills it), so after each problem's items the time is the work
- * so far in whole rounds of that item. 64 / 32 / 16 everywhere / this rule, us:
- * 2048^3 222 x1 15204 / 13633 / 16552 / 13638; 512^3 222 x1 2019 / 586 / 319 /
- * 319; eight classical 700^3 4957 / 4629 / 5308 / 4631; 200 of 100^3 222 x1
- * 1033 / 826 / 962 / 829. */
-template <class TilesOf>
-void batch_tiles(const F64BatchItem* items, const std::vector<int>& order, bool mma, int slots, TilesOf tiles_of,
-                 std::vector<int>& tile, std::vector<double>& cost)
+/* Time of n like items on `sms` SMs, in times of one item with an SM's FP64
+ * pipe to itself: two CTAs of an SM share the pipe, the items of a last part
+ * round are alone on their SM or nearly, and a CTA alone does not fill the
+ * pipe, the less the smaller its tile and the more terms its packs have. */
+double batch_rounds(double n, int sms, int tile, double nn)
 {
-    struct Choice {
-        double cost[3], items[3];   /* at tiles of 64, 32, 16 */
+    const double alone = tile == 64 ? std::max(1.05, 1.0 + 0.1 * (nn - 2.0))
+                                    : tile == 32 ? 1.15 + 0.16 * (nn - 2.0) : 1.5 + 0.35 * (nn - 2.0);
+    if (n <= sms) return alone;
+    const double full = std::floor(n / (2.0 * sms)), left = n - full * 2.0 * sms;
+    return 2.0 * full + (left <= 0.0 ? 0.0 : left <= sms ? std::min(2.0, 1.08 * alone) : 2.0);
+}
+
+/* each problem's tile, by the rule above, for `ctas` CTAs on `sms` SMs; items(i, tile): a problem's items */
+template <class Items>
+void batch_tiles(const F64BatchItem* p, const std::vector<int>& order, bool mma, int64_t ctas, int sms, Items items,
+                 std::vector<int>& tile)
+{
+    const int least = mma ? 32 : 16;
+    auto idle = [&](int i) { return p[i].k == 0 || p[i].alpha == 0.0; };   /* C := beta*C only */
+    auto fmas = [&](int i, int t) {
+        return idle(i) ? 1.0 : (double)t * t * p[i].alg.R * (double)((p[i].k + p[i].alg.kt - 1) / p[i].alg.kt + 1);
     };
-    const int sizes = mma ? 2 : 3;
-    std::vector<Choice> ch(order.size());
-    double longest = 0.0, total = 0.0;
-    for (size_t q = 0; q < order.size(); ++q) {
-        for (int t = 0; t < sizes; ++t) {
-            int64_t tm = 0;
-            ch[q].cost[t] = batch_item_cost(items[order[q]], 64 >> t, mma);
-            ch[q].items[t] = (double)tiles_of(order[q], 64 >> t, &tm);
-        }
-        longest = std::max(longest, ch[q].cost[0]);
-        total += ch[q].cost[1] * ch[q].items[1];
-    }
-    std::vector<int> pick(order.size()), best(order.size(), 0);
-    std::vector<std::pair<double, double>> cls(order.size());   /* (item cost, items) */
-    double least = 0.0;
-    for (int x = 0; x <= 6; ++x) {
-        const double limit = x < 6 ? longest / (1 << x) : total / slots / 16;
-        for (size_t q = 0; q < order.size(); ++q) {
-            pick[q] = 0;
-            while (pick[q] + 1 < sizes && ch[q].cost[pick[q]] > limit) ++pick[q];
-            cls[q] = {ch[q].cost[pick[q]], ch[q].items[pick[q]]};
-        }
-        std::sort(cls.begin(), cls.end(), [](auto& a, auto& b) { return a.first > b.first; });
-        double work = 0.0, est = 0.0;
-        for (const auto& c : cls) {
-            work += c.first * c.second;
-            est = std::max(est, c.first * std::ceil(work / (slots * c.first)));
-        }
-        if (x == 0 || est < (x < 6 ? 0.98 : 1.0) * least) {   /* larger tiles at a near tie */
-            least = est;
-            best = pick;
+    double total = 0.0, work = 0.0, most = 0.0;
+    int heavy = -1;   /* the problem with the most work */
+    for (int i : order) {
+        total += fmas(i, 32) * (double)items(i, 32);
+        const double w = fmas(i, 64) * (double)items(i, 64);
+        work += w;
+        if (!idle(i) && w > most) {
+            most = w;
+            heavy = i;
         }
     }
-    for (size_t q = 0; q < order.size(); ++q) {
-        tile[order[q]] = 64 >> best[q];
-        cost[order[q]] = ch[q].cost[best[q]];
+    for (int i : order) {
+        tile[i] = 64;
+        while (tile[i] > least && fmas(i, tile[i]) > total / (double)ctas / 8) tile[i] /= 2;
     }
+    if (heavy < 0) return;
+    /* the problems whose items are within a tenth of the heavy one's */
+    const double len = fmas(heavy, 64);
+    auto alike = [&](int i) { return !idle(i) && fmas(i, 64) <= len * 1.1 && fmas(i, 64) >= len / 1.1; };
+    double part = 0.0;
+    for (int i : order)
+        if (alike(i)) part += fmas(i, 64) * (double)items(i, 64);
+    if (part < 0.95 * work) return;
+    const int slots = (int)std::min<int64_t>(ctas, sms);
+    auto estimate = [&](int t) {
+        double n = 0.0, longest = 0.0;
+        for (int i : order)
+            if (alike(i)) {
+                n += (double)items(i, t);
+                longest = std::max(longest, batch_item_cost(p[i], t, mma));
+            }
+        return longest * batch_rounds(n, slots, t, p[heavy].alg.avg_nnz_u + p[heavy].alg.avg_nnz_v);
+    };
+    double best = 0.95 * estimate(tile[heavy]);
+    int to = tile[heavy];
+    for (int t = 64; t >= least; t /= 2) {
+        const double e = t == tile[heavy] ? best : estimate(t);
+        if (e < best) {
+            best = e;
+            to = t;
+        }
+    }
+    if (to != tile[heavy])
+        for (int i : order)
+            if (alike(i)) tile[i] = to;
 }
 
 }  // namespace
@@ -1419,8 +1438,13 @@ int fmm_f64_batch_launch(int count, const F64BatchItem* items, void* ws, size_t 
         return *tm * ((ne + tile - 1) / tile);
     };
     std::vector<int> tile(count, 64);
-    batch_tiles(items, order, mma, (int)std::min<int64_t>(ctas, sms), tiles_of, tile, cost);
     int64_t tm = 0;
+    batch_tiles(items, order, mma, ctas, sms, [&](int i, int t) { return tiles_of(i, t, &tm); }, tile);
+    for (int i : order) {
+        const F64BatchItem& it = items[i];
+        cost[i] = it.k == 0 || it.alpha == 0.0
+                      ? 1.0 : (double)tile[i] * tile[i] * it.alg.R * (double)((it.k + it.alg.kt - 1) / it.alg.kt + 1);
+    }
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
     std::vector<F64Prob> tab(order.size());
     int64_t items_total = 0;

@@ -80,6 +80,7 @@ def test_batch_of_unlike_small_c_updates(fmm, torch_cuda):
     ("222", [(2048, 2048, 2048, 1)], 15000),                    # tiles of 32: 13.6 ms; of 64 15.2, of 16 16.6
     ("232", [(1912, 2475, 97, 1), (169, 242, 116, 0)], 1800),   # tiles of 64: 1.5 ms; of 16 2.0
     ("222", [(512, 512, 512, 1)], 450),                         # tiles of 16: 0.32 ms; of 32 0.59, of 64 2.0
+    ("333", [(1380, 185, 323, 1), (534, 382, 1340, 0)], 1200),  # unlike items on tiles of 16: 0.78 ms; of 32 1.7
 ])
 def test_fp64_batch_tiles(fmm, torch_cuda, alg, shapes, bound):
     torch = torch_cuda
