@@ -3464,17 +3464,18 @@ static int split_launch_budget(const AlgView& alg, int64_t m, int64_t n, int64_t
 /* ---------------------------------------------------------------------------
  * Host-buffer entry.
  *
- * Operands in host memory: the call owns the device copies and overlaps the
- * host<->device traffic with the device work. Copies run on s[1] in the
- * order A, B, C (with the blocked schedule below: A's first row half, B's
- * first column half, A's second half, B's second half, C); the A side (row
- * maxima, row exponents, A slices) starts as soon as its rows have arrived,
- * the B side on s[0] as soon as its columns have, and C is only needed by the
- * C updates, so its upload runs under the GEMM. The host enqueues in the same
- * order, which keeps the overlap when a copy from pageable memory blocks the
- * host until it is staged. Every host copy touches its host pages first
- * (fmm_touch_host). The operand and workspace buffers are kept per device
- * (grow-only) until fmm_gpu_release_host_buffers.
+ * Operands in host memory: the call owns the device copies and, unless they
+ * are small, overlaps the host<->device traffic with the device work. Uploads
+ * run on s[1] in the order A, B, C (with the blocked schedule below: A's first
+ * row half, B's first column part, A's second half, B's other parts, each
+ * block's C before its updates); the A side (row maxima, row exponents, A
+ * slices) starts as soon as its rows have arrived, the B side on another stream
+ * as soon as its columns have, and C is only needed by the C updates, so its
+ * upload runs under the GEMM. The host enqueues in the same order, which keeps
+ * the overlap when a copy from pageable memory blocks the host until it is
+ * staged. Every host copy touches its host pages first (fmm_touch_host). The
+ * operand and workspace buffers are kept per device (grow-only) until
+ * fmm_gpu_release_host_buffers.
  * ------------------------------------------------------------------------- */
 struct HostBuffers {
     uint8_t* p = nullptr;
