@@ -1909,25 +1909,27 @@ __device__ __forceinline__ double beta_c(double beta, const double* c)
     return beta == 0.0 ? 0.0 : beta * *c;
 }
 
-/* C updates of one C sub-block p = blockIdx.y: tiles of tr rows (a power of two,
- * 8 to 128) x 512 / tr columns, a thread a row of a 4-column group. For
- * algorithms of more than 16 sub-blocks (scatter_all_better). One thread
- * gathers the sub-block's entries for each tile, which bounds narrow product
- * grids: with 128 rows x 4 columns on 8 rows, 444 x2 on an 8 x 600 grid takes
- * 8.5 ms a call instead of 5.2. */
+/* C updates of one C sub-block p: tiles of tr rows (a power of two, 8 to 128) x
+ * 512 / tr columns, a thread a row of a 4-column group. Where scatter_all_better
+ * says so. One thread gathers the sub-block's entries for each tile, which
+ * bounds narrow product grids: with 128 rows x 4 columns on 8 rows, 444 x2 on an
+ * 8 x 600 grid takes 8.5 ms a call instead of 5.2. */
 constexpr int kScatterThreads = 128;
 
+struct ScatterEntries {
+    double lam[kScatterMaxEnt];
+    int prod[kScatterMaxEnt];
+    int n;
+};
+
+/* tile bx of sub-block p */
 template <int FMT>
-__global__ void __launch_bounds__(kScatterThreads)
-scatter_kernel(const int* __restrict__ tab, int r0, int nprod, int64_t m, int64_t n, double alpha, double beta,
-               const ZView Z, const int* __restrict__ e_row, const int* __restrict__ f_col, double* __restrict__ C,
-               int64_t ldc, int tr)
+__device__ __forceinline__ void scatter_part_body(ScatterEntries& sh, const int* __restrict__ tab, int r0, int nprod,
+                                                  int64_t m, int64_t n, double alpha, double beta, const ZView& Z,
+                                                  const int* __restrict__ e_row, const int* __restrict__ f_col,
+                                                  double* __restrict__ C, int64_t ldc, int tr, int p, uint32_t bx)
 {
-    __shared__ double lam[kScatterMaxEnt];
-    __shared__ int prod[kScatterMaxEnt];
-    __shared__ int nsel;
     const Tab t = tab_view(tab);
-    const int p = blockIdx.y;
     int ro, rl, co, cl;
     fmm_part_geom32((int)m, t.mt, p / t.nt, &ro, &rl);
     fmm_part_geom32((int)n, t.nt, p % t.nt, &co, &cl);
@@ -1939,34 +1941,46 @@ scatter_kernel(const int* __restrict__ tab, int r0, int nprod, int64_t m, int64_
             const int r = t.wp_ent[2 * e] - r0;
             if (r < 0) continue;
             if (r >= nprod) break;
-            prod[q] = r;
-            lam[q] = alpha * (double)t.wp_ent[2 * e + 1];
+            sh.prod[q] = r;
+            sh.lam[q] = alpha * (double)t.wp_ent[2 * e + 1];
             ++q;
         }
-        nsel = q;
+        sh.n = q;
     }
     __syncthreads();
-    const int ne = nsel;
+    const int ne = sh.n;
     const uint32_t me = (uint32_t)((m + t.mt - 1) / t.mt), tiles_i = (me + tr - 1) / tr;
-    const int i = (int)(blockIdx.x % tiles_i * tr + threadIdx.x % tr);
-    const int j = (int)(blockIdx.x / tiles_i * (kScatterThreads / tr) + threadIdx.x / tr) * 4;
+    const int i = (int)(bx % tiles_i * tr + threadIdx.x % tr);
+    const int j = (int)(bx / tiles_i * (kScatterThreads / tr) + threadIdx.x / tr) * 4;
     if ((ne == 0 && beta == 1.0) || i >= rl || j >= cl) return;
     double* cp = C + ro + i + (int64_t)(co + j) * ldc;
     double c[kScatterCols];
 #pragma unroll
     for (int u = 0; u < 4; ++u) c[u] = j + u < cl ? beta_c(beta, cp + u * ldc) : 0.0;
     ZRow<FMT> z;
-    if (ne > 0) z.load(Z, e_row, f_col, prod[0], i, j);
+    if (ne > 0) z.load(Z, e_row, f_col, sh.prod[0], i, j);
     for (int q = 0; q < ne; ++q) {
         double M[kScatterCols];
         z.values(Z, M);
-        if (q + 1 < ne) z.load(Z, e_row, f_col, prod[q + 1], i, j);   /* in flight under this product's updates */
+        if (q + 1 < ne) z.load(Z, e_row, f_col, sh.prod[q + 1], i, j);   /* in flight under this product's updates */
 #pragma unroll
-        for (int u = 0; u < 4; ++u) c[u] = fma(lam[q], M[u], c[u]);
+        for (int u = 0; u < 4; ++u) c[u] = fma(sh.lam[q], M[u], c[u]);
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u)
         if (j + u < cl) cp[u * ldc] = c[u];
+}
+
+/* grid: tiles x sub-blocks */
+template <int FMT>
+__global__ void __launch_bounds__(kScatterThreads)
+scatter_kernel(const int* __restrict__ tab, int r0, int nprod, int64_t m, int64_t n, double alpha, double beta,
+               const ZView Z, const int* __restrict__ e_row, const int* __restrict__ f_col, double* __restrict__ C,
+               int64_t ldc, int tr)
+{
+    __shared__ ScatterEntries sh;
+    scatter_part_body<FMT>(sh, tab, r0, nprod, m, n, alpha, beta, Z, e_row, f_col, C, ldc, tr, (int)blockIdx.y,
+                           blockIdx.x);
 }
 
 /* Multi-C epilogue, element-major: a thread takes a row of a 4-column group, or
@@ -2214,7 +2228,7 @@ struct WaveProb {
     int64_t nb;   /* its blocks */
     int64_t gx;   /* blocks along the first coordinate of its per-problem grid */
     double alpha, beta;
-    int R, kt, fmt;
+    int R, kt, fmt, tr;   /* tr: rows of a tile of the C updates by sub-block */
 };
 struct WaveLaunch {
     int nprob;
@@ -2330,6 +2344,20 @@ __global__ void __launch_bounds__(256, 4) wave_scatter_kernel(const __grid_const
     } else {
         if (P.fmt) go(fp8, pair); else go(bf16, pair);
     }
+}
+
+/* the rest, by sub-block: gx tiles for each */
+__global__ void __launch_bounds__(kScatterThreads, 8) wave_scatter_part_kernel(const __grid_constant__ WaveLaunch W)
+{
+    __shared__ ScatterEntries sh;
+    const WaveProb& P = W.p[wave_find(W, blockIdx.x)];
+    const int64_t vb = blockIdx.x - P.b0;
+    const int p = (int)(vb / P.gx);
+    const uint32_t bx = (uint32_t)(vb % P.gx);
+    if (P.fmt)
+        scatter_part_body<1>(sh, P.tab, 0, P.R, P.m, P.n, P.alpha, P.beta, P.Z, P.e_row, P.f_col, P.C, P.ldc, P.tr, p, bx);
+    else
+        scatter_part_body<0>(sh, P.tab, 0, P.R, P.m, P.n, P.alpha, P.beta, P.Z, P.e_row, P.f_col, P.C, P.ldc, P.tr, p, bx);
 }
 
 /* --------------------------------------------------------- host -------- */
@@ -3147,23 +3175,37 @@ static void job_scatter_cols(const SplitJob& j, int r0, int np, int64_t j0, int6
     job_scatter_block(j, r0, np, 0, j.d.me, j0, j1, st);
 }
 
+/* tiles of one sub-block in scatter_kernel, and their rows */
+static int64_t scatter_part_tiles(const SplitJob& j, int* tr)
+{
+    int t = 8;
+    while (t < kScatterThreads && t < j.d.me) t *= 2;
+    *tr = t;
+    const int64_t groups = kScatterThreads / t;
+    return (j.d.me + t - 1) / t * (((j.d.ne + 3) / 4 + groups - 1) / groups);
+}
+
+/* the C updates of products [r0, r0 + np) by sub-block */
+static void job_scatter_parts(const SplitJob& j, int r0, int np, cudaStream_t st)
+{
+    int tr;
+    const int64_t tiles = scatter_part_tiles(j, &tr);
+    auto* k = j.fmt ? scatter_kernel<1> : scatter_kernel<0>;
+    k<<<dim3((unsigned)tiles, (unsigned)(j.alg.mt * j.alg.nt)), kScatterThreads, 0, st>>>(
+        j.alg.tab, r0, np, j.m, j.n, j.alpha, job_beta(j, r0), job_zview(j), (const int*)(j.w + j.L.erow),
+        (const int*)(j.w + j.L.fcol), j.C, j.ldc, tr);
+    fmm_count_launch(1);
+}
+
+/* the C updates of products [r0, r0 + np), in the faster form */
 static void job_scatter(const SplitJob& j, int r0, int np, cudaStream_t st, bool small = false)
 {
     int T;
     size_t smem;
-    if (job_scatter_all(j, r0, np, &T, &smem) && scatter_all_better(j, scatter_tiles(j, j.d.me, j.d.ne, T))) {
+    if (job_scatter_all(j, r0, np, &T, &smem) && scatter_all_better(j, scatter_tiles(j, j.d.me, j.d.ne, T)))
         job_scatter_block(j, r0, np, 0, j.d.me, 0, j.d.ne, st, small);
-        return;
-    }
-    auto* k = j.fmt ? scatter_kernel<1> : scatter_kernel<0>;
-    int tr = 8;
-    while (tr < kScatterThreads && tr < j.d.me) tr *= 2;
-    const int64_t groups = kScatterThreads / tr;
-    k<<<dim3((unsigned)((j.d.me + tr - 1) / tr * (((j.d.ne + 3) / 4 + groups - 1) / groups)),
-             (unsigned)(j.alg.mt * j.alg.nt)),
-        kScatterThreads, 0, st>>>(j.alg.tab, r0, np, j.m, j.n, j.alpha, job_beta(j, r0), job_zview(j),
-                                  (const int*)(j.w + j.L.erow), (const int*)(j.w + j.L.fcol), j.C, j.ldc, tr);
-    fmm_count_launch(1);
+    else
+        job_scatter_parts(j, r0, np, st);
 }
 
 /* dynamic shared memory limits of this file's kernels: per-device attributes, set once per device */
@@ -4053,74 +4095,94 @@ static int wave_side_pack(const std::vector<SplitJob*>& all, cudaStream_t st)
     return cudaGetLastError() == cudaSuccess ? FMM_OK : FMM_ERR_CUDA;
 }
 
-/* The C updates after a wave's GEMM, on up to kWaveStreams streams `on(x)`:
- * classical jobs (bound by HBM, no shared memory, full blocks) in one
- * element-major launch, the other jobs that it is better for in a second one,
- * the rest each by its own launch. One launch for all of them would run every job with
- * the fewest threads and the most shared memory any of them needs: 322 x2 at
- * 963 x 267 x 134 with a classical 675 x 2091 x 595, 829 us for the batch
- * against 380. Within a launch the blocks, at most 16 per SM in all, are shared
- * out by work, so a block's set-up serves several tiles in a wave of many
- * problems and no job is left with a few long blocks. */
-template <class On>
-static int wave_side_scatter(const std::vector<SplitJob*>& qs, On on)
+/* The C updates after a wave's GEMM, a launch per kind: classical jobs (bound by
+ * HBM, no shared memory, full blocks), the other jobs that the element-major
+ * form is better for, those of many products among them apart (on st_long), and
+ * the rest by sub-block. One element-major launch for all of them would run
+ * every job with the fewest threads and the most shared memory any of them
+ * needs: 322 x2 at 963 x 267 x 134 with a classical 675 x 2091 x 595, 829 us for
+ * the batch against 205. The launches of short blocks run one after the other
+ * on one stream: on one each they cost a batch of two kinds 6 us more. */
+static int wave_side_scatter(const std::vector<SplitJob*>& qs, cudaStream_t st, cudaStream_t st_long)
 {
-    std::vector<SplitJob*> kinds[2], other;   /* classical, element-major */
-    int T[2] = {256, 256};
+    /* Classical, element-major (up to kLongProducts products, and more), by sub-block. A job of many products has long
+     * blocks; where the launch is about one round of blocks (six per SM), other jobs' blocks in front of them push its
+     * last ones into a second round: five problems, 861 of 940 blocks of 232 x2 at 1654 x 1967, 771 us for the batch,
+     * 653 with that one in a launch of its own. */
+    constexpr int kLongProducts = 64, kBySubBlock = 3;
+    std::vector<SplitJob*> kinds[4];
+    int T[3] = {256, 256, 256};
     for (SplitJob* j : qs) {
         int Tj;
         size_t sm;
         if (job_scatter_all(*j, 0, j->alg.R, &Tj, &sm) && scatter_all_better(*j, INT64_MAX)) {
-            const int x = j->classical ? 0 : 1;
+            const int x = j->classical ? 0 : j->alg.R <= kLongProducts ? 1 : 2;
             kinds[x].push_back(j);
             T[x] = std::min(T[x], Tj);
         } else {
-            other.push_back(j);
+            kinds[kBySubBlock].push_back(j);
         }
     }
+    auto tiles_of = [&](const SplitJob& j, int x) { return scatter_tiles(j, j.d.me, j.d.ne, T[x]); };
     int64_t together = 0;
-    for (SplitJob* j : kinds[1]) together += scatter_tiles(*j, j->d.me, j->d.ne, T[1]);
-    /* A job of many products has long blocks; where the launch is about one round of blocks (six per SM), other
-     * jobs' blocks push its last ones into a second round: five problems, 861 of 940 blocks of 232 x2 at 1654 x
-     * 1967, 774 us for the batch, 698 with that one by sub-block (alone it takes 356 this way and 397 by sub-block). */
-    const bool unlike = kinds[1].size() > 1;
-    const auto apart = std::stable_partition(kinds[1].begin(), kinds[1].end(), [&](SplitJob* j) {
-        return scatter_all_better(*j, unlike && j->alg.R > 64 ? together / 4 : together);
-    });
-    other.insert(other.end(), apart, kinds[1].end());
-    kinds[1].erase(apart, kinds[1].end());
-    auto entries = [](const SplitJob& j) {
-        const Tab ht = tab_view(j.alg.htab);
-        return ht.w_off[j.alg.R] - ht.w_off[0];
-    };
-    for (int x = 0; x < 2; ++x) {
+    for (SplitJob* j : kinds[1]) together += tiles_of(*j, 1);
+    for (int x = 1; x < kBySubBlock; ++x) {
+        const auto rest = std::stable_partition(kinds[x].begin(), kinds[x].end(), [&](SplitJob* j) {
+            return scatter_all_better(*j, x == 1 ? together : tiles_of(*j, x));
+        });
+        kinds[kBySubBlock].insert(kinds[kBySubBlock].end(), rest, kinds[x].end());
+        kinds[x].erase(rest, kinds[x].end());
+    }
+    /* the only job of a kind: the kernel of single calls, with one form's registers and a hundredth of the parameters */
+    for (int x = 0; x <= kBySubBlock; ++x) {
+        if (kinds[x].size() != 1) continue;
+        const SplitJob& j = *kinds[x][0];
+        if (x == kBySubBlock)
+            job_scatter_parts(j, 0, j.alg.R, st);
+        else
+            job_scatter_block(j, 0, j.alg.R, 0, j.d.me, 0, j.d.ne, x == 2 ? st_long : st);
+        kinds[x].clear();
+    }
+    WaveLaunch L;
+    for (int x = 0; x < kBySubBlock; ++x) {
         if (kinds[x].empty()) continue;
-        /* a job's tiles, and its work: per tile each product's Z, each W entry's update, each sub-block's C in and out */
-        auto tiles = [&](const SplitJob& j) { return scatter_tiles(j, j.d.me, j.d.ne, T[x]); };
-        auto work = [&](const SplitJob& j) {
-            return (double)tiles(j) * (double)(j.alg.R + entries(j) + 2 * j.alg.mt * j.alg.nt);
-        };
+        /* a job's work: per tile each product's Z, each W entry's update, each sub-block's C in and out */
+        std::vector<double> work;
         size_t smem = 0;
         int64_t all_tiles = 0;
         double all_work = 0.0;
         for (SplitJob* j : kinds[x]) {
-            const int P = j->alg.mt * j->alg.nt;
-            if (x == 1)
-                smem = std::max(smem, scatter_all_smem(P, T[x], entries(*j), j->alg.R));
-            all_tiles += tiles(*j);
-            all_work += work(*j);
+            const Tab ht = tab_view(j->alg.htab);
+            const int P = j->alg.mt * j->alg.nt, E = ht.w_off[j->alg.R] - ht.w_off[0];
+            if (x > 0) smem = std::max(smem, scatter_all_smem(P, T[x], E, j->alg.R));
+            const int64_t t = tiles_of(*j, x);
+            work.push_back((double)t * (double)(j->alg.R + E + 2 * P));
+            all_tiles += t;
+            all_work += work.back();
         }
-        WaveLaunch L;
+        /* a block per tile, or the most blocks of a launch shared out by work, so that a block's set-up serves several
+         * tiles in a wave of many problems and no job is left with a few long blocks */
+        const double per_work = (double)scatter_blocks(INT64_MAX) / all_work;
+        const bool fits = scatter_blocks(all_tiles) == all_tiles;
+        size_t q = 0;
         const int64_t nb = wave_table(L, kinds[x], [&](const SplitJob& j, WaveProb& w) {
+            const int64_t t = tiles_of(j, x);
             w.gx = 1;
-            w.nb = std::min<int64_t>(
-                std::max<int64_t>(1, (int64_t)((double)scatter_blocks(all_tiles) * work(j) / all_work)), tiles(j));
+            w.nb = fits ? t : std::min(std::max<int64_t>(1, (int64_t)(per_work * work[q])), t);
+            ++q;
         });
-        (x == 0 ? wave_scatter_one_kernel : wave_scatter_kernel)<<<(unsigned)nb, (unsigned)T[x], smem, on(x)>>>(L);
+        (x == 0 ? wave_scatter_one_kernel : wave_scatter_kernel)<<<(unsigned)nb, (unsigned)T[x], smem,
+                                                                     x == 2 ? st_long : st>>>(L);
         fmm_count_launch(1);
     }
-    for (size_t q = 0; q < other.size(); ++q)
-        job_scatter(*other[q], 0, other[q]->alg.R, on(2 + (int)(q % (kWaveStreams - 2))));
+    if (!kinds[kBySubBlock].empty()) {
+        const int64_t nb = wave_table(L, kinds[kBySubBlock], [&](const SplitJob& j, WaveProb& w) {
+            w.gx = scatter_part_tiles(j, &w.tr);
+            w.nb = w.gx * j.alg.mt * j.alg.nt;
+        });
+        wave_scatter_part_kernel<<<(unsigned)nb, kScatterThreads, 0, st>>>(L);
+        fmm_count_launch(1);
+    }
     return cudaGetLastError() == cudaSuccess ? FMM_OK : FMM_ERR_CUDA;
 }
 
@@ -4220,7 +4282,7 @@ int fmm_split_batch(int count, const SplitJob* jobs_in, void* ws, size_t ws_byte
                 if (!ok(cudaStreamWaitEvent(scat_st(y), sp->wave_gm[W.h], 0))) return FMM_ERR_CUDA;
         std::vector<SplitJob*> qs;
         for (int q = W.i; q < W.e; ++q) qs.push_back(&jobs[q]);
-        if (int rc = wave_side_scatter(qs, scat_st); rc != FMM_OK) return rc;
+        if (int rc = wave_side_scatter(qs, scat_st(0), scat_st(1)); rc != FMM_OK) return rc;
         if (sp)
             for (int y = 0; y < kWaveStreams; ++y)
                 if (!ok(cudaEventRecord(sp->wave_sc[W.h][y], scat_st(y)))) return FMM_ERR_CUDA;

@@ -162,3 +162,47 @@ def test_c_updates_of_many_products_on_small_grids(fmm, torch_cuda):
     A, B, C = operand(torch, m, k), operand(torch, k, n), operand(torch, m, n)
     ws = torch.empty(fmm.split_workspace_size(m, n, k, f, 2, 6), dtype=torch.uint8, device="cuda")
     assert device_us(torch, lambda: fmm.split_dgemm(A, B, C, f, 2, 6, 1.0, 0.5, ws)) < 135
+
+
+def test_batch_of_many_small_c_updates(fmm, torch_cuda):
+    """20 problems of a handful of C update blocks: 145 us with one launch for
+    all of them, 203 with one each."""
+    torch = torch_cuda
+    f = fmm.new_fmm(COEFFS / "333.txt")
+    ps = [{"A": operand(torch, 33, 90), "B": operand(torch, 90, 101), "C": operand(torch, 33, 101), "fmm": f, "levels": 1,
+           "slices": 3} for _ in range(20)]
+    b = fmm.make_batch(ps)
+    ws = torch.empty(fmm.batch_workspace_size(b), dtype=torch.uint8, device="cuda")
+    assert device_us(torch, lambda: fmm.batch_dgemm(b, workspace=ws)) < 175
+
+
+@pytest.mark.parametrize("kinds", [
+    [("322", 2), ("222", 3), ("444", 2), ("333", 2)],                         # by sub-block, in one launch
+    [("322", 2), (None, 0), ("222", 1), ("232", 2), ("333", 1)],              # each kind once
+    [("222", 1), ("322", 1), ("222", 2), (None, 0), (None, 0), ("232", 2)],
+])
+@pytest.mark.parametrize("big", [False, True])
+def test_batch_c_update_forms_equal_single_calls(fmm, torch_cuda, kinds, big):
+    """every kind of C update launch of a batch, small product grids and some
+    above two blocks per SM, gives the single calls' bits"""
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(5)
+
+    def rnd(r, c):
+        return (torch.rand((c, r), generator=g, device="cuda", dtype=torch.float64) * 2 - 1).t()
+
+    probs, want = [], []
+    for i, (a, lv) in enumerate(kinds * 2):
+        f = fmm.new_fmm(COEFFS / f"{a}.txt") if a else None
+        m, n, k = (1500 + 61 * i, 1300 + 37 * i, 90) if big and i % 3 == 0 else (130 + 17 * i, 97 + 29 * i, 70 + 13 * i)
+        p = {"A": rnd(m, k), "B": rnd(k, n), "C": rnd(m, n), "fmm": f, "levels": lv, "slices": 3 + i % 5,
+             "fmt": "fp8" if i % 2 else "bf16", "alpha": -0.75, "beta": [1.0, 0.5, 0.0][i % 3]}
+        c = p["C"].clone()
+        fmm.split_dgemm(p["A"], p["B"], c, f, lv, p["slices"], alpha=p["alpha"], beta=p["beta"], fmt=p["fmt"])
+        probs.append(p)
+        want.append(c)
+    fmm.batch_dgemm(probs)
+    torch.cuda.synchronize()
+    for i, (p, w) in enumerate(zip(probs, want)):
+        assert torch.equal(p["C"], w), f"problem {i}"
+    assert fmm.take_device_error() == 0
