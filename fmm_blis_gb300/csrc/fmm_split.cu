@@ -1922,8 +1922,8 @@ struct ScatterEntries {
     int n;
 };
 
-/* tile bx of sub-block p */
-template <int FMT>
+/* tile bx of sub-block p; WIDE: tr is 128, so a block's columns are the same for all its threads (3% of the kernel) */
+template <int FMT, bool WIDE>
 __device__ __forceinline__ void scatter_part_body(ScatterEntries& sh, const int* __restrict__ tab, int r0, int nprod,
                                                   int64_t m, int64_t n, double alpha, double beta, const ZView& Z,
                                                   const int* __restrict__ e_row, const int* __restrict__ f_col,
@@ -1949,9 +1949,10 @@ __device__ __forceinline__ void scatter_part_body(ScatterEntries& sh, const int*
     }
     __syncthreads();
     const int ne = sh.n;
-    const uint32_t me = (uint32_t)((m + t.mt - 1) / t.mt), tiles_i = (me + tr - 1) / tr;
-    const int i = (int)(bx % tiles_i * tr + threadIdx.x % tr);
-    const int j = (int)(bx / tiles_i * (kScatterThreads / tr) + threadIdx.x / tr) * 4;
+    const int TR = WIDE ? kScatterThreads : tr;
+    const uint32_t me = (uint32_t)((m + t.mt - 1) / t.mt), tiles_i = (me + TR - 1) / TR;
+    const int i = (int)(bx % tiles_i * TR) + (int)(WIDE ? threadIdx.x : threadIdx.x % TR);
+    const int j = (int)(WIDE ? bx / tiles_i : bx / tiles_i * (kScatterThreads / TR) + threadIdx.x / TR) * 4;
     if ((ne == 0 && beta == 1.0) || i >= rl || j >= cl) return;
     double* cp = C + ro + i + (int64_t)(co + j) * ldc;
     double c[kScatterCols];
@@ -1972,14 +1973,14 @@ __device__ __forceinline__ void scatter_part_body(ScatterEntries& sh, const int*
 }
 
 /* grid: tiles x sub-blocks */
-template <int FMT>
+template <int FMT, bool WIDE>
 __global__ void __launch_bounds__(kScatterThreads)
 scatter_kernel(const int* __restrict__ tab, int r0, int nprod, int64_t m, int64_t n, double alpha, double beta,
                const ZView Z, const int* __restrict__ e_row, const int* __restrict__ f_col, double* __restrict__ C,
                int64_t ldc, int tr)
 {
     __shared__ ScatterEntries sh;
-    scatter_part_body<FMT>(sh, tab, r0, nprod, m, n, alpha, beta, Z, e_row, f_col, C, ldc, tr, (int)blockIdx.y,
+    scatter_part_body<FMT, WIDE>(sh, tab, r0, nprod, m, n, alpha, beta, Z, e_row, f_col, C, ldc, tr, (int)blockIdx.y,
                            blockIdx.x);
 }
 
@@ -2355,9 +2356,9 @@ __global__ void __launch_bounds__(kScatterThreads, 8) wave_scatter_part_kernel(c
     const int p = (int)(vb / P.gx);
     const uint32_t bx = (uint32_t)(vb % P.gx);
     if (P.fmt)
-        scatter_part_body<1>(sh, P.tab, 0, P.R, P.m, P.n, P.alpha, P.beta, P.Z, P.e_row, P.f_col, P.C, P.ldc, P.tr, p, bx);
+        scatter_part_body<1, false>(sh, P.tab, 0, P.R, P.m, P.n, P.alpha, P.beta, P.Z, P.e_row, P.f_col, P.C, P.ldc, P.tr, p, bx);
     else
-        scatter_part_body<0>(sh, P.tab, 0, P.R, P.m, P.n, P.alpha, P.beta, P.Z, P.e_row, P.f_col, P.C, P.ldc, P.tr, p, bx);
+        scatter_part_body<0, false>(sh, P.tab, 0, P.R, P.m, P.n, P.alpha, P.beta, P.Z, P.e_row, P.f_col, P.C, P.ldc, P.tr, p, bx);
 }
 
 /* --------------------------------------------------------- host -------- */
@@ -3190,7 +3191,9 @@ static void job_scatter_parts(const SplitJob& j, int r0, int np, cudaStream_t st
 {
     int tr;
     const int64_t tiles = scatter_part_tiles(j, &tr);
-    auto* k = j.fmt ? scatter_kernel<1> : scatter_kernel<0>;
+    const bool wide = tr == kScatterThreads;
+    auto* k = j.fmt ? (wide ? scatter_kernel<1, true> : scatter_kernel<1, false>)
+                    : (wide ? scatter_kernel<0, true> : scatter_kernel<0, false>);
     k<<<dim3((unsigned)tiles, (unsigned)(j.alg.mt * j.alg.nt)), kScatterThreads, 0, st>>>(
         j.alg.tab, r0, np, j.m, j.n, j.alpha, job_beta(j, r0), job_zview(j), (const int*)(j.w + j.L.erow),
         (const int*)(j.w + j.L.fcol), j.C, j.ldc, tr);
