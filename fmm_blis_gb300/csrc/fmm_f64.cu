@@ -1306,7 +1306,7 @@ namespace {
  * with 64 x 64 alone. That is within 3% of the best limit for 258 drawn
  * batches but for those whose items are nearly all alike, where smaller tiles
  * only cost more and whole rounds of items decide: for these the tile with the
- * least batch_rounds times batch_item_cost is taken if it saves 5%. Tiles of 64
+ * least batch_rounds times batch_item_cost is taken if it saves 3%. Tiles of 64
  * / 32 / 16 / the rule, us: 2048^3 222 x1 15204 / 13633 / 16552 / 13640; 1912 x
  * 2475 x 97 232 x1 1522 / 1580 / 2015 / 1522; 1024^3 222 x1 3992 / 1966 / 2388
  * / 1966; 512^3 222 x1 2019 / 586 / 319 / 319; classical 1216 x 1024 x 500 1048
@@ -1321,7 +1321,7 @@ double batch_item_cost(const F64BatchItem& it, int tile, bool mma)
     const double ke = (double)((it.k + it.alg.kt - 1) / it.alg.kt), nn = it.alg.avg_nnz_u + it.alg.avg_nnz_v;
     double rel = 1.0;
     if (tile == 32)
-        rel = mma ? 1.01 + 0.11 * (nn - 2.0) : 1.0 + 0.016 * (nn - 2.0) + 1.6 / ke;
+        rel = mma ? 1.01 + 0.11 * (nn - 2.0) : 1.01 + 0.016 * (nn - 2.0) + 3.0 / ke;
     else if (tile == 16)
         rel = 1.14 + 0.085 * (nn - 2.0) + 11.0 / ke;
     return rel * tile * tile * it.alg.R * (ke + 1.0);
@@ -1383,7 +1383,7 @@ void batch_tiles(const F64BatchItem* p, const std::vector<int>& order, bool mma,
             }
         return longest * batch_rounds(n, slots, t, p[heavy].alg.avg_nnz_u + p[heavy].alg.avg_nnz_v);
     };
-    double best = 0.95 * estimate(tile[heavy]);
+    double best = 0.97 * estimate(tile[heavy]);
     int to = tile[heavy];
     for (int t = 64; t >= least; t /= 2) {
         const double e = t == tile[heavy] ? best : estimate(t);
